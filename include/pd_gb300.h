@@ -176,7 +176,10 @@ typedef struct pd_solver_options {
      * iterations launched from the host, each followed by a read-back of the
      * test.  Both run the same kernels in the same order, so the results are
      * identical.  Default 0; a device where the graph cannot be built falls
-     * back to 1 (pd_step_stats.cg_graph_solves stays 0). */
+     * back to 1 (pd_step_stats.cg_graph_solves stays 0).  Small bodies (those
+     * whose blocks' shares fit in shared memory, on the gather product without
+     * a preconditioner) run their iterations in one cooperative launch instead
+     * of the graph, and in host-checked batches of such launches with 1. */
     int cg_loop;
     /* CG preconditioner (the reference's cusp::precond::diagonal is
      * commented out, simulator.cu:767-769, so it runs plain CG): 0 = none, as
@@ -230,7 +233,8 @@ typedef struct pd_step_stats {
                                       adaptive time step's test (Newmark-beta or adaptive_integration)
                                       and the read-back of each solve's result, plus one per host
                                       batch with cg_loop 1 */
-    long long cg_graph_solves;     /* solves whose iterations ran in the CG graph (cg_loop 0) */
+    long long cg_graph_solves;     /* solves whose iterations ran in the CG graph or, for a small
+                                      body, in one cooperative launch (cg_loop 0) */
     long long ws_guesses_skipped;  /* batch learned warm start: steps whose learned pass was paused
                                       (3 guesses rejected in a row; retried every 16 steps) */
 } pd_step_stats;

@@ -1,0 +1,697 @@
+// cg_persist.cu -- the CG iterations of a small body in one cooperative launch.
+//
+// The solve of the reference (CUSP krylov::cg, driven by
+// Simulator::solveLinearSystem, src/core/simulator.cu:735-799) needs two
+// grid-wide sums per iteration.  As separate launches (product, solution
+// update, direction update) an iteration of a body of a few thousand particles
+// costs the launches and the tails of three nearly empty kernels; here every
+// block keeps its rows for the whole solve:
+//   * x, r, p and A p of the block's own rows stay in shared memory, and so
+//     does p of its halo (the distinct neighbours of its rows);
+//   * what a bond contributes to the product does not change inside a solve
+//     (the positions do not move): where they fit, every bond's geometry (FP64:
+//     its Jacobian) and halo index are kept in shared memory;
+//   * a grid-wide sum is one exchange of (partial sum, epoch) records, one
+//     16-byte store from every block into every block's inbox: a block polls
+//     only its own inbox and adds the partials in block order, so the sum and
+//     the barrier are the same round trip and no line is polled by two blocks;
+//   * the residual r is the only vector that travels: each row publishes (r,
+//     epoch) in 16-byte records, which the blocks that have it in their halo
+//     poll while <r, r> is being summed, and p = r + beta p of the halo is then
+//     formed by every block for itself.
+// An iteration takes two exchanges (<p, A p>, <r, r>) and no memory fence.
+//
+// Memory ordering.  Every value that another block reads is in a record of
+// one 16-byte access together with the epoch it belongs to, so a reader never
+// needs what was written before or after it.  A record is overwritten only
+// after all its readers have it: the next r of a row follows the exchange of
+// <p, A p>, whose partials depend on every record read for them, and inbox
+// records alternate by epoch parity.  Every wait is bounded: after 5 s a
+// thread records the error and its block returns, and so does every block that
+// sees the error.
+#include <algorithm>
+
+#include "step_rows.cuh"
+
+namespace pdgb {
+
+namespace {
+
+constexpr int kPersistThreads = 512;
+constexpr int kPersistWarps = kPersistThreads / 32;
+constexpr int kPersistMaxGrid = 256;
+constexpr unsigned long long kPersistTimeoutNs = 5000000000ull;   // 5 s
+
+__device__ __forceinline__ unsigned long long now_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// 16 bytes in one access: a reader sees the value that belongs to the epoch
+__device__ __forceinline__ void publish(ulonglong2* slot, unsigned long long value, unsigned long long epoch)
+{
+    asm volatile("{ .reg .b128 v; mov.b128 v, {%1, %2}; st.relaxed.gpu.global.b128 [%0], v; }"
+                 ::"l"(slot), "l"(value), "l"(epoch)
+                 : "memory");
+}
+__device__ __forceinline__ ulonglong2 observe(const ulonglong2* slot)
+{
+    ulonglong2 v;
+    asm volatile("{ .reg .b128 v; ld.relaxed.gpu.global.b128 v, [%2]; mov.b128 {%0, %1}, v; }"
+                 : "=l"(v.x), "=l"(v.y)
+                 : "l"(slot)
+                 : "memory");
+    return v;
+}
+
+struct PersistArgs {
+    StepParams P;
+    DeviceState S;
+    ulonglong2* rec;            // published r: one record per row (FP64: two)
+    ulonglong2* inbox;          // [2][grid][grid]: records by epoch parity, reader, writer
+    unsigned long long epoch;   // the last epoch of earlier launches
+    int rows;                   // rows per block
+    int halo;                   // halo entries of a block at most
+    int bonds;                  // bond slots kept in shared memory per block (0: none)
+    int max_iters;              // iterations of this launch at most
+    int profile;
+};
+
+// Sums travel as their accumulator's own form: double-float for FP32 data.
+__device__ __forceinline__ unsigned long long pack(DF v)
+{
+    return ((unsigned long long)__float_as_uint(v.hi) << 32) | __float_as_uint(v.lo);
+}
+__device__ __forceinline__ unsigned long long pack(double v) { return (unsigned long long)__double_as_longlong(v); }
+template <typename T> __device__ __forceinline__ T unpack(unsigned long long v);
+template <> __device__ __forceinline__ DF unpack<DF>(unsigned long long v)
+{
+    return DF{__uint_as_float((unsigned)(v >> 32)), __uint_as_float((unsigned)v)};
+}
+template <> __device__ __forceinline__ double unpack<double>(unsigned long long v)
+{
+    return __longlong_as_double((long long)v);
+}
+__device__ __forceinline__ void add_to(DF& a, DF b) { df_add(a, b); }
+__device__ __forceinline__ void add_to(double& a, double b) { a = __dadd_rn(a, b); }
+__device__ __forceinline__ DF shfl_xor(DF a, int off)
+{
+    return DF{__shfl_xor_sync(0xffffffffu, a.hi, off), __shfl_xor_sync(0xffffffffu, a.lo, off)};
+}
+__device__ __forceinline__ double shfl_xor(double a, int off) { return __shfl_xor_sync(0xffffffffu, a, off); }
+// sum over the lanes whose index is a multiple of `step` (a power of two)
+template <typename T>
+__device__ __forceinline__ void warp_sum(T& v, int step)
+{
+    for (int off = 16; off >= step; off >>= 1) add_to(v, shfl_xor(v, off));
+}
+
+struct Exchange {
+    unsigned long long warp[kPersistWarps];
+    unsigned long long from[kPersistMaxGrid];
+    int error;
+};
+
+// Polls a record until `arrived` accepts it; false when the wait ran out of
+// time (here or in another thread).
+template <typename Ok>
+__device__ __forceinline__ bool await(const ulonglong2* rec, CgScalars* sc, Exchange& e, ulonglong2& r, Ok arrived)
+{
+    r = observe(rec);
+    if (arrived(r)) return true;
+    unsigned spins = 0;
+    const unsigned long long t0 = now_ns();
+    for (;;) {
+        r = observe(rec);
+        if (arrived(r)) return true;
+        if ((++spins & 255u) == 0) {
+            if (((volatile CgScalars*)sc)->wait_error || now_ns() - t0 > kPersistTimeoutNs) {
+                ((volatile CgScalars*)sc)->wait_error = 1;
+                e.error = 1;
+                return false;
+            }
+        }
+    }
+}
+
+// The sum over all blocks of v (which only lanes at multiples of `step` hold);
+// every thread of the block calls it and gets the sum.  The warps that do not
+// poll the inbox run help(thread, threads) meanwhile.  Returns false when a
+// wait ran out of time.
+template <typename T, typename Help>
+__device__ __forceinline__ bool exchange_sum(Exchange& e, T& v, int step, const PersistArgs& A, unsigned long long epoch,
+                                             Help help)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int grid = gridDim.x;
+    const int polling = (grid + 31) / 32 * 32;   // threads with an inbox record, in whole warps
+    warp_sum(v, step);
+    if (lane == 0) e.warp[warp] = pack(v);
+    __syncthreads();
+    if ((int)threadIdx.x < polling) {
+        T t = unpack<T>(e.warp[lane & (kPersistWarps - 1)]);   // both halves of the warp form the same sum
+#pragma unroll
+        for (int off = kPersistWarps / 2; off > 0; off >>= 1) add_to(t, shfl_xor(t, off));
+        const int b = threadIdx.x;
+        if (b < grid) {
+            ulonglong2* box = A.inbox + (size_t)(epoch & 1) * grid * grid;
+            publish(box + (size_t)b * grid + blockIdx.x, pack(t), epoch);
+            ulonglong2 r;
+            await(box + (size_t)blockIdx.x * grid + b, A.S.sc, e, r, [epoch](const ulonglong2& x) { return x.y == epoch; });
+            e.from[b] = r.x;
+        }
+    } else {
+        help((int)threadIdx.x - polling, kPersistThreads - polling);
+    }
+    __syncthreads();
+    v = T();
+    for (int b = lane; b < grid; b += 32) add_to(v, unpack<T>(e.from[b]));
+    warp_sum(v, 1);
+    return e.error == 0;
+}
+
+// The quotient a / b rounded to FP32 (a, b in double-float): the FP32 quotient
+// and one correction by its remainder, as accurate as the rounded FP64
+// quotient to 2^-40, at a fifth of an FP64 division's latency (573 cycles).
+// Sums whose FP32 words leave the range of the steps take the FP64 division.
+__device__ __forceinline__ float df_quotient(DF a, DF b)
+{
+    const float fa = fabsf(a.hi), fb = fabsf(b.hi);
+    if (!(fa > 1e-25f && fa < 1e25f && fb > 1e-25f && fb < 1e25f)) return (float)(df_to_double(a) / df_to_double(b));
+    const float q = __fdiv_rn(a.hi, b.hi);
+    const float p = __fmul_rn(q, b.hi);
+    const float pe = __fmaf_rn(q, b.hi, -p);
+    // a - q b: the leading words cancel exactly
+    const float r = __fadd_rn(__fsub_rn(a.hi, p), __fsub_rn(__fsub_rn(a.lo, pe), __fmul_rn(q, b.lo)));
+    return __fadd_rn(q, __fdividef(r, b.hi));
+}
+
+// One iteration's convergence test (as cg_fin_axpy): ||r|| <= tol, the square
+// root only where the squares are too near to tell.
+__device__ __forceinline__ bool below_tolerance(double rr, double tol)
+{
+    const double t2 = tol * tol;
+    if (rr > t2 * (1.0 + 1e-12)) return false;
+    if (rr < t2 * (1.0 - 1e-12)) return true;
+    return sqrt(rr) <= tol;
+}
+
+struct __align__(16) BondGeometry {   // one bond of the mixed-precision product, formed once per solve
+    float x, y, z;   // x_q - x_p
+    float i3;        // 1 / d^3
+};
+__device__ __forceinline__ BondGeometry bond_geometry(const float4& Xq, const float4& xp, float sup, float inv_d0,
+                                                      float& a1)
+{
+    BondGeometry g;
+    float cx, cy, cz;
+    supercell_delta(__float_as_int(Xq.w), __float_as_int(xp.w), sup, cx, cy, cz);
+    g.x = (Xq.x - xp.x) + cx;
+    g.y = (Xq.y - xp.y) + cy;
+    g.z = (Xq.z - xp.z) + cz;
+    const float inv_d = rsqrtf(fmaf(g.x, g.x, fmaf(g.y, g.y, g.z * g.z)));
+    g.i3 = inv_d * inv_d * inv_d;
+    a1 = inv_d0 - inv_d;
+    return g;
+}
+
+// Mixed precision, G lanes per row, U bonds in flight per lane.  The halo is
+// S.halo of a tile per block, a bond's index into it S.lidx.
+// CACHED: the bonds' geometry stays in shared memory; else the halo's
+// positions do, and the index and 1/d0 of a bond are read from global memory
+// (6 bytes per bond, from L2).
+template <bool CACHED, int G, int U>
+__global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist32(PersistArgs A)
+{
+    CgScalars* sc = A.S.sc;
+    // (the scalars change only after every block's last exchange)
+    if (((volatile CgScalars*)sc)->done) return;
+    extern __shared__ __align__(32) unsigned char smem[];
+    __shared__ Exchange ex;
+    const StepParams& P = A.P;
+    const DeviceState& S = A.S;
+    const int lo = blockIdx.x * A.rows;
+    const int nr = min(A.rows, P.n - lo);
+    float4* sx = (float4*)smem;
+    float4* sr = sx + A.rows;
+    float4* sp = sr + A.rows;
+    float4* sy = sp + A.rows;
+    float4* sw = sy + A.rows;                            // the halo's p
+    float4* sh = sw + A.halo;                            // the halo's r
+    float4* shx = sh + A.halo;                           // the halo's positions (not CACHED)
+    BondGeometry* sg = (BondGeometry*)(CACHED ? shx : shx + A.halo);
+    float* sa1 = (float*)(sg + A.bonds);                 // 1/d0 - 1/d
+    int* srow = (int*)(sa1 + A.bonds);                   // first slot of the row
+    int* scnt = srow + A.rows;                           // live bonds, -1 for a Dirichlet row
+    int* sq = scnt + A.rows;                             // the halo's slots
+    uint16_t* sl = (uint16_t*)(sq + A.halo);             // a bond's halo index
+
+    const int lane = threadIdx.x & (G - 1);
+    const unsigned gmask = group_mask<G>();
+    constexpr int NG = kPersistThreads / G;
+    const int first = CACHED ? S.row_ptr[lo] : 0;
+    for (int t = threadIdx.x; t < nr; t += kPersistThreads) {
+        const int p = lo + t;
+        sx[t] = ((const float4*)S.sol)[p];
+        sr[t] = ((const float4*)S.r)[p];
+        sp[t] = ((const float4*)S.p)[p];
+        scnt[t] = is_dirichlet(S.act[p] & kActMask) ? -1 : S.cnt[p];
+        srow[t] = S.row_ptr[p] - first;
+    }
+    const int h0 = S.halo_ptr[blockIdx.x], nh = S.halo_ptr[blockIdx.x + 1] - h0;
+    for (int h = threadIdx.x; h < nh; h += kPersistThreads) {
+        const int q = S.halo[h0 + h];
+        sq[h] = q;
+        sw[h] = ((const float4*)S.p)[q];
+        sh[h] = ((const float4*)S.r)[q];
+        if (!CACHED) shx[h] = S.xs4[q];
+    }
+    if (threadIdx.x == 0) ex.error = 0;
+    __syncthreads();
+    const float sup = (float)P.sup;
+    if (CACHED) {
+        for (int i = threadIdx.x / G; i < nr; i += NG) {
+            const int cn = scnt[i], base = srow[i];
+            const float4 xp = S.xs4[lo + i];
+            for (int j = lane; j < cn; j += G) {
+                const int l = S.lidx[first + base + j];
+                sg[base + j] = bond_geometry(S.xs4[sq[l]], xp, sup, S.inv_d0[first + base + j], sa1[base + j]);
+                sl[base + j] = (uint16_t)l;
+            }
+        }
+    }
+    const double tol = sc->tol;
+    const float tol2_far = (float)(tol * tol * 1.0001);   // a sum of squares above it is above tol^2
+    const int max_iter = sc->max_iter;
+    const double rz0 = sc->rz;
+    DF rz{(float)rz0, (float)(rz0 - (double)(float)rz0)};
+    float alpha = 0.f, beta = (float)sc->beta;
+    int iter = sc->iter;
+    bool done = false, converged = false;
+
+    unsigned long long epoch = A.epoch;
+    unsigned long long t_mark = 0, ns_spmv = 0, ns_vec = 0;
+    const bool timed = A.profile && blockIdx.x == 0 && threadIdx.x == 0;
+    DF pAp{0.f, 0.f};
+    for (int it = 0; it < A.max_iters && !done; ++it) {
+        if (timed) t_mark = now_ns();
+        // ---- p = r + beta p of the halo and the own rows; y = A p
+        for (int h = threadIdx.x; h < nh; h += kPersistThreads) {
+            const float4 r = sh[h], w = sw[h];
+            sw[h] = make_float4(r.x + beta * w.x, r.y + beta * w.y, r.z + beta * w.z, 0.f);
+        }
+        __syncthreads();
+        DotAcc32 acc;
+        for (int i = threadIdx.x / G; i < nr; i += NG) {
+            const int cn = scnt[i], base = srow[i], p = lo + i;
+            float4 w = sp[i];
+            const float4 r = sr[i];
+            w = make_float4(r.x + beta * w.x, r.y + beta * w.y, r.z + beta * w.z, 0.f);
+            float ax = 0.f, ay = 0.f, az = 0.f;
+            float4 xp = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (!CACHED && cn > 0) xp = __ldg(S.xs4 + p);
+            for (int j0 = lane; j0 < cn; j0 += G * U) {
+                int l[U];
+                float a1[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int j = j0 + u * G;
+                    l[u] = 0;
+                    a1[u] = 0.f;
+                    if (j < cn) {
+                        l[u] = CACHED ? sl[base + j] : __ldg(S.lidx + base + j);
+                        a1[u] = CACHED ? sa1[base + j] : __ldg(S.inv_d0 + base + j);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int j = j0 + u * G;
+                    if (j >= cn) continue;
+                    const float4 Wq = sw[l[u]];
+                    BondGeometry g;
+                    if constexpr (CACHED) {
+                        g = sg[base + j];
+                    } else {
+                        const float inv_d0 = a1[u];
+                        g = bond_geometry(shx[l[u]], xp, sup, inv_d0, a1[u]);
+                    }
+                    const float wx = w.x - Wq.x, wy = w.y - Wq.y, wz = w.z - Wq.z;
+                    const float d = fmaf(g.x, wx, fmaf(g.y, wy, g.z * wz)) * g.i3;
+                    ax = fmaf(a1[u], wx, fmaf(d, g.x, ax));
+                    ay = fmaf(a1[u], wy, fmaf(d, g.y, ay));
+                    az = fmaf(a1[u], wz, fmaf(d, g.z, az));
+                }
+            }
+            if (cn >= 0) spmv_finish_mixed<G, true>(P, S, p, S.act[p], w, ax, ay, az, lane, gmask, sy - lo, acc);
+            else if (lane == 0) sy[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            __syncwarp(gmask);   // every lane has read sp[i]
+            if (lane == 0) sp[i] = w;
+        }
+        pAp = acc.v;
+        if (!exchange_sum(ex, pAp, G, A, ++epoch, [](int, int) {})) return;
+        alpha = df_quotient(rz, pAp);
+        if (timed) {
+            const unsigned long long t = now_ns();
+            ns_spmv += t - t_mark;
+            t_mark = t;
+        }
+        // ---- x += alpha p ; r -= alpha A p, by the lanes that formed the rows
+        ++epoch;
+        const unsigned tag = (unsigned)epoch;
+        DotAcc32 rr;
+        if (lane == 0) {
+            for (int i = threadIdx.x / G; i < nr; i += NG) {
+                const float4 pv = sp[i], yv = sy[i];
+                float4 xv = sx[i], rv = sr[i];
+                xv.x += alpha * pv.x; xv.y += alpha * pv.y; xv.z += alpha * pv.z;
+                rv.x -= alpha * yv.x; rv.y -= alpha * yv.y; rv.z -= alpha * yv.z;
+                sx[i] = xv;
+                sr[i] = rv;
+                publish(A.rec + lo + i, pack(DF{rv.y, rv.x}), ((unsigned long long)tag << 32) | __float_as_uint(rv.z));
+                rr.fma(rv.x, rv.x);
+                rr.fma(rv.y, rv.y);
+                rr.fma(rv.z, rv.z);
+            }
+        }
+        DF total = rr.v;
+        const auto gather = [&](int t, int threads) {   // the halo's new r
+            for (int h = t; h < nh; h += threads) {
+                ulonglong2 v;
+                if (!await(A.rec + sq[h], sc, ex, v, [tag](const ulonglong2& x) { return (unsigned)(x.y >> 32) == tag; }))
+                    return;
+                const DF yx = unpack<DF>(v.x);
+                sh[h] = make_float4(yx.lo, yx.hi, __uint_as_float((unsigned)v.y), 0.f);
+            }
+        };
+        if (!exchange_sum(ex, total, G, A, epoch, gather)) return;
+        beta = df_quotient(total, rz);
+        rz = total;
+        ++iter;
+        if (!(total.hi > tol2_far)) converged = below_tolerance(df_to_double(total), tol);
+        done = converged || iter >= max_iter;
+        if (timed) ns_vec += now_ns() - t_mark;
+    }
+    for (int t = threadIdx.x; t < nr; t += kPersistThreads) {
+        ((float4*)S.sol)[lo + t] = sx[t];
+        ((float4*)S.r)[lo + t] = sr[t];
+        ((float4*)S.p)[lo + t] = sp[t];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        sc->pAp = df_to_double(pAp);
+        sc->rz = df_to_double(rz);
+        sc->alpha = alpha;
+        sc->beta = beta;
+        sc->rnorm = sqrt(sc->rz);
+        sc->iter = iter;
+        sc->converged = converged;
+        sc->done = done;
+        sc->ns_spmv = (double)ns_spmv;
+        sc->ns_vec = (double)ns_vec;
+    }
+}
+
+struct __align__(8) Vec3d {
+    double x, y, z;
+};
+
+// FP64, G lanes per row (at least 4), U bonds in flight per lane.  The product
+// is bound by the FP64 pipe (1.7 multiply-adds per cycle and SM measured, 9 per
+// bond).
+template <bool CACHED, int G, int U>
+__global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist64(PersistArgs A)
+{
+    CgScalars* sc = A.S.sc;
+    if (((volatile CgScalars*)sc)->done) return;
+    extern __shared__ __align__(32) unsigned char smem[];
+    __shared__ Exchange ex;
+    __shared__ double s_alpha, s_beta, s_rz;
+    __shared__ int s_done, s_converged;
+    const StepParams& P = A.P;
+    const DeviceState& S = A.S;
+    const int lo = blockIdx.x * A.rows;
+    const int nr = min(A.rows, P.n - lo);
+    double2* sJ = (double2*)smem;                        // three per bond: xx yy | zz xy | xz yz
+    Vec3d* sx = (Vec3d*)(sJ + 3 * (size_t)A.bonds);
+    Vec3d* sr = sx + A.rows;
+    Vec3d* sp = sr + A.rows;
+    Vec3d* sy = sp + A.rows;
+    Vec3d* sw = sy + A.rows;                             // the halo's p
+    Vec3d* sh = sw + A.halo;                             // the halo's r
+    int* srow = (int*)(sh + A.halo);
+    int* scnt = srow + A.rows;
+    int* sq = scnt + A.rows;
+    uint16_t* sl = (uint16_t*)(sq + A.halo);
+
+    const int lane = threadIdx.x & (G - 1);
+    const unsigned gmask = group_mask<G>();
+    constexpr int NG = kPersistThreads / G;
+    const int first = CACHED ? S.row_ptr[lo] : 0;
+    const auto load3 = [](const void* v, int p) {
+        const dbl4 a = ((const dbl4*)v)[p];
+        return Vec3d{a.x, a.y, a.z};
+    };
+    for (int t = threadIdx.x; t < nr; t += kPersistThreads) {
+        const int p = lo + t;
+        sx[t] = load3(S.sol, p);
+        sr[t] = load3(S.r, p);
+        sp[t] = load3(S.p, p);
+        scnt[t] = is_dirichlet(S.act[p] & kActMask) ? -1 : S.cnt[p];
+        srow[t] = S.row_ptr[p] - first;
+    }
+    const int h0 = S.halo_ptr[blockIdx.x], nh = S.halo_ptr[blockIdx.x + 1] - h0;
+    for (int h = threadIdx.x; h < nh; h += kPersistThreads) {
+        const int q = S.halo[h0 + h];
+        sq[h] = q;
+        sw[h] = load3(S.p, q);
+        sh[h] = load3(S.r, q);
+    }
+    if (threadIdx.x == 0) {
+        ex.error = 0;
+        s_rz = sc->rz;
+        s_beta = sc->beta;
+        s_done = 0;
+        s_converged = 0;
+    }
+    __syncthreads();
+    if (CACHED) {
+        for (int i = threadIdx.x / G; i < nr; i += NG) {
+            const int cn = scnt[i], base = srow[i];
+            for (int j = lane; j < cn; j += G) {
+                const double2* J = (const double2*)(S.jac + 6ll * (first + base + j));
+                sJ[3 * (base + j)] = J[0];
+                sJ[3 * (base + j) + 1] = J[1];
+                sJ[3 * (base + j) + 2] = J[2];
+                sl[base + j] = S.lidx[first + base + j];
+            }
+        }
+    }
+    const double tol = sc->tol;
+    const int max_iter = sc->max_iter;
+    int iter = sc->iter;
+
+    unsigned long long epoch = A.epoch;
+    unsigned long long t_mark = 0, ns_spmv = 0, ns_vec = 0;
+    const bool timed = A.profile && blockIdx.x == 0 && threadIdx.x == 0;
+    double pAp = 0.0;
+    const auto next_p = [](const Vec3d& r, const Vec3d& p, double beta) {
+        return Vec3d{r.x + beta * p.x, r.y + beta * p.y, r.z + beta * p.z};
+    };
+    for (int it = 0; it < A.max_iters && !s_done; ++it) {
+        if (timed) t_mark = now_ns();
+        const double beta = s_beta;
+        for (int h = threadIdx.x; h < nh; h += kPersistThreads) sw[h] = next_p(sh[h], sw[h], beta);
+        for (int t = threadIdx.x; t < nr; t += kPersistThreads) sp[t] = next_p(sr[t], sp[t], beta);
+        __syncthreads();
+        double acc = 0.0;
+        for (int i = threadIdx.x / G; i < nr; i += NG) {
+            const int cn = scnt[i], base = srow[i], p = lo + i;
+            double ax = 0, ay = 0, az = 0;
+            for (int j0 = lane; j0 < cn; j0 += G * U) {
+                int l[U];
+                double2 J[U][3];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int j = j0 + u * G;
+                    if (j < cn) {
+                        l[u] = CACHED ? sl[base + j] : __ldg(S.lidx + base + j);
+                        const double2* s = CACHED ? sJ + 3 * (base + j) : (const double2*)(S.jac + 6ll * (base + j));
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) J[u][k] = CACHED ? s[k] : __ldg(s + k);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (j0 + u * G >= cn) continue;
+                    const Vec3d w = sw[l[u]];
+                    const double2 a = J[u][0], b = J[u][1], c = J[u][2];
+                    ax = fma(a.x, w.x, fma(b.y, w.y, fma(c.x, w.z, ax)));
+                    ay = fma(b.y, w.x, fma(a.y, w.y, fma(c.y, w.z, ay)));
+                    az = fma(c.x, w.x, fma(c.y, w.y, fma(b.x, w.z, az)));
+                }
+            }
+            if (cn < 0) {
+                if (lane < 3) ((double*)(sy + i))[lane] = 0.0;
+                continue;
+            }
+            ax = group_sum<G>(ax, gmask);
+            ay = group_sum<G>(ay, gmask);
+            az = group_sum<G>(az, gmask);
+            if (lane < 3) {   // one component per lane: a third of the FP64 instructions
+                const double* D = S.jdiag + 6ll * p;
+                const Vec3d w = sp[i];
+                const double d0 = D[lane == 0 ? 0 : lane == 1 ? 3 : 4], d1 = D[lane == 0 ? 3 : lane == 1 ? 1 : 5],
+                             d2 = D[lane == 0 ? 4 : lane == 1 ? 5 : 2];
+                const double s = lane == 0 ? ax : lane == 1 ? ay : az;
+                const double wk = lane == 0 ? w.x : lane == 1 ? w.y : w.z;
+                const double k = fma(d0, w.x, fma(d1, w.y, fma(d2, w.z, -s)));
+                const double y = fma(P.t2, k, P.mass * wk);
+                ((double*)(sy + i))[lane] = y;
+                acc = fma(wk, y, acc);
+            }
+        }
+        pAp = acc;
+        if (!exchange_sum(ex, pAp, 1, A, ++epoch, [](int, int) {})) return;
+        if (threadIdx.x == 0) s_alpha = s_rz / pAp;
+        __syncthreads();
+        if (timed) {
+            const unsigned long long t = now_ns();
+            ns_spmv += t - t_mark;
+            t_mark = t;
+        }
+        ++epoch;
+        const unsigned tag = (unsigned)epoch;
+        const double alpha = s_alpha;
+        double rr = 0.0;
+        for (int t = threadIdx.x; t < nr; t += kPersistThreads) {
+            const Vec3d pv = sp[t], yv = sy[t];
+            Vec3d xv = sx[t], rv = sr[t];
+            xv.x += alpha * pv.x; xv.y += alpha * pv.y; xv.z += alpha * pv.z;
+            rv.x -= alpha * yv.x; rv.y -= alpha * yv.y; rv.z -= alpha * yv.z;
+            sx[t] = xv;
+            sr[t] = rv;
+            // 24 bytes and the tag in two records: (x, y low), (z, y high)
+            const unsigned long long y = (unsigned long long)__double_as_longlong(rv.y), hi = (unsigned long long)tag << 32;
+            ulonglong2* rec = A.rec + 2 * (size_t)(lo + t);
+            publish(rec, pack(rv.x), hi | (y & 0xffffffffull));
+            publish(rec + 1, pack(rv.z), hi | (y >> 32));
+            rr = fma(rv.x, rv.x, fma(rv.y, rv.y, fma(rv.z, rv.z, rr)));
+        }
+        const auto gather = [&](int t, int threads) {
+            const auto arrived = [tag](const ulonglong2& x) { return (unsigned)(x.y >> 32) == tag; };
+            for (int h = t; h < nh; h += threads) {
+                const ulonglong2* rec = A.rec + 2 * (size_t)sq[h];
+                ulonglong2 a, b;
+                if (!await(rec, sc, ex, a, arrived) || !await(rec + 1, sc, ex, b, arrived)) return;
+                sh[h] = Vec3d{unpack<double>(a.x), unpack<double>((b.y << 32) | (a.y & 0xffffffffull)), unpack<double>(b.x)};
+            }
+        };
+        if (!exchange_sum(ex, rr, 1, A, epoch, gather)) return;
+        ++iter;
+        if (threadIdx.x == 0) {
+            s_beta = rr / s_rz;
+            s_rz = rr;
+            s_converged = below_tolerance(rr, tol);
+            s_done = s_converged || iter >= max_iter;
+        }
+        __syncthreads();
+        if (timed) ns_vec += now_ns() - t_mark;
+    }
+    for (int t = threadIdx.x; t < nr; t += kPersistThreads) {
+        ((dbl4*)S.sol)[lo + t] = make_dbl4(sx[t].x, sx[t].y, sx[t].z, 0.0);
+        ((dbl4*)S.r)[lo + t] = make_dbl4(sr[t].x, sr[t].y, sr[t].z, 0.0);
+        ((dbl4*)S.p)[lo + t] = make_dbl4(sp[t].x, sp[t].y, sp[t].z, 0.0);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        sc->pAp = pAp;
+        sc->rz = s_rz;
+        sc->alpha = s_alpha;
+        sc->beta = s_beta;
+        sc->rnorm = sqrt(s_rz);
+        sc->iter = iter;
+        sc->converged = s_converged;
+        sc->done = s_done;
+        sc->ns_spmv = (double)ns_spmv;
+        sc->ns_vec = (double)ns_vec;
+    }
+}
+
+size_t persist_smem(bool fp64, int rows, int halo, int bonds)
+{
+    const size_t v = fp64 ? sizeof(Vec3d) : sizeof(float4);
+    const size_t bond = (fp64 ? 6 * sizeof(double) : sizeof(BondGeometry) + sizeof(float)) + sizeof(uint16_t);
+    return (4 * v + 2 * sizeof(int)) * rows + (v * (fp64 || bonds > 0 ? 2 : 3) + sizeof(int)) * halo + bond * (size_t)bonds;
+}
+
+template <bool CACHED>
+const void* persist_kernel_t(bool fp64, int lanes)
+{
+    switch (lanes) {
+    case 4: return fp64 ? (const void*)k_cg_persist64<CACHED, 4, 4> : (const void*)k_cg_persist32<CACHED, 4, 4>;
+    case 8: return fp64 ? (const void*)k_cg_persist64<CACHED, 8, 4> : (const void*)k_cg_persist32<CACHED, 8, 4>;
+    case 16: return fp64 ? (const void*)k_cg_persist64<CACHED, 16, 4> : (const void*)k_cg_persist32<CACHED, 16, 4>;
+    default: return fp64 ? (const void*)k_cg_persist64<CACHED, 32, 2> : (const void*)k_cg_persist32<CACHED, 32, 2>;
+    }
+}
+
+const void* persist_kernel(bool fp64, const CgPersistPlan& pl)
+{
+    return pl.bonds > 0 ? persist_kernel_t<true>(fp64, pl.lanes) : persist_kernel_t<false>(fp64, pl.lanes);
+}
+
+}  // namespace
+
+CgPersistPlan cg_persist_rows(bool fp64, int n, int sm_count, int device)
+{
+    CgPersistPlan pl{};
+    int coop = 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
+    if (!coop || n <= 0 || n > kPersistMaxRows) return pl;
+    const int most = std::min(sm_count, kPersistMaxGrid);
+    // An exchange costs 1.2 us among 64 blocks and 1.8 among 152, so mixed
+    // precision spreads thin only down to 32 rows per block: 4096 particles
+    // take 6.0 us per iteration at 32 rows, 6.7 at 27 (152 blocks) and 8.6 at
+    // 64; 512 take 5.2 (5.5 at 4 rows).  FP64, bound by its pipe, goes down to
+    // 8 rows: 3000 particles take 15.0 us at 20 rows and 17.1 at 32.
+    pl.rows = std::max(fp64 ? 8 : 32, (n + most - 1) / most);
+    pl.grid = (n + pl.rows - 1) / pl.rows;
+    return pl;
+}
+
+bool cg_persist_plan(bool fp64, int max_halo, int max_bonds, int device, CgPersistPlan* plan)
+{
+    CgPersistPlan pl = *plan;
+    int optin = 0;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    const int room = optin - (int)sizeof(Exchange) - 1024;
+    pl.halo = max_halo;
+    const long long bonds = (long long)pl.rows * ((max_bonds + 7) / 8 * 8);
+    pl.bonds = bonds < (1 << 20) && persist_smem(fp64, pl.rows, pl.halo, (int)bonds) <= (size_t)room ? (int)bonds : 0;
+    pl.smem = persist_smem(fp64, pl.rows, pl.halo, pl.bonds);
+    if (pl.smem > (size_t)room) return false;
+    pl.lanes = 32;
+    while (pl.lanes > 4 && kPersistThreads / pl.lanes < pl.rows) pl.lanes /= 2;
+    const void* k = persist_kernel(fp64, pl);
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, room) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kPersistThreads, pl.smem);
+    if (per_sm < 1) return false;
+    *plan = pl;
+    return true;
+}
+
+cudaError_t launch_cg_persist(bool fp64, const StepParams& P, const DeviceState& S, const CgPersistPlan& plan,
+                              ulonglong2* rec, ulonglong2* inbox, unsigned long long epoch, int max_iters, bool profile,
+                              cudaStream_t st)
+{
+    PersistArgs A{P, S, rec, inbox, epoch, plan.rows, plan.halo, plan.bonds, max_iters, profile ? 1 : 0};
+    void* args[] = {&A};
+    return cudaLaunchCooperativeKernel(persist_kernel(fp64, plan), dim3(plan.grid), dim3(kPersistThreads), args, plan.smem,
+                                       st);
+}
+
+}  // namespace pdgb

@@ -459,11 +459,10 @@ pd_status Engine::dataio_load_state(size_t timestep)
         launch_refresh(fp64_, P, S_, L_, stream_);
         launch_stretch_limits(S_, (int)std::min<long long>(((long long)n_ + kBlock - 1) / kBlock, 4096), stream_);
         launches_ += 2;
-        if (S_.lidx && S_.n_tiles > 0) {
-            int max_halo = 0;
-            CK(build_tiles(S_, n_, &max_halo, stream_), "rebuild tiles");
-            S_.halo_cap = std::min(max_halo, kMaxHaloCap);
-        }
+    }
+    if (S_.lidx && S_.n_tiles > 0) {
+        const pd_status hs = build_halos();
+        if (hs != PD_OK) return hs;
     }
     if (lat_ok_ && !same_order) {
         lattice_free(&latb_);
@@ -923,11 +922,10 @@ pd_status Engine::dataio_load_state_reference(size_t timestep)
         launch_refresh(fp64_, P, S_, L_, stream_);
         launch_stretch_limits(S_, (int)std::min<long long>(((long long)n_ + kBlock - 1) / kBlock, 4096), stream_);
         launches_ += 2;
-        if (S_.lidx && S_.n_tiles > 0) {
-            int max_halo = 0;
-            CK(build_tiles(S_, n_, &max_halo, stream_), "rebuild tiles");
-            S_.halo_cap = std::min(max_halo, kMaxHaloCap);
-        }
+    }
+    if (S_.lidx && S_.n_tiles > 0) {
+        const pd_status hs = build_halos();
+        if (hs != PD_OK) return hs;
     }
     lattice_resync(true);
     last_params_ = P;

@@ -147,6 +147,9 @@ void Engine::free_all()
     lat_fixed_built_ = false;
     if (d_p2_) cudaFree(d_p2_);
     d_p2_ = nullptr;
+    if (d_inbox_) cudaFree(d_inbox_);
+    d_inbox_ = nullptr;
+    persist_ = CgPersistPlan{};
     L_.lattice = 0;
     L_.lat = nullptr;
     cudaFree(contact_.counts);
@@ -320,10 +323,9 @@ pd_status Engine::make_ready()
         if (n > 0 && opt_.spmv_path == 1) {
             CK(dalloc(&S_.lidx, slots), "alloc local indices");
             S_.tile_rows = kTileRows;
-            int max_halo = 0;
-            CK(build_tiles(S_, n, &max_halo, stream_), "build tiles");
+            s = build_halos();
+            if (s != PD_OK) return s;
             launches_ += 2;
-            S_.halo_cap = std::min(max_halo, kMaxHaloCap);
         }
     }
     // PD-PD contact hash: a power-of-two bucket count >= 2 n
@@ -369,6 +371,8 @@ pd_status Engine::make_ready()
         }
     }
     s = tune_spmv();
+    if (s != PD_OK) return s;
+    s = persist_prepare();
     if (s != PD_OK) return s;
     if (opt_.warm_start == 2 || opt_.warm_start == 3) {
         s = hist_prepare();
@@ -525,6 +529,45 @@ void Engine::apply_op(const StepParams& P, const void* in, void* out, ReduceSlot
     if (L_.lattice)
         launch_spmv_lattice(dot_out != nullptr, P, S_, lat_, in, out, slot, nullptr, dot_out, nullptr, nullptr, stream_);
     else launch_operator_u(fp64_, P, S_, L_.lanes, L_.unroll, L_.grid_bonds, in, out, slot, dot_out, stream_);
+}
+
+// Small bodies on the gather product: the iterations of a solve in one
+// cooperative launch (cg_persist.cu).
+pd_status Engine::persist_prepare()
+{
+    if (n_ <= 0 || batch_member_ || L_.lattice || L_.tiled || opt_.preconditioner || S_.lidx) return PD_OK;
+    CgPersistPlan plan = cg_persist_rows(fp64_, n_, sm_count_, device_);
+    if (plan.grid == 0) return PD_OK;
+    int max_halo = 0, unfit = 0;
+    // each block's halo, and every bond's index into it
+    CK(dalloc(&S_.lidx, (size_t)std::max<long long>(total_slots_, 1)), "alloc local indices");
+    S_.tile_rows = plan.rows;
+    CK(build_tiles(S_, n_, &max_halo, &unfit, stream_), "build tiles");
+    launches_ += 2;
+    if (unfit > 0 || !cg_persist_plan(fp64_, max_halo, sim_.pd_max_num_bonds, device_, &plan)) {
+        if (S_.lidx) cudaFree(S_.lidx);
+        S_.lidx = nullptr;
+        free_tiles(S_);
+        return PD_OK;
+    }
+    const size_t inbox = 2 * (size_t)plan.grid * plan.grid, rec = (fp64_ ? 2 : 1) * (size_t)n_;
+    CK(dalloc(&d_inbox_, inbox + rec), "alloc records");
+    CK(cudaMemsetAsync(d_inbox_, 0, sizeof(ulonglong2) * (inbox + rec), stream_), "memset records");
+    persist_epoch_ = 0;
+    persist_ = plan;
+    return PD_OK;
+}
+
+// The tiles' halos and local indices of the CSR rows as they are.  A body
+// whose blocks' halos no longer fit (a checkpoint in another slot order) leaves
+// the one-launch solve.
+pd_status Engine::build_halos()
+{
+    int max_halo = 0, unfit = 0;
+    CK(build_tiles(S_, n_, &max_halo, &unfit, stream_), "build tiles");
+    S_.halo_cap = std::min(max_halo, kMaxHaloCap);
+    if (persist_.grid > 0 && (unfit > 0 || max_halo > persist_.halo)) persist_ = CgPersistPlan{};
+    return PD_OK;
 }
 
 void Engine::lattice_resync(bool force)
@@ -958,6 +1001,11 @@ pd_status Engine::solve(const StepParams& P)
         launch_pcg_start(fp64_, P, S_, L_, stream_);
         launches_ += 2;
     }
+    if (persist_.grid > 0) {
+        pd_status s = cg_persist_loop(P);
+        if (s != PD_OK) return s;
+        return solve_finish(P);
+    }
     // iteration 0 from the host: the sample of the profiled kernel times (a
     // live launch unless the guess had already converged)
     cg_iteration(P, 0, 0, true);
@@ -987,6 +1035,12 @@ pd_status Engine::solve(const StepParams& P)
         pd_status s = cg_host_loop(P);
         if (s != PD_OK) return s;
     }
+    return solve_finish(P);
+}
+
+// After the read-back of a solve's scalars.
+pd_status Engine::solve_finish(const StepParams& P)
+{
     last_iters_ = h_sc_->iter;
     last_res_ = h_sc_->rnorm;
     last_tol_ = h_sc_->tol;
@@ -1117,6 +1171,46 @@ pd_status Engine::cg_host_loop(const StepParams& P)
             return PD_ERR_STATE;
         }
         batch = std::max(check, launched / 8);
+    }
+    return PD_OK;
+}
+
+pd_status Engine::cg_persist_loop(const StepParams& P)
+{
+    const int check = opt_.cg_check_interval > 0 ? opt_.cg_check_interval : 8;
+    const bool whole = opt_.cg_loop == 0;
+    int batch = whole ? std::max(1, opt_.cg_max_iterations) : std::max(1, predicted_iters_ - 1);
+    double ns_spmv = 0.0, ns_vec = 0.0;
+    for (long long run = 0;;) {
+        CK(launch_cg_persist(fp64_, P, S_, persist_, d_inbox_ + 2 * (size_t)persist_.grid * persist_.grid, d_inbox_,
+                             persist_epoch_, batch, profiling_, stream_),
+           "cg launch");
+        persist_epoch_ += 2ull * (unsigned long long)batch;
+        ++launches_;
+        CK(cudaMemcpyAsync(h_sc_, S_.sc, sizeof(CgScalars), cudaMemcpyDeviceToHost, stream_), "read cg scalars");
+        CK(cudaStreamSynchronize(stream_), "cg sync");
+        ++host_syncs_;
+        if (h_sc_->wait_error) {
+            err_ = "cg: a grid-wide wait ran out of time";
+            return PD_ERR_CUDA;
+        }
+        ns_spmv += h_sc_->ns_spmv;
+        ns_vec += h_sc_->ns_vec;
+        if (h_sc_->done) break;
+        run += batch;
+        if (run > opt_.cg_max_iterations + 2LL * check) {
+            err_ = "cg: iteration count not advancing";
+            return PD_ERR_STATE;
+        }
+        batch = (int)std::max<long long>(check, run / 8);
+    }
+    if (whole) ++cg_graph_solves_;
+    if (profiling_ && h_sc_->iter > 0) {   // one sample per solve: the mean over its iterations
+        const double ms = 1e-6 / h_sc_->iter;
+        kc_sample_ms_[PD_KC_SPMV] += ns_spmv * ms;
+        kc_sample_ms_[PD_KC_CG_VECTOR] += ns_vec * ms;
+        kc_samples_[PD_KC_SPMV] += 1;
+        kc_samples_[PD_KC_CG_VECTOR] += 1;
     }
     return PD_OK;
 }

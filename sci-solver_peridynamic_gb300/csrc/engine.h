@@ -71,6 +71,8 @@ private:
     pd_status tune_spmv();
     // y = A in with this handle's product (lattice stencil or CSR rows)
     void apply_op(const StepParams& P, const void* in, void* out, ReduceSlot slot, double* dot_out);
+    pd_status persist_prepare();
+    pd_status build_halos();
     void lattice_resync(bool force);   // the lattice product's 1/d0 table from the live CSR bonds
     // mixed mode: reorders every row's live bonds for the (g, u) SpMV shape
     void relayout_bonds(int g, int u);
@@ -91,6 +93,7 @@ private:
     void* hist_vec(int j) const;
     pd_status integrate(bool* advanced);
     pd_status solve(const StepParams& P);
+    pd_status solve_finish(const StepParams& P);
     // one CG iteration's launches (iteration k of the solve: on lattice bodies
     // its parity picks the direction buffers); cond: the CG graph's while
     // condition when captured into it, else 0
@@ -101,6 +104,9 @@ private:
     // cg_graph_body() iterations until the device-side test stops it
     cudaError_t cg_graph_launch(const StepParams& P);
     pd_status cg_host_loop(const StepParams& P);   // the same iterations in host-checked batches
+    // a small body's iterations in one cooperative launch (cg_loop 0) or in
+    // host-checked batches of it (cg_loop 1)
+    pd_status cg_persist_loop(const StepParams& P);
     void hist_collect();   // the projection's statistics, after the solve's read-back
     template <typename T>
     pd_status download_scatter(const T* dev, T* host_out, size_t count_per, size_t elem_count);
@@ -193,6 +199,9 @@ private:
     long long host_syncs_ = 0;         // stream synchronisations of the step loop
     long long cg_graph_solves_ = 0;    // solves whose iterations ran in the CG graph
     bool cg_graph_failed_ = false;     // the graph could not be built: host-checked batches
+    CgPersistPlan persist_{};          // one-launch solve of a small body (grid 0: not used)
+    ulonglong2* d_inbox_ = nullptr;    // its records: partial sums (2 grid^2), then r
+    unsigned long long persist_epoch_ = 0;
     // profiling
     bool profiling_ = false;
     std::vector<cudaEvent_t> event_pool_;

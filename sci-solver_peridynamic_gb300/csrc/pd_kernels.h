@@ -50,6 +50,9 @@ struct CgScalars {
     int ws_rejects;        // batch: consecutive rejected guesses (and paused steps since)
     int ws_skip;           // batch: 1 while this step's learned pass is paused
     int ws_skipped;        // batch: steps whose learned pass was paused
+    int wait_error;        // cg_persist.cu: a wait of the one-launch solve ran out of time
+    double ns_spmv;        // cg_persist.cu, profiling: ns of the latest launch's products
+    double ns_vec;         // ... and of its vector phases
 };
 
 // Partial-sum scratch of a reducing launch: one double per block and an
@@ -244,6 +247,29 @@ void launch_spmv(bool fp64, bool dot, const StepParams& P, const DeviceState& S,
 void launch_operator(bool fp64, const StepParams& P, const DeviceState& S, int lanes, int grid, const void* in,
                      void* out, ReduceSlot slot, double* dot_out, cudaStream_t st);
 void launch_cg_residual(bool fp64, const StepParams& P, const DeviceState& S, const LaunchCfg& L, cudaStream_t st);
+// The CG iterations of a small body in one cooperative launch (cg_persist.cu).
+constexpr int kPersistMaxRows = 200000;   // (a block's share of more does not fit in shared memory)
+struct CgPersistPlan {
+    int grid = 0;        // blocks (0: the body does not qualify)
+    int rows = 0;        // rows per block
+    int halo = 0;        // the largest number of distinct neighbours of a block's rows
+    int bonds = 0;       // bond slots kept in shared memory per block (0: read from global memory)
+    int lanes = 0;       // lanes per row
+    size_t smem = 0;
+};
+// rows per block and grid for a body of n rows (grid 0: does not qualify)
+CgPersistPlan cg_persist_rows(bool fp64, int n, int sm_count, int device);
+// the rest of the plan, from the blocks' largest halo (S.halo built for tiles
+// of plan->rows) and the largest row; false when a block's share does not
+// fit in shared memory
+bool cg_persist_plan(bool fp64, int max_halo, int max_bonds, int device, CgPersistPlan* plan);
+// At most max_iters iterations from the state of S (x, r, p and the scalars,
+// as the residual kernel or an earlier launch left them).  rec: n records (FP64:
+// 2 n); inbox: 2 x grid^2 records; epoch: no smaller than any epoch of earlier
+// launches on them, of which a launch uses at most 2 max_iters.
+cudaError_t launch_cg_persist(bool fp64, const StepParams& P, const DeviceState& S, const CgPersistPlan& plan,
+                              ulonglong2* rec, ulonglong2* inbox, unsigned long long epoch, int max_iters, bool profile,
+                              cudaStream_t st);
 // Preconditioned CG (no reference counterpart in use: the reference's
 // cusp::precond::diagonal is commented out, simulator.cu:767-769): mode 1 =
 // inverse diagonal of A, 2 = inverse 3x3 diagonal blocks; the stopping test
@@ -270,8 +296,9 @@ void launch_bond_relayout(const DeviceState& S, int grid, int g_from, int u_from
                           cudaStream_t st);
 // Shared-memory tile SpMV (tiles.cu).  build_tiles fills halo / halo_ptr /
 // tile_info / lidx of S (allocating them) for tiles of S.tile_rows rows and
-// returns the largest halo in *max_halo.
-cudaError_t build_tiles(DeviceState& S, int n, int* max_halo, cudaStream_t st);
+// returns the largest halo in *max_halo and the tiles whose halo did not fit
+// the builder's hash set in *unfit.
+cudaError_t build_tiles(DeviceState& S, int n, int* max_halo, int* unfit, cudaStream_t st);
 void free_tiles(DeviceState& S);
 // Tile SpMV: blocks per SM for a shared-memory halo of halo_cap entries, and the launch.
 int tile_spmv_blocks_per_sm(int lanes, int unroll, int halo_cap);

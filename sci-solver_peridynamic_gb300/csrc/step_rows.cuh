@@ -400,11 +400,11 @@ __device__ __forceinline__ void force_row(const StepParams& P, const DeviceState
                         const float2 t2 = S.d0sq[rs + bond];
                         S.d0sq[rs + bond] = S.d0sq[rs + top];
                         S.d0sq[rs + top] = t2;
-                        if (S.lidx) {
-                            const uint16_t l = S.lidx[rs + bond];
-                            S.lidx[rs + bond] = S.lidx[rs + top];
-                            S.lidx[rs + top] = l;
-                        }
+                    }
+                    if (S.lidx) {
+                        const uint16_t l = S.lidx[rs + bond];
+                        S.lidx[rs + bond] = S.lidx[rs + top];
+                        S.lidx[rs + top] = l;
                     }
                     --top;
                     continue;

@@ -12,7 +12,10 @@
 // gathering 32 bytes from L1/L2.
 //
 // Built once per make_ready (bonds are never added; a broken bond only moves
-// within its row, and its local index moves with it).
+// within its row, and its local index moves with it: every slot of a row has
+// one, so a rollback that restores broken bonds finds theirs).  The one-launch
+// solve of small bodies (cg_persist.cu) uses the same halos and indices, with a
+// tile per block.
 #include <vector>
 
 #include "pd_device.cuh"
@@ -23,11 +26,12 @@ namespace pdgb {
 
 namespace {
 
-constexpr int kHashCap = 4096;                    // per-tile hash set of neighbour slots
+constexpr int kHashBits = 13;
+constexpr int kHashCap = 1 << kHashBits;          // per-tile hash set of neighbour slots
 constexpr int kHashLimit = (kHashCap * 3) / 4;    // larger halos use the global path
 constexpr unsigned kEmpty = 0xffffffffu;
 
-__device__ __forceinline__ unsigned hash_slot(unsigned q) { return (q * 2654435761u) >> (32 - 12); }
+__device__ __forceinline__ unsigned hash_slot(unsigned q) { return (q * 2654435761u) >> (32 - kHashBits); }
 
 // Inserts the neighbour slots of rows [r0, r1) into the shared hash set;
 // returns the number of distinct slots (kHashCap + 1 when the set is full).
@@ -39,7 +43,7 @@ __device__ int tile_collect(const DeviceState& S, int r0, int r1, unsigned* tabl
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     for (int p = r0 + warp; p < r1; p += nw) {
-        const int rs = S.row_ptr[p], cn = S.cnt[p];
+        const int rs = S.row_ptr[p], cn = S.row_ptr[p + 1] - rs;
         for (int j = lane; j < cn; j += 32) {
             const unsigned q = (unsigned)S.col[rs + j];
             unsigned h = hash_slot(q);
@@ -111,7 +115,7 @@ __global__ void __launch_bounds__(kBlock) k_tile_fill(DeviceState S, int n)
         // local index of every bond: binary search in the sorted halo
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
         for (int p = r0 + warp; p < r1; p += nw) {
-            const int rs = S.row_ptr[p], cn = S.cnt[p];
+            const int rs = S.row_ptr[p], cn = S.row_ptr[p + 1] - rs;
             for (int j = lane; j < cn; j += 32) {
                 const unsigned q = (unsigned)S.col[rs + j];
                 int lo = 0, hi = info - 1;
@@ -287,10 +291,11 @@ int tile_blocks(int halo_cap)
 
 }  // namespace
 
-cudaError_t build_tiles(DeviceState& S, int n, int* max_halo, cudaStream_t st)
+cudaError_t build_tiles(DeviceState& S, int n, int* max_halo, int* unfit, cudaStream_t st)
 {
     free_tiles(S);
     *max_halo = 0;
+    *unfit = 0;
     if (n <= 0 || S.tile_rows <= 0) return cudaSuccess;
     S.n_tiles = (n + S.tile_rows - 1) / S.tile_rows;
     const size_t nt = (size_t)S.n_tiles;
@@ -321,7 +326,10 @@ cudaError_t build_tiles(DeviceState& S, int n, int* max_halo, cudaStream_t st)
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     cudaFree(counts);
     if (e != cudaSuccess) return e;
-    for (int v : info) *max_halo = v > *max_halo ? v : *max_halo;
+    for (int v : info) {
+        *max_halo = v > *max_halo ? v : *max_halo;
+        if (v < 0) ++*unfit;
+    }
     return cudaSuccess;
 }
 
