@@ -144,9 +144,6 @@ void Engine::free_all()
     sph_buffers_free(&sph_);
     lat_ = LatticeParams{};
     lat_ok_ = false;
-    lat_fixed_built_ = false;
-    if (d_p2_) cudaFree(d_p2_);
-    d_p2_ = nullptr;
     if (d_inbox_) cudaFree(d_inbox_);
     d_inbox_ = nullptr;
     persist_ = CgPersistPlan{};
@@ -267,8 +264,6 @@ pd_status Engine::make_ready()
                          total_slots_, &lat_, &latb_, &ok, stream_),
            "lattice build");
         lat_ok_ = ok != 0;
-        lat_fixed_built_ = lat_ok_ && lat_.fixed != 0;
-        if (lat_ok_) CK(cudaMalloc(&d_p2_, sizeof(float4) * N), "alloc second direction buffer");
     }
     if (n > 0) {
         CK(cudaMemcpyAsync(S_.X64, S_.x64, sizeof(dbl4) * N, cudaMemcpyDeviceToDevice, stream_), "copy X");
@@ -367,7 +362,7 @@ pd_status Engine::make_ready()
         ++launches_;
         if (lat_ok_) {   // and the lattice product's deviations (its candidates are timed next)
             launch_lattice_delta(S_, lat_, sup_, stream_);
-            ++launches_;
+            launches_ += 2;
         }
     }
     s = tune_spmv();
@@ -440,16 +435,12 @@ pd_status Engine::tune_spmv()
         // bond reorderings would cost make_ready ~45 ms: the stencil only
         if (opt_.spmv_path == 3 || n_ >= kLatticeOnlyRows) cand.clear();
         cand.push_back({0, 1, 1, 1});
-        // the 80-entry stencil also runs on the general kernel (offsets from
-        // the launch parameters instead of compile-time constants)
-        if (lat_fixed_built_ && n_ >= 20000) cand.push_back({0, 1, 1, 2});
     }
     if (cand.empty()) cand.push_back({0, fixed_lanes ? fixed_lanes : 8, fixed_unroll ? fixed_unroll : 1});
     auto apply = [&](const Cand& c) {
         L_.lattice = c.lattice ? 1 : 0;
         L_.lat = c.lattice ? &lat_ : nullptr;
         if (c.lattice) {
-            lat_.fixed = (c.lattice == 1 && lat_fixed_built_) ? 1 : 0;
             L_.tiled = 0;
             L_.lanes = 1;
             L_.unroll = 1;
@@ -485,13 +476,10 @@ pd_status Engine::tune_spmv()
     Cand best_c = cand[0];
     // each candidate: one warm-up launch, then the best of three timed pairs
     // of the CG iteration's product as the CG loop launches it (y = A p with
-    // <p, y>; the lattice product with the direction update fused in; the
-    // scalars and the second direction buffer it writes are reset by the
-    // first solve)
+    // <p, y>; the scalars it writes are reset by the first solve)
     const auto cg_product = [&]() {
-        if (L_.lattice && d_p2_)
-            launch_spmv_lattice(true, P, S_, lat_, S_.p, S_.y, ReduceSlot{S_.partials, S_.counters + 1}, S_.sc,
-                                nullptr, S_.r, d_p2_, stream_);
+        if (L_.lattice)
+            launch_spmv_lattice(true, P, S_, lat_, S_.y, ReduceSlot{S_.partials, S_.counters + 1}, S_.sc, nullptr, stream_);
         else
             launch_spmv(fp64_, true, P, S_, L_, stream_);
     };
@@ -526,8 +514,11 @@ pd_status Engine::tune_spmv()
 
 void Engine::apply_op(const StepParams& P, const void* in, void* out, ReduceSlot slot, double* dot_out)
 {
-    if (L_.lattice)
-        launch_spmv_lattice(dot_out != nullptr, P, S_, lat_, in, out, slot, nullptr, dot_out, nullptr, nullptr, stream_);
+    if (L_.lattice) {
+        launch_lattice_scatter(S_, lat_, in, stream_);
+        launch_spmv_lattice(dot_out != nullptr, P, S_, lat_, out, slot, nullptr, dot_out, stream_);
+        ++launches_;
+    }
     else launch_operator_u(fp64_, P, S_, L_.lanes, L_.unroll, L_.grid_bonds, in, out, slot, dot_out, stream_);
 }
 
@@ -926,7 +917,7 @@ pd_status Engine::integrate(bool* advanced)
     mark_begin(PD_KC_FORCE, -1);
     launch_force(fp64_, Pf, S_, L_, stream_);
     mark_end();
-    launches_ += fp64_ ? 1 : (L_.lattice ? 3 : 2);   // mixed: the supercell words (+ lattice deviations), the pass
+    launches_ += fp64_ ? 1 : (L_.lattice ? 4 : 2);   // mixed: the supercell words (+ lattice deviations and halos), the pass
     lattice_resync(false);        // only where the pass broke a bond (read on the device)
     const bool adaptive = run_.integrator == PD_NEWMARK_BETA || run_.adaptive_integration != 0;
     if (adaptive) {
@@ -942,7 +933,7 @@ pd_status Engine::integrate(bool* advanced)
             CK(cudaMemcpyAsync(S_.x64, S_.x64_bk, sizeof(dbl4) * N, cudaMemcpyDeviceToDevice, stream_), "restore x");
             CK(cudaMemcpyAsync(S_.v64, S_.v64_bk, sizeof(dbl4) * N, cudaMemcpyDeviceToDevice, stream_), "restore v");
             launch_refresh(fp64_, Pf, S_, L_, stream_);
-            launches_ += L_.lattice ? 2 : 1;
+            launches_ += L_.lattice ? 3 : 1;
             lattice_resync(true);   // the restored live sets
             return PD_OK;
         }
@@ -1006,6 +997,10 @@ pd_status Engine::solve(const StepParams& P)
         if (s != PD_OK) return s;
         return solve_finish(P);
     }
+    if (L_.lattice) {   // the first direction onto the lattice's grid
+        launch_lattice_scatter(S_, lat_, S_.p, stream_);
+        ++launches_;
+    }
     // iteration 0 from the host: the sample of the profiled kernel times (a
     // live launch unless the guess had already converged)
     cg_iteration(P, 0, 0, true);
@@ -1041,6 +1036,10 @@ pd_status Engine::solve(const StepParams& P)
 // After the read-back of a solve's scalars.
 pd_status Engine::solve_finish(const StepParams& P)
 {
+    if (h_sc_->wait_error) {
+        err_ = "cg: a bounded wait of a kernel ran out of time";
+        return PD_ERR_CUDA;
+    }
     last_iters_ = h_sc_->iter;
     last_res_ = h_sc_->rnorm;
     last_tol_ = h_sc_->tol;
@@ -1054,7 +1053,7 @@ pd_status Engine::solve_finish(const StepParams& P)
     }
     if (profiling_) {
         kc_launches_[PD_KC_SPMV] += last_iters_;
-        kc_launches_[PD_KC_CG_VECTOR] += (L_.lattice && d_p2_ ? 1LL : 2LL) * last_iters_;
+        kc_launches_[PD_KC_CG_VECTOR] += 2LL * last_iters_;
     }
     if (!h_sc_->converged) cg_converged_ = false;
     if (ws_features_needed()) return ws_after_cg(P);
@@ -1067,22 +1066,15 @@ void Engine::cg_iteration(const StepParams& P, int k, cudaGraphConditionalHandle
     // index, so that the event records barely perturb the solve they measure;
     // the mean sampled duration is scaled to the exact launch count
     sample = sample && profiling_ && cond == 0 && (k % kMarkStride) == 0;
-    if (L_.lattice && d_p2_) {
-        // the direction update p = r + beta p is fused into the product, which
-        // reads the previous direction from one buffer and writes the new one
-        // to the other (buffer 0 = S_.p, set to r by the residual kernel)
-        // (preconditioned: p = z + beta p, from the z buffer)
-        void* p_prev = (k & 1) ? d_p2_ : S_.p;
-        void* p_new = (k & 1) ? S_.p : d_p2_;
+    if (L_.lattice) {
+        // the direction lives in slot order and on the lattice's dense grid
         if (sample) mark_begin(PD_KC_SPMV, k);
-        launch_spmv_lattice(true, P, S_, lat_, p_prev, S_.y, ReduceSlot{S_.partials, S_.counters + 1}, S_.sc, nullptr,
-                            opt_.preconditioner ? S_.z : S_.r, p_new, stream_);
+        launch_spmv_lattice(true, P, S_, lat_, S_.y, ReduceSlot{S_.partials, S_.counters + 1}, S_.sc, nullptr, stream_);
         if (sample) mark_end();
-        DeviceState Sj = S_;
-        Sj.p = p_new;
         if (sample) mark_begin(PD_KC_CG_VECTOR, k);
-        if (opt_.preconditioner) launch_cg_axpy_pc(fp64_, P, Sj, L_, stream_, cond);
-        else launch_cg_axpy(fp64_, P, Sj, L_, stream_, cond);
+        if (opt_.preconditioner) launch_cg_axpy_pc(fp64_, P, S_, L_, stream_, cond);
+        else launch_cg_axpy(fp64_, P, S_, L_, stream_, cond);
+        launch_lattice_xpby(S_, lat_, opt_.preconditioner ? S_.z : S_.r, L_.grid_vec, stream_);
         if (sample) mark_end();
     } else {
         if (sample) mark_begin(PD_KC_SPMV, k);
@@ -1102,8 +1094,8 @@ void Engine::cg_iteration(const StepParams& P, int k, cudaGraphConditionalHandle
     }
 }
 
-// Iterations per while-node body: an even count (the lattice product's
-// direction buffers alternate), 4 unless cg_check_interval asks otherwise.
+// Iterations per while-node body: an even count, 4 unless cg_check_interval
+// asks otherwise.
 int Engine::cg_graph_body() const
 {
     const int k = opt_.cg_check_interval > 0 ? opt_.cg_check_interval : 4;
@@ -1190,10 +1182,7 @@ pd_status Engine::cg_persist_loop(const StepParams& P)
         CK(cudaMemcpyAsync(h_sc_, S_.sc, sizeof(CgScalars), cudaMemcpyDeviceToHost, stream_), "read cg scalars");
         CK(cudaStreamSynchronize(stream_), "cg sync");
         ++host_syncs_;
-        if (h_sc_->wait_error) {
-            err_ = "cg: a grid-wide wait ran out of time";
-            return PD_ERR_CUDA;
-        }
+        if (h_sc_->wait_error) break;
         ns_spmv += h_sc_->ns_spmv;
         ns_vec += h_sc_->ns_vec;
         if (h_sc_->done) break;

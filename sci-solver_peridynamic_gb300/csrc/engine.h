@@ -98,7 +98,7 @@ private:
     // its parity picks the direction buffers); cond: the CG graph's while
     // condition when captured into it, else 0
     void cg_iteration(const StepParams& P, int k, cudaGraphConditionalHandle cond, bool sample);
-    int cg_kernels_per_iteration() const { return (L_.lattice && d_p2_) ? 2 : 3; }
+    int cg_kernels_per_iteration() const { return 3; }
     int cg_graph_body() const;
     // iterations 1.. of a solve as one graph launch: a while node repeating
     // cg_graph_body() iterations until the device-side test stops it
@@ -216,8 +216,6 @@ private:
     LatticeParams lat_{};
     LatticeBuffers latb_{};
     bool lat_ok_ = false;
-    bool lat_fixed_built_ = false;     // the stencil is the 80-entry one (compile-time kernel available)
-    void* d_p2_ = nullptr;             // second CG direction buffer of the lattice product's fused update
     bool batch_member_ = false;        // set by Batch: its scenes keep the builder's slot order
     ContactBuffers contact_{};         // PD-PD contact hash (when enabled)
     SphBuffers sph_{};                 // SPH <-> PD collision scratch

@@ -8,11 +8,13 @@
 // entry per bond.  Here, when every particle sits within 0.3 spacings of a
 // distinct lattice site, each bond joins two sites whose offset lies in a
 // small stencil (80 offsets for a horizon of 2.5 spacings).  The slots are
-// renumbered brick by brick (bricks of 32 x 4 x bz sites, x fastest), and the
+// renumbered brick by brick (bricks of 16 x 8 x 4 sites, x fastest), and the
 // product runs one brick per block iteration: the block stages the halo of
 // the brick's sites (each particle's deviation from its site and its entry of
-// w) in shared memory, then each thread walks its row's stencil.  Rows of a
-// warp are x-consecutive sites, so the neighbours at one stencil entry are
+// w) in shared memory, then each thread walks the stencil of one z column of
+// the brick -- its four rows at once, so that a neighbour read from shared
+// memory serves every row of the column whose stencil it is in.  Threads take
+// x-consecutive columns, so the neighbours at one stencil entry are
 // x-consecutive shared-memory words (no bank conflicts), and the only per-bond
 // stream is 1/d0 per (row, stencil entry), 0 where there is no live bond
 // (stored scaled by 2^100, see kLatScale).
@@ -40,62 +42,39 @@ namespace {
         if (e_ != cudaSuccess) return e_;      \
     } while (0)
 
-constexpr int kLatBX = 32;
-constexpr int kLatBY = 4;
-constexpr float kLatEmpty = 1.0e4f;   // deviation of an empty site (any far, finite position)
+// Bricks of 16 x 8 x 4 sites (8 x 8 x 4 for a reach of 3 sites), a thread per
+// pair of z-adjacent rows, a warp per chunk of 32 pairs.  Runs of 8 pairs in x
+// keep every 8 lanes of a 16-byte shared-memory access consecutive.
+constexpr int kLatBY = 8;
+constexpr int kLatBZ = 4;
+constexpr int kLatRZ = 2;             // rows of a thread
+__host__ __device__ constexpr int lat_bx(int R) { return R <= 2 ? 16 : 8; }
+constexpr int kLatMaxPairs = 16 * kLatBY * (kLatBZ / kLatRZ);   // of a brick
+__host__ __device__ constexpr int lat_warps(int R) { return lat_bx(R) * kLatBY * (kLatBZ / kLatRZ) / 32; }
+// the table of a chunk comes in slabs of whole stencil columns: so many of each
+// reach, at most kLatSlab entries (of 256 bytes)
+constexpr int kLatSlab = 12;
+__host__ __device__ constexpr int lat_slab_columns(int RC) { return RC >= 2 ? kLatSlab / (2 * RC + 1) : 4; }
 // The table holds 2^100 / d0: then min(1/d, entry) is 1/d for a live bond (its
 // entry is near 1e31 or more) and 0 for "no bond" (entry 0), one instruction,
 // and 1/d0 - 1/d = fma(entry, 2^-100, -1/d) is exact scaling by a power of two.
 constexpr float kLatScale = 1.2676506002282294e30f;     // 2^100
 constexpr float kLatUnscale = 7.888609052210118e-31f;   // 2^-100
-// the largest halo: R = 3, bricks of 32 x 4 x 2 sites -> 38 x 10 x 8 sites of 24 bytes
-constexpr int kLatHaloMax = 38 * 10 * 8;
-constexpr int kLatSiteBytes = sizeof(float4) + sizeof(float2);
-constexpr int kLatSmemMax = kLatHaloMax * kLatSiteBytes;
-constexpr int kLatHaloPerThread = (kLatHaloMax + kBlock - 1) / kBlock;
-
-// The stencil of a horizon of 2.5 spacings (the benchmark's 5 r): every lattice
-// offset with |v|^2 <= 6 (80 offsets, reach 2 per axis), in (dz, dy, dx)
-// order.  Bodies whose bonds all fall in it use a product specialised for it:
-// bricks of 32 x 4 x 4 sites, a 36 x 8 x 8 halo, and shared-memory offsets
-// known at compile time.
-constexpr int kS80 = 80;
-constexpr int kS80Hx = kLatBX + 4, kS80Hy = kLatBY + 4, kS80Hz = 4 + 4;
-struct Stencil80 {
-    int off[kS80];
-    int dx[kS80], dy[kS80], dz[kS80];
-};
-__host__ __device__ constexpr bool in_s80(int dx, int dy, int dz)
+__host__ __device__ constexpr int lat_halo_sites(int R)
 {
-    return (dx || dy || dz) && dx * dx + dy * dy + dz * dz <= 6 && dx >= -2 && dx <= 2 && dy >= -2 && dy <= 2 &&
-           dz >= -2 && dz <= 2;
+    return (lat_bx(R) + 2 * R) * (kLatBY + 2 * R) * (kLatBZ + 2 * R);
 }
-__host__ __device__ constexpr Stencil80 make_stencil80()
+// shared memory: barriers, the halo (a box of the direction, float4 per site,
+// then the deviations as they lie in the image: x, y pairs, then z), and two
+// slabs of the table per warp
+__host__ __device__ constexpr int lat_image_bytes(int R) { return 12 * lat_halo_sites(R); }
+__host__ __device__ constexpr int lat_halo_bytes(int R) { return (28 * lat_halo_sites(R) + 127) / 128 * 128; }
+constexpr int kLatBarrierBytes = 256;
+constexpr int kLatSlabBytes = kLatSlab * 32 * (int)sizeof(float2);
+__host__ __device__ constexpr int lat_smem(int R)
 {
-    Stencil80 t{};
-    int k = 0;
-    for (int dz = -2; dz <= 2; ++dz)
-        for (int dy = -2; dy <= 2; ++dy)
-            for (int dx = -2; dx <= 2; ++dx)
-                if (in_s80(dx, dy, dz)) {
-                    t.off[k] = (dz * kS80Hy + dy) * kS80Hx + dx;
-                    t.dx[k] = dx;
-                    t.dy[k] = dy;
-                    t.dz[k] = dz;
-                    ++k;
-                }
-    return t;
+    return kLatBarrierBytes + lat_halo_bytes(R) + 2 * lat_warps(R) * kLatSlabBytes;
 }
-__host__ __device__ constexpr int count_s80()
-{
-    int k = 0;
-    for (int dz = -2; dz <= 2; ++dz)
-        for (int dy = -2; dy <= 2; ++dy)
-            for (int dx = -2; dx <= 2; ++dx)
-                if (in_s80(dx, dy, dz)) ++k;
-    return k;
-}
-static_assert(count_s80() == kS80, "the |v|^2 <= 6 stencil has 80 offsets");
 
 // 1/sqrt(x) by the hardware approximation without a denormal path: a live
 // bond's d^2 is far above the FP32 denormal range, and an empty or padding
@@ -185,7 +164,7 @@ __global__ void __launch_bounds__(kBlock) k_lat_offsets(int n, const int4* __res
 }
 
 // shifted sites and the brick-major sort key of every slot
-__global__ void __launch_bounds__(kBlock) k_lat_keys(int n, int4* __restrict__ site, int3 lo, int bz, int3 nb,
+__global__ void __launch_bounds__(kBlock) k_lat_keys(int n, int4* __restrict__ site, int3 lo, int bx, int3 nb,
                                                      unsigned* __restrict__ key, int* __restrict__ val)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -194,11 +173,11 @@ __global__ void __launch_bounds__(kBlock) k_lat_keys(int n, int4* __restrict__ s
         s.y -= lo.y;
         s.z -= lo.z;
         site[i] = s;
-        const unsigned brick = ((unsigned)(s.z / bz) * (unsigned)nb.y + (unsigned)(s.y / kLatBY)) * (unsigned)nb.x +
-                               (unsigned)(s.x / kLatBX);
-        const unsigned local = ((unsigned)(s.z % bz) * kLatBY + (unsigned)(s.y % kLatBY)) * kLatBX +
-                               (unsigned)(s.x % kLatBX);
-        key[i] = brick * (unsigned)(kLatBX * kLatBY * bz) + local;
+        const unsigned brick = ((unsigned)(s.z / kLatBZ) * (unsigned)nb.y + (unsigned)(s.y / kLatBY)) * (unsigned)nb.x +
+                               (unsigned)(s.x / bx);
+        const unsigned local = ((unsigned)(s.z % kLatBZ) * kLatBY + (unsigned)(s.y % kLatBY)) * (unsigned)bx +
+                               (unsigned)(s.x % bx);
+        key[i] = brick * (unsigned)(bx * kLatBY * kLatBZ) + local;
         val[i] = i;
     }
 }
@@ -243,45 +222,44 @@ __global__ void k_lat_remap_col(const int* __restrict__ row_ptr_old, const int* 
     }
 }
 
-__global__ void k_lat_map(const int4* __restrict__ site, int n, int R, int mx, int my, int* __restrict__ map)
+__global__ void __launch_bounds__(kBlock) k_lat_dense(const int4* __restrict__ site, int n, int R, int mx, int my,
+                                                      int* __restrict__ dense)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int4 s = site[i];
-        map[((long long)(s.z + R) * my + (s.y + R)) * mx + (s.x + R)] = i;
+        dense[i] = (int)(((long long)(s.z + R) * my + (s.y + R)) * mx + (s.x + R));
     }
 }
 
 // ---- 1/d0 table ------------------------------------------------------------------------
-__global__ void __launch_bounds__(kBlock) k_lat_ell(DeviceState S, LatticeParams lp, int force)
+// [chunk][entry][32 pairs] words of a pair's two rows.
+__global__ void __launch_bounds__(kBlock) k_lat_ell(DeviceState S, const __grid_constant__ LatticeParams lp, int force)
 {
     if (!force && ((volatile int*)S.flags)[1] == 0) return;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < S.n; p += gridDim.x * blockDim.x) {
-        const int b = lp.row_brick[p];
-        const int start = lp.brick_start[b];
-        const int rows = lp.brick_start[b + 1] - start;
-        const int l = p - start;
-        float* e = lp.ell + (size_t)lp.K * start;
-        for (int k4 = 0; k4 < lp.K / 4; ++k4)
-            ((float4*)e)[(size_t)k4 * rows + l] = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int rp = lp.row_pair[p];   // 64 chunk + 2 lane + row
+        float* e = lp.ell + (size_t)(rp >> 6) * lp.K * 64 + (rp & 63);
+        for (int k = 0; k < lp.K; ++k) e[k * 64] = 0.f;
         const int4 sp = lp.site[p];
         const int rs = S.row_ptr[p], cn = S.cnt[p];
         for (int j = 0; j < cn; ++j) {
             const int4 sq = lp.site[S.col[rs + j]];
             const int t = ((sq.z - sp.z + kLatRmax) * kLatTab + (sq.y - sp.y + kLatRmax)) * kLatTab +
                           (sq.x - sp.x + kLatRmax);
-            const int k = lp.offk[t];
-            e[((size_t)(k >> 2) * rows + l) * 4 + (k & 3)] = S.inv_d0[rs + j] * kLatScale;
+            e[lp.offk[t] * 64] = S.inv_d0[rs + j] * kLatScale;
         }
     }
 }
 
 // ---- deviations from the lattice sites ------------------------------------------------
-// dl[i] = (d, n): x - (org + h site) = d + sup n per axis with n = rint(. / sup)
-// (FP64, exact: sup is a power of two), d rounded once to FP32; n packed in
-// 10 bits per axis (+512).  |n| stays below 512 for displacements below
-// 500 supercells; larger ones are clamped (the deviation then loses digits).
-__global__ void __launch_bounds__(kBlock) k_lat_delta(const dbl4* __restrict__ x64, int n, LatticeParams lp,
-                                                      double sup, float4* __restrict__ dl)
+// grid_d[site of i] = (d, n): x - (org + h site) = d + sup n per axis with n =
+// rint(. / sup) (FP64, exact: sup is a power of two), d rounded once to FP32;
+// n packed in 10 bits per axis (+512).  |n| stays below 512 for displacements
+// below 500 supercells; larger ones are clamped (the deviation then loses
+// digits).  (Sites without a particle keep 0: their table entries are 0, so any
+// finite deviation does.)
+__global__ void __launch_bounds__(kBlock) k_lat_delta(const dbl4* __restrict__ x64, int n,
+                                                      const __grid_constant__ LatticeParams lp, double sup)
 {
     const double inv_sup = 1.0 / sup;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -297,179 +275,348 @@ __global__ void __launch_bounds__(kBlock) k_lat_delta(const dbl4* __restrict__ x
             d[k] = (float)(dev[k] - m * sup);
             packed |= ((int)m + 512) << (10 * k);
         }
-        dl[i] = make_float4(d[0], d[1], d[2], __int_as_float(packed));
+        lp.grid_d[lp.dense[i]] = make_float4(d[0], d[1], d[2], __int_as_float(packed));
     }
 }
 
-// ---- the product -----------------------------------------------------------------------
-// Shared memory per halo site: A = (d.x, d.y, w.x, w.y), B = (d.z, w.z)
-// (24 bytes), d the site particle's deviation re-referenced to the brick:
-// d + sup (n - n_brick), n_brick the wrap counts of the brick's first slot
-// (within a brick's halo they differ by at most one for any strain a bond
-// survives, so |d| stays within 1.5 sup).  Entry k's bond vector is then
-// xi = h v_k + (d_q - d_p), formed in FP32 pairs with the differences of w.
-//
-// Blocks take bricks from a counter (lp.sched[0]) in brick order, so that
-// bricks of uneven fill balance over the blocks; the last block to finish
-// resets the counter for the next launch.  (An L2 prefetch of the next
-// brick's 1/d0 block, issued when the brick is taken, measured 3 % slower at
-// three blocks per SM; ordering the bricks by row count made no difference.)
-//
-// FIXED: the 80-entry stencil with its compile-time halo (lp.K == 80, halo
-// 36 x 8 x 8).  FUSE (a CG iteration): the direction is updated on the way
-// in, w = r + beta p_prev for every halo site (beta = 0 on the first
-// iteration, which cg_fin_residual sets), and each brick writes its rows' new
-// direction to p_out (p_prev and p_out are different buffers, so blocks that
-// still stage halos read the old direction).
+// The deviations of every brick's halo as the product copies them into shared
+// memory, once per step (every product of a solve reads them): re-referenced
+// to the brick, d + sup (n - n_brick) with n_brick the wrap counts of the
+// brick's first slot (within a brick's halo they differ by at most one for any
+// strain a bond survives, so |d| stays within 1.5 sup).  12 bytes per halo site
+// in two runs cost the product less than a box of grid_d (16 bytes per site in
+// shared memory and its reads): 134 against 143 us at 1M particles.
 __device__ __forceinline__ float wrap_delta(int nq, int nb, int shift, float sup)
 {
     return sup * small_int_to_float(((nq >> shift) & 1023) - ((nb >> shift) & 1023));
 }
 
-// Three blocks per SM (80 registers, a 55 KB halo each): at 1M particles 173 us
-// per product against 184 at two blocks (128 registers) and 178 at four (64).
-template <bool DOT, bool FIXED, bool FUSE>
-__global__ void __launch_bounds__(kBlock, 3) k_spmv_lattice(StepParams P, DeviceState S, LatticeParams lp,
-                                                           const float4* __restrict__ in, float4* __restrict__ out,
-                                                           ReduceSlot slot, CgScalars* cg, double* dot_out,
-                                                           const float4* __restrict__ r_in, float4* __restrict__ p_out)
+template <int R>
+__global__ void __launch_bounds__(kBlock) k_lat_image(const __grid_constant__ LatticeParams lp, float sup)
+{
+    constexpr int HX = lat_bx(R) + 2 * R, HY = kLatBY + 2 * R, HXY = HX * HY, H = lat_halo_sites(R);
+    const int mx = lp.map_dim[0], mxy = lp.map_dim[0] * lp.map_dim[1];
+    for (int b = blockIdx.x; b < lp.n_bricks; b += gridDim.x) {
+        const int corner = lp.brick_corner[b];
+        const int nb = __float_as_int(lp.grid_d[lp.dense[lp.brick_start[b]]].w);
+        float2* xy = (float2*)(lp.image + (size_t)b * 3 * H);
+        float* z = (float*)(xy + H);
+        for (int h = threadIdx.x; h < H; h += kBlock) {
+            const int iz = h / HXY;
+            const int r2 = h - iz * HXY;
+            const int iy = r2 / HX;
+            const float4 d = lp.grid_d[corner + iz * mxy + iy * mx + (r2 - iy * HX)];
+            const int nq = __float_as_int(d.w);
+            xy[h] = make_float2(d.x + wrap_delta(nq, nb, 0, sup), d.y + wrap_delta(nq, nb, 10, sup));
+            z[h] = d.z + wrap_delta(nq, nb, 20, sup);
+        }
+    }
+}
+
+// ---- the direction on the dense grid of sites --------------------------------------------
+// The product reads its vector from a dense grid of the map's extent (lp.grid_w,
+// zero where there is no particle), so that a brick's halo is one box.
+__global__ void __launch_bounds__(kBlock) k_lat_scatter(int n, const int* __restrict__ dense, float4* __restrict__ grid_w,
+                                                        const float4* __restrict__ in)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const float4 v = in[i];
+        grid_w[dense[i]] = make_float4(v.x, v.y, v.z, 0.f);
+    }
+}
+
+// p = r + beta p (xpby_elem), in slot order and on the grid
+__global__ void __launch_bounds__(kBlock) k_lat_xpby(int n, const int* __restrict__ dense, float4* __restrict__ grid_w,
+                                                     const CgScalars* sc, const float4* __restrict__ r,
+                                                     float4* __restrict__ p)
+{
+    if (((volatile const CgScalars*)sc)->done) return;
+    const float beta = (float)sc->beta;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const float4 ri = r[i], pi = p[i];
+        const float4 q = make_float4(ri.x + beta * pi.x, ri.y + beta * pi.y, ri.z + beta * pi.z, 0.f);
+        p[i] = q;
+        grid_w[dense[i]] = q;
+    }
+}
+
+// ---- the product -----------------------------------------------------------------------
+// Blocks take bricks from a counter (lp.sched[0]) in brick order, a warp per
+// chunk of 32 row pairs.  Everything the computation reads comes by bulk
+// copies: the halo of a brick (a box of the direction's grid, the deviations as
+// one run of the image) once the block is done with the brick before, and each warp's table in slabs, two ahead and across bricks, so that
+// some 70 KB per SM are in flight at any time -- at a DRAM latency of 1 us
+// (2.5 us under a full stream) loads into registers cannot hold that many: with
+// one stencil column (40 bytes a thread) loaded ahead the product took 150 us at
+// 1M particles however few instructions it had, 105 us without the table.
+// Entry k's bond vector is xi = d_q - (d_p - h v_k), formed in FP32 with the
+// differences of w.  Every wait is bounded (a second): on expiry the block
+// records the error in the handle's scalars, waits once more for its copies
+// and returns.
+
+constexpr unsigned long long kLatTimeoutNs = 1000000000ull;
+__device__ __forceinline__ unsigned long long lat_now_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+__device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(uint32_t bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity)
+{
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity)
+{
+    if (bar_try(bar, parity)) return true;
+    const unsigned long long t0 = lat_now_ns();
+    while (!bar_try(bar, parity))
+        if (lat_now_ns() - t0 > kLatTimeoutNs) return false;
+    return true;
+}
+
+// The rows of a thread: their sites' words and the sums of a1 (w_q - w_p) + g xi
+// with g = xi . (w_q - w_p) / d^3 (the row's term with the sign of w_q - w_p,
+// negated at the end).
+struct LatRows {
+    float2 d[kLatRZ], w[kLatRZ];   // (d.x, d.y), (w.x, w.y)
+    float dz[kLatRZ], wz[kLatRZ];
+    float2 sxy[kLatRZ];
+    float sz[kLatRZ];
+};
+struct LatHalo {
+    const float4* w;
+    const float2* xy;
+    const float* z;
+};
+
+// The stencil's column (dx, dy) of reach RC: entries dz = -RC .. RC of the
+// thread's rows, e[dz + RC] one word each.  Every site of the column is read
+// once and serves the rows it is a neighbour of.
+// q: shared-memory index of the site (dx, dy) from the thread's lowest row.
+template <int R, int RC>
+__device__ __forceinline__ void lat_column(const LatHalo& halo, int q, const float2 (&e)[2 * RC + 1], float2 cxy,
+                                           const float (&cz)[kLatTab], LatRows& row)
+{
+    constexpr int HXY = (lat_bx(R) + 2 * R) * (kLatBY + 2 * R);
+    const float2 m1 = make_float2(-1.f, -1.f);
+    float2 pxy[kLatRZ];
+#pragma unroll
+    for (int i = 0; i < kLatRZ; ++i) pxy[i] = __ffma2_rn(cxy, m1, row.d[i]);   // d_p - h v
+#pragma unroll
+    for (int j = -RC; j < kLatRZ + RC; ++j) {
+        const float4 qw4 = halo.w[q + j * HXY];
+        const float2 qd = halo.xy[q + j * HXY];
+        const float qz = halo.z[q + j * HXY];
+        const float2 qw = make_float2(qw4.x, qw4.y);
+#pragma unroll
+        for (int i = 0; i < kLatRZ; ++i) {
+            const int dz = j - i;
+            if (dz < -RC || dz > RC) continue;
+            const float s = i == 0 ? e[dz + RC].x : e[dz + RC].y;
+            const float2 xy = __ffma2_rn(pxy[i], m1, qd);      // d_q - (d_p - h v)
+            const float2 wxy = __ffma2_rn(row.w[i], m1, qw);   // w_q - w_p
+            const float zs = qz - (row.dz[i] - cz[dz + kLatRmax]);
+            const float wz = qw4.z - row.wz[i];
+            float inv_d = rsqrt_ftz(fmaf(xy.x, xy.x, fmaf(xy.y, xy.y, zs * zs)));
+            inv_d = fminf(inv_d, s);   // no live bond (s = 0): the term vanishes
+            const float a1 = fmaf(s, kLatUnscale, -inv_d);
+            const float g = fmaf(xy.x, wxy.x, fmaf(xy.y, wxy.y, zs * wz)) * (inv_d * inv_d * inv_d);
+            row.sxy[i] = __ffma2_rn(make_float2(a1, a1), wxy, __ffma2_rn(make_float2(g, g), xy, row.sxy[i]));
+            row.sz[i] = fmaf(a1, wz, fmaf(g, zs, row.sz[i]));
+        }
+    }
+}
+
+// bulk copy of `bytes` from global memory to shared memory, completing on `bar`,
+// with the table's lines first to leave L2
+__device__ __forceinline__ void copy_slab(uint32_t dst, const void* src, int bytes, uint32_t bar, uint64_t policy)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(dst),
+        "l"((uint64_t)src), "r"(bytes), "r"(bar), "l"(policy)
+        : "memory");
+}
+
+// One warp's stream of slabs: the chunk's, in the order of lp.slab_entry, then
+// those of the chunk it will take from the next brick.
+struct LatStream {
+    uint32_t ring, bars;    // the warp's two slabs and their barriers (shared-memory addresses)
+    uint64_t policy;
+    int issued = 0, used = 0;
+};
+__device__ __forceinline__ void lat_issue(LatStream& s, const LatticeParams& lp, int chunk, int slab)
+{
+    const int slot = s.issued & 1;
+    const int e0 = lp.slab_entry[slab], e1 = lp.slab_entry[slab + 1];
+    copy_slab(s.ring + slot * kLatSlabBytes, (const float2*)lp.ell + ((size_t)chunk * lp.K + e0) * 32, (e1 - e0) * 256,
+              s.bars + 8 * slot, s.policy);
+    ++s.issued;
+}
+
+// The stencil's columns of reach RC, the first one c, slab by slab; after a slab
+// the one two further on is asked for, of the next chunk at the end.
+template <int R, int RC>
+__device__ __forceinline__ bool lat_columns(const LatticeParams& lp, const LatHalo& halo, int base, const float2* ring,
+                                            LatStream& s, int chunk, int next, int& slab, int& c, int count,
+                                            const float (&cz)[kLatTab], LatRows& row)
+{
+    constexpr int N = 2 * RC + 1, M = lat_slab_columns(RC);
+    const int lane = threadIdx.x & 31;
+    for (; count > 0; count -= M) {
+        const int slot = s.used & 1;
+        if (!bar_wait(s.bars + 8 * slot, (s.used >> 1) & 1)) return false;
+        ++s.used;
+        const float2* e2 = ring + slot * (kLatSlabBytes / (int)sizeof(float2)) + lane;
+#pragma unroll 1
+        for (int m = 0; m < min(M, count); ++m, ++c, e2 += N * 32) {
+            float2 e[N];
+#pragma unroll
+            for (int k = 0; k < N; ++k) e[k] = e2[k * 32];
+            lat_column<R, RC>(halo, base + lp.coff[c], e, make_float2(lp.ccx[c], lp.ccy[c]), cz, row);
+        }
+        __syncwarp();   // every lane is done with the slab
+        const int ahead = ++slab + 1;
+        if (lane == 0) {
+            if (ahead < lp.slabs) lat_issue(s, lp, chunk, ahead);
+            else if (next >= 0) lat_issue(s, lp, next, ahead - lp.slabs);
+        }
+    }
+    return true;
+}
+
+template <int R, bool DOT>
+__global__ void __launch_bounds__(32 * lat_warps(R), 2)
+    k_spmv_lattice(StepParams P, DeviceState S, const __grid_constant__ LatticeParams lp, float4* __restrict__ out,
+                   ReduceSlot slot, CgScalars* cg, double* dot_out)
 {
     if (DOT && cg && ((volatile CgScalars*)cg)->done) return;
-    extern __shared__ float4 lat_smem[];
-    __shared__ int s_next;
-    const int H = FIXED ? kS80Hx * kS80Hy * kS80Hz : lp.hx * lp.hy * lp.hz;
-    float4* sA = lat_smem;
-    float2* sB = (float2*)(sA + H);
-    const float sup = (float)P.sup;
-    const int hx = FIXED ? kS80Hx : lp.hx, hxy = FIXED ? kS80Hx * kS80Hy : lp.hx * lp.hy;
-    const int mx = lp.map_dim[0], mxy = lp.map_dim[0] * lp.map_dim[1];
-    const int K = FIXED ? kS80 : lp.K;
-    const float beta = FUSE ? (float)((volatile CgScalars*)cg)->beta : 0.f;
-    const float2 m1 = make_float2(-1.f, -1.f);
-    DotAcc32 acc;
+    constexpr int HX = lat_bx(R) + 2 * R, HY = kLatBY + 2 * R, HXY = HX * HY, H = lat_halo_sites(R);
+    extern __shared__ __align__(128) unsigned char lat_smem_raw[];
+    __shared__ int s_ahead;
+    const uint32_t bars = (uint32_t)__cvta_generic_to_shared(lat_smem_raw);   // the halo's, then two per warp
+    const unsigned char* stage = lat_smem_raw + kLatBarrierBytes;
+    const LatHalo halo{(const float4*)stage, (const float2*)(stage + 16 * H), (const float*)(stage + 24 * H)};
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned char* ring = stage + lat_halo_bytes(R) + warp * 2 * kLatSlabBytes;
+    LatStream s;
+    s.ring = (uint32_t)__cvta_generic_to_shared(ring);
+    s.bars = bars + 8 + 16 * warp;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(s.policy));
+    const auto load_halo = [&](int b) {   // thread 0
+        const int corner = lp.brick_corner[b];
+        const int mx = lp.map_dim[0], my = lp.map_dim[1];
+        const int cx = corner % mx, cy = corner / mx % my, cz = corner / mx / my;
+        const uint32_t dst = bars + kLatBarrierBytes;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bars), "r"(28 * H) : "memory");
+        asm volatile(
+            "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+            "[%6];" ::"r"(dst),
+            "l"((uint64_t)&lp.box_w), "r"(0), "r"(cx), "r"(cy), "r"(cz), "r"(bars)
+            : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst + 16 * H),
+                     "l"((uint64_t)(lp.image + (size_t)b * 3 * H)), "r"(lat_image_bytes(R)), "r"(bars)
+                     : "memory");
+    };
+    // this warp's chunk of a brick, or -1
+    const auto chunk_of = [&](int b) {
+        if (b >= lp.n_bricks) return -1;
+        const int c = __ldg(lp.chunk_start + b) + warp;
+        return c < __ldg(lp.chunk_start + b + 1) ? c : -1;
+    };
+    int b = 0;
     if (threadIdx.x == 0) {
-        s_next = (int)atomicAdd(&lp.sched[0], 1u);
+        for (int k = 0; k < 1 + 2 * lat_warps(R); ++k) bar_init(bars + 8 * k, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        b = (int)atomicAdd(&lp.sched[0], 1u);
+        s_ahead = b;
     }
     __syncthreads();
-    int b = s_next;
-    while (b < lp.n_bricks) {
-        const int corner = lp.brick_corner[b];
-        const int start = lp.brick_start[b];
-        const int rows = lp.brick_start[b + 1] - start;
-        const int nb = __float_as_int(__ldg(&lp.dl[start].w));
-        // the map entries of this thread's halo sites first (independent
-        // loads), then their deviations and w entries
-        int qs[kLatHaloPerThread];
-#pragma unroll
-        for (int t = 0; t < kLatHaloPerThread; ++t) {
-            const int h = threadIdx.x + t * kBlock;
-            qs[t] = -1;
-            if (h < H) {
-                const int iz = h / hxy;
-                const int r2 = h - iz * hxy;
-                const int iy = r2 / hx;
-                const int ix = r2 - iy * hx;
-                qs[t] = __ldg(lp.map + corner + iz * mxy + iy * mx + ix);
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < kLatHaloPerThread; ++t) {
-            const int h = threadIdx.x + t * kBlock;
-            if (h >= H) continue;
-            const int q = qs[t];
-            float4 a = make_float4(kLatEmpty, kLatEmpty, 0.f, 0.f);
-            float2 bb = make_float2(kLatEmpty, 0.f);
-            if (q >= 0) {
-                const float4 dq = __ldg(lp.dl + q);
-                float4 w = __ldg(in + q);
-                if (FUSE) {   // xpby_elem: p = r + beta p
-                    const float4 r = __ldg(r_in + q);
-                    w.x = r.x + beta * w.x;
-                    w.y = r.y + beta * w.y;
-                    w.z = r.z + beta * w.z;
-                }
-                const int nq = __float_as_int(dq.w);
-                a = make_float4(dq.x + wrap_delta(nq, nb, 0, sup), dq.y + wrap_delta(nq, nb, 10, sup), w.x, w.y);
-                bb = make_float2(dq.z + wrap_delta(nq, nb, 20, sup), w.z);
-            }
-            sA[h] = a;
-            sB[h] = bb;
-        }
-        __syncthreads();   // halo staged; every thread has read s_next
-        if (threadIdx.x == 0) {
-            s_next = (int)atomicAdd(&lp.sched[0], 1u);
-        }
-        for (int l = threadIdx.x; l < rows; l += blockDim.x) {
-            const int p = start + l;
-            const uint8_t ab = S.act[p];
-            const int c = lp.row_local[p];
-            const float4 pa = sA[c];
-            const float2 pb = sB[c];
-            const float4 w = make_float4(pa.z, pa.w, pb.y, 0.f);
-            if (FUSE) p_out[p] = w;
-            if (is_dirichlet(ab & kActMask)) {
-                out[p] = make_float4(0.f, 0.f, 0.f, 0.f);
-                continue;
-            }
-            const float2 pd = make_float2(pa.x, pa.y), pw = make_float2(pa.z, pa.w);
-            // this row's 1/d0 stream: 16 bytes (4 stencil entries) per load
-            const float4* __restrict__ e4 = (const float4*)(lp.ell + (size_t)K * start) + l;
-            // sums of a1 (w_q - w_p) + g xi with g = xi . (w_q - w_p) / d^3: the
-            // row's term with the sign of w_q - w_p, negated at the end
-            float2 sxy = make_float2(0.f, 0.f);
-            float sz = 0.f;
-            constexpr Stencil80 s80 = make_stencil80();
-            const auto bond = [&](int k, float s) {
-                const int q = c + (FIXED ? s80.off[k] : lp.off[k]);
-                const float4 qa = sA[q];
-                const float2 qb = sB[q];
-                float2 xy = __ffma2_rn(pd, m1, make_float2(qa.x, qa.y));    // d_q - d_p
-                const float2 wxy = __ffma2_rn(pw, m1, make_float2(qa.z, qa.w));   // w_q - w_p
-                const float2 zz = __ffma2_rn(pb, m1, qb);                        // (d_q - d_p, w_q - w_p).z
-                float zs = zz.x;
-                if (FIXED) {   // h v_k: compile-time zeros drop out
-                    if (s80.dx[k] != 0) xy.x += lp.cx[k];
-                    if (s80.dy[k] != 0) xy.y += lp.cy[k];
-                    if (s80.dz[k] != 0) zs += lp.cz[k];
-                } else {
-                    xy.x += lp.cx[k];
-                    xy.y += lp.cy[k];
-                    zs += lp.cz[k];
-                }
-                const float2 sq = __fmul2_rn(xy, xy);
-                float inv_d = rsqrt_ftz(fmaf(zs, zs, sq.x + sq.y));
-                inv_d = fminf(inv_d, s);   // no live bond (s = 0): the term vanishes
-                const float a1 = fmaf(s, kLatUnscale, -inv_d);
-                const float2 t = __fmul2_rn(xy, wxy);
-                const float g = fmaf(zs, zz.y, t.x + t.y) * (inv_d * inv_d * inv_d);
-                sxy = __ffma2_rn(make_float2(a1, a1), wxy, __ffma2_rn(make_float2(g, g), xy, sxy));
-                sz = fmaf(a1, zz.y, fmaf(g, zs, sz));
-            };
-            // (loading each table chunk one chunk ahead measured slower: 181 against 173 us)
-            if constexpr (FIXED) {
-#pragma unroll
-                for (int k4 = 0; k4 < kS80 / 4; ++k4) {
-                    const float4 s4 = __ldcs(e4 + (size_t)k4 * rows);
-                    bond(4 * k4, s4.x);
-                    bond(4 * k4 + 1, s4.y);
-                    bond(4 * k4 + 2, s4.z);
-                    bond(4 * k4 + 3, s4.w);
-                }
-            } else {
-#pragma unroll 10   // 160 us at 1M against 163 (5), 168 (4), 171 (2) and 174 (20)
-                for (int k4 = 0; k4 < K / 4; ++k4) {
-                    const float4 s4 = __ldcs(e4 + (size_t)k4 * rows);
-                    bond(4 * k4, s4.x);
-                    bond(4 * k4 + 1, s4.y);
-                    bond(4 * k4 + 2, s4.z);
-                    bond(4 * k4 + 3, s4.w);
-                }
-            }
-            spmv_finish_mixed<1, DOT>(P, S, p, ab, w, -sxy.x, -sxy.y, -sz, 0, 0xffffffffu, out, acc);
-        }
-        __syncthreads();   // the rows are done with the halo; s_next is visible
-        b = s_next;
+    b = s_ahead;
+    __syncthreads();
+    if (threadIdx.x == 0 && b < lp.n_bricks) {
+        s_ahead = (int)atomicAdd(&lp.sched[0], 1u);
+        load_halo(b);
     }
+    int chunk = chunk_of(b);
+    if (lane == 0 && chunk >= 0)
+        for (int k = 0; k < min(2, lp.slabs); ++k) lat_issue(s, lp, chunk, k);
+    DotAcc32 acc;
+    bool ok = true;
+    const float c0 = (float)P.bond_coeff, t2 = (float)P.t2, m = (float)P.mass;
+    float cz[kLatTab];
+#pragma unroll
+    for (int k = 0; k < kLatTab; ++k) cz[k] = lp.cz[k];
+    for (int it = 0; b < lp.n_bricks; ++it) {
+        ok = bar_wait(bars, it & 1);
+        const int ahead = *(volatile int*)&s_ahead;   // the next brick
+        const int next = chunk_of(ahead);
+        if (ok && chunk >= 0) {
+            const int base = __ldg(lp.pair_base + chunk * 32 + lane);   // halo index of the lower site
+            const int2 slots = __ldg((const int2*)lp.pair_slot + chunk * 32 + lane);
+            LatRows row;
+#pragma unroll
+            for (int i = 0; i < kLatRZ; ++i) {
+                const float4 w = halo.w[base + i * HXY];
+                row.d[i] = halo.xy[base + i * HXY];
+                row.dz[i] = halo.z[base + i * HXY];
+                row.w[i] = make_float2(w.x, w.y);
+                row.wz[i] = w.z;
+                row.sxy[i] = make_float2(0.f, 0.f);
+                row.sz[i] = 0.f;
+            }
+            const float2* ring2 = (const float2*)ring;
+            int c = 0, slab = 0;
+            if constexpr (R >= 3) ok = ok && lat_columns<R, 3>(lp, halo, base, ring2, s, chunk, next, slab, c, lp.ncol[3], cz, row);
+            if constexpr (R >= 2) ok = ok && lat_columns<R, 2>(lp, halo, base, ring2, s, chunk, next, slab, c, lp.ncol[2], cz, row);
+            ok = ok && lat_columns<R, 1>(lp, halo, base, ring2, s, chunk, next, slab, c, lp.ncol[1], cz, row);
+            ok = ok && lat_columns<R, 0>(lp, halo, base, ring2, s, chunk, next, slab, c, lp.ncol[0], cz, row);
+#pragma unroll
+            for (int i = 0; i < kLatRZ; ++i) {
+                const int p = i == 0 ? slots.x : slots.y;
+                if (p < 0) continue;
+                const uint8_t ab = S.act[p];
+                if (is_dirichlet(ab & kActMask))
+                    out[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+                else
+                    mixed_row_result<DOT>(P, S, p, ab, c0, t2, m, make_float4(row.w[i].x, row.w[i].y, row.wz[i], 0.f),
+                                          -row.sxy[i].x, -row.sxy[i].y, -row.sz[i], out, acc);
+            }
+        } else if (lane == 0 && next >= 0) {
+            for (int k = 0; k < min(2, lp.slabs); ++k) lat_issue(s, lp, next, k);
+        }
+        if (__syncthreads_or(ok ? 0 : 1)) {   // the block is done with the halo, or gave up
+            ok = false;
+            break;
+        }
+        b = ahead;
+        chunk = next;
+        if (threadIdx.x == 0 && b < lp.n_bricks) {
+            s_ahead = (int)atomicAdd(&lp.sched[0], 1u);
+            load_halo(b);
+        }
+    }
+    if (!ok) {   // record it, and wait once more for the copies in flight
+        ((volatile CgScalars*)S.sc)->wait_error = 1;
+        if (lane == 0)
+            for (; s.used < s.issued; ++s.used) bar_wait(s.bars + 8 * (s.used & 1), (s.used >> 1) & 1);
+    }
+    __syncthreads();
     // every block has taken its last brick index: the last to arrive resets the counter
     if (threadIdx.x == 0) {
         __threadfence();
@@ -490,26 +637,37 @@ __global__ void __launch_bounds__(kBlock, 3) k_spmv_lattice(StepParams P, Device
 
 size_t lattice_smem_bytes(const LatticeParams& lp)
 {
-    return (size_t)lp.hx * lp.hy * lp.hz * kLatSiteBytes;
+    return (size_t)lat_smem(lp.R);
 }
 
 void launch_lattice_delta(const DeviceState& S, const LatticeParams& lp, double sup, cudaStream_t st)
 {
-    if (S.n > 0 && lp.dl) k_lat_delta<<<blocks_for(S.n), kBlock, 0, st>>>(S.x64, S.n, lp, sup, lp.dl);
+    if (S.n <= 0 || !lp.grid_d) return;
+    k_lat_delta<<<blocks_for(S.n), kBlock, 0, st>>>(S.x64, S.n, lp, sup);
+    const int grid = std::min(lp.n_bricks, 8192);
+    if (lp.R == 1) k_lat_image<1><<<grid, kBlock, 0, st>>>(lp, (float)sup);
+    else if (lp.R == 2) k_lat_image<2><<<grid, kBlock, 0, st>>>(lp, (float)sup);
+    else k_lat_image<3><<<grid, kBlock, 0, st>>>(lp, (float)sup);
 }
 
-template <bool FIXED>
+void launch_lattice_scatter(const DeviceState& S, const LatticeParams& lp, const void* in, cudaStream_t st)
+{
+    k_lat_scatter<<<blocks_for(S.n), kBlock, 0, st>>>(S.n, lp.dense, lp.grid_w, (const float4*)in);
+}
+
+void launch_lattice_xpby(const DeviceState& S, const LatticeParams& lp, const void* r, int grid, cudaStream_t st)
+{
+    k_lat_xpby<<<grid, kBlock, 0, st>>>(S.n, lp.dense, lp.grid_w, S.sc, (const float4*)r, (float4*)S.p);
+}
+
+template <int R>
 int lattice_blocks(size_t smem)
 {
-    const void* ks[3] = {(const void*)k_spmv_lattice<false, FIXED, false>, (const void*)k_spmv_lattice<true, FIXED, false>,
-                         (const void*)k_spmv_lattice<true, FIXED, true>};
     int m = 1 << 30;
-    for (const void* k : ks) {
-        // the attribute is per kernel and process: set to the largest halo any
-        // handle can need, so that every handle's launch fits
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kLatSmemMax);
+    for (const void* k : {(const void*)k_spmv_lattice<R, false>, (const void*)k_spmv_lattice<R, true>}) {
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int a = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k, kBlock, smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k, 32 * lat_warps(R), smem);
         m = std::min(m, a);
     }
     return m > 0 ? m : 1;
@@ -517,39 +675,51 @@ int lattice_blocks(size_t smem)
 
 int lattice_spmv_blocks_per_sm(const LatticeParams& lp)
 {
-    // both variants get the shared-memory attribute: the autotuner may run
-    // the general kernel on a stencil the compile-time one also covers
     const size_t smem = lattice_smem_bytes(lp);
-    const int general = lattice_blocks<false>(smem);
-    return lp.fixed ? std::min(general, lattice_blocks<true>(smem)) : general;
+    return lp.R == 1 ? lattice_blocks<1>(smem) : lp.R == 2 ? lattice_blocks<2>(smem) : lattice_blocks<3>(smem);
 }
 
-template <bool FIXED>
-void launch_lattice_t(bool dot, const StepParams& P, const DeviceState& S, const LatticeParams& lp, const void* in,
-                      void* out, ReduceSlot slot, CgScalars* cg, double* dot_out, const void* r_in, void* p_out,
-                      int grid, size_t smem, cudaStream_t st)
+template <int R>
+void launch_lattice_t(bool dot, const StepParams& P, const DeviceState& S, const LatticeParams& lp, void* out,
+                      ReduceSlot slot, CgScalars* cg, double* dot_out, int grid, size_t smem, cudaStream_t st)
 {
-    const float4* x = (const float4*)in;
     float4* y = (float4*)out;
-    if (r_in)
-        k_spmv_lattice<true, FIXED, true><<<grid, kBlock, smem, st>>>(P, S, lp, x, y, slot, cg, dot_out,
-                                                                      (const float4*)r_in, (float4*)p_out);
-    else if (dot)
-        k_spmv_lattice<true, FIXED, false><<<grid, kBlock, smem, st>>>(P, S, lp, x, y, slot, cg, dot_out, nullptr,
-                                                                       nullptr);
-    else
-        k_spmv_lattice<false, FIXED, false><<<grid, kBlock, smem, st>>>(P, S, lp, x, y, slot, nullptr, nullptr,
-                                                                        nullptr, nullptr);
+    const int threads = 32 * lat_warps(R);
+    if (dot) k_spmv_lattice<R, true><<<grid, threads, smem, st>>>(P, S, lp, y, slot, cg, dot_out);
+    else k_spmv_lattice<R, false><<<grid, threads, smem, st>>>(P, S, lp, y, slot, nullptr, nullptr);
 }
 
-void launch_spmv_lattice(bool dot, const StepParams& P, const DeviceState& S, const LatticeParams& lp,
-                         const void* in, void* out, ReduceSlot slot, CgScalars* cg, double* dot_out,
-                         const void* r_in, void* p_out, cudaStream_t st)
+void launch_spmv_lattice(bool dot, const StepParams& P, const DeviceState& S, const LatticeParams& lp, void* out,
+                         ReduceSlot slot, CgScalars* cg, double* dot_out, cudaStream_t st)
 {
     const size_t smem = lattice_smem_bytes(lp);
     const int grid = std::max(1, std::min(lp.grid, std::max(lp.n_bricks, 1)));
-    if (lp.fixed) launch_lattice_t<true>(dot, P, S, lp, in, out, slot, cg, dot_out, r_in, p_out, grid, smem, st);
-    else launch_lattice_t<false>(dot, P, S, lp, in, out, slot, cg, dot_out, r_in, p_out, grid, smem, st);
+    if (lp.R == 1) launch_lattice_t<1>(dot, P, S, lp, out, slot, cg, dot_out, grid, smem, st);
+    else if (lp.R == 2) launch_lattice_t<2>(dot, P, S, lp, out, slot, cg, dot_out, grid, smem, st);
+    else launch_lattice_t<3>(dot, P, S, lp, out, slot, cg, dot_out, grid, smem, st);
+}
+
+// the direction's grid as a TMA tensor of 4 floats per site, in boxes of a brick's halo
+static cudaError_t grid_box(LatticeParams* lp)
+{
+    using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    const cudaError_t e = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q);
+    if (e != cudaSuccess) return e;
+    if (q != cudaDriverEntryPointSuccess || !fn) return cudaErrorNotSupported;
+    const int R = lp->R;
+    const cuuint64_t dims[4] = {4, (cuuint64_t)lp->map_dim[0], (cuuint64_t)lp->map_dim[1], (cuuint64_t)lp->map_dim[2]};
+    const cuuint64_t strides[3] = {16, 16 * dims[1], 16 * dims[1] * dims[2]};
+    const cuuint32_t box[4] = {4, (cuuint32_t)(lat_bx(R) + 2 * R), (cuuint32_t)(kLatBY + 2 * R),
+                               (cuuint32_t)(kLatBZ + 2 * R)};
+    const cuuint32_t one[4] = {1, 1, 1, 1};
+    const CUresult r = ((EncodeFn)fn)(&lp->box_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, lp->grid_w, dims, strides, box, one,
+                                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
 void launch_lattice_ell(const DeviceState& S, const LatticeParams& lp, int force, int grid, cudaStream_t st)
@@ -561,13 +731,17 @@ void lattice_free(LatticeBuffers* lb)
 {
     cudaFree(lb->brick_start);
     cudaFree(lb->brick_corner);
-    cudaFree(lb->row_local);
-    cudaFree(lb->row_brick);
+    cudaFree(lb->chunk_start);
+    cudaFree(lb->pair_base);
+    cudaFree(lb->pair_slot);
+    cudaFree(lb->row_pair);
     cudaFree(lb->site);
-    cudaFree(lb->map);
     cudaFree(lb->offk);
     cudaFree(lb->ell);
-    cudaFree(lb->dl);
+    cudaFree(lb->dense);
+    cudaFree(lb->grid_w);
+    cudaFree(lb->grid_d);
+    cudaFree(lb->image);
     cudaFree(lb->sched);
     *lb = LatticeBuffers{};
 }
@@ -620,46 +794,47 @@ cudaError_t lattice_build(int n, double spacing, dbl4* x64, float4* X32, int* pe
     LT_TRY(cudaMemcpyAsync(ext, t.ext, sizeof(ext), cudaMemcpyDeviceToHost, st));
     LT_TRY(cudaStreamSynchronize(st));
     if (ext[7]) return cudaSuccess;   // a bond longer than the stencil reach
-    // the stencil: offsets in (dz, dy, dx) order
+    // the stencil: the bonds' offsets as z columns (dx, dy), a column of reach
+    // r covering dz = -r .. r (entries without a bond, the row itself among
+    // them, hold 0), columns of the largest reach first
     LatticeParams L{};
-    int R = 1;
+    int R = 1, offsets = 0;
+    int reach[kLatTab * kLatTab];
+    for (int dy = -kLatRmax; dy <= kLatRmax; ++dy)
+        for (int dx = -kLatRmax; dx <= kLatRmax; ++dx) {
+            int& r = reach[(dy + kLatRmax) * kLatTab + dx + kLatRmax];
+            r = -1;
+            for (int dz = -kLatRmax; dz <= kLatRmax; ++dz)
+                if (tab[((dz + kLatRmax) * kLatTab + (dy + kLatRmax)) * kLatTab + (dx + kLatRmax)]) {
+                    r = std::max(r, std::abs(dz));
+                    R = std::max(R, std::max(std::abs(dx), std::max(std::abs(dy), std::abs(dz))));
+                    ++offsets;
+                }
+        }
+    if (offsets > kLatMaxOffsets) return cudaSuccess;
+    L.R = R;
+    const int BX = lat_bx(R), HX = BX + 2 * R, HY = kLatBY + 2 * R;
     std::vector<int> offk(tab.size(), -1);
-    std::vector<int3> sten;
-    // every offset inside the 80-entry stencil: take that stencil whole (absent
-    // offsets get 1/d0 = 0) so that the specialised product applies
-    bool in80 = true;
-    for (int dz = -kLatRmax; dz <= kLatRmax; ++dz)
-        for (int dy = -kLatRmax; dy <= kLatRmax; ++dy)
-            for (int dx = -kLatRmax; dx <= kLatRmax; ++dx)
-                if (tab[((dz + kLatRmax) * kLatTab + (dy + kLatRmax)) * kLatTab + (dx + kLatRmax)] && !in_s80(dx, dy, dz))
-                    in80 = false;
-    for (int dz = -kLatRmax; dz <= kLatRmax; ++dz)
+    int cols = 0;
+    for (int r = kLatRmax; r >= 0; --r)
         for (int dy = -kLatRmax; dy <= kLatRmax; ++dy)
             for (int dx = -kLatRmax; dx <= kLatRmax; ++dx) {
-                const int i = ((dz + kLatRmax) * kLatTab + (dy + kLatRmax)) * kLatTab + (dx + kLatRmax);
-                if (in80 ? !in_s80(dx, dy, dz) : !tab[i]) continue;
-                if ((int)sten.size() >= kLatMaxK) return cudaSuccess;   // (kLatMaxK is a multiple of 4)
-                offk[i] = (int)sten.size();
-                sten.push_back(make_int3(dx, dy, dz));
-                R = std::max(R, std::max(std::abs(dx), std::max(std::abs(dy), std::abs(dz))));
+                if (reach[(dy + kLatRmax) * kLatTab + dx + kLatRmax] != r) continue;
+                for (int dz = -r; dz <= r; ++dz)
+                    offk[((dz + kLatRmax) * kLatTab + (dy + kLatRmax)) * kLatTab + (dx + kLatRmax)] = L.K++;
+                L.coff[cols] = dy * HX + dx;
+                L.ccx[cols] = (float)(spacing * dx);
+                L.ccy[cols] = (float)(spacing * dy);
+                ++cols;
+                ++L.ncol[r];
             }
-    L.K = ((int)sten.size() + 3) / 4 * 4;   // padding entries: offset 0 (the row's own site), 1/d0 = 0
-    if (in80) R = 2;
-    L.R = R;
-    L.fixed = in80 ? 1 : 0;
-    L.bx = kLatBX;
-    L.by = kLatBY;
-    L.bz = R <= 2 ? 4 : 2;
-    L.hx = L.bx + 2 * R;
-    L.hy = L.by + 2 * R;
-    L.hz = L.bz + 2 * R;
-    for (int k = 0; k < L.K; ++k) {
-        const int3 v = k < (int)sten.size() ? sten[k] : make_int3(0, 0, 0);
-        L.off[k] = (v.z * L.hy + v.y) * L.hx + v.x;
-        L.cx[k] = (float)(spacing * v.x);
-        L.cy[k] = (float)(spacing * v.y);
-        L.cz[k] = (float)(spacing * v.z);
-    }
+    for (int k = 0; k < kLatTab; ++k) L.cz[k] = (float)(spacing * (k - kLatRmax));
+    for (int r = kLatRmax, k = 0; r >= 0; --r)
+        for (int left = L.ncol[r]; left > 0; left -= lat_slab_columns(r)) {
+            k += (2 * r + 1) * std::min(left, lat_slab_columns(r));
+            L.slab_entry[++L.slabs] = k;
+        }
+    if (L.slabs < 2) return cudaSuccess;   // (bonds along one axis only)
     // site s (from the minimum site) lies at anchor + h (s + min)
     L.h = spacing;
     L.org[0] = anchor.x + spacing * ext[0];
@@ -667,23 +842,23 @@ cudaError_t lattice_build(int n, double spacing, dbl4* x64, float4* X32, int* pe
     L.org[2] = anchor.z + spacing * ext[2];
     const long long D[3] = {(long long)ext[3] - ext[0] + 1, (long long)ext[4] - ext[1] + 1,
                             (long long)ext[5] - ext[2] + 1};
-    const long long NB[3] = {(D[0] + L.bx - 1) / L.bx, (D[1] + L.by - 1) / L.by, (D[2] + L.bz - 1) / L.bz};
-    const long long M[3] = {NB[0] * L.bx + 2 * R, NB[1] * L.by + 2 * R, NB[2] * L.bz + 2 * R};
+    const long long NB[3] = {(D[0] + BX - 1) / BX, (D[1] + kLatBY - 1) / kLatBY, (D[2] + kLatBZ - 1) / kLatBZ};
+    const long long M[3] = {NB[0] * BX + 2 * R, NB[1] * kLatBY + 2 * R, NB[2] * kLatBZ + 2 * R};
     const long long map_size = M[0] * M[1] * M[2];
     const long long bricks_total = NB[0] * NB[1] * NB[2];
     // a dense site map of modest size (the body fills a good part of its box)
     if (map_size > std::max<long long>(16LL * n, 1LL << 22) || map_size >= (1LL << 31) ||
-        bricks_total * L.bx * L.by * L.bz >= (1LL << 32))
+        bricks_total * BX * kLatBY * kLatBZ >= (1LL << 32))
         return cudaSuccess;
     for (int k = 0; k < 3; ++k) L.map_dim[k] = (int)M[k];
     // brick-major keys, sorted; two particles on one site: not a lattice fill
     LT_TRY(cudaMalloc(&t.key, sizeof(unsigned) * (size_t)n));
     LT_TRY(cudaMalloc(&t.n2o, sizeof(int) * (size_t)n));
-    k_lat_keys<<<G, kBlock, 0, st>>>(n, t.lb.site, make_int3(ext[0], ext[1], ext[2]), L.bz,
+    k_lat_keys<<<G, kBlock, 0, st>>>(n, t.lb.site, make_int3(ext[0], ext[1], ext[2]), BX,
                                      make_int3((int)NB[0], (int)NB[1], (int)NB[2]), t.key, t.n2o);
     LT_TRY(cudaGetLastError());
     int key_bits = 0;
-    while (key_bits < 32 && (1ULL << key_bits) < (unsigned long long)(bricks_total * L.bx * L.by * L.bz)) ++key_bits;
+    while (key_bits < 32 && (1ULL << key_bits) < (unsigned long long)(bricks_total * BX * kLatBY * kLatBZ)) ++key_bits;
     key_bits = (key_bits + 7) / 8 * 8;
     LT_TRY(sort_pairs_u32(t.key, t.n2o, n, std::max(key_bits, 8), st));
     LT_TRY(cudaMemsetAsync(t.ext + 7, 0, sizeof(int), st));
@@ -693,6 +868,44 @@ cudaError_t lattice_build(int n, double spacing, dbl4* x64, float4* X32, int* pe
     LT_TRY(cudaMemcpyAsync(keys.data(), t.key, sizeof(unsigned) * (size_t)n, cudaMemcpyDeviceToHost, st));
     LT_TRY(cudaStreamSynchronize(st));
     if (ext[7]) return cudaSuccess;
+    // bricks, their pairs of z-adjacent rows (rows of a brick come z, then y,
+    // then x) and the chunks of 32 pairs: a body so thin along z that most pairs
+    // lack a row, or so scattered that most bricks hold a few rows, keeps the
+    // gather product
+    const unsigned bxy = (unsigned)(BX * kLatBY), bsz = bxy * kLatBZ;
+    std::vector<int> bstart, bcorner, chunk_start(1, 0), pair_base, pair_slot, row_pair(n);
+    for (int i = 0; i < n;) {
+        const unsigned brick = keys[i] / bsz;
+        const auto pair_of = [&](unsigned local) { return (int)(local / bxy / kLatRZ * bxy + local % bxy); };
+        int e = i;
+        unsigned char seen[kLatMaxPairs] = {};
+        for (; e < n && keys[e] / bsz == brick; ++e) seen[pair_of(keys[e] % bsz)] = 1;
+        int index[kLatMaxPairs];
+        for (int t = 0; t < kLatMaxPairs; ++t)
+            if (seen[t]) {
+                const int xy = t % (int)bxy, z = t / (int)bxy * kLatRZ;
+                index[t] = (int)pair_base.size();
+                pair_base.push_back(((z + R) * HY + (xy / BX + R)) * HX + (xy % BX + R));
+                pair_slot.insert(pair_slot.end(), kLatRZ, -1);
+            }
+        while (pair_base.size() % 32) {   // spare lanes repeat a pair and write nothing
+            pair_base.push_back(pair_base.back());
+            pair_slot.insert(pair_slot.end(), kLatRZ, -1);
+        }
+        for (int k = i; k < e; ++k) {
+            const unsigned local = keys[k] % bsz;
+            row_pair[(size_t)k] = kLatRZ * index[pair_of(local)] + (int)(local / bxy % kLatRZ);
+            pair_slot[(size_t)row_pair[(size_t)k]] = k;
+        }
+        bstart.push_back(i);
+        const long long bxi = brick % NB[0], byi = (brick / NB[0]) % NB[1], bzi = brick / (NB[0] * NB[1]);
+        bcorner.push_back((int)(((bzi * kLatBZ) * M[1] + byi * kLatBY) * M[0] + bxi * BX));
+        chunk_start.push_back((int)(pair_base.size() / 32));
+        i = e;
+    }
+    L.n_bricks = (int)bstart.size();
+    const size_t n_pairs = pair_base.size();
+    if (n_pairs * kLatRZ > std::max<size_t>((size_t)n * 5 / 2, 8192) || n_pairs >= (1u << 30)) return cudaSuccess;
     // ---- from here on the particles are renumbered: no more early returns ----
     LT_TRY(cudaMalloc(&t.o2n, sizeof(int) * (size_t)n));
     LT_TRY(cudaMalloc(&t.len, sizeof(unsigned) * ((size_t)n + 1)));
@@ -717,52 +930,48 @@ cudaError_t lattice_build(int n, double spacing, dbl4* x64, float4* X32, int* pe
     LT_TRY(cudaMemcpyAsync(row_ptr, t.len, sizeof(int) * ((size_t)n + 1), cudaMemcpyDeviceToDevice, st));
     LT_TRY(cudaGetLastError());
     std::swap(*col, t.col_new);   // the old column array is freed with the temporaries
-    // bricks, each row's halo index, the site map and the stencil lookup
-    const unsigned bsz = (unsigned)(L.bx * L.by * L.bz);
-    std::vector<int> bstart, bcorner, rlocal(n), rbrick(n);
-    for (int i = 0; i < n; ++i) {
-        const unsigned brick = keys[i] / bsz, local = keys[i] % bsz;
-        if (i == 0 || brick != keys[i - 1] / bsz) {
-            bstart.push_back(i);
-            const long long bxi = brick % NB[0], byi = (brick / NB[0]) % NB[1], bzi = brick / (NB[0] * NB[1]);
-            bcorner.push_back((int)(((bzi * L.bz) * M[1] + byi * L.by) * M[0] + bxi * L.bx));
-        }
-        const int lx = (int)(local % L.bx), ly = (int)((local / L.bx) % L.by), lz = (int)(local / (L.bx * L.by));
-        rlocal[i] = ((lz + R) * L.hy + (ly + R)) * L.hx + (lx + R);
-        rbrick[i] = (int)bstart.size() - 1;
-    }
-    L.n_bricks = (int)bstart.size();
-    bstart.push_back(n);
     LT_TRY(cudaMalloc(&t.lb.brick_start, sizeof(int) * bstart.size()));
     LT_TRY(cudaMalloc(&t.lb.brick_corner, sizeof(int) * bcorner.size()));
-    LT_TRY(cudaMalloc(&t.lb.row_local, sizeof(int) * (size_t)n));
-    LT_TRY(cudaMalloc(&t.lb.row_brick, sizeof(int) * (size_t)n));
-    LT_TRY(cudaMalloc(&t.lb.map, sizeof(int) * (size_t)map_size));
+    LT_TRY(cudaMalloc(&t.lb.chunk_start, sizeof(int) * chunk_start.size()));
+    LT_TRY(cudaMalloc(&t.lb.pair_base, sizeof(int) * n_pairs));
+    LT_TRY(cudaMalloc(&t.lb.pair_slot, sizeof(int) * pair_slot.size()));
+    LT_TRY(cudaMalloc(&t.lb.row_pair, sizeof(int) * (size_t)n));
     LT_TRY(cudaMalloc(&t.lb.offk, sizeof(int) * offk.size()));
-    LT_TRY(cudaMalloc(&t.lb.ell, sizeof(float) * (size_t)L.K * (size_t)n));
-    LT_TRY(cudaMalloc(&t.lb.dl, sizeof(float4) * (size_t)n));
-    LT_TRY(cudaMemsetAsync(t.lb.dl, 0, sizeof(float4) * (size_t)n, st));
+    LT_TRY(cudaMalloc(&t.lb.ell, sizeof(float2) * (size_t)L.K * n_pairs));
+    LT_TRY(cudaMemsetAsync(t.lb.ell, 0, sizeof(float2) * (size_t)L.K * n_pairs, st));   // rows that do not exist stay 0
+    LT_TRY(cudaMalloc(&t.lb.dense, sizeof(int) * (size_t)n));
+    LT_TRY(cudaMalloc(&t.lb.grid_w, sizeof(float4) * (size_t)map_size));
+    LT_TRY(cudaMemsetAsync(t.lb.grid_w, 0, sizeof(float4) * (size_t)map_size, st));
+    LT_TRY(cudaMalloc(&t.lb.grid_d, sizeof(float4) * (size_t)map_size));
+    LT_TRY(cudaMemsetAsync(t.lb.grid_d, 0, sizeof(float4) * (size_t)map_size, st));
+    LT_TRY(cudaMalloc(&t.lb.image, (size_t)lat_image_bytes(R) * (size_t)L.n_bricks));
     LT_TRY(cudaMalloc(&t.lb.sched, sizeof(unsigned) * 2));
     LT_TRY(cudaMemsetAsync(t.lb.sched, 0, sizeof(unsigned) * 2, st));
     LT_TRY(cudaMemcpyAsync(t.lb.brick_start, bstart.data(), sizeof(int) * bstart.size(), cudaMemcpyHostToDevice, st));
     LT_TRY(cudaMemcpyAsync(t.lb.brick_corner, bcorner.data(), sizeof(int) * bcorner.size(), cudaMemcpyHostToDevice, st));
-    LT_TRY(cudaMemcpyAsync(t.lb.row_local, rlocal.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, st));
-    LT_TRY(cudaMemcpyAsync(t.lb.row_brick, rbrick.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, st));
+    LT_TRY(cudaMemcpyAsync(t.lb.chunk_start, chunk_start.data(), sizeof(int) * chunk_start.size(), cudaMemcpyHostToDevice, st));
+    LT_TRY(cudaMemcpyAsync(t.lb.pair_base, pair_base.data(), sizeof(int) * n_pairs, cudaMemcpyHostToDevice, st));
+    LT_TRY(cudaMemcpyAsync(t.lb.pair_slot, pair_slot.data(), sizeof(int) * pair_slot.size(), cudaMemcpyHostToDevice, st));
+    LT_TRY(cudaMemcpyAsync(t.lb.row_pair, row_pair.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, st));
     LT_TRY(cudaMemcpyAsync(t.lb.offk, offk.data(), sizeof(int) * offk.size(), cudaMemcpyHostToDevice, st));
-    LT_TRY(cudaMemsetAsync(t.lb.map, 0xff, sizeof(int) * (size_t)map_size, st));
-    k_lat_map<<<G, kBlock, 0, st>>>(t.lb.site, n, R, (int)M[0], (int)M[1], t.lb.map);
+    k_lat_dense<<<G, kBlock, 0, st>>>(t.lb.site, n, R, (int)M[0], (int)M[1], t.lb.dense);
     LT_TRY(cudaGetLastError());
     LT_TRY(cudaStreamSynchronize(st));   // the host vectors above are read by the copies
     L.brick_start = t.lb.brick_start;
     L.brick_corner = t.lb.brick_corner;
-    L.row_local = t.lb.row_local;
-    L.row_brick = t.lb.row_brick;
+    L.chunk_start = t.lb.chunk_start;
+    L.pair_base = t.lb.pair_base;
+    L.pair_slot = t.lb.pair_slot;
+    L.row_pair = t.lb.row_pair;
     L.site = t.lb.site;
-    L.map = t.lb.map;
     L.offk = t.lb.offk;
     L.ell = t.lb.ell;
-    L.dl = t.lb.dl;
     L.sched = t.lb.sched;
+    L.dense = t.lb.dense;
+    L.grid_w = t.lb.grid_w;
+    L.grid_d = t.lb.grid_d;
+    L.image = t.lb.image;
+    LT_TRY(grid_box(&L));
     int dev = 0, sms = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -156,7 +156,7 @@ __device__ __forceinline__ double warp_total(DotAcc64 a)
 template <typename Acc, typename Fin>
 __device__ __forceinline__ void block_reduce_finish(Acc acc, ReduceSlot slot, Fin fin)
 {
-    __shared__ double warp_sums[kBlock / 32];
+    __shared__ double warp_sums[32];
     __shared__ bool is_last;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;

@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cstdint>
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -50,7 +51,7 @@ struct CgScalars {
     int ws_rejects;        // batch: consecutive rejected guesses (and paused steps since)
     int ws_skip;           // batch: 1 while this step's learned pass is paused
     int ws_skipped;        // batch: steps whose learned pass was paused
-    int wait_error;        // cg_persist.cu: a wait of the one-launch solve ran out of time
+    int wait_error;        // a bounded wait of a kernel ran out of time (cg_persist.cu, lattice.cu)
     double ns_spmv;        // cg_persist.cu, profiling: ns of the latest launch's products
     double ns_vec;         // ... and of its vector phases
 };
@@ -150,54 +151,63 @@ struct DeviceState {
 // body that way, src/examples/scene.cpp:33-135) keep each particle within a
 // fraction of a spacing of its lattice site, and every bond joins two sites
 // whose offset lies in a small stencil.  For such bodies the slots are
-// renumbered brick by brick (bricks of bx x by x bz sites, x fastest), and the
-// product runs brick-wise with the brick's halo of sites staged in shared
-// memory: a row's neighbour at stencil entry k sits at a fixed shared-memory
-// offset, and 1/d0 per (row, stencil entry) streams from a table in which 0
-// marks "no live bond" (no particle there, beyond the horizon, or broken).
-constexpr int kLatMaxK = 160;        // stencil entries at most
+// renumbered brick by brick (x fastest), and the product runs brick-wise with
+// the brick's halo of sites staged in shared memory: a row's neighbour at a
+// stencil entry sits at a fixed shared-memory offset, and 1/d0 per (row,
+// stencil entry) streams from a table in which 0 marks "no live bond" (no
+// particle there, beyond the horizon, or broken).
+constexpr int kLatMaxOffsets = 160;  // distinct bond offsets at most
 constexpr int kLatticeMinRows = 20000;   // automatic choice: smaller bodies keep the gather product
 constexpr int kLatticeOnlyRows = 250000; // automatic choice: larger lattice bodies time only the stencil variants
 constexpr int kLatRmax = 3;          // largest offset per axis (sites)
 constexpr int kLatTab = 2 * kLatRmax + 1;
 
 struct LatticeParams {
-    int K;                    // stencil entries, padded to a multiple of 4 (padding: offset 0, 1/d0 = 0)
+    int K;                    // stencil entries per row (2 r + 1 per z column of reach r)
     int R;                    // halo width (sites)
-    int bx, by, bz;           // brick extent (sites)
-    int hx, hy, hz;           // halo extent = brick + 2R
     int n_bricks;
     int grid;                 // blocks of the product
-    int fixed;                // 1: the 80-entry stencil of a 2.5-spacing horizon (compile-time offsets)
-    int map_dim[3];           // site map extent (bricks + R on each side)
+    int map_dim[3];           // extent of the grids of sites (bricks + R on each side)
     const int* brick_start;   // n_bricks + 1: slot range of each brick
-    const int* brick_corner;  // n_bricks: map index of the halo's first site
-    const int* row_local;     // n: halo index of the row's own site
-    const int* row_brick;     // n: brick of each slot
-    const int4* site;         // n: site coordinates (x, y, z) of each slot, from the map's first site
-    const int* map;           // site map: slot or -1
+    const int* brick_corner;  // n_bricks: grid index of the halo's first site
+    const int* chunk_start;   // n_bricks + 1: range of each brick's chunks of 32 pairs of z-adjacent rows
+    const int* pair_base;     // 32 per chunk: halo index of the pair's lower site
+    const int* pair_slot;     // 64 per chunk: slots of the pair's rows, -1 where there is none
+    const int* row_pair;      // n: 64 * chunk + 2 * lane + row of the pair
+    const int4* site;         // n: site coordinates (x, y, z) of each slot, from the body's first site
     const int* offk;          // kLatTab^3: stencil entry of an offset, or -1
     unsigned* sched;          // [0] next brick, [1] blocks finished (zero between launches)
-    float* ell;               // K per row, brick-major, in chunks of 4 entries:
-                              // [K * start_b + (k / 4) * 4 rows_b + 4 l + k % 4]
-    float4* dl;               // n, per step: the particle's deviation from its site, x - (org + h site)
+    float* ell;               // float2 [chunk][K][32]: 2^100 / d0 of the pair's two rows
+    int slabs;                // copies of a chunk's table, whole stencil columns each:
+    int slab_entry[kLatTab * kLatTab + 1];   // their first entries, and K
+    const int* dense;         // n: grid index of every slot
+    float4* grid_w;           // the product's vector on the grid of sites, 0 where there is no particle
+    float4* grid_d;           // per step: the particle's deviation from its site there, x - (org + h site)
                               // = d + sup n (|d| <= sup / 2 per axis): (d.x, d.y, d.z, packed n + 512)
+    float* image;             // per step, per brick: the deviations of its halo (x, y pairs, then z)
+    CUtensorMap box_w;        // grid_w in boxes of a brick's halo
     double org[3];            // position of site (0, 0, 0)
     double h;                 // lattice spacing
-    int off[kLatMaxK];        // halo index offset of each stencil entry
-    float cx[kLatMaxK], cy[kLatMaxK], cz[kLatMaxK];   // h * (lattice offset) of each stencil entry
+    int ncol[kLatRmax + 1];   // the stencil's z columns (dx, dy) of each reach, the largest reach first in:
+    int coff[kLatTab * kLatTab];                              // halo index offset
+    float ccx[kLatTab * kLatTab], ccy[kLatTab * kLatTab];     // h dx, h dy
+    float cz[kLatTab];        // h dz, dz = -kLatRmax .. kLatRmax
 };
 
 struct LatticeBuffers {       // device allocations owned by the engine
     int* brick_start = nullptr;
     int* brick_corner = nullptr;
-    int* row_local = nullptr;
-    int* row_brick = nullptr;
+    int* chunk_start = nullptr;
+    int* pair_base = nullptr;
+    int* pair_slot = nullptr;
+    int* row_pair = nullptr;
     int4* site = nullptr;
-    int* map = nullptr;
     int* offk = nullptr;
     float* ell = nullptr;
-    float4* dl = nullptr;
+    int* dense = nullptr;
+    float4* grid_w = nullptr;
+    float4* grid_d = nullptr;
+    float* image = nullptr;
     unsigned* sched = nullptr;
 };
 
@@ -225,13 +235,15 @@ cudaError_t lattice_build(int n, double spacing, dbl4* x64, float4* X32, int* pe
 // 1/d0 table from the live CSR bonds (force = 0: only when the force pass
 // reported a broken bond, read from S.flags[1] on the device)
 void launch_lattice_ell(const DeviceState& S, const LatticeParams& lp, int force, int grid, cudaStream_t st);
-// y = A(in) by the lattice stencil; dot as launch_operator (cg: CG iteration).
-// r_in set (a CG iteration): the direction p = r_in + beta in is formed on the
-// way in (beta from cg) and written to p_out (a buffer other than in); y = A p.
-void launch_spmv_lattice(bool dot, const StepParams& P, const DeviceState& S, const LatticeParams& lp,
-                         const void* in, void* out, ReduceSlot slot, CgScalars* cg, double* dot_out,
-                         const void* r_in, void* p_out, cudaStream_t st);
-// lp.dl from the positions x64 (with the supercell edge sup): after every
+// y = A w by the lattice stencil, w the vector on lp.grid_w; dot as
+// launch_operator (cg: CG iteration)
+void launch_spmv_lattice(bool dot, const StepParams& P, const DeviceState& S, const LatticeParams& lp, void* out,
+                         ReduceSlot slot, CgScalars* cg, double* dot_out, cudaStream_t st);
+// a vector in slot order onto lp.grid_w
+void launch_lattice_scatter(const DeviceState& S, const LatticeParams& lp, const void* in, cudaStream_t st);
+// S.p = r + beta S.p, in slot order and onto lp.grid_w
+void launch_lattice_xpby(const DeviceState& S, const LatticeParams& lp, const void* r, int grid, cudaStream_t st);
+// lp.grid_d and lp.image from the positions x64 (with the supercell edge sup): after every
 // change of the positions the product's operator is taken at
 void launch_lattice_delta(const DeviceState& S, const LatticeParams& lp, double sup, cudaStream_t st);
 int lattice_spmv_blocks_per_sm(const LatticeParams& lp);

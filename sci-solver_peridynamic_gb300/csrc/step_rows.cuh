@@ -505,8 +505,38 @@ __device__ __forceinline__ dbl4 ld_in(const dbl4* p)
     return make_dbl4(a.x, a.y, b.x, b.y);
 }
 
-// Mixed-precision row result from the group's partial bond sums:
-// y_p = m w_p + t2 (c sum_q J'(w_p - w_q) + k_contact n n^T w_p).
+// Mixed-precision row result from the row's bond sum (ax, ay, az):
+// y_p = m w_p + t2 (c sum_q J'(w_p - w_q) + k_contact n n^T w_p), with c, t2
+// and m rounded to FP32 by the caller.
+template <bool DOT, typename Acc>
+__device__ __forceinline__ void mixed_row_result(const StepParams& P, const DeviceState& S, int p, uint8_t ab, float c,
+                                                 float t2, float m, const float4& w, float ax, float ay, float az,
+                                                 float4* __restrict__ out, Acc& acc)
+{
+    float kx = c * ax, ky = c * ay, kz = c * az;
+    if (ab & kActContact) {
+        const float4 Xp = S.X32[p];
+        const float4 Up = S.u32[p];
+        const float dx = Xp.x + Up.x - (float)P.sphere_c_local[0];
+        const float dy = Xp.y + Up.y - (float)P.sphere_c_local[1];
+        const float dz = Xp.z + Up.z - (float)P.sphere_c_local[2];
+        const float inv = rsqrtf(dx * dx + dy * dy + dz * dz);
+        const float nx = dx * inv, ny = dy * inv, nz = dz * inv;
+        const float kn = (float)P.sphere_k * (nx * w.x + ny * w.y + nz * w.z);
+        kx += kn * nx; ky += kn * ny; kz += kn * nz;
+    }
+    const float yx = m * w.x + t2 * kx;
+    const float yy = m * w.y + t2 * ky;
+    const float yz = m * w.z + t2 * kz;
+    out[p] = make_float4(yx, yy, yz, 0.f);
+    if (DOT) {
+        acc.fma(w.x, yx);
+        acc.fma(w.y, yy);
+        acc.fma(w.z, yz);
+    }
+}
+
+// The same from a G-lane group's partial bond sums.
 template <int G, bool DOT, typename Acc>
 __device__ __forceinline__ void spmv_finish_mixed(const StepParams& P, const DeviceState& S, int p, uint8_t ab,
                                                   const float4& w, float ax, float ay, float az, int lane,
@@ -518,29 +548,7 @@ __device__ __forceinline__ void spmv_finish_mixed(const StepParams& P, const Dev
     ax = group_sum<G>(ax, gmask);
     ay = group_sum<G>(ay, gmask);
     az = group_sum<G>(az, gmask);
-    if (lane == 0) {
-        float kx = c * ax, ky = c * ay, kz = c * az;
-        if (ab & kActContact) {
-            const float4 Xp = S.X32[p];
-            const float4 Up = S.u32[p];
-            const float dx = Xp.x + Up.x - (float)P.sphere_c_local[0];
-            const float dy = Xp.y + Up.y - (float)P.sphere_c_local[1];
-            const float dz = Xp.z + Up.z - (float)P.sphere_c_local[2];
-            const float inv = rsqrtf(dx * dx + dy * dy + dz * dz);
-            const float nx = dx * inv, ny = dy * inv, nz = dz * inv;
-            const float kn = (float)P.sphere_k * (nx * w.x + ny * w.y + nz * w.z);
-            kx += kn * nx; ky += kn * ny; kz += kn * nz;
-        }
-        const float yx = m * w.x + t2 * kx;
-        const float yy = m * w.y + t2 * ky;
-        const float yz = m * w.z + t2 * kz;
-        out[p] = make_float4(yx, yy, yz, 0.f);
-        if (DOT) {
-            acc.fma(w.x, yx);
-            acc.fma(w.y, yy);
-            acc.fma(w.z, yz);
-        }
-    }
+    if (lane == 0) mixed_row_result<DOT>(P, S, p, ab, c, t2, m, w, ax, ay, az, out, acc);
 }
 
 // U bonds of one lane in mixed precision: gathers of the neighbours'
