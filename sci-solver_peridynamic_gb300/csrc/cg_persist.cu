@@ -40,6 +40,8 @@ namespace {
 constexpr int kPersistThreads = 512;
 constexpr int kPersistWarps = kPersistThreads / 32;
 constexpr int kPersistMaxGrid = 256;
+constexpr int kTileLanes = 4;        // lanes per row where the bonds are read from global memory
+constexpr int kTileBlock = 1024;     // threads of a product outside a solve
 constexpr unsigned long long kPersistTimeoutNs = 5000000000ull;   // 5 s
 
 __device__ __forceinline__ unsigned long long now_ns()
@@ -217,11 +219,25 @@ __device__ __forceinline__ BondGeometry bond_geometry(const float4& Xq, const fl
     return g;
 }
 
+// Four consecutive bonds' halo indices and 1/d0.
+__device__ __forceinline__ void load_bonds(const DeviceState& S, int slot, int (&l)[4], float (&id0)[4])
+{
+    const ushort4 i = __ldg((const ushort4*)(S.lidx + slot));
+    const float4 d = __ldg((const float4*)(S.inv_d0 + slot));
+    l[0] = i.x; l[1] = i.y; l[2] = i.z; l[3] = i.w;
+    id0[0] = d.x; id0[1] = d.y; id0[2] = d.z; id0[3] = d.w;
+}
+
 // Mixed precision, G lanes per row, U bonds in flight per lane.  The halo is
 // S.halo of a tile per block, a bond's index into it S.lidx.
 // CACHED: the bonds' geometry stays in shared memory; else the halo's
 // positions do, and the index and 1/d0 of a bond are read from global memory
-// (6 bytes per bond, from L2).
+// (6 bytes per bond, from L2).  Not cached, the product is bound by the
+// shared-memory pipe and by latency (one block per SM): four consecutive bonds
+// per lane and load, the next four in flight, and the rows' order from
+// k_bank_order take an iteration at 100k particles (76 bonds) from 38.2 us to
+// 31.2; with 8 lanes per row 34.9 (37.5 without the order), with 1024 threads
+// 30.3 (but 24.0 against 21.8 at 50k and 104 bonds).
 template <bool CACHED, int G, int U>
 __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist32(PersistArgs A)
 {
@@ -244,7 +260,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist32(PersistArgs
     BondGeometry* sg = (BondGeometry*)(CACHED ? shx : shx + A.halo);
     float* sa1 = (float*)(sg + A.bonds);                 // 1/d0 - 1/d
     int* srow = (int*)(sa1 + A.bonds);                   // first slot of the row
-    int* scnt = srow + A.rows;                           // live bonds, -1 for a Dirichlet row
+    int* scnt = srow + A.rows;                           // live bonds << 8 | activity, -1 for a Dirichlet row
     int* sq = scnt + A.rows;                             // the halo's slots
     uint16_t* sl = (uint16_t*)(sq + A.halo);             // a bond's halo index
 
@@ -257,7 +273,8 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist32(PersistArgs
         sx[t] = ((const float4*)S.sol)[p];
         sr[t] = ((const float4*)S.r)[p];
         sp[t] = ((const float4*)S.p)[p];
-        scnt[t] = is_dirichlet(S.act[p] & kActMask) ? -1 : S.cnt[p];
+        const uint8_t ab = S.act[p];
+        scnt[t] = is_dirichlet(ab & kActMask) ? -1 : S.cnt[p] << 8 | ab;
         srow[t] = S.row_ptr[p] - first;
     }
     const int h0 = S.halo_ptr[blockIdx.x], nh = S.halo_ptr[blockIdx.x + 1] - h0;
@@ -273,7 +290,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist32(PersistArgs
     const float sup = (float)P.sup;
     if (CACHED) {
         for (int i = threadIdx.x / G; i < nr; i += NG) {
-            const int cn = scnt[i], base = srow[i];
+            const int cn = scnt[i] < 0 ? 0 : scnt[i] >> 8, base = srow[i];
             const float4 xp = S.xs4[lo + i];
             for (int j = lane; j < cn; j += G) {
                 const int l = S.lidx[first + base + j];
@@ -305,46 +322,62 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist32(PersistArgs
         __syncthreads();
         DotAcc32 acc;
         for (int i = threadIdx.x / G; i < nr; i += NG) {
-            const int cn = scnt[i], base = srow[i], p = lo + i;
+            const int cn = scnt[i] >> 8, base = srow[i], p = lo + i;
+            int l[U];
+            float a1[U];
+            // the bond records of one step: index, and 1/d0 - 1/d (CACHED) or
+            // 1/d0; U consecutive slots in one load each (not CACHED: rows start
+            // 32-byte aligned and hold a multiple of 8 slots)
+            const auto load = [&](int j0) {
+                if constexpr (CACHED) {
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const int j = j0 + u * G;
+                        l[u] = 0;
+                        a1[u] = 0.f;
+                        if (j < cn) {
+                            l[u] = sl[base + j];
+                            a1[u] = sa1[base + j];
+                        }
+                    }
+                } else if (j0 < cn) {
+                    load_bonds(S, base + j0, l, a1);
+                }
+            };
+            constexpr int LS = CACHED ? 1 : U, US = CACHED ? G : 1;   // slots between lanes, between a lane's bonds
+            load(lane * LS);
+            float4 xp = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (!CACHED && cn > 0) xp = __ldg(S.xs4 + p);
             float4 w = sp[i];
             const float4 r = sr[i];
             w = make_float4(r.x + beta * w.x, r.y + beta * w.y, r.z + beta * w.z, 0.f);
             float ax = 0.f, ay = 0.f, az = 0.f;
-            float4 xp = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (!CACHED && cn > 0) xp = __ldg(S.xs4 + p);
-            for (int j0 = lane; j0 < cn; j0 += G * U) {
-                int l[U];
-                float a1[U];
+            for (int j0 = lane * LS; j0 < cn; j0 += G * U) {
+                int lc[U];
+                float ac[U];
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    const int j = j0 + u * G;
-                    l[u] = 0;
-                    a1[u] = 0.f;
-                    if (j < cn) {
-                        l[u] = CACHED ? sl[base + j] : __ldg(S.lidx + base + j);
-                        a1[u] = CACHED ? sa1[base + j] : __ldg(S.inv_d0 + base + j);
-                    }
+                    lc[u] = l[u];
+                    ac[u] = a1[u];
                 }
+                load(j0 + G * U);   // in flight while this step's bonds are added
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    const int j = j0 + u * G;
+                    const int j = j0 + u * US;
                     if (j >= cn) continue;
-                    const float4 Wq = sw[l[u]];
+                    const float4 Wq = sw[lc[u]];
                     BondGeometry g;
-                    if constexpr (CACHED) {
-                        g = sg[base + j];
-                    } else {
-                        const float inv_d0 = a1[u];
-                        g = bond_geometry(shx[l[u]], xp, sup, inv_d0, a1[u]);
-                    }
+                    float a = ac[u];
+                    if constexpr (CACHED) g = sg[base + j];
+                    else g = bond_geometry(shx[lc[u]], xp, sup, ac[u], a);
                     const float wx = w.x - Wq.x, wy = w.y - Wq.y, wz = w.z - Wq.z;
                     const float d = fmaf(g.x, wx, fmaf(g.y, wy, g.z * wz)) * g.i3;
-                    ax = fmaf(a1[u], wx, fmaf(d, g.x, ax));
-                    ay = fmaf(a1[u], wy, fmaf(d, g.y, ay));
-                    az = fmaf(a1[u], wz, fmaf(d, g.z, az));
+                    ax = fmaf(a, wx, fmaf(d, g.x, ax));
+                    ay = fmaf(a, wy, fmaf(d, g.y, ay));
+                    az = fmaf(a, wz, fmaf(d, g.z, az));
                 }
             }
-            if (cn >= 0) spmv_finish_mixed<G, true>(P, S, p, S.act[p], w, ax, ay, az, lane, gmask, sy - lo, acc);
+            if (cn >= 0) spmv_finish_mixed<G, true>(P, S, p, (uint8_t)scnt[i], w, ax, ay, az, lane, gmask, sy - lo, acc);
             else if (lane == 0) sy[i] = make_float4(0.f, 0.f, 0.f, 0.f);
             __syncwarp(gmask);   // every lane has read sp[i]
             if (lane == 0) sp[i] = w;
@@ -410,6 +443,85 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist32(PersistArgs
         sc->ns_spmv = (double)ns_spmv;
         sc->ns_vec = (double)ns_vec;
     }
+}
+
+// One product y = A w outside a solve by the same rows and halos, bonds read as
+// the uncached solve reads them, and bound like it.  The gather product, whose
+// every bond reads two 16-byte records through L1, takes 45.3 us at 100k
+// particles of 104 bonds, this one 38.8 (41.1 with 512 threads).
+template <bool DOT>
+__global__ void __launch_bounds__(kTileBlock, 1)
+    k_tile_product32(StepParams P, DeviceState S, int rows, int halo, const float4* __restrict__ in,
+                     float4* __restrict__ out, ReduceSlot slot, double* dot_out)
+{
+    constexpr int G = kTileLanes;
+    extern __shared__ __align__(32) unsigned char smem[];
+    float4* sw = (float4*)smem;
+    float4* shx = sw + halo;
+    const int lo = blockIdx.x * rows;
+    const int nr = min(rows, P.n - lo);
+    const int lane = threadIdx.x & (G - 1);
+    const unsigned gmask = group_mask<G>();
+    // a row's own data and its first bonds, in flight while the halo is staged
+    // (the block's later rows: while the row before them is finished)
+    int rs = 0, cn = -1, l[4];
+    float id0[4];
+    uint8_t ab = 0;
+    float4 w, xp;
+    const auto fetch = [&](int i) {
+        if (i >= nr) return;
+        const int p = lo + i;
+        rs = __ldg(S.row_ptr + p);
+        cn = S.cnt[p];
+        ab = S.act[p];
+        w = __ldg(in + p);
+        xp = __ldg(S.xs4 + p);
+        if (is_dirichlet(ab & kActMask)) cn = -1;
+        if (lane * 4 < cn) load_bonds(S, rs + lane * 4, l, id0);
+    };
+    fetch(threadIdx.x / G);
+    const int h0 = S.halo_ptr[blockIdx.x], nh = S.halo_ptr[blockIdx.x + 1] - h0;
+    for (int h = threadIdx.x; h < nh; h += kTileBlock) {
+        const int q = __ldg(S.halo + h0 + h);
+        sw[h] = __ldg(in + q);
+        shx[h] = __ldg(S.xs4 + q);
+    }
+    __syncthreads();
+    const float sup = (float)P.sup;
+    DotAcc32 acc;
+    for (int i = threadIdx.x / G; i < nr; i += kTileBlock / G) {
+        float ax = 0.f, ay = 0.f, az = 0.f;
+        for (int j0 = lane * 4; j0 < cn; j0 += G * 4) {
+            int lc[4];
+            float ic[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                lc[u] = l[u];
+                ic[u] = id0[u];
+            }
+            if (j0 + G * 4 < cn) load_bonds(S, rs + j0 + G * 4, l, id0);   // in flight while this step's bonds are added
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (j0 + u >= cn) continue;
+                const float4 Wq = sw[lc[u]];
+                float a1;
+                const BondGeometry g = bond_geometry(shx[lc[u]], xp, sup, ic[u], a1);
+                const float wx = w.x - Wq.x, wy = w.y - Wq.y, wz = w.z - Wq.z;
+                const float d = fmaf(g.x, wx, fmaf(g.y, wy, g.z * wz)) * g.i3;
+                ax = fmaf(a1, wx, fmaf(d, g.x, ax));
+                ay = fmaf(a1, wy, fmaf(d, g.y, ay));
+                az = fmaf(a1, wz, fmaf(d, g.z, az));
+            }
+        }
+        const int p = lo + i;
+        const uint8_t row_ab = ab;
+        const float4 row_w = w;
+        const bool fixed = cn < 0;
+        fetch(i + kTileBlock / G);
+        if (!fixed) spmv_finish_mixed<G, DOT>(P, S, p, row_ab, row_w, ax, ay, az, lane, gmask, out, acc);
+        else if (lane == 0) out[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (DOT) block_reduce_finish(acc, slot, [dot_out](double pAp) { *dot_out = pAp; });
 }
 
 struct __align__(8) Vec3d {
@@ -624,20 +736,32 @@ size_t persist_smem(bool fp64, int rows, int halo, int bonds)
     return (4 * v + 2 * sizeof(int)) * rows + (v * (fp64 || bonds > 0 ? 2 : 3) + sizeof(int)) * halo + bond * (size_t)bonds;
 }
 
+const void* persist_kernel32(const CgPersistPlan& pl)
+{
+    if (pl.bonds == 0) return (const void*)k_cg_persist32<false, kTileLanes, 4>;
+    switch (pl.lanes) {
+    case 4: return (const void*)k_cg_persist32<true, 4, 4>;
+    case 8: return (const void*)k_cg_persist32<true, 8, 4>;
+    case 16: return (const void*)k_cg_persist32<true, 16, 4>;
+    default: return (const void*)k_cg_persist32<true, 32, 2>;
+    }
+}
+
 template <bool CACHED>
-const void* persist_kernel_t(bool fp64, int lanes)
+const void* persist_kernel64(int lanes)
 {
     switch (lanes) {
-    case 4: return fp64 ? (const void*)k_cg_persist64<CACHED, 4, 4> : (const void*)k_cg_persist32<CACHED, 4, 4>;
-    case 8: return fp64 ? (const void*)k_cg_persist64<CACHED, 8, 4> : (const void*)k_cg_persist32<CACHED, 8, 4>;
-    case 16: return fp64 ? (const void*)k_cg_persist64<CACHED, 16, 4> : (const void*)k_cg_persist32<CACHED, 16, 4>;
-    default: return fp64 ? (const void*)k_cg_persist64<CACHED, 32, 2> : (const void*)k_cg_persist32<CACHED, 32, 2>;
+    case 4: return (const void*)k_cg_persist64<CACHED, 4, 4>;
+    case 8: return (const void*)k_cg_persist64<CACHED, 8, 4>;
+    case 16: return (const void*)k_cg_persist64<CACHED, 16, 4>;
+    default: return (const void*)k_cg_persist64<CACHED, 32, 2>;
     }
 }
 
 const void* persist_kernel(bool fp64, const CgPersistPlan& pl)
 {
-    return pl.bonds > 0 ? persist_kernel_t<true>(fp64, pl.lanes) : persist_kernel_t<false>(fp64, pl.lanes);
+    if (!fp64) return persist_kernel32(pl);
+    return pl.bonds > 0 ? persist_kernel64<true>(pl.lanes) : persist_kernel64<false>(pl.lanes);
 }
 
 }  // namespace
@@ -670,8 +794,11 @@ bool cg_persist_plan(bool fp64, int max_halo, int max_bonds, int device, CgPersi
     pl.bonds = bonds < (1 << 20) && persist_smem(fp64, pl.rows, pl.halo, (int)bonds) <= (size_t)room ? (int)bonds : 0;
     pl.smem = persist_smem(fp64, pl.rows, pl.halo, pl.bonds);
     if (pl.smem > (size_t)room) return false;
+    // a cached row is spread over as many lanes as one pass of the block allows
     pl.lanes = 32;
     while (pl.lanes > 4 && kPersistThreads / pl.lanes < pl.rows) pl.lanes /= 2;
+    pl.tiled_products = !fp64 && pl.bonds == 0;
+    if (pl.tiled_products) pl.lanes = kTileLanes;
     const void* k = persist_kernel(fp64, pl);
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, room) != cudaSuccess) {
         cudaGetLastError();
@@ -680,8 +807,25 @@ bool cg_persist_plan(bool fp64, int max_halo, int max_bonds, int device, CgPersi
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kPersistThreads, pl.smem);
     if (per_sm < 1) return false;
+    if (pl.tiled_products)
+        for (const void* t : {(const void*)k_tile_product32<true>, (const void*)k_tile_product32<false>})
+            if (cudaFuncSetAttribute(t, cudaFuncAttributeMaxDynamicSharedMemorySize, room) != cudaSuccess) {
+                cudaGetLastError();
+                return false;
+            }
     *plan = pl;
     return true;
+}
+
+cudaError_t launch_tile_product(const StepParams& P, const DeviceState& S, const CgPersistPlan& plan, const void* in,
+                                void* out, ReduceSlot slot, double* dot_out, cudaStream_t st)
+{
+    StepParams p = P;
+    DeviceState s = S;
+    int rows = plan.rows, halo = plan.halo;
+    void* args[] = {&p, &s, &rows, &halo, &in, &out, &slot, &dot_out};
+    const void* k = dot_out ? (const void*)k_tile_product32<true> : (const void*)k_tile_product32<false>;
+    return cudaLaunchKernel(k, dim3(plan.grid), dim3(kTileBlock), args, 2 * sizeof(float4) * (size_t)plan.halo, st);
 }
 
 cudaError_t launch_cg_persist(bool fp64, const StepParams& P, const DeviceState& S, const CgPersistPlan& plan,

@@ -253,12 +253,19 @@ pd_status Engine::make_ready()
     total_slots_ = out.total;
     bonds_initial_ = out.bonds;
     sim_.pd_max_num_bonds = out.max_bonds;
-    // lattice-filled bodies: slots renumbered brick by brick for the stencil
+    // bodies small enough for the one-launch solve keep the builder's order;
+    // larger lattice-filled bodies are renumbered brick by brick for the stencil
     // product (mixed mode; automatic above kLatticeMinRows particles, or asked
-    // for with spmv_path 3).  Bodies that are not a lattice fill keep the
-    // builder's order and the gather product.
+    // for with spmv_path 3).  Other bodies keep the builder's order and the
+    // gather product.  (Per CG iteration, one launch against the stencil: 27
+    // us against 44 at 50k particles and a horizon of 3 spacings, 38 against
+    // 50 at 100k and 2.5.)
+    if (opt_.spmv_path == 0 || opt_.spmv_path == 2) {
+        s = persist_prepare();
+        if (s != PD_OK) return s;
+    }
     if (!fp64_ && n > 0 && !batch_member_ &&
-        (opt_.spmv_path == 3 || (opt_.spmv_path == 0 && n >= kLatticeMinRows))) {
+        (opt_.spmv_path == 3 || (opt_.spmv_path == 0 && n >= kLatticeMinRows && persist_.grid == 0))) {
         int ok = 0;
         CK(lattice_build(n, 2.0 * sim_.pd_particle_radius, S_.x64, S_.X32, d_perm_, S_.row_ptr, S_.cnt, &S_.col,
                          total_slots_, &lat_, &latb_, &ok, stream_),
@@ -367,8 +374,6 @@ pd_status Engine::make_ready()
     }
     s = tune_spmv();
     if (s != PD_OK) return s;
-    s = persist_prepare();
-    if (s != PD_OK) return s;
     if (opt_.warm_start == 2 || opt_.warm_start == 3) {
         s = hist_prepare();
         if (s != PD_OK) return s;
@@ -447,7 +452,7 @@ pd_status Engine::tune_spmv()
             L_.grid_bonds = lat_.grid;
             return;
         }
-        if (c.tiled) relayout_bonds(1, 1);
+        if (c.tiled || persist_.tiled_products) relayout_bonds(1, 1);   // (the tile product has its own order)
         else relayout_bonds(c.g, c.u);
         L_.tiled = c.tiled;
         L_.lanes = c.g;
@@ -459,7 +464,7 @@ pd_status Engine::tune_spmv()
             L_.grid_bonds = grid_for_rows(c.g, row_kernel_blocks_per_sm(fp64_, c.g, c.u));
         }
     };
-    if (cand.size() == 1 || n_ < 20000) {
+    if (cand.size() == 1 || n_ < 20000 || persist_.tiled_products) {
         // small problems: launch overhead dominates, keep the default (the
         // tiled path when it was asked for)
         Cand c = cand.size() == 1 ? cand[0] : Cand{0, 8, fp64_ ? 1 : 2};
@@ -512,12 +517,22 @@ pd_status Engine::tune_spmv()
     return PD_OK;
 }
 
+// y = A x for the solve's first residual
+void Engine::product_of_guess(const StepParams& P)
+{
+    if (persist_.tiled_products)
+        launch_tile_product(P, S_, persist_, S_.sol, S_.y, ReduceSlot{S_.partials, S_.counters + 1}, nullptr, stream_);
+    else launch_spmv(fp64_, false, P, S_, L_, stream_);
+}
+
 void Engine::apply_op(const StepParams& P, const void* in, void* out, ReduceSlot slot, double* dot_out)
 {
     if (L_.lattice) {
         launch_lattice_scatter(S_, lat_, in, stream_);
         launch_spmv_lattice(dot_out != nullptr, P, S_, lat_, out, slot, nullptr, dot_out, stream_);
         ++launches_;
+    } else if (persist_.tiled_products) {
+        launch_tile_product(P, S_, persist_, in, out, slot, dot_out, stream_);
     }
     else launch_operator_u(fp64_, P, S_, L_.lanes, L_.unroll, L_.grid_bonds, in, out, slot, dot_out, stream_);
 }
@@ -526,7 +541,7 @@ void Engine::apply_op(const StepParams& P, const void* in, void* out, ReduceSlot
 // cooperative launch (cg_persist.cu).
 pd_status Engine::persist_prepare()
 {
-    if (n_ <= 0 || batch_member_ || L_.lattice || L_.tiled || opt_.preconditioner || S_.lidx) return PD_OK;
+    if (n_ <= 0 || batch_member_ || opt_.preconditioner) return PD_OK;
     CgPersistPlan plan = cg_persist_rows(fp64_, n_, sm_count_, device_);
     if (plan.grid == 0) return PD_OK;
     int max_halo = 0, unfit = 0;
@@ -541,6 +556,14 @@ pd_status Engine::persist_prepare()
         free_tiles(S_);
         return PD_OK;
     }
+    // Below kTileMinSlots bond slots the gather product is the faster one outside
+    // the solve: 12.4 us against 15.1 at 18k particles and 76 bonds each, 15.0
+    // against 16.5 at 40k and 29; above, 20.3 against 19.8 at 30k and 104, 35.9
+    // against 31.8 at 100k and 76, 45.3 against 38.8 at 100k and 104.
+    // (A fixed lanes_per_particle or spmv_unroll names a shape of the gather.)
+    plan.tiled_products = plan.tiled_products && total_slots_ >= kTileMinSlots && !opt_.lanes_per_particle && !opt_.spmv_unroll;
+    if (plan.tiled_products)
+        CK(launch_bank_order(S_, n_, plan.lanes, 4, total_slots_, stream_), "order bonds");
     const size_t inbox = 2 * (size_t)plan.grid * plan.grid, rec = (fp64_ ? 2 : 1) * (size_t)n_;
     CK(dalloc(&d_inbox_, inbox + rec), "alloc records");
     CK(cudaMemsetAsync(d_inbox_, 0, sizeof(ulonglong2) * (inbox + rec), stream_), "memset records");
@@ -718,7 +741,7 @@ pd_status Engine::ws_before_cg(const StepParams& P)
         launch_ws_save_plain(S_, stream_);
         CK(mlp_infer_tc(mlp_, W_.features, n_, mlp_work_.y, stream_), "network launch");
         launch_ws_apply(P, S_, W_, mlp_work_.y, L_.grid_vec, stream_);
-        launch_spmv(fp64_, false, P, S_, L_, stream_);
+        product_of_guess(P);
         launch_cg_residual(fp64_, P, S_, L_, stream_);
         launch_ws_guard(P, S_, W_.xsave, ws_rsave_, L_.grid_vec, stream_);
         launches_ += 14;
@@ -969,7 +992,7 @@ pd_status Engine::integrate(bool* advanced)
 pd_status Engine::solve(const StepParams& P)
 {
     launch_cg_init(fp64_, P, S_, L_, stream_);
-    launch_spmv(fp64_, false, P, S_, L_, stream_);
+    product_of_guess(P);
     launch_cg_residual(fp64_, P, S_, L_, stream_);
     launches_ += 3;
     if (opt_.warm_start == 3) {   // network column first, then the projection over history + column
@@ -1303,7 +1326,7 @@ pd_status Engine::hist_project(const StepParams& P)
     // x1 + H y and its residual (the apply returns at once when no column was
     // used; the residual is then that of x1 again)
     launch_hist_apply(fp64_, n_, m, H, d_hsol_, S_.sol, L_.grid_vec, stream_);
-    launch_spmv(fp64_, false, P, S_, L_, stream_);
+    product_of_guess(P);
     launch_cg_residual(fp64_, P, S_, L_, stream_);
     launches_ += m + 5;
     CK(cudaMemcpyAsync(h_sc_hist_, S_.sc, sizeof(CgScalars), cudaMemcpyDeviceToHost, stream_),

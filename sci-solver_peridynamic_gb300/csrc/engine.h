@@ -69,6 +69,7 @@ private:
     StepParams step_params() const;
     int grid_for_rows(int lanes, int blocks_per_sm) const;
     pd_status tune_spmv();
+    void product_of_guess(const StepParams& P);
     // y = A in with this handle's product (lattice stencil or CSR rows)
     void apply_op(const StepParams& P, const void* in, void* out, ReduceSlot slot, double* dot_out);
     pd_status persist_prepare();

@@ -556,6 +556,14 @@ __global__ void __launch_bounds__(32 * lat_warps(R), 2)
     int chunk = chunk_of(b);
     if (lane == 0 && chunk >= 0)
         for (int k = 0; k < min(2, lp.slabs); ++k) lat_issue(s, lp, chunk, k);
+    // the chunk's row pair of this lane, read a brick ahead: the halo index of
+    // the lower site and the slots (139 -> 134 us at 1M particles)
+    int base_n = 0;
+    int2 slots_n = make_int2(-1, -1);
+    if (chunk >= 0) {
+        base_n = __ldg(lp.pair_base + chunk * 32 + lane);
+        slots_n = __ldg((const int2*)lp.pair_slot + chunk * 32 + lane);
+    }
     DotAcc32 acc;
     bool ok = true;
     const float c0 = (float)P.bond_coeff, t2 = (float)P.t2, m = (float)P.mass;
@@ -567,8 +575,13 @@ __global__ void __launch_bounds__(32 * lat_warps(R), 2)
         const int ahead = *(volatile int*)&s_ahead;   // the next brick
         const int next = chunk_of(ahead);
         if (ok && chunk >= 0) {
-            const int base = __ldg(lp.pair_base + chunk * 32 + lane);   // halo index of the lower site
-            const int2 slots = __ldg((const int2*)lp.pair_slot + chunk * 32 + lane);
+            const int base = base_n;
+            const int2 slots = slots_n;
+            const uint8_t ab2[2] = {slots.x >= 0 ? S.act[slots.x] : (uint8_t)0, slots.y >= 0 ? S.act[slots.y] : (uint8_t)0};
+            if (next >= 0) {
+                base_n = __ldg(lp.pair_base + next * 32 + lane);
+                slots_n = __ldg((const int2*)lp.pair_slot + next * 32 + lane);
+            }
             LatRows row;
 #pragma unroll
             for (int i = 0; i < kLatRZ; ++i) {
@@ -590,15 +603,18 @@ __global__ void __launch_bounds__(32 * lat_warps(R), 2)
             for (int i = 0; i < kLatRZ; ++i) {
                 const int p = i == 0 ? slots.x : slots.y;
                 if (p < 0) continue;
-                const uint8_t ab = S.act[p];
+                const uint8_t ab = ab2[i];
                 if (is_dirichlet(ab & kActMask))
                     out[p] = make_float4(0.f, 0.f, 0.f, 0.f);
                 else
                     mixed_row_result<DOT>(P, S, p, ab, c0, t2, m, make_float4(row.w[i].x, row.w[i].y, row.wz[i], 0.f),
                                           -row.sxy[i].x, -row.sxy[i].y, -row.sz[i], out, acc);
             }
-        } else if (lane == 0 && next >= 0) {
-            for (int k = 0; k < min(2, lp.slabs); ++k) lat_issue(s, lp, next, k);
+        } else if (next >= 0) {
+            if (lane == 0)
+                for (int k = 0; k < min(2, lp.slabs); ++k) lat_issue(s, lp, next, k);
+            base_n = __ldg(lp.pair_base + next * 32 + lane);
+            slots_n = __ldg((const int2*)lp.pair_slot + next * 32 + lane);
         }
         if (__syncthreads_or(ok ? 0 : 1)) {   // the block is done with the halo, or gave up
             ok = false;

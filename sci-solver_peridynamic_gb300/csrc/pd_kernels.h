@@ -157,6 +157,7 @@ struct DeviceState {
 // stencil entry) streams from a table in which 0 marks "no live bond" (no
 // particle there, beyond the horizon, or broken).
 constexpr int kLatMaxOffsets = 160;  // distinct bond offsets at most
+constexpr long long kTileMinSlots = 3000000;   // bond slots from which the one-launch bodies' other products use its tiles
 constexpr int kLatticeMinRows = 20000;   // automatic choice: smaller bodies keep the gather product
 constexpr int kLatticeOnlyRows = 250000; // automatic choice: larger lattice bodies time only the stencil variants
 constexpr int kLatRmax = 3;          // largest offset per axis (sites)
@@ -266,6 +267,7 @@ struct CgPersistPlan {
     int rows = 0;        // rows per block
     int halo = 0;        // the largest number of distinct neighbours of a block's rows
     int bonds = 0;       // bond slots kept in shared memory per block (0: read from global memory)
+    bool tiled_products = false;   // launch_tile_product serves the body's other products
     int lanes = 0;       // lanes per row
     size_t smem = 0;
 };
@@ -282,6 +284,10 @@ bool cg_persist_plan(bool fp64, int max_halo, int max_bonds, int device, CgPersi
 cudaError_t launch_cg_persist(bool fp64, const StepParams& P, const DeviceState& S, const CgPersistPlan& plan,
                               ulonglong2* rec, ulonglong2* inbox, unsigned long long epoch, int max_iters, bool profile,
                               cudaStream_t st);
+// y = A in by the same blocks (mixed precision, a plan with a grid); *dot_out
+// (may be null) receives <in, A in>
+cudaError_t launch_tile_product(const StepParams& P, const DeviceState& S, const CgPersistPlan& plan, const void* in,
+                                void* out, ReduceSlot slot, double* dot_out, cudaStream_t st);
 // Preconditioned CG (no reference counterpart in use: the reference's
 // cusp::precond::diagonal is commented out, simulator.cu:767-769): mode 1 =
 // inverse diagonal of A, 2 = inverse 3x3 diagonal blocks; the stopping test
@@ -311,6 +317,10 @@ void launch_bond_relayout(const DeviceState& S, int grid, int g_from, int u_from
 // returns the largest halo in *max_halo and the tiles whose halo did not fit
 // the builder's hash set in *unfit.
 cudaError_t build_tiles(DeviceState& S, int n, int* max_halo, int* unfit, cudaStream_t st);
+// Reorders every row's bonds (col, lidx; the geometry arrays not yet formed) for
+// few bank conflicts among those that `lanes` lanes, each reading `unroll`
+// consecutive slots, look up together.
+cudaError_t launch_bank_order(const DeviceState& S, int n, int lanes, int unroll, long long slots, cudaStream_t st);
 void free_tiles(DeviceState& S);
 // Tile SpMV: blocks per SM for a shared-memory halo of halo_cap entries, and the launch.
 int tile_spmv_blocks_per_sm(int lanes, int unroll, int halo_cap);

@@ -131,6 +131,52 @@ __global__ void __launch_bounds__(kBlock) k_tile_fill(DeviceState S, int n)
     }
 }
 
+// ---- order of a row's bonds -------------------------------------------------------------
+// A halo entry is 16 bytes, so eight lanes that read entries of eight different
+// residues mod 8 take one pass through shared memory, and eight arbitrary ones
+// 2.6 on average.  Lane k of a row's G reads U consecutive slots of every G*U,
+// one after another; the bonds that the lanes read together are given different
+// residues as far as the row's bonds allow: one of each residue that is left,
+// then of the residues with most left.  Thread per row; `scratch` holds (slot,
+// local index) of the row's bonds by residue.
+__global__ void __launch_bounds__(kBlock) k_bank_order(DeviceState S, int n, int G, int U, int2* __restrict__ scratch)
+{
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
+        const int rs = S.row_ptr[p], cn = S.cnt[p];
+        int left[8], at[8];
+        for (int c = 0; c < 8; ++c) left[c] = 0;
+        for (int j = 0; j < cn; ++j) ++left[S.lidx[rs + j] & 7];
+        int sum = rs;
+        for (int c = 0; c < 8; ++c) {
+            at[c] = sum;
+            sum += left[c];
+        }
+        for (int j = 0; j < cn; ++j) {
+            const int l = S.lidx[rs + j];
+            scratch[at[l & 7]++] = make_int2(S.col[rs + j], l);
+        }
+        for (int b = 0; b < cn; b += G * U)
+            for (int u = 0; u < U; ++u) {
+                int c = 0;
+                for (int j = b + u; j < min(b + G * U, cn); j += U) {
+                    while (c < 8 && left[c] == 0) ++c;
+                    int take = c;
+                    if (c == 8) {
+                        take = 0;
+                        for (int k = 1; k < 8; ++k)
+                            if (left[k] > left[take]) take = k;
+                    } else {
+                        ++c;
+                    }
+                    --left[take];
+                    const int2 bond = scratch[--at[take]];
+                    S.col[rs + j] = bond.x;
+                    S.lidx[rs + j] = (uint16_t)bond.y;
+                }
+            }
+    }
+}
+
 // ---- the tile SpMV ------------------------------------------------------------------
 template <int G, int U, bool DOT>
 __device__ __forceinline__ void tile_row(const StepParams& P, const DeviceState& S, const float4* __restrict__ in,
@@ -290,6 +336,17 @@ int tile_blocks(int halo_cap)
 }
 
 }  // namespace
+
+cudaError_t launch_bank_order(const DeviceState& S, int n, int lanes, int unroll, long long slots, cudaStream_t st)
+{
+    int2* scratch = nullptr;
+    cudaError_t e = cudaMalloc((void**)&scratch, sizeof(int2) * (size_t)(slots > 0 ? slots : 1));
+    if (e != cudaSuccess) return e;
+    k_bank_order<<<(n + kBlock - 1) / kBlock, kBlock, 0, st>>>(S, n, lanes, unroll, scratch);
+    e = cudaGetLastError();
+    const cudaError_t f = cudaFree(scratch);
+    return e != cudaSuccess ? e : f;
+}
 
 cudaError_t build_tiles(DeviceState& S, int n, int* max_halo, int* unfit, cudaStream_t st)
 {
