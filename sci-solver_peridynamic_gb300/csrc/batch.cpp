@@ -53,6 +53,7 @@ private:
     pd_status build_items(int item_rows);
     BatchArgs args(int tune_reps) const;
     pd_status enqueue_step();
+    pd_status plan_gangs();
     pd_status tune();
     pd_status build_graph();
     pd_status pull_state();
@@ -80,6 +81,11 @@ private:
     int grid_pre_ = 0, grid_cg_ = 0;
     bool autotuned_ = false;
     double tuned_ms_ = 0.0;
+    // gangs' solve (gangs_ 0: not used); its records, order and counter in one block
+    int gangs_ = 0, gang_ = 0;
+    size_t gang_smem_ = 0, gang_zero_ = 0;   // zeroed before each launch: the first gang_zero_ bytes
+    unsigned char* d_gang_ = nullptr;
+    GangArgs gang_args_{};
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t exec_ = nullptr;
     // learned warm start: one network for all scenes, run once per step over
@@ -127,6 +133,9 @@ void Batch::free_device()
     d_counters_ = nullptr;
     d_sync_ = nullptr;
     items_cap_ = 0;
+    cudaFree(d_gang_);
+    d_gang_ = nullptr;
+    gangs_ = 0;
 }
 
 pd_status Batch::fail(cudaError_t e, const char* what)
@@ -251,7 +260,109 @@ pd_status Batch::enqueue_step()
         const int grid_ws = std::max(1, batch_ws_blocks_per_sm(lanes_, unroll_)) * sm_count_;
         BCK(launch_batch_ws_guess(lanes_, unroll_, A, grid_ws, stream_), "k_batch_ws_guess launch");
     }
-    BCK(launch_batch_cg(fp64_, lanes_, unroll_, A, grid_cg_, stream_), "k_batch_cg launch");
+    if (gangs_ > 0) {
+        BCK(cudaMemsetAsync(d_gang_, 0, gang_zero_, stream_), "reset records");
+        GangArgs G = gang_args_;
+        G.scenes = d_desc_;
+        G.run = d_run_;
+        G.error = &d_sync_->error;
+        BCK(launch_gang_solve(G, gangs_, gang_smem_, stream_), "k_gang_solve32 launch");
+    } else {
+        BCK(launch_batch_cg(fp64_, lanes_, unroll_, A, grid_cg_, stream_), "k_batch_cg launch");
+    }
+    return PD_OK;
+}
+
+// The gangs of the solve: how many blocks to each, from the makespan of the
+// scenes (the largest first to the gang that is free first) with one scene's
+// iteration modelled as below, among the gang sizes whose shares of every scene
+// fit in shared memory.  No gangs: the phases of k_batch_cg.
+pd_status Batch::plan_gangs()
+{
+    gangs_ = 0;
+    const int ns = (int)eng_.size();
+    if (fp64_) return PD_OK;
+    struct Choice {
+        double time;
+        int gangs;
+    };
+    std::vector<Choice> choices;
+    std::vector<int> order(ns);
+    for (int s = 0; s < ns; ++s) order[s] = s;
+    std::sort(order.begin(), order.end(), [&](int a, int b) {
+        const long long x = eng_[a]->total_slots_, y = eng_[b]->total_slots_;
+        return x != y ? x > y : a < b;
+    });
+    for (int k = std::min(ns, sm_count_); k >= 1; --k) {
+        const int g = std::min(sm_count_ / k, 256);
+        bool fits = true;
+        std::vector<double> busy(k, 0.0);
+        for (int s : order) {
+            const Engine& e = *eng_[s];
+            const int rows = (e.n_ + g - 1) / g;
+            const double spacing = 2.0 * e.sim_.pd_particle_radius;
+            if (e.n_ > 0 && !cg_persist_may_fit(rows, spacing > 0 ? e.sim_.pd_horizon / spacing : 0.0, device_)) fits = false;
+            // us: two exchanges and the serial part, rows, bond slots (fitted to
+            // one-launch solves of 4k to 130k particles and 29 to 104 bonds each)
+            const double slots = e.n_ > 0 ? (double)e.total_slots_ / e.n_ : 0.0;
+            const double t = 3.3 + 0.008 * g + rows * (7.2e-3 + 0.42e-3 * slots);
+            *std::min_element(busy.begin(), busy.end()) += t;
+        }
+        if (fits) choices.push_back(Choice{*std::max_element(busy.begin(), busy.end()), k});
+    }
+    std::stable_sort(choices.begin(), choices.end(), [](const Choice& a, const Choice& b) { return a.time < b.time; });
+    std::vector<CgPersistPlan> plan(ns);
+    int tries = 0;
+    for (const Choice& c : choices) {
+        if (++tries > 4) break;
+        const int g = std::min(sm_count_ / c.gangs, 256);
+        bool all = true;
+        for (int s = 0; s < ns && all; ++s) {
+            pd_status st = eng_[s]->gang_tiles(std::max(1, (eng_[s]->n_ + g - 1) / g), g, &plan[s], &all);
+            if (st != PD_OK) {
+                err_ = "scene " + std::to_string(s) + ": " + eng_[s]->error();
+                return st;
+            }
+        }
+        if (all) {
+            gangs_ = c.gangs;
+            gang_ = g;
+            break;
+        }
+    }
+    if (gangs_ == 0) {
+        for (auto& e : eng_) e->gang_tiles_free();
+        return PD_OK;
+    }
+    std::vector<GangScene> gs(ns);
+    long long rec = 0;
+    gang_smem_ = 0;
+    for (int s = 0; s < ns; ++s) {
+        gs[s] = GangScene{plan[s].rows, plan[s].halo, plan[s].bonds, plan[s].lanes, rec};
+        rec += eng_[s]->n_;
+        gang_smem_ = std::max(gang_smem_, plan[s].smem);
+        h_desc_[s].S = eng_[s]->S_;
+    }
+    // one allocation: [records | inboxes | turns | counter] zeroed, [plan | order]
+    const size_t r16 = sizeof(ulonglong2);
+    const size_t inbox = 2 * (size_t)gang_ * gang_ * gangs_, turns = (size_t)gangs_ * (ns + 1);
+    gang_zero_ = r16 * ((size_t)rec + inbox + turns + 1);
+    const size_t plan_bytes = sizeof(GangScene) * ns;
+    BCK(cudaMalloc((void**)&d_gang_, gang_zero_ + plan_bytes + sizeof(int) * ns), "alloc gangs");
+    GangArgs& G = gang_args_;
+    G = GangArgs{};
+    G.rec = (ulonglong2*)d_gang_;
+    G.inbox = G.rec + rec;
+    G.turns = G.inbox + inbox;
+    G.next = (int*)(G.turns + turns);
+    G.plan = (const GangScene*)(d_gang_ + gang_zero_);
+    G.order = (const int*)(d_gang_ + gang_zero_ + plan_bytes);
+    G.n_scenes = ns;
+    G.gang = gang_;
+    BCK(cudaMemcpyAsync((void*)G.plan, gs.data(), plan_bytes, cudaMemcpyHostToDevice, stream_), "upload gangs");
+    BCK(cudaMemcpyAsync((void*)G.order, order.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, stream_), "upload gangs");
+    for (auto& e : eng_) BCK(cudaStreamSynchronize(e->stream_), "gang tiles sync");
+    BCK(cudaStreamSynchronize(stream_), "gang tiles sync");
     return PD_OK;
 }
 
@@ -321,6 +432,7 @@ pd_status Batch::ws_set_params(const float* params, size_t count)
 // scenes' own streams, waited for before the batch's next launch).
 pd_status Batch::relayout(int lanes, int unroll)
 {
+    if (gangs_ > 0) return PD_OK;
     for (auto& e : eng_) e->relayout_bonds(lanes, fp64_ ? 1 : unroll);
     for (auto& e : eng_) BCK(cudaStreamSynchronize(e->stream_), "relayout sync");
     return PD_OK;
@@ -331,6 +443,7 @@ pd_status Batch::relayout(int lanes, int unroll)
 pd_status Batch::tune()
 {
     std::vector<int> lanes_c = {4, 8}, unroll_c = {2, 4}, rows_c = {64, 128, 256, 512};
+    if (gangs_ > 0) lanes_c = {8}, unroll_c = {2};   // (the products outside the solve; the rows keep the gangs' bond order)
     if (opt_.lanes_per_particle) lanes_c = {opt_.lanes_per_particle};
     if (opt_.spmv_unroll || fp64_) unroll_c = {fp64_ ? 2 : opt_.spmv_unroll};
     if (opt_.item_rows) rows_c = {opt_.item_rows};
@@ -485,8 +598,10 @@ pd_status Batch::make_ready()
     BCK(cudaMemsetAsync(d_sync_, 0, sizeof(BatchSync), stream_), "reset barrier");
     BCK(cudaMemcpyAsync(d_run_, h_run_.data(), sizeof(SceneRun) * ns, cudaMemcpyHostToDevice, stream_), "upload run");
     grid_pre_ = std::max(1, batch_pre_blocks_per_sm(fp64_)) * sm_count_;
-    pd_status st = tune();
+    pd_status st = plan_gangs();
+    if (st == PD_OK) st = tune();
     if (st != PD_OK) return st;
+    if (gangs_ > 0) grid_cg_ = gangs_ * gang_;
     if (opt_.use_graph) {
         st = build_graph();
         if (st != PD_OK) return st;

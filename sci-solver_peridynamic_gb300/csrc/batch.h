@@ -6,6 +6,9 @@
 //   k_batch_pre  step start, rounds of { force pass ; adaptive decision ;
 //                rollback restore or backup }, CG set-up (b, x0, r0)
 //   k_batch_cg   CG iterations of every scene until all have converged, update
+// In mixed precision, where a share of every scene fits in a block's shared
+// memory, k_gang_solve32 (cg_persist.cu) takes the place of k_batch_cg: gangs of
+// blocks solve the scenes one after another.
 // With the learned warm start on, k_batch_pre ends with the features of every
 // solving scene, one network launch over the rows of all scenes follows, and
 // k_batch_ws_guess forms the learned guess, its residual and the guard before
@@ -93,6 +96,26 @@ struct BatchArgs {
     int tune_reps;         // > 0: only time the SpMV phase this many times
     int warm_start;        // 1: learned CG initial guess (mixed precision)
 };
+
+// A scene's part in k_gang_solve32 (cg_persist.cu).
+struct GangScene {
+    int rows, halo, bonds, lanes;   // of its CgPersistPlan
+    long long rec;                  // its first record
+};
+struct GangArgs {
+    SceneDesc* scenes;
+    SceneRun* run;
+    const GangScene* plan;
+    const int* order;       // scenes, the largest first
+    int n_scenes;
+    int gang;               // blocks per gang
+    int* next;              // scenes taken (0 before the launch)
+    ulonglong2* turns;      // [gangs][n_scenes + 1] (zero before the launch)
+    ulonglong2* inbox;      // [gangs][2][gang][gang] (zero before the launch)
+    ulonglong2* rec;        // a record per row (zero before the launch)
+    int* error;
+};
+cudaError_t launch_gang_solve(const GangArgs& A, int gangs, size_t smem, cudaStream_t st);
 
 // Launchers (batch.cu).  Both kernels are cooperative launches: `grid` must
 // not exceed the co-resident block count (blocks per SM x SMs).

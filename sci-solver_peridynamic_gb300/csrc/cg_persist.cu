@@ -30,7 +30,9 @@
 // thread records the error and its block returns, and so does every block that
 // sees the error.
 #include <algorithm>
+#include <cmath>
 
+#include "batch.h"
 #include "step_rows.cuh"
 
 namespace pdgb {
@@ -81,6 +83,20 @@ struct PersistArgs {
     int profile;
 };
 
+// A block's part in a solve.
+struct PersistRun {
+    ulonglong2* rec;
+    ulonglong2* inbox;
+    int rows, halo, bonds, max_iters;
+    int block, grid;            // this block among those of the solve
+    int* error;                 // set when a wait ran out of time
+};
+__device__ __forceinline__ PersistRun persist_run(const PersistArgs& A)
+{
+    return PersistRun{A.rec, A.inbox, A.rows, A.halo, A.bonds, A.max_iters, (int)blockIdx.x, (int)gridDim.x,
+                      &A.S.sc->wait_error};
+}
+
 // Sums travel as their accumulator's own form: double-float for FP32 data.
 __device__ __forceinline__ unsigned long long pack(DF v)
 {
@@ -119,7 +135,7 @@ struct Exchange {
 // Polls a record until `arrived` accepts it; false when the wait ran out of
 // time (here or in another thread).
 template <typename Ok>
-__device__ __forceinline__ bool await(const ulonglong2* rec, CgScalars* sc, Exchange& e, ulonglong2& r, Ok arrived)
+__device__ __forceinline__ bool await(const ulonglong2* rec, int* error, Exchange& e, ulonglong2& r, Ok arrived)
 {
     r = observe(rec);
     if (arrived(r)) return true;
@@ -129,8 +145,8 @@ __device__ __forceinline__ bool await(const ulonglong2* rec, CgScalars* sc, Exch
         r = observe(rec);
         if (arrived(r)) return true;
         if ((++spins & 255u) == 0) {
-            if (((volatile CgScalars*)sc)->wait_error || now_ns() - t0 > kPersistTimeoutNs) {
-                ((volatile CgScalars*)sc)->wait_error = 1;
+            if (*(volatile int*)error || now_ns() - t0 > kPersistTimeoutNs) {
+                *(volatile int*)error = 1;
                 e.error = 1;
                 return false;
             }
@@ -143,11 +159,11 @@ __device__ __forceinline__ bool await(const ulonglong2* rec, CgScalars* sc, Exch
 // poll the inbox run help(thread, threads) meanwhile.  Returns false when a
 // wait ran out of time.
 template <typename T, typename Help>
-__device__ __forceinline__ bool exchange_sum(Exchange& e, T& v, int step, const PersistArgs& A, unsigned long long epoch,
+__device__ __forceinline__ bool exchange_sum(Exchange& e, T& v, int step, const PersistRun& A, unsigned long long epoch,
                                              Help help)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int grid = gridDim.x;
+    const int grid = A.grid;
     const int polling = (grid + 31) / 32 * 32;   // threads with an inbox record, in whole warps
     warp_sum(v, step);
     if (lane == 0) e.warp[warp] = pack(v);
@@ -159,9 +175,9 @@ __device__ __forceinline__ bool exchange_sum(Exchange& e, T& v, int step, const 
         const int b = threadIdx.x;
         if (b < grid) {
             ulonglong2* box = A.inbox + (size_t)(epoch & 1) * grid * grid;
-            publish(box + (size_t)b * grid + blockIdx.x, pack(t), epoch);
+            publish(box + (size_t)b * grid + A.block, pack(t), epoch);
             ulonglong2 r;
-            await(box + (size_t)blockIdx.x * grid + b, A.S.sc, e, r, [epoch](const ulonglong2& x) { return x.y == epoch; });
+            await(box + (size_t)A.block * grid + b, A.error, e, r, [epoch](const ulonglong2& x) { return x.y == epoch; });
             e.from[b] = r.x;
         }
     } else {
@@ -238,18 +254,17 @@ __device__ __forceinline__ void load_bonds(const DeviceState& S, int slot, int (
 // k_bank_order take an iteration at 100k particles (76 bonds) from 38.2 us to
 // 31.2; with 8 lanes per row 34.9 (37.5 without the order), with 1024 threads
 // 30.3 (but 24.0 against 21.8 at 50k and 104 bonds).
+// `epoch` is the last epoch used in the inbox and the records.  Blocks beyond the
+// last row only exchange.  Returns false when a wait ran out of time.
 template <bool CACHED, int G, int U>
-__global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist32(PersistArgs A)
+__device__ __forceinline__ bool persist_solve32(const StepParams& P, const DeviceState& S, const PersistRun& A,
+                                                unsigned char* smem, Exchange& ex, unsigned long long& epoch, bool timed)
 {
-    CgScalars* sc = A.S.sc;
+    CgScalars* sc = S.sc;
     // (the scalars change only after every block's last exchange)
-    if (((volatile CgScalars*)sc)->done) return;
-    extern __shared__ __align__(32) unsigned char smem[];
-    __shared__ Exchange ex;
-    const StepParams& P = A.P;
-    const DeviceState& S = A.S;
-    const int lo = blockIdx.x * A.rows;
-    const int nr = min(A.rows, P.n - lo);
+    if (((volatile CgScalars*)sc)->done) return true;
+    const int lo = A.block * A.rows;
+    const int nr = max(0, min(A.rows, P.n - lo));
     float4* sx = (float4*)smem;
     float4* sr = sx + A.rows;
     float4* sp = sr + A.rows;
@@ -267,7 +282,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist32(PersistArgs
     const int lane = threadIdx.x & (G - 1);
     const unsigned gmask = group_mask<G>();
     constexpr int NG = kPersistThreads / G;
-    const int first = CACHED ? S.row_ptr[lo] : 0;
+    const int first = CACHED && nr > 0 ? S.row_ptr[lo] : 0;
     for (int t = threadIdx.x; t < nr; t += kPersistThreads) {
         const int p = lo + t;
         sx[t] = ((const float4*)S.sol)[p];
@@ -277,7 +292,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist32(PersistArgs
         scnt[t] = is_dirichlet(ab & kActMask) ? -1 : S.cnt[p] << 8 | ab;
         srow[t] = S.row_ptr[p] - first;
     }
-    const int h0 = S.halo_ptr[blockIdx.x], nh = S.halo_ptr[blockIdx.x + 1] - h0;
+    const int h0 = nr > 0 ? S.halo_ptr[A.block] : 0, nh = nr > 0 ? S.halo_ptr[A.block + 1] - h0 : 0;
     for (int h = threadIdx.x; h < nh; h += kPersistThreads) {
         const int q = S.halo[h0 + h];
         sq[h] = q;
@@ -308,9 +323,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist32(PersistArgs
     int iter = sc->iter;
     bool done = false, converged = false;
 
-    unsigned long long epoch = A.epoch;
     unsigned long long t_mark = 0, ns_spmv = 0, ns_vec = 0;
-    const bool timed = A.profile && blockIdx.x == 0 && threadIdx.x == 0;
     DF pAp{0.f, 0.f};
     for (int it = 0; it < A.max_iters && !done; ++it) {
         if (timed) t_mark = now_ns();
@@ -383,7 +396,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist32(PersistArgs
             if (lane == 0) sp[i] = w;
         }
         pAp = acc.v;
-        if (!exchange_sum(ex, pAp, G, A, ++epoch, [](int, int) {})) return;
+        if (!exchange_sum(ex, pAp, G, A, ++epoch, [](int, int) {})) return false;
         alpha = df_quotient(rz, pAp);
         if (timed) {
             const unsigned long long t = now_ns();
@@ -412,13 +425,13 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist32(PersistArgs
         const auto gather = [&](int t, int threads) {   // the halo's new r
             for (int h = t; h < nh; h += threads) {
                 ulonglong2 v;
-                if (!await(A.rec + sq[h], sc, ex, v, [tag](const ulonglong2& x) { return (unsigned)(x.y >> 32) == tag; }))
+                if (!await(A.rec + sq[h], A.error, ex, v, [tag](const ulonglong2& x) { return (unsigned)(x.y >> 32) == tag; }))
                     return;
                 const DF yx = unpack<DF>(v.x);
                 sh[h] = make_float4(yx.lo, yx.hi, __uint_as_float((unsigned)v.y), 0.f);
             }
         };
-        if (!exchange_sum(ex, total, G, A, epoch, gather)) return;
+        if (!exchange_sum(ex, total, G, A, epoch, gather)) return false;
         beta = df_quotient(total, rz);
         rz = total;
         ++iter;
@@ -431,7 +444,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist32(PersistArgs
         ((float4*)S.r)[lo + t] = sr[t];
         ((float4*)S.p)[lo + t] = sp[t];
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (A.block == 0 && threadIdx.x == 0) {
         sc->pAp = df_to_double(pAp);
         sc->rz = df_to_double(rz);
         sc->alpha = alpha;
@@ -443,6 +456,16 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist32(PersistArgs
         sc->ns_spmv = (double)ns_spmv;
         sc->ns_vec = (double)ns_vec;
     }
+    return true;
+}
+
+template <bool CACHED, int G, int U>
+__global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist32(PersistArgs A)
+{
+    extern __shared__ __align__(32) unsigned char smem[];
+    __shared__ Exchange ex;
+    unsigned long long epoch = A.epoch;
+    persist_solve32<CACHED, G, U>(A.P, A.S, persist_run(A), smem, ex, epoch, A.profile && blockIdx.x == 0 && threadIdx.x == 0);
 }
 
 // One product y = A w outside a solve by the same rows and halos, bonds read as
@@ -538,6 +561,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist64(PersistArgs
     if (((volatile CgScalars*)sc)->done) return;
     extern __shared__ __align__(32) unsigned char smem[];
     __shared__ Exchange ex;
+    const PersistRun run = persist_run(A);
     __shared__ double s_alpha, s_beta, s_rz;
     __shared__ int s_done, s_converged;
     const StepParams& P = A.P;
@@ -664,7 +688,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist64(PersistArgs
             }
         }
         pAp = acc;
-        if (!exchange_sum(ex, pAp, 1, A, ++epoch, [](int, int) {})) return;
+        if (!exchange_sum(ex, pAp, 1, run, ++epoch, [](int, int) {})) return;
         if (threadIdx.x == 0) s_alpha = s_rz / pAp;
         __syncthreads();
         if (timed) {
@@ -695,11 +719,11 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist64(PersistArgs
             for (int h = t; h < nh; h += threads) {
                 const ulonglong2* rec = A.rec + 2 * (size_t)sq[h];
                 ulonglong2 a, b;
-                if (!await(rec, sc, ex, a, arrived) || !await(rec + 1, sc, ex, b, arrived)) return;
+                if (!await(rec, run.error, ex, a, arrived) || !await(rec + 1, run.error, ex, b, arrived)) return;
                 sh[h] = Vec3d{unpack<double>(a.x), unpack<double>((b.y << 32) | (a.y & 0xffffffffull)), unpack<double>(b.x)};
             }
         };
-        if (!exchange_sum(ex, rr, 1, A, epoch, gather)) return;
+        if (!exchange_sum(ex, rr, 1, run, epoch, gather)) return;
         ++iter;
         if (threadIdx.x == 0) {
             s_beta = rr / s_rz;
@@ -726,6 +750,69 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist64(PersistArgs
         sc->done = s_done;
         sc->ns_spmv = (double)ns_spmv;
         sc->ns_vec = (double)ns_vec;
+    }
+}
+
+// The solves and updates of a batch's scenes (batch.h) in one cooperative launch.
+// The blocks form gangs of A.gang; a gang takes the next scene of the list
+// (largest first) when it has finished one, solves it as k_cg_persist32 does, and
+// advances its rows.  Scenes meet no barrier of other scenes, and each runs only
+// its own iterations.  Every block of a gang takes part in every exchange, so
+// the epochs of its inbox go on from scene to scene; which scene comes next is
+// a record of its own per turn.  Against phases of all scenes between grid
+// barriers (k_batch_cg): 12 steps of 24 bodies of 4k to 24k particles take 97 ms
+// against 226, of 8 of 1k to 4k 13.5 against 65.
+__global__ void __launch_bounds__(kPersistThreads, 1) k_gang_solve32(GangArgs A)
+{
+    extern __shared__ __align__(32) unsigned char smem[];
+    __shared__ Exchange ex;
+    __shared__ int s_turn;
+    const int gang = blockIdx.x / A.gang, block = blockIdx.x % A.gang;
+    ulonglong2* inbox = A.inbox + (size_t)gang * 2 * A.gang * A.gang;
+    ulonglong2* turns = A.turns + (size_t)gang * (A.n_scenes + 1);
+    unsigned long long epoch = 0;
+    for (int turn = 0; turn <= A.n_scenes; ++turn) {
+        if (threadIdx.x == 0) {
+            if (block == 0) {
+                const int i = atomicAdd(A.next, 1);
+                s_turn = i < A.n_scenes ? A.order[i] : A.n_scenes;
+                publish(turns + turn, (unsigned long long)s_turn, 1ull);
+            } else {
+                ulonglong2 r;
+                s_turn = await(turns + turn, A.error, ex, r, [](const ulonglong2& x) { return x.y == 1ull; }) ? (int)r.x
+                                                                                                          : A.n_scenes;
+            }
+        }
+        __syncthreads();
+        const int scene = s_turn;
+        __syncthreads();
+        if (scene >= A.n_scenes) return;
+        SceneRun& R = A.run[scene];
+        if (!*(volatile int*)&R.solving) continue;
+        const SceneDesc& D = A.scenes[scene];
+        const GangScene g = A.plan[scene];
+        const StepParams P = D.P;
+        const DeviceState S = D.S;
+        const PersistRun run{A.rec + g.rec, inbox, g.rows, g.halo, g.bonds, 0x7fffffff, block, A.gang, A.error};
+        bool ok;
+        if (g.bonds == 0) ok = persist_solve32<false, kTileLanes, 4>(P, S, run, smem, ex, epoch, false);
+        else if (g.lanes == 4) ok = persist_solve32<true, 4, 4>(P, S, run, smem, ex, epoch, false);
+        else if (g.lanes == 8) ok = persist_solve32<true, 8, 4>(P, S, run, smem, ex, epoch, false);
+        else if (g.lanes == 16) ok = persist_solve32<true, 16, 4>(P, S, run, smem, ex, epoch, false);
+        else ok = persist_solve32<true, 32, 2>(P, S, run, smem, ex, epoch, false);
+        if (!ok) return;
+        __syncthreads();   // the block's rows of the solution
+        const int lo = block * g.rows, hi = min(P.n, lo + g.rows);
+        for (int r = lo + (int)threadIdx.x; r < hi; r += kPersistThreads) update_elem<false>(P, S, r);
+        if (block == 0 && threadIdx.x == 0) {
+            const volatile CgScalars* sc = S.sc;
+            R.last_iters = sc->iter;
+            R.total_iters += sc->iter;
+            R.last_res = sc->rnorm;
+            R.last_tol = sc->tol;
+            if (!sc->converged) R.cg_converged = 0;
+            R.sim_time += P.h;
+        }
     }
 }
 
@@ -815,6 +902,23 @@ bool cg_persist_plan(bool fp64, int max_halo, int max_bonds, int device, CgPersi
             }
     *plan = pl;
     return true;
+}
+
+bool cg_persist_may_fit(int rows, double reach, int device)
+{
+    int optin = 0;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    const double side = std::cbrt((double)rows) + 2.0 * reach;   // a compact block of rows and its halo
+    return persist_smem(false, rows, (int)std::min(side * side * side, 1e6), 0) <= (size_t)(optin - (int)sizeof(Exchange) - 1024);
+}
+
+cudaError_t launch_gang_solve(const GangArgs& A, int gangs, size_t smem, cudaStream_t st)
+{
+    GangArgs a = A;
+    void* args[] = {&a};
+    cudaError_t e = cudaFuncSetAttribute((const void*)k_gang_solve32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    return cudaLaunchCooperativeKernel((const void*)k_gang_solve32, dim3(gangs * A.gang), dim3(kPersistThreads), args, smem, st);
 }
 
 cudaError_t launch_tile_product(const StepParams& P, const DeviceState& S, const CgPersistPlan& plan, const void* in,

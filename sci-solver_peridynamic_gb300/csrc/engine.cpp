@@ -572,6 +572,40 @@ pd_status Engine::persist_prepare()
     return PD_OK;
 }
 
+// A batch scene's tiles of `rows` rows for the gangs' solve (mixed precision;
+// k_gang_solve32), and its rows' bond order; *fits is false (and nothing kept)
+// when a block's share does not fit.
+pd_status Engine::gang_tiles(int rows, int blocks, CgPersistPlan* plan, bool* fits)
+{
+    *plan = CgPersistPlan{};
+    *fits = true;
+    if (n_ <= 0) return PD_OK;
+    int max_halo = 0, unfit = 0;
+    if (!S_.lidx) CK(dalloc(&S_.lidx, (size_t)std::max<long long>(total_slots_, 1)), "alloc local indices");
+    S_.tile_rows = plan->rows = rows;
+    plan->grid = blocks;
+    CK(build_tiles(S_, n_, &max_halo, &unfit, stream_), "build tiles");
+    launches_ += 2;
+    *fits = unfit == 0 && cg_persist_plan(false, max_halo, sim_.pd_max_num_bonds, device_, plan);
+    if (!*fits) {
+        gang_tiles_free();
+        return PD_OK;
+    }
+    if (plan->bonds == 0) {
+        CK(launch_bank_order(S_, n_, plan->lanes, 4, total_slots_, stream_), "order bonds");
+        launch_bond_geometry(S_, (int)std::min<long long>(((long long)n_ + kBlock - 1) / kBlock, kMaxPartials), stream_);
+        launches_ += 2;
+    }
+    return PD_OK;
+}
+
+void Engine::gang_tiles_free()
+{
+    if (S_.lidx) cudaFree(S_.lidx);
+    S_.lidx = nullptr;
+    free_tiles(S_);
+}
+
 // The tiles' halos and local indices of the CSR rows as they are.  A body
 // whose blocks' halos no longer fit (a checkpoint in another slot order) leaves
 // the one-launch solve.

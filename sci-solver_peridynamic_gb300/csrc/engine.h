@@ -73,6 +73,8 @@ private:
     // y = A in with this handle's product (lattice stencil or CSR rows)
     void apply_op(const StepParams& P, const void* in, void* out, ReduceSlot slot, double* dot_out);
     pd_status persist_prepare();
+    pd_status gang_tiles(int rows, int blocks, CgPersistPlan* plan, bool* fits);
+    void gang_tiles_free();
     pd_status build_halos();
     void lattice_resync(bool force);   // the lattice product's 1/d0 table from the live CSR bonds
     // mixed mode: reorders every row's live bonds for the (g, u) SpMV shape

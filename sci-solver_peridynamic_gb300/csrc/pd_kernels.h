@@ -277,6 +277,9 @@ CgPersistPlan cg_persist_rows(bool fp64, int n, int sm_count, int device);
 // of plan->rows) and the largest row; false when a block's share does not
 // fit in shared memory
 bool cg_persist_plan(bool fp64, int max_halo, int max_bonds, int device, CgPersistPlan* plan);
+// whether a compact block of `rows` rows with neighbours within `reach` spacings
+// is likely to fit (mixed precision, before its halo is known)
+bool cg_persist_may_fit(int rows, double reach, int device);
 // At most max_iters iterations from the state of S (x, r, p and the scalars,
 // as the residual kernel or an earlier launch left them).  rec: n records (FP64:
 // 2 n); inbox: 2 x grid^2 records; epoch: no smaller than any epoch of earlier
