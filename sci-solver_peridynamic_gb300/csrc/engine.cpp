@@ -467,7 +467,14 @@ pd_status Engine::tune_spmv()
     if (cand.size() == 1 || n_ < 20000 || persist_.tiled_products) {
         // small problems: launch overhead dominates, keep the default (the
         // tiled path when it was asked for)
-        Cand c = cand.size() == 1 ? cand[0] : Cand{0, 8, fp64_ ? 1 : 2};
+        // As many lanes per row as one block per SM holds: FP64 10.4 us at 500
+        // particles with 32 lanes (14.8 with 8), 13.1 at 2000 with 16 (18.0), 35.0 at
+        // 18k with 4 (49.4); mixed precision 8.4 at 500 with 16 (10.3 with 8), but
+        // 10.4 at 4096 with either and 10.5 (12.4) at 8000: never below 8.
+        int lanes = 32;
+        while (lanes > (fp64_ ? 4 : 8) && (long long)n_ * lanes > (long long)sm_count_ * kBlock) lanes /= 2;
+        if (!fp64_ && lanes == 32) lanes = 16;   // (as fast, and fewer shuffles)
+        Cand c = cand.size() == 1 ? cand[0] : Cand{0, lanes, fp64_ ? 1 : 2};
         if (lat_ok_ && opt_.spmv_path == 3) c = Cand{0, 1, 1, 1};
         if (opt_.spmv_path == 1 && can_tile && cand.size() > 1) c = Cand{1, fixed_lanes ? fixed_lanes : 8, fixed_unroll ? fixed_unroll : 2};
         apply(c);

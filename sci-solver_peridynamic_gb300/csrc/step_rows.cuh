@@ -605,15 +605,63 @@ __device__ __forceinline__ void spmv_row(const StepParams& P, const DeviceState&
     const int rs = S.row_ptr[p];
     const int cn = S.cnt[p];
     Real ax = 0, ay = 0, az = 0;
-    if (FP64) {
-        for (int j = lane; j < cn; j += G) {
-            const int q = S.col[rs + j];
-            const V4 wq = ld_in<LD>(in + q);
-            const double* J = S.jac + 6ll * (rs + j);
-            ax += J[0] * wq.x + J[3] * wq.y + J[4] * wq.z;
-            ay += J[3] * wq.x + J[1] * wq.y + J[5] * wq.z;
-            az += J[4] * wq.x + J[5] * wq.y + J[2] * wq.z;
+    if constexpr (FP64) {
+        // Bound by the FP64 pipe (9 multiply-adds per bond, 527 G/s: 178 us at 100k
+        // particles of 104 bonds) and by the latency of the Jacobians, which a row
+        // reads once: xx yy | zz xy | xz yz in three 16-byte loads, two bonds in
+        // flight.  209 us there, against 335 with one bond in flight, 8-byte loads
+        // and the row finished by one lane.
+        const auto load = [&](int j, double2& a, double2& b, double2& c, V4& wq) {
+            const double2* J = (const double2*)(S.jac + 6ll * (rs + j));
+            a = __ldcs(J);
+            b = __ldcs(J + 1);
+            c = __ldcs(J + 2);
+            wq = ld_in<LD>(in + __ldcs(S.col + rs + j));
+        };
+        const auto add = [&](const double2& a, const double2& b, const double2& c, const V4& wq) {
+            ax = fma(a.x, wq.x, fma(b.y, wq.y, fma(c.x, wq.z, ax)));
+            ay = fma(b.y, wq.x, fma(a.y, wq.y, fma(c.y, wq.z, ay)));
+            az = fma(c.x, wq.x, fma(c.y, wq.y, fma(b.x, wq.z, az)));
+        };
+        int j = lane;
+        for (; j + G < cn; j += 2 * G) {
+            double2 a0, b0, c0, a1, b1, c1;
+            V4 w0, w1;
+            load(j, a0, b0, c0, w0);
+            load(j + G, a1, b1, c1, w1);
+            add(a0, b0, c0, w0);
+            add(a1, b1, c1, w1);
         }
+        if (j < cn) {
+            double2 a0, b0, c0;
+            V4 w0;
+            load(j, a0, b0, c0, w0);
+            add(a0, b0, c0, w0);
+        }
+        // The sums by halving: after two steps lane & 3 holds one component (3:
+        // none), so an FP64 instruction of the rest serves all three.
+        static_assert(G >= 4, "a lane per component");
+        const bool hi = lane & 2, odd = lane & 1;
+        const double first = (hi ? az : ax) + __shfl_xor_sync(gmask, hi ? ax : az, 2);
+        const double second = __shfl_xor_sync(gmask, hi ? ay : 0.0, 2) + (hi ? 0.0 : ay);
+        double v = (odd ? second : first) + __shfl_xor_sync(gmask, odd ? first : second, 1);
+#pragma unroll
+        for (int off = 4; off < G; off <<= 1) v += __shfl_xor_sync(gmask, v, off);
+        if (lane < 4) {
+            const double* D = S.jdiag + 6ll * p;
+            double y = 0.0;
+            if (lane < 3) {
+                // row `lane` of the symmetric diagonal block
+                const double k = fma(D[lane == 0 ? 0 : lane + 2], w.x,
+                                     fma(D[lane == 0 ? 3 : lane == 1 ? 1 : 5], w.y,
+                                         fma(D[lane == 0 ? 4 : lane == 1 ? 5 : 2], w.z, -v)));
+                const double wc = lane == 0 ? w.x : lane == 1 ? w.y : w.z;
+                y = fma(t2, k, m * wc);
+                if (DOT) acc.fma(wc, y);
+            }
+            ((double*)(out + p))[lane] = y;
+        }
+        return;
     } else {
         // per bond: the column index and 1/d0 stream in coalesced; the
         // neighbour's supercell position and its CG entry are gathered
@@ -655,46 +703,7 @@ __device__ __forceinline__ void spmv_row(const StepParams& P, const DeviceState&
                                     qq, id0, ax, ay, az);
         }
     }
-    if constexpr (!FP64) {
-        spmv_finish_mixed<G, DOT>(P, S, p, ab, w, ax, ay, az, lane, gmask, out, acc);
-        return;
-    }
-    ax = group_sum<G>(ax, gmask);
-    ay = group_sum<G>(ay, gmask);
-    az = group_sum<G>(az, gmask);
-    if (lane == 0) {
-        Real kx, ky, kz;
-        if (FP64) {
-            const double* D = S.jdiag + 6ll * p;
-            kx = D[0] * w.x + D[3] * w.y + D[4] * w.z - ax;
-            ky = D[3] * w.x + D[1] * w.y + D[5] * w.z - ay;
-            kz = D[4] * w.x + D[5] * w.y + D[2] * w.z - az;
-        } else {
-            kx = c * ax; ky = c * ay; kz = c * az;
-            if (ab & kActContact) {
-                const float4 Xp = S.X32[p];
-                const float4 Up = S.u32[p];
-                const float dx = Xp.x + Up.x - (float)P.sphere_c_local[0];
-                const float dy = Xp.y + Up.y - (float)P.sphere_c_local[1];
-                const float dz = Xp.z + Up.z - (float)P.sphere_c_local[2];
-                const float inv = rsqrtf(dx * dx + dy * dy + dz * dz);
-                const float nx = dx * inv, ny = dy * inv, nz = dz * inv;
-                const float kn = (float)P.sphere_k * (nx * (float)w.x + ny * (float)w.y + nz * (float)w.z);
-                kx += kn * nx; ky += kn * ny; kz += kn * nz;
-            }
-        }
-        const Real yx = m * (Real)w.x + t2 * kx;
-        const Real yy = m * (Real)w.y + t2 * ky;
-        const Real yz = m * (Real)w.z + t2 * kz;
-        V4 yv;
-        yv.x = yx; yv.y = yy; yv.z = yz; yv.w = 0;
-        out[p] = yv;
-        if (DOT) {
-            acc.fma(w.x, yx);
-            acc.fma(w.y, yy);
-            acc.fma(w.z, yz);
-        }
-    }
+    if constexpr (!FP64) spmv_finish_mixed<G, DOT>(P, S, p, ab, w, ax, ay, az, lane, gmask, out, acc);
 }
 
 // ---- CG vector bodies (CUSP krylov::cg, identity preconditioner) -----------------
