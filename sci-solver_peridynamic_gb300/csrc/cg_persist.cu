@@ -671,18 +671,11 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist64(PersistArgs
                 if (lane < 3) ((double*)(sy + i))[lane] = 0.0;
                 continue;
             }
-            ax = group_sum<G>(ax, gmask);
-            ay = group_sum<G>(ay, gmask);
-            az = group_sum<G>(az, gmask);
-            if (lane < 3) {   // one component per lane: a third of the FP64 instructions
-                const double* D = S.jdiag + 6ll * p;
+            const double s = component_sum<G>(ax, ay, az, lane, gmask);
+            if (lane < 3) {
                 const Vec3d w = sp[i];
-                const double d0 = D[lane == 0 ? 0 : lane == 1 ? 3 : 4], d1 = D[lane == 0 ? 3 : lane == 1 ? 1 : 5],
-                             d2 = D[lane == 0 ? 4 : lane == 1 ? 5 : 2];
-                const double s = lane == 0 ? ax : lane == 1 ? ay : az;
-                const double wk = lane == 0 ? w.x : lane == 1 ? w.y : w.z;
-                const double k = fma(d0, w.x, fma(d1, w.y, fma(d2, w.z, -s)));
-                const double y = fma(P.t2, k, P.mass * wk);
+                double wk;
+                const double y = fp64_row_result(P, S, p, lane, w.x, w.y, w.z, s, wk);
                 ((double*)(sy + i))[lane] = y;
                 acc = fma(wk, y, acc);
             }

@@ -361,8 +361,12 @@ pd_status Engine::make_ready()
     // 4 blocks per SM: the CG vector kernels measured 0.090 of the 1M step
     // against 0.099 at 8, 0.097 at 2 and 0.125 at 16
     L_.grid_vec = (int)std::max<long long>(1, std::min<long long>({need_vec, (long long)sm_count_ * 4, (long long)kMaxPartials}));
-    // 4 lanes per row: at 1M particles 1.25 ms per force pass against 1.74 (8) and 2.9 (16)
-    L_.force_lanes = 4;
+    // as many lanes per row as one block per SM holds (mixed precision: 34.0 us
+    // at 512 particles with 4, 21.0 with 32, 35.3 and 23.1 with 16 at 1500; FP64:
+    // 200 us and 39), at least 4 (1.25 ms at 1M against 1.74 with 8), FP64 at least
+    // 8 (1025 us at 30k with 4, 833 with 8)
+    L_.force_lanes = 32;
+    while (L_.force_lanes > (fp64_ ? 8 : 4) && (long long)n * L_.force_lanes > (long long)sm_count_ * kBlock) L_.force_lanes /= 2;
     L_.grid_force = grid_for_rows(L_.force_lanes, force_kernel_blocks_per_sm(fp64_, L_.force_lanes));
     if (!fp64_ && n > 0) {   // supercell positions of the initial state (read by the SpMV)
         launch_refresh(fp64_, step_params(), S_, L_, stream_);

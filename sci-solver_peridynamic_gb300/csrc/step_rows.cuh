@@ -585,6 +585,34 @@ __device__ __forceinline__ void mixed_bond_chunk(const float4* __restrict__ xs4,
     }
 }
 
+// A group's sums of three components by halving: after two steps lane & 3 holds
+// one component (3: none), so that an FP64 instruction of the rest of the row
+// serves all three.
+template <int G>
+__device__ __forceinline__ double component_sum(double ax, double ay, double az, int lane, unsigned gmask)
+{
+    static_assert(G >= 4, "a lane per component");
+    const bool hi = lane & 2, odd = lane & 1;
+    const double first = (hi ? az : ax) + __shfl_xor_sync(gmask, hi ? ax : az, 2);
+    const double second = __shfl_xor_sync(gmask, hi ? ay : 0.0, 2) + (hi ? 0.0 : ay);
+    double v = (odd ? second : first) + __shfl_xor_sync(gmask, odd ? first : second, 1);
+#pragma unroll
+    for (int off = 4; off < G; off <<= 1) v += __shfl_xor_sync(gmask, v, off);
+    return v;
+}
+
+// Component k (0 to 2) of an FP64 row's result from the sum over its bonds; wk
+// receives that component of w.
+__device__ __forceinline__ double fp64_row_result(const StepParams& P, const DeviceState& S, int p, int k, double wx,
+                                                  double wy, double wz, double sum, double& wk)
+{
+    const double* D = S.jdiag + 6ll * p;   // xx yy zz xy xz yz
+    const double d = fma(D[k == 0 ? 0 : k + 2], wx,
+                         fma(D[k == 0 ? 3 : k == 1 ? 1 : 5], wy, fma(D[k == 0 ? 4 : k == 1 ? 5 : 2], wz, -sum)));
+    wk = k == 0 ? wx : k == 1 ? wy : wz;
+    return fma(P.t2, d, P.mass * wk);
+}
+
 // y_p = (A w)_p by particle p's G-lane group: mass + (beta h^2) stiffness with
 // Dirichlet rows projected out.  DOT: lane 0 adds w_p . y_p to acc.
 // LD: load path of the positions and of w (kLd*).
@@ -638,25 +666,12 @@ __device__ __forceinline__ void spmv_row(const StepParams& P, const DeviceState&
             load(j, a0, b0, c0, w0);
             add(a0, b0, c0, w0);
         }
-        // The sums by halving: after two steps lane & 3 holds one component (3:
-        // none), so an FP64 instruction of the rest serves all three.
-        static_assert(G >= 4, "a lane per component");
-        const bool hi = lane & 2, odd = lane & 1;
-        const double first = (hi ? az : ax) + __shfl_xor_sync(gmask, hi ? ax : az, 2);
-        const double second = __shfl_xor_sync(gmask, hi ? ay : 0.0, 2) + (hi ? 0.0 : ay);
-        double v = (odd ? second : first) + __shfl_xor_sync(gmask, odd ? first : second, 1);
-#pragma unroll
-        for (int off = 4; off < G; off <<= 1) v += __shfl_xor_sync(gmask, v, off);
+        const double sum = component_sum<G>(ax, ay, az, lane, gmask);
         if (lane < 4) {
-            const double* D = S.jdiag + 6ll * p;
             double y = 0.0;
             if (lane < 3) {
-                // row `lane` of the symmetric diagonal block
-                const double k = fma(D[lane == 0 ? 0 : lane + 2], w.x,
-                                     fma(D[lane == 0 ? 3 : lane == 1 ? 1 : 5], w.y,
-                                         fma(D[lane == 0 ? 4 : lane == 1 ? 5 : 2], w.z, -v)));
-                const double wc = lane == 0 ? w.x : lane == 1 ? w.y : w.z;
-                y = fma(t2, k, m * wc);
+                double wc;
+                y = fp64_row_result(P, S, p, lane, w.x, w.y, w.z, sum, wc);
                 if (DOT) acc.fma(wc, y);
             }
             ((double*)(out + p))[lane] = y;
