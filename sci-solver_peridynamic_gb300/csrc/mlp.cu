@@ -77,20 +77,48 @@ __global__ void k_gelu_back(const float* __restrict__ dH, const float* __restric
         dZ[i] = __float2bfloat16_rn(dH[i] * gelu_grad(Z[i]));
 }
 
-// column sums of a BF16 [M x N] matrix into f32 (bias gradients)
-__global__ void k_colsum(const __nv_bfloat16* __restrict__ X, int M, int N, int ldx, float* __restrict__ out)
+// Column sums of rows [z rows_per, (z + 1) rows_per) of a BF16 [M x N] matrix
+// into out[z][N] (bias gradients); N <= 128, two threads per column.
+__global__ void __launch_bounds__(256) k_colsum_slices(const __nv_bfloat16* __restrict__ X, int M, int N, int ldx,
+                                                       int rows_per, float* __restrict__ out)
 {
-    const int c = blockIdx.x;
+    __shared__ float sh[128];
+    const int c = threadIdx.x & 127, half = threadIdx.x >> 7;
+    const int r0 = blockIdx.x * rows_per, r1 = min(M, r0 + rows_per);
     float s = 0.f;
-    for (int r = threadIdx.x; r < M; r += blockDim.x) s += __bfloat162float(X[(size_t)r * ldx + c]);
-    __shared__ float sh[256];
-    sh[threadIdx.x] = s;
+    if (c < N)
+        for (int r = r0 + half; r < r1; r += 2) s += __bfloat162float(X[(size_t)r * ldx + c]);
+    if (half) sh[c] = s;
     __syncthreads();
-    for (int off = blockDim.x / 2; off > 0; off >>= 1) {
-        if ((int)threadIdx.x < off) sh[threadIdx.x] += sh[threadIdx.x + off];
-        __syncthreads();
+    if (!half && c < N) out[(size_t)blockIdx.x * N + c] = s + sh[c];
+}
+
+// The sums of the slices, in order;
+// the first count_a values go to a, the rest to b (a layer's weight and bias
+// gradients).
+__global__ void __launch_bounds__(256) k_sum_slices(const float* __restrict__ wa, int count_a, int slices_a,
+                                                    const float* __restrict__ wb, int count_b, int slices_b,
+                                                    float* __restrict__ a, float* __restrict__ b)
+{
+    // (a warp reads 32 consecutive values of a slice; the block's 8 warps take a run of slices each)
+    __shared__ float sh[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
+    const bool is_a = i < count_a;
+    const int j = is_a ? i : i - count_a;
+    const bool in = is_a || j < count_b;
+    const float* p = is_a ? wa + j : wb + j;
+    const int stride = is_a ? count_a : count_b, slices = is_a ? slices_a : slices_b;
+    const int per = (slices + 7) / 8, z1 = min(slices, (warp + 1) * per);
+    float s = 0.f;
+    if (in)
+        for (int z = warp * per; z < z1; ++z) s += p[(size_t)z * stride];
+    sh[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && in) {
+        for (int w = 1; w < 8; ++w) s += sh[w][lane];
+        (is_a ? a : b)[j] = s;
     }
-    if (threadIdx.x == 0 && c < N) out[c] = sh[0];
 }
 
 // Adam on the FP32 master parameters, refreshing the BF16 weight copies
@@ -166,6 +194,30 @@ void mlp_forward(const MlpDev& m, const __nv_bfloat16* X, int B, MlpWork& ws, fl
     k_bias_gelu<<<blocks_for((long long)B * kMlpOutPad), 256, 0, st>>>(Y, b3, nullptr, B, kMlpOutPad, kMlpOut, 0);
 }
 
+// Rows of a slice of the gradient sums: eight slices up to 20480 rows (12,000
+// rows: 45 us per layer; one slice 1.6 ms), of 2560 rows beyond.  The tensor cores
+// truncate as they accumulate: at 20,000 rows eight slices move the sums by
+// 1.7e-5 towards the exact ones, 94 slices by 1.95e-5.
+static int slice_rows(int B)
+{
+    const int rows = ((B + 7) / 8 + kMlpSliceRows - 1) / kMlpSliceRows * kMlpSliceRows;
+    return std::min(rows, 20 * kMlpSliceRows);
+}
+
+// dW = H^T dZ [in x out] and db = the column sums of dZ over B rows, by slices of
+// rows: a CTA each, summed in slice order (db: up to 128 slices, a block each).
+static void layer_gradients(int in, int out, int B, const __nv_bfloat16* H, const __nv_bfloat16* dZ, int lddz, float* dW,
+                            float* db, MlpWork& ws, cudaStream_t st)
+{
+    const int rows = slice_rows(B), slices = (B + rows - 1) / rows;
+    const int rows_b = ((B + 127) / 128 + kMlpSliceRows - 1) / kMlpSliceRows * kMlpSliceRows, slices_b = (B + rows_b - 1) / rows_b;
+    float* part_b = ws.part + (size_t)slices * in * out;
+    gemm_tc_slices(in, out, B, H, in, dZ, lddz, slices > 1 ? ws.part : dW, slices, rows, st);
+    k_colsum_slices<<<slices_b, 256, 0, st>>>(dZ, B, out, lddz, rows_b, slices > 1 ? part_b : db);
+    if (slices > 1)
+        k_sum_slices<<<(in * out + out + 31) / 32, 256, 0, st>>>(ws.part, in * out, slices, part_b, out, slices_b, dW, db);
+}
+
 // Loss and gradients (into m.grad) for a batch; returns nothing, loss accumulates in *loss (device double).
 void mlp_backward(const MlpDev& m, const __nv_bfloat16* X, const float* T, int B, MlpWork& ws, const float* Y,
                   double* loss, cudaStream_t st)
@@ -179,18 +231,15 @@ void mlp_backward(const MlpDev& m, const __nv_bfloat16* X, const float* T, int B
     // dY [B x 8] BF16
     k_mse_grad<<<blocks_for(B), 256, 0, st>>>(Y, kMlpOutPad, T, kMlpOut, B, ws.dy, kMlpOutPad, loss);
     // layer 3: dW3 = H2^T dY  [128 x 3], db3 = colsum(dY), dH2 = dY W3^T
-    gemm<true, false>(kMlpHidden, kMlpOut, B, ws.h2, kMlpHidden, ws.dy, kMlpOutPad, gw3, kMlpOut, false, st);
-    k_colsum<<<kMlpOut, 256, 0, st>>>(ws.dy, B, kMlpOut, kMlpOutPad, gb3);
+    layer_gradients(kMlpHidden, kMlpOut, B, ws.h2, ws.dy, kMlpOutPad, gw3, gb3, ws, st);
     gemm<false, true>(B, kMlpHidden, kMlpOutPad, ws.dy, kMlpOutPad, m.w3b, kMlpOutPad, ws.dh, kMlpHidden, false, st);
     k_gelu_back<<<blocks_for((long long)B * kMlpHidden), 256, 0, st>>>(ws.dh, ws.z2, ws.dz, (long long)B * kMlpHidden);
     // layer 2
-    gemm<true, false>(kMlpHidden, kMlpHidden, B, ws.h1, kMlpHidden, ws.dz, kMlpHidden, gw2, kMlpHidden, false, st);
-    k_colsum<<<kMlpHidden, 256, 0, st>>>(ws.dz, B, kMlpHidden, kMlpHidden, gb2);
+    layer_gradients(kMlpHidden, kMlpHidden, B, ws.h1, ws.dz, kMlpHidden, gw2, gb2, ws, st);
     gemm<false, true>(B, kMlpHidden, kMlpHidden, ws.dz, kMlpHidden, m.w2b, kMlpHidden, ws.dh, kMlpHidden, false, st);
     k_gelu_back<<<blocks_for((long long)B * kMlpHidden), 256, 0, st>>>(ws.dh, ws.z1, ws.dz, (long long)B * kMlpHidden);
     // layer 1
-    gemm<true, false>(kMlpIn, kMlpHidden, B, X, kMlpIn, ws.dz, kMlpHidden, gw1, kMlpHidden, false, st);
-    k_colsum<<<kMlpHidden, 256, 0, st>>>(ws.dz, B, kMlpHidden, kMlpHidden, gb1);
+    layer_gradients(kMlpIn, kMlpHidden, B, X, ws.dz, kMlpHidden, gw1, gb1, ws, st);
 }
 
 void mlp_adam(MlpDev& m, float lr, int t, cudaStream_t st)
@@ -224,6 +273,13 @@ __global__ void k_gather_rows(const __nv_bfloat16* __restrict__ X, const float* 
     }
 }
 
+// the columns in use of padded output rows
+__global__ void k_pack_rows(const float* __restrict__ y, float* __restrict__ out, int B)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < B; i += gridDim.x * blockDim.x)
+        for (int c = 0; c < kMlpOut; ++c) out[(size_t)i * kMlpOut + c] = y[(size_t)i * kMlpOutPad + c];
+}
+
 struct Xorshift {
     uint64_t s;
     explicit Xorshift(uint64_t seed) : s(seed * 0x9E3779B97F4A7C15ull + 0x2545F4914F6CDD1Dull) {}
@@ -238,58 +294,90 @@ struct Xorshift {
 };
 }  // namespace
 
+namespace {
+// Sections of one allocation, each on a 256-byte boundary: an allocation costs
+// 5 us and more by its size, and giving it back as much again.
+struct Sections {
+    size_t bytes = 0;
+    size_t add(size_t n)
+    {
+        const size_t at = bytes;
+        bytes += (n + 255) / 256 * 256;
+        return at;
+    }
+};
+}  // namespace
+
 cudaError_t mlp_alloc(MlpDev* m, bool training)
 {
     *m = MlpDev{};
-    const size_t P = mlp_param_count();
-    cudaError_t e;
-    if ((e = cudaMalloc(&m->params, P * sizeof(float))) != cudaSuccess) return e;
+    const size_t P = mlp_param_count() * sizeof(float), H = sizeof(__nv_bfloat16) * kMlpHidden;
+    Sections s;
+    s.add(P);
+    const size_t grad = s.add(training ? P : 0), m1 = s.add(training ? P : 0), m2 = s.add(training ? P : 0), end = s.bytes;
+    const size_t w1 = s.add(H * kMlpIn), w2 = s.add(H * kMlpHidden), w3 = s.add(H * kMlpOutPad);
+    unsigned char* base = nullptr;
+    const cudaError_t e = cudaMalloc((void**)&base, s.bytes);
+    if (e != cudaSuccess) return e;
+    m->params = (float*)base;
     if (training) {
-        if ((e = cudaMalloc(&m->grad, P * sizeof(float))) != cudaSuccess) return e;
-        if ((e = cudaMalloc(&m->m1, P * sizeof(float))) != cudaSuccess) return e;
-        if ((e = cudaMalloc(&m->m2, P * sizeof(float))) != cudaSuccess) return e;
-        cudaMemset(m->grad, 0, P * sizeof(float));
-        cudaMemset(m->m1, 0, P * sizeof(float));
-        cudaMemset(m->m2, 0, P * sizeof(float));
+        m->grad = (float*)(base + grad);
+        m->m1 = (float*)(base + m1);
+        m->m2 = (float*)(base + m2);
+        cudaMemset(base + grad, 0, end - grad);
     }
-    if ((e = cudaMalloc(&m->w1b, sizeof(__nv_bfloat16) * kMlpIn * kMlpHidden)) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&m->w2b, sizeof(__nv_bfloat16) * kMlpHidden * kMlpHidden)) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&m->w3b, sizeof(__nv_bfloat16) * kMlpHidden * kMlpOutPad)) != cudaSuccess) return e;
+    m->w1b = (__nv_bfloat16*)(base + w1);
+    m->w2b = (__nv_bfloat16*)(base + w2);
+    m->w3b = (__nv_bfloat16*)(base + w3);
     return cudaSuccess;
 }
 
 void mlp_free(MlpDev* m)
 {
-    void* p[] = {m->params, m->grad, m->m1, m->m2, m->w1b, m->w2b, m->w3b};
-    for (void* q : p)
-        if (q) cudaFree(q);
+    cudaFree(m->params);
     *m = MlpDev{};
 }
 
+// Inference needs the output rows only.  dh and the partial gradients are never
+// live together.
 cudaError_t mlp_work_alloc(MlpWork* w, long long rows, bool training)
 {
     *w = MlpWork{};
     w->rows = rows;
-    const size_t r = (size_t)(rows > 0 ? rows : 1);
-    cudaError_t e;
-    if ((e = cudaMalloc(&w->z1, r * kMlpHidden * sizeof(float))) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&w->z2, r * kMlpHidden * sizeof(float))) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&w->h1, r * kMlpHidden * sizeof(__nv_bfloat16))) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&w->h2, r * kMlpHidden * sizeof(__nv_bfloat16))) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&w->y, r * kMlpOutPad * sizeof(float))) != cudaSuccess) return e;
+    const size_t r = (size_t)(rows > 0 ? rows : 1), h = r * kMlpHidden;
+    Sections s;
+    s.add(r * kMlpOutPad * sizeof(float));
+    size_t z1 = 0, z2 = 0, h1 = 0, h2 = 0, dy = 0, dz = 0, dh = 0;
     if (training) {
-        if ((e = cudaMalloc(&w->dy, r * kMlpOutPad * sizeof(__nv_bfloat16))) != cudaSuccess) return e;
-        if ((e = cudaMalloc(&w->dh, r * kMlpHidden * sizeof(float))) != cudaSuccess) return e;
-        if ((e = cudaMalloc(&w->dz, r * kMlpHidden * sizeof(__nv_bfloat16))) != cudaSuccess) return e;
+        z1 = s.add(h * sizeof(float));
+        z2 = s.add(h * sizeof(float));
+        h1 = s.add(h * sizeof(__nv_bfloat16));
+        h2 = s.add(h * sizeof(__nv_bfloat16));
+        dy = s.add(r * kMlpOutPad * sizeof(__nv_bfloat16));
+        dz = s.add(h * sizeof(__nv_bfloat16));
+        const size_t slices = (r + kMlpSliceRows - 1) / kMlpSliceRows;
+        dh = s.add(std::max(h, slices * kMlpHidden * (kMlpHidden + 1)) * sizeof(float));
+    }
+    unsigned char* base = nullptr;
+    const cudaError_t e = cudaMalloc((void**)&base, s.bytes);
+    if (e != cudaSuccess) return e;
+    w->y = (float*)base;
+    if (training) {
+        w->z1 = (float*)(base + z1);
+        w->z2 = (float*)(base + z2);
+        w->h1 = (__nv_bfloat16*)(base + h1);
+        w->h2 = (__nv_bfloat16*)(base + h2);
+        w->dy = (__nv_bfloat16*)(base + dy);
+        w->dz = (__nv_bfloat16*)(base + dz);
+        w->dh = (float*)(base + dh);
+        w->part = w->dh;
     }
     return cudaSuccess;
 }
 
 void mlp_work_free(MlpWork* w)
 {
-    void* p[] = {w->z1, w->z2, w->h1, w->h2, w->dy, w->dh, w->dz, w->y};
-    for (void* q : p)
-        if (q) cudaFree(q);
+    cudaFree(w->y);
     *w = MlpWork{};
 }
 
@@ -316,7 +404,7 @@ struct Session {
     cudaStream_t st = nullptr;
     pdgb::MlpDev m{};
     pdgb::MlpWork w{};
-    __nv_bfloat16* X = nullptr;
+    __nv_bfloat16* X = nullptr;   // (one allocation with the three below)
     float* T = nullptr;
     float* Xf = nullptr;
     double* loss = nullptr;
@@ -325,9 +413,6 @@ struct Session {
         pdgb::mlp_work_free(&w);
         pdgb::mlp_free(&m);
         if (X) cudaFree(X);
-        if (T) cudaFree(T);
-        if (Xf) cudaFree(Xf);
-        if (loss) cudaFree(loss);
         if (st) cudaStreamDestroy(st);
     }
 };
@@ -345,25 +430,53 @@ pd_status mlp_fail(cudaError_t e)
         if (e_ != cudaSuccess) return mlp_fail(e_); \
     } while (0)
 
-// uploads X (f32 -> BF16 on the device) and T
-pd_status session_setup(Session& s, int device, const float* X, const float* T, long long rows, long long work_rows,
-                        bool training, const float* params)
+// Rows of X uploaded at a time, which bounds the session's buffers (100,000 rows:
+// 628 us in one part, 657 in parts of 32768, 740 in parts of 16384: a copy from
+// pageable memory returns when it is done).
+constexpr long long kUploadRows = 131072;
+
+// The network, and room for `rows` rows of X in BF16, `parts` rows of them in
+// FP32 on their way, `t_rows` rows of T (or of the result) and the loss.
+pd_status session_setup(Session& s, int device, long long rows, long long t_rows, long long parts, bool training,
+                        const float* params)
 {
     MLP_TRY(cudaSetDevice(device));
     MLP_TRY(cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking));
     MLP_TRY(pdgb::mlp_alloc(&s.m, training));
-    MLP_TRY(pdgb::mlp_work_alloc(&s.w, work_rows, training));
-    const size_t nx = (size_t)rows * pdgb::kMlpIn;
-    MLP_TRY(cudaMalloc(&s.X, (nx ? nx : 1) * sizeof(__nv_bfloat16)));
-    MLP_TRY(cudaMalloc(&s.Xf, (nx ? nx : 1) * sizeof(float)));
-    MLP_TRY(cudaMalloc(&s.T, ((size_t)rows * pdgb::kMlpOut + 1) * sizeof(float)));
-    MLP_TRY(cudaMalloc(&s.loss, sizeof(double)));
-    if (nx) MLP_TRY(cudaMemcpyAsync(s.Xf, X, nx * sizeof(float), cudaMemcpyHostToDevice, s.st));
-    if (T && rows) MLP_TRY(cudaMemcpyAsync(s.T, T, (size_t)rows * pdgb::kMlpOut * sizeof(float), cudaMemcpyHostToDevice, s.st));
-    if (nx) pdgb::k_f32_to_bf16<<<pdgb::blocks_for((long long)nx), 256, 0, s.st>>>(s.Xf, s.X, (long long)nx);
+    pdgb::Sections sec;
+    sec.add((size_t)std::max(rows, 1LL) * pdgb::kMlpIn * sizeof(__nv_bfloat16));
+    const size_t xf = sec.add((size_t)std::max(parts, 1LL) * pdgb::kMlpIn * sizeof(float));
+    const size_t t = sec.add((size_t)t_rows * pdgb::kMlpOut * sizeof(float));
+    const size_t loss = sec.add(sizeof(double));
+    unsigned char* base = nullptr;
+    MLP_TRY(cudaMalloc((void**)&base, sec.bytes));
+    s.X = (__nv_bfloat16*)base;
+    s.Xf = (float*)(base + xf);
+    s.T = (float*)(base + t);
+    s.loss = (double*)(base + loss);
     MLP_TRY(cudaMemcpyAsync(s.m.params, params, pdgb::mlp_param_count() * sizeof(float), cudaMemcpyHostToDevice, s.st));
     pdgb::mlp_refresh_bf16(s.m, s.st);
     MLP_TRY(cudaGetLastError());
+    return PD_OK;
+}
+
+// `rows` rows of X (f32) to dst (BF16) through s.Xf
+cudaError_t upload_rows(Session& s, const float* X, __nv_bfloat16* dst, long long rows)
+{
+    const size_t nx = (size_t)rows * pdgb::kMlpIn;
+    const cudaError_t e = cudaMemcpyAsync(s.Xf, X, nx * sizeof(float), cudaMemcpyHostToDevice, s.st);
+    if (e == cudaSuccess) pdgb::k_f32_to_bf16<<<pdgb::blocks_for((long long)nx), 256, 0, s.st>>>(s.Xf, dst, (long long)nx);
+    return e;
+}
+
+// X and T of a training session, and its activations for work_rows rows
+pd_status session_data(Session& s, const float* X, const float* T, long long rows, long long work_rows)
+{
+    for (long long r0 = 0; r0 < rows; r0 += kUploadRows)
+        MLP_TRY(upload_rows(s, X + (size_t)r0 * pdgb::kMlpIn, s.X + (size_t)r0 * pdgb::kMlpIn,
+                            std::min(kUploadRows, rows - r0)));
+    MLP_TRY(cudaMemcpyAsync(s.T, T, (size_t)rows * pdgb::kMlpOut * sizeof(float), cudaMemcpyHostToDevice, s.st));
+    MLP_TRY(pdgb::mlp_work_alloc(&s.w, work_rows, true));
     return PD_OK;
 }
 
@@ -382,21 +495,23 @@ extern "C" pd_status pd_mlp_predict(int device, const float* X, long long rows, 
 {
     if (rows < 0 || (rows > 0 && (!X || !Y)) || !params) return PD_ERR_INVALID_ARGUMENT;
     Session s;
-    const long long chunk = rows < 65536 ? (rows > 0 ? rows : 1) : 65536;
-    pd_status st = session_setup(s, device, X, nullptr, rows, chunk, false, params);
+    const long long part = std::min(rows, kUploadRows);
+    pd_status st = session_setup(s, device, part, rows, part, false, params);
     if (st != PD_OK) return st;
-    std::vector<float> yb((size_t)chunk * pdgb::kMlpOutPad);
-    for (long long r0 = 0; r0 < rows; r0 += chunk) {
-        const int B = (int)std::min(chunk, rows - r0);
-        MLP_TRY(pdgb::mlp_infer_tc(s.m, s.X + (size_t)r0 * pdgb::kMlpIn, B, s.w.y, s.st));
-        MLP_TRY(cudaMemcpyAsync(yb.data(), s.w.y, (size_t)B * pdgb::kMlpOutPad * sizeof(float), cudaMemcpyDeviceToHost, s.st));
-        MLP_TRY(cudaStreamSynchronize(s.st));
-        if (pdgb::mlp_tc_take_error()) {
-            pdgb::set_handleless_error("pd_mlp_predict: a tensor-core wait ran out of time");
-            return PD_ERR_CUDA;
-        }
-        for (int i = 0; i < B; ++i)
-            for (int c = 0; c < pdgb::kMlpOut; ++c) Y[(size_t)(r0 + i) * pdgb::kMlpOut + c] = yb[(size_t)i * pdgb::kMlpOutPad + c];
+    MLP_TRY(pdgb::mlp_work_alloc(&s.w, part, false));
+    for (long long r0 = 0; r0 < rows; r0 += part) {
+        const int B = (int)std::min(part, rows - r0);
+        MLP_TRY(upload_rows(s, X + (size_t)r0 * pdgb::kMlpIn, s.X, B));
+        MLP_TRY(pdgb::mlp_infer_tc(s.m, s.X, B, s.w.y, s.st));
+        pdgb::k_pack_rows<<<pdgb::blocks_for(B), 256, 0, s.st>>>(s.w.y, s.T + (size_t)r0 * pdgb::kMlpOut, B);
+    }
+    if (rows)
+        MLP_TRY(cudaMemcpyAsync(Y, s.T, (size_t)rows * pdgb::kMlpOut * sizeof(float), cudaMemcpyDeviceToHost, s.st));
+    MLP_TRY(cudaStreamSynchronize(s.st));
+    MLP_TRY(cudaGetLastError());
+    if (pdgb::mlp_tc_take_error()) {
+        pdgb::set_handleless_error("pd_mlp_predict: a tensor-core wait ran out of time");
+        return PD_ERR_CUDA;
     }
     return PD_OK;
 }
@@ -406,7 +521,8 @@ extern "C" pd_status pd_mlp_loss_grad(int device, const float* X, const float* T
 {
     if (rows <= 0 || !X || !T || !params || !grad || !loss) return PD_ERR_INVALID_ARGUMENT;
     Session s;
-    pd_status st = session_setup(s, device, X, T, rows, rows, true, params);
+    pd_status st = session_setup(s, device, rows, rows, std::min<long long>(rows, kUploadRows), true, params);
+    if (st == PD_OK) st = session_data(s, X, T, rows, rows);
     if (st != PD_OK) return st;
     pdgb::mlp_forward(s.m, s.X, rows, s.w, s.w.y, s.st);
     MLP_TRY(cudaMemsetAsync(s.loss, 0, sizeof(double), s.st));
@@ -428,8 +544,8 @@ extern "C" pd_status pd_mlp_train(int device, const float* X, const float* T, lo
     if (rows <= 0 || !X || !T || !params || iterations < 0 || batch <= 0) return PD_ERR_INVALID_ARGUMENT;
     if (batch > rows) batch = (int)rows;
     Session s;
-    pd_status st = session_setup(s, device, X, T, rows, std::max<long long>(batch, std::min<long long>(rows, 65536)),
-                                 true, params);
+    pd_status st = session_setup(s, device, rows, rows, std::min(rows, kUploadRows), true, params);
+    if (st == PD_OK) st = session_data(s, X, T, rows, std::max<long long>(batch, std::min<long long>(rows, 65536)));
     if (st != PD_OK) return st;
     __nv_bfloat16* Xb = nullptr;
     float* Tb = nullptr;

@@ -359,26 +359,89 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 // ---- general GEMM of the training passes ----------------------------------------------
 // C[M x N] (FP32, row-major, ldc) = op(A)[M x K] op(B)[K x N] (+ C), BF16
 // operands; op(P) is P (row-major) or, with TA / TB, its transpose.  One CTA
-// per 128 x 128 tile of C: K in slabs of 64, each slab's operands written by
-// the threads into K-major core-matrix tiles (transposing where asked), four
-// tcgen05.mma (K = 16) accumulating in TMEM, then the epilogue.
+// per 128 x 128 tile of C: K in slabs of 64, four tcgen05.mma (K = 16) each,
+// accumulating in TMEM, then the epilogue.  An operand is staged as it lies in
+// memory, 16 bytes per access into tiles of core matrices -- K-major where its
+// rows run along K, MN-major where they run along M or N -- and the next slab's
+// loads are in flight during the MMAs: latency-bound, 1.9 us per slab (8.7 with
+// 2-byte accesses and a transposing store).  12,000 rows: forward products 20 us
+// together (52), those of the output gradients 14 (38).
+// blockIdx.z takes the slice [z kslice, (z + 1) kslice) of K into its own copy
+// of C (`cstride` apart): the weight gradients sum over all rows of a batch into
+// one or two tiles, which one CTA would walk alone (12,000 rows: 1.6 ms each).
 constexpr int kGemmSlab = 64;
-constexpr int kGemmOffA = 0;                                   // 128 x 64
+constexpr int kGemmOffA = 0;                                   // 128 x 64 (core_off's or the MN-major order)
 constexpr int kGemmOffB = kGemmOffA + 128 * kGemmSlab * 2;     // 128 x 64
 constexpr int kGemmOffBar = kGemmOffB + 128 * kGemmSlab * 2;   // mbarrier, TMEM address
 // requested shared memory: limits residency to 3 CTAs per SM (3 x 128 TMEM columns)
-constexpr int kGemmSmemBytes = 58 * 1024;
+constexpr int kGemmSmemBytes = 66 * 1024;
+
+// A 128 (M or N) x 64 (K) operand tile, four 16-byte pieces per thread.  MN: rows
+// of P run along M / N (MN-major core matrices, 8 K rows of 8 elements each, K
+// groups 2048 bytes apart), else along K (8 M / N rows, K groups 128 bytes apart).
+template <bool MN>
+struct OperandTile {
+    uint4 v[4];
+
+    static __device__ __forceinline__ void place(int c, int& r, int& a, int& b)
+    {
+        r = c & 7;                          // row of the core matrix
+        a = (c >> 3) & (MN ? 15 : 7);       // group along the contiguous direction
+        b = c >> (MN ? 7 : 6);              // group along the other one
+    }
+    __device__ __forceinline__ void load(const __nv_bfloat16* __restrict__ P, int ld, int mn0, int mn_end, int k0, int k_end,
+                                         bool vec)
+    {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            int r, a, b;
+            place((int)threadIdx.x + i * kTcThreads, r, a, b);
+            const int row = (MN ? k0 : mn0) + 8 * b + r, col = (MN ? mn0 : k0) + 8 * a;
+            const int row_end = MN ? k_end : mn_end, col_end = MN ? mn_end : k_end;
+            v[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (row >= row_end || col >= col_end) continue;
+            const __nv_bfloat16* src = P + (size_t)row * ld + col;
+            if (vec && col + 8 <= col_end) {
+                v[i] = __ldg((const uint4*)src);
+            } else {
+                unsigned w[4] = {0u, 0u, 0u, 0u};
+                const unsigned short* s16 = (const unsigned short*)src;
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    if (col + e < col_end) w[e >> 1] |= (unsigned)__ldg(s16 + e) << (16 * (e & 1));
+                v[i] = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+        }
+    }
+    __device__ __forceinline__ void store(unsigned char* tile) const
+    {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            int r, a, b;
+            place((int)threadIdx.x + i * kTcThreads, r, a, b);
+            *(uint4*)(tile + ((b * (MN ? 16 : 8) + a) << 7) + (r << 4)) = v[i];
+        }
+    }
+    // descriptor of K step s (16 of the slab's 64)
+    static __device__ __forceinline__ uint64_t desc(uint32_t tile, int s)
+    {
+        return MN ? smem_desc(tile + 4096 * s, 2048, 128) : smem_desc(tile + 256 * s, 128, kGemmSlab * 16);
+    }
+};
 
 template <bool TA, bool TB>
 __global__ void __launch_bounds__(kTcThreads, 1)
     k_gemm_tc(int M, int N, int K, const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ B,
-              int ldb, float* __restrict__ C, int ldc, int accumulate)
+              int ldb, float* __restrict__ C, int ldc, int accumulate, int kslice, size_t cstride)
 {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.x * 128, n0 = blockIdx.y * 128;
+    const int kbegin = blockIdx.z * kslice;
+    K = K - kbegin < kslice ? K : kbegin + kslice;
+    C += blockIdx.z * cstride;
     const int nt = (N - n0 < 128 ? N - n0 : 128);
     const int nmma = (nt + 15) & ~15;   // MMA N: a multiple of 16
     const uint32_t bar = sbase + kGemmOffBar;
@@ -394,49 +457,49 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     }
     bool ok = tc_sync(true);
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(sm + kGemmOffBar + 8);
-    const uint32_t idesc = instr_desc(128, nmma);
+    // (bits 15, 16: A, B MN-major)
+    const uint32_t idesc = instr_desc(128, nmma) | (TA ? 1u << 15 : 0u) | (TB ? 0u : 1u << 16);
     uint32_t parity = 0;
     bool pending = false;
-    for (int k0 = 0; k0 < K && ok; k0 += kGemmSlab) {
-        // op(A) rows m0.., columns k0..: consecutive threads walk the
-        // contiguous direction of A in memory
-        for (int i = tid; i < 128 * kGemmSlab; i += blockDim.x) {
-            const int m = TA ? (i & 127) : (i >> 6), kk = TA ? (i >> 7) : (i & 63);
-            const int gm = m0 + m, gk = k0 + kk;
-            __nv_bfloat16 v = __float2bfloat16_rn(0.f);
-            if (gm < M && gk < K) v = TA ? A[(size_t)gk * lda + gm] : A[(size_t)gm * lda + gk];
-            *reinterpret_cast<__nv_bfloat16*>(sm + kGemmOffA + core_off(m, kk, kGemmSlab)) = v;
-        }
-        // the B operand is op(B)^T: row n holds op(B)[k0.., n0 + n]
-        for (int i = tid; i < 128 * kGemmSlab; i += blockDim.x) {
-            const int n = TB ? (i >> 6) : (i & 127), kk = TB ? (i & 63) : (i >> 7);
-            const int gn = n0 + n, gk = k0 + kk;
-            __nv_bfloat16 v = __float2bfloat16_rn(0.f);
-            if (gn < N && gk < K) v = TB ? B[(size_t)gn * ldb + gk] : B[(size_t)gk * ldb + gn];
-            *reinterpret_cast<__nv_bfloat16*>(sm + kGemmOffB + core_off(n, kk, kGemmSlab)) = v;
-        }
+    OperandTile<TA> ta;
+    OperandTile<!TB> tb;
+    const bool va = lda % 8 == 0 && ((uintptr_t)A & 15u) == 0, vb = ldb % 8 == 0 && ((uintptr_t)B & 15u) == 0;
+    ta.load(A, lda, m0, M, kbegin, K, va);
+    tb.load(B, ldb, n0, N, kbegin, K, vb);
+    for (int k0 = kbegin; k0 < K && ok; k0 += kGemmSlab) {
+        ta.store(sm + kGemmOffA);
+        tb.store(sm + kGemmOffB);
         ok = tc_sync(ok);
         if (!ok) break;
         if (tid == 0) {
 #pragma unroll
             for (int s = 0; s < kGemmSlab / 16; ++s)
-                mma_bf16(tmem, smem_desc(sbase + kGemmOffA + 256 * s, 128, kGemmSlab * 16),
-                         smem_desc(sbase + kGemmOffB + 256 * s, 128, kGemmSlab * 16), idesc, (k0 > 0 || s > 0) ? 1u : 0u);
+                mma_bf16(tmem, OperandTile<TA>::desc(sbase + kGemmOffA, s), OperandTile<!TB>::desc(sbase + kGemmOffB, s), idesc,
+                         (k0 > kbegin || s > 0) ? 1u : 0u);
             mma_commit(bar);
         }
         pending = true;
+        if (k0 + kGemmSlab < K) {
+            ta.load(A, lda, m0, M, k0 + kGemmSlab, K, va);
+            tb.load(B, ldb, n0, N, k0 + kGemmSlab, K, vb);
+        }
         ok = mbar_wait(bar, parity);
         if (ok) { parity ^= 1u; pending = false; }
         ok = tc_sync(ok);
     }
+    const bool vc = !accumulate && ldc % 4 == 0 && ((uintptr_t)C & 15u) == 0;
     if (ok && warp < 4) {
         const int row = 32 * warp + lane, gm = m0 + row;
         for (int c0 = 0; c0 < nmma; c0 += 16) {
             float v[16];
-            if (K > 0) tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)c0, v);
+            if (K > kbegin) tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)c0, v);
             else
                 for (int i = 0; i < 16; ++i) v[i] = 0.f;
-            if (gm < M)
+            if (gm < M && vc && n0 + c0 + 16 <= N) {
+                float4* dst = (float4*)(C + (size_t)gm * ldc + n0 + c0);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            } else if (gm < M)
                 for (int i = 0; i < 16; ++i) {
                     const int gn = n0 + c0 + i;
                     if (gn >= N) break;
@@ -458,7 +521,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 
 template <bool TA, bool TB>
 static cudaError_t gemm_tc_t(int M, int N, int K, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb,
-                             float* C, int ldc, bool accumulate, cudaStream_t st)
+                             float* C, int ldc, bool accumulate, int slices, int kslice, size_t cstride, cudaStream_t st)
 {
     static std::mutex mtx;
     static bool configured[kMaxDevices] = {};
@@ -474,8 +537,9 @@ static cudaError_t gemm_tc_t(int M, int N, int K, const __nv_bfloat16* A, int ld
             configured[dev] = true;
         }
     }
-    const dim3 grid((unsigned)((M + 127) / 128), (unsigned)((N + 127) / 128));
-    k_gemm_tc<TA, TB><<<grid, kTcThreads, kGemmSmemBytes, st>>>(M, N, K, A, lda, B, ldb, C, ldc, accumulate ? 1 : 0);
+    const dim3 grid((unsigned)((M + 127) / 128), (unsigned)((N + 127) / 128), (unsigned)slices);
+    k_gemm_tc<TA, TB><<<grid, kTcThreads, kGemmSmemBytes, st>>>(M, N, K, A, lda, B, ldb, C, ldc, accumulate ? 1 : 0, kslice,
+                                                                cstride);
     return cudaGetLastError();
 }
 
@@ -483,10 +547,18 @@ cudaError_t gemm_tc(bool ta, bool tb, int M, int N, int K, const __nv_bfloat16* 
                     int ldb, float* C, int ldc, bool accumulate, cudaStream_t st)
 {
     if (M <= 0 || N <= 0) return cudaSuccess;
-    if (!ta && !tb) return gemm_tc_t<false, false>(M, N, K, A, lda, B, ldb, C, ldc, accumulate, st);
-    if (ta && !tb) return gemm_tc_t<true, false>(M, N, K, A, lda, B, ldb, C, ldc, accumulate, st);
-    if (!ta && tb) return gemm_tc_t<false, true>(M, N, K, A, lda, B, ldb, C, ldc, accumulate, st);
-    return gemm_tc_t<true, true>(M, N, K, A, lda, B, ldb, C, ldc, accumulate, st);
+    const int ks = K > 0 ? K : 1;
+    if (!ta && !tb) return gemm_tc_t<false, false>(M, N, K, A, lda, B, ldb, C, ldc, accumulate, 1, ks, 0, st);
+    if (ta && !tb) return gemm_tc_t<true, false>(M, N, K, A, lda, B, ldb, C, ldc, accumulate, 1, ks, 0, st);
+    if (!ta && tb) return gemm_tc_t<false, true>(M, N, K, A, lda, B, ldb, C, ldc, accumulate, 1, ks, 0, st);
+    return gemm_tc_t<true, true>(M, N, K, A, lda, B, ldb, C, ldc, accumulate, 1, ks, 0, st);
+}
+
+// A^T B by slices of K into part[slices][M x N]
+cudaError_t gemm_tc_slices(int M, int N, int K, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb,
+                           float* part, int slices, int kslice, cudaStream_t st)
+{
+    return gemm_tc_t<true, false>(M, N, K, A, lda, B, ldb, part, N, false, slices, kslice, (size_t)M * N, st);
 }
 
 // Y[B x kMlpOutPad] (columns 0..2 used) = network(X[B x 64]) on the tensor

@@ -458,6 +458,7 @@ constexpr int kMlpHidden = 128;
 constexpr int kMlpOut = 3;
 constexpr int kMlpOutPad = 8;
 
+constexpr int kMlpSliceRows = 128;    // rows of a slice of the gradient sums, or a multiple
 struct MlpDev {
     float* params;            // FP32 master parameters (mlp_param_count())
     float* grad;
@@ -476,6 +477,7 @@ struct MlpWork {              // activations for up to `rows` rows
     __nv_bfloat16* dy;        // [rows x 8]
     float* dh;
     __nv_bfloat16* dz;
+    float* part;              // partial weight and bias gradients (shares dh)
     float* y;                 // [rows x 8]
     long long rows;
 };
@@ -506,6 +508,8 @@ void mlp_forward(const MlpDev& m, const __nv_bfloat16* X, int B, MlpWork& ws, fl
 // C[M x N] (f32, ldc) = op(A) op(B) (+ C) on tcgen05, op = transpose when ta / tb (mlp_tc.cu)
 cudaError_t gemm_tc(bool ta, bool tb, int M, int N, int K, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B,
                     int ldb, float* C, int ldc, bool accumulate, cudaStream_t st);
+cudaError_t gemm_tc_slices(int M, int N, int K, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb,
+                           float* part, int slices, int kslice, cudaStream_t st);
 // inference only (mlp_tc.cu): all layers in one tcgen05 kernel, Y [B x 8]
 cudaError_t mlp_infer_tc(const MlpDev& m, const __nv_bfloat16* X, int B, float* Y, cudaStream_t st);
 // 1 if a wait of the tensor-core kernel ran out of time since the last call
