@@ -271,12 +271,22 @@ __global__ void __launch_bounds__(kBlock) k_bond_query(const dbl4* __restrict__ 
 __global__ void k_pad_counts(const unsigned* __restrict__ cnt, int n, int max_bonds, unsigned* __restrict__ padded,
                              int* __restrict__ cnt_out, int* __restrict__ flags)
 {
+    unsigned long long bonds = 0ull;
+    int most = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const unsigned c = cnt[i];
+        bonds += c;
+        most = max(most, (int)c);
         padded[i] = (c + kRowAlign - 1) / kRowAlign * kRowAlign;
         cnt_out[i] = (int)c;
         if ((int)c > max_bonds) flags[0] = 1;
-        atomicMax(&flags[1], (int)c);
+    }
+    // one update per warp: the counters are one address
+    most = __reduce_max_sync(0xffffffffu, most);
+    for (int off = 16; off > 0; off >>= 1) bonds += __shfl_xor_sync(0xffffffffu, bonds, off);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&flags[1], most);
+        atomicAdd((unsigned long long*)(flags + 2), bonds);
     }
 }
 
@@ -356,50 +366,75 @@ int grid_for(long long n, int threads = kBlock)
         if (e_ != cudaSuccess) return e_;          \
     } while (0)
 
-// Exclusive scan of n unsigned values (in may equal out).  Temporary storage
-// is allocated per level.
-cudaError_t exclusive_scan(const unsigned* in, unsigned* out, long long n, cudaStream_t st)
+// Words of scratch that a scan of n values takes.
+size_t scan_scratch(long long n)
+{
+    size_t words = 0;
+    while (n > 1) words += (size_t)(n = (n + kScanTile - 1) / kScanTile);
+    return words > 0 ? words : 1;
+}
+
+// Exclusive scan of n unsigned values (in may equal out); tmp: scan_scratch(n) words.
+cudaError_t exclusive_scan(const unsigned* in, unsigned* out, long long n, unsigned* tmp, cudaStream_t st)
 {
     if (n <= 0) return cudaSuccess;
     const long long tiles = (n + kScanTile - 1) / kScanTile;
-    unsigned* sums = nullptr;
-    PD_TRY(cudaMalloc(&sums, sizeof(unsigned) * (size_t)tiles));
-    k_scan_tiles<<<(unsigned)tiles, kScanThreads, 0, st>>>(in, out, n, sums);
+    k_scan_tiles<<<(unsigned)tiles, kScanThreads, 0, st>>>(in, out, n, tmp);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess && tiles > 1) {
-        e = exclusive_scan(sums, sums, tiles, st);
+        e = exclusive_scan(tmp, tmp, tiles, tmp + tiles, st);
         if (e == cudaSuccess) {
-            k_scan_add<<<grid_for(n), kBlock, 0, st>>>(out, n, sums);
+            k_scan_add<<<grid_for(n), kBlock, 0, st>>>(out, n, tmp);
             e = cudaGetLastError();
         }
     }
-    cudaError_t e2 = cudaStreamSynchronize(st);
-    cudaFree(sums);
-    return e != cudaSuccess ? e : e2;
+    return e;
 }
+
+// Sections of one allocation, given back with it.
+struct Workspace {
+    unsigned char* base = nullptr;
+    size_t bytes = 0;
+    ~Workspace() { cudaFree(base); }
+    size_t add(size_t n)
+    {
+        const size_t at = bytes;
+        bytes += (n + 255) / 256 * 256;
+        return at;
+    }
+    cudaError_t alloc() { return cudaMalloc((void**)&base, bytes > 0 ? bytes : 1); }
+    template <typename T>
+    T* at(size_t offset) const { return (T*)(base + offset); }
+};
 
 }  // namespace
 
 cudaError_t scan_exclusive_u32(const unsigned* in, unsigned* out, long long n, cudaStream_t st)
 {
-    return exclusive_scan(in, out, n, st);
+    if (n <= 0) return cudaSuccess;
+    Workspace ws;
+    ws.add(sizeof(unsigned) * scan_scratch(n));
+    PD_TRY(ws.alloc());
+    const cudaError_t e = exclusive_scan(in, out, n, ws.at<unsigned>(0), st);
+    const cudaError_t e2 = cudaStreamSynchronize(st);
+    return e != cudaSuccess ? e : e2;
 }
 
 cudaError_t sort_pairs_u32(unsigned* keys, int* vals, int n, int key_bits, cudaStream_t st)
 {
     if (n <= 1) return cudaSuccess;
     const int tiles = (n + kSortTile - 1) / kSortTile;
-    unsigned *k1 = nullptr, *hist = nullptr;
-    int* v1 = nullptr;
-    PD_TRY(cudaMalloc(&k1, sizeof(unsigned) * n));
-    PD_TRY(cudaMalloc(&v1, sizeof(int) * n));
-    PD_TRY(cudaMalloc(&hist, sizeof(unsigned) * 256 * (size_t)tiles));
-    unsigned *ka = keys, *kb = k1;
-    int *va = vals, *vb = v1;
+    Workspace ws;
+    const size_t k1 = ws.add(sizeof(unsigned) * n), v1 = ws.add(sizeof(int) * n);
+    const size_t oh = ws.add(sizeof(unsigned) * 256 * (size_t)tiles), os = ws.add(sizeof(unsigned) * scan_scratch(256LL * tiles));
+    PD_TRY(ws.alloc());
+    unsigned *hist = ws.at<unsigned>(oh), *scan = ws.at<unsigned>(os);
+    unsigned *ka = keys, *kb = ws.at<unsigned>(k1);
+    int *va = vals, *vb = ws.at<int>(v1);
     cudaError_t e = cudaSuccess;
     for (int shift = 0; shift < key_bits && e == cudaSuccess; shift += 8) {
         k_radix_hist<<<tiles, kSortThreads, 0, st>>>(ka, n, shift, tiles, hist);
-        e = exclusive_scan(hist, hist, 256LL * tiles, st);
+        e = exclusive_scan(hist, hist, 256LL * tiles, scan, st);
         if (e != cudaSuccess) break;
         k_radix_scatter<<<tiles, kSortThreads, 0, st>>>(ka, va, n, shift, tiles, hist, kb, vb);
         std::swap(ka, kb);
@@ -411,9 +446,6 @@ cudaError_t sort_pairs_u32(unsigned* keys, int* vals, int n, int key_bits, cudaS
     }
     if (e == cudaSuccess) e = cudaGetLastError();
     cudaError_t e2 = cudaStreamSynchronize(st);
-    cudaFree(k1);
-    cudaFree(v1);
-    cudaFree(hist);
     return e != cudaSuccess ? e : e2;
 }
 
@@ -503,38 +535,36 @@ cudaError_t build_bonds(const dbl4* pos_orig, int n, double horizon, int max_bon
     const int key_bits = 3 * std::max(bits, 1);
 
     // keys + sort
-    unsigned *k0 = nullptr, *k1 = nullptr, *hist = nullptr;
-    int *v0 = nullptr, *v1 = nullptr;
     const int tiles = (n + kSortTile - 1) / kSortTile;
-    PD_TRY(cudaMalloc(&k0, sizeof(unsigned) * n));
-    PD_TRY(cudaMalloc(&k1, sizeof(unsigned) * n));
-    PD_TRY(cudaMalloc(&v0, sizeof(int) * n));
-    PD_TRY(cudaMalloc(&v1, sizeof(int) * n));
-    PD_TRY(cudaMalloc(&hist, sizeof(unsigned) * 256 * (size_t)tiles));
+    Workspace ws;
+    const size_t words = sizeof(unsigned) * (size_t)n;
+    const size_t ok0 = ws.add(words), ok1 = ws.add(words), ov1 = ws.add(words);
+    const size_t oh = ws.add(sizeof(unsigned) * 256 * (size_t)tiles);
+    const size_t os = ws.add(sizeof(unsigned) * scan_scratch(std::max(256LL * tiles, (long long)n + 1)));
+    const size_t ocell = ws.add(sizeof(int) * 2 * (size_t)ncell), opad = ws.add(words + sizeof(unsigned));
+    const size_t oflag = ws.add(4 * sizeof(int));
+    PD_TRY(ws.alloc());
+    unsigned *k0 = ws.at<unsigned>(ok0), *k1 = ws.at<unsigned>(ok1), *hist = ws.at<unsigned>(oh), *scan = ws.at<unsigned>(os);
+    int *v0 = nullptr, *v1 = ws.at<int>(ov1);
+    PD_TRY(cudaMalloc(&out->perm, words));   // slot -> caller index (owned by the caller from here)
+    v0 = out->perm;
     k_cell_keys<<<grid_for(n), kBlock, 0, st>>>(pos_orig, n, g, k0, v0);
     for (int shift = 0; shift < key_bits; shift += 8) {
         k_radix_hist<<<tiles, kSortThreads, 0, st>>>(k0, n, shift, tiles, hist);
-        PD_TRY(exclusive_scan(hist, hist, 256LL * tiles, st));
+        PD_TRY(exclusive_scan(hist, hist, 256LL * tiles, scan, st));
         k_radix_scatter<<<tiles, kSortThreads, 0, st>>>(k0, v0, n, shift, tiles, hist, k1, v1);
         std::swap(k0, k1);
         std::swap(v0, v1);
     }
     PD_TRY(cudaGetLastError());
-    cudaFree(hist);
-    cudaFree(k1);
-    cudaFree(v1);
-    out->perm = v0;   // slot -> caller index (owned by the caller from here)
+    if (v0 != out->perm) PD_TRY(cudaMemcpyAsync(out->perm, v0, words, cudaMemcpyDeviceToDevice, st));
     gather_double4(pos_orig, out->perm, pos_sorted, n, st);
     make_local32(pos_sorted, origin[0], origin[1], origin[2], x32_sorted, nullptr, n, st);
 
     // cell ranges
-    int *cstart = nullptr, *cend = nullptr;
-    PD_TRY(cudaMalloc(&cstart, sizeof(int) * (size_t)ncell));
-    PD_TRY(cudaMalloc(&cend, sizeof(int) * (size_t)ncell));
-    PD_TRY(cudaMemsetAsync(cstart, 0, sizeof(int) * (size_t)ncell, st));
-    PD_TRY(cudaMemsetAsync(cend, 0, sizeof(int) * (size_t)ncell, st));
+    int *cstart = ws.at<int>(ocell), *cend = cstart + ncell;
+    PD_TRY(cudaMemsetAsync(cstart, 0, sizeof(int) * 2 * (size_t)ncell, st));
     k_cell_ranges<<<grid_for(n), kBlock, 0, st>>>(pos_sorted, k0, n, g, cstart, cend);
-    cudaFree(k0);
 
     // FP32 prefilter bounds: positions relative to the box centre carry a
     // rounding error below 2^-24 |x| per coordinate; the margin covers 4x the
@@ -550,24 +580,25 @@ cudaError_t build_bonds(const dbl4* pos_orig, int n, double horizon, int max_bon
     Q.h2_out = (float)(h2 * (1.0 + eps));
     if (!(horizon > 0)) { Q.h2_in = -1.f; Q.h2_out = -1.f; }
 
-    unsigned* cnt = nullptr;
-    unsigned* padded = nullptr;
-    int* flags = nullptr;
-    PD_TRY(cudaMalloc(&cnt, sizeof(unsigned) * n));
-    PD_TRY(cudaMalloc(&padded, sizeof(unsigned) * ((size_t)n + 1)));
-    PD_TRY(cudaMalloc(&flags, sizeof(int) * 2));
-    PD_TRY(cudaMemsetAsync(flags, 0, sizeof(int) * 2, st));
+    unsigned* cnt = k1;   // (the sort is done with it)
+    unsigned* padded = ws.at<unsigned>(opad);
+    int* flags = ws.at<int>(oflag);   // overflow, largest row, bonds (64 bits)
+    PD_TRY(cudaMemsetAsync(flags, 0, sizeof(int) * 4, st));
     k_bond_query<false><<<grid_for(n), kBlock, 0, st>>>(pos_sorted, x32_sorted, n, Q, cstart, cend, cnt, nullptr, nullptr);
     k_pad_counts<<<grid_for(n), kBlock, 0, st>>>(cnt, n, max_bonds, padded, out->cnt, flags);
     PD_TRY(cudaMemsetAsync(padded + n, 0, sizeof(unsigned), st));
-    PD_TRY(exclusive_scan(padded, padded, (long long)n + 1, st));
-    int hflags[2] = {0, 0};
+    PD_TRY(exclusive_scan(padded, padded, (long long)n + 1, scan, st));
+    struct {
+        int overflow, most;
+        unsigned long long bonds;
+    } hflags = {0, 0, 0ull};
     unsigned total = 0;
-    PD_TRY(cudaMemcpyAsync(hflags, flags, sizeof(hflags), cudaMemcpyDeviceToHost, st));
+    PD_TRY(cudaMemcpyAsync(&hflags, flags, sizeof(hflags), cudaMemcpyDeviceToHost, st));
     PD_TRY(cudaMemcpyAsync(&total, padded + n, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     PD_TRY(cudaStreamSynchronize(st));
-    out->overflow = hflags[0];
-    out->max_bonds = hflags[1];
+    out->overflow = hflags.overflow;
+    out->max_bonds = hflags.most;
+    out->bonds = (long long)hflags.bonds;
     // row_ptr (int) from the padded scan
     PD_TRY(cudaMemcpyAsync(out->row_ptr, padded, sizeof(int) * ((size_t)n + 1), cudaMemcpyDeviceToDevice, st));
     out->total = total;
@@ -581,19 +612,6 @@ cudaError_t build_bonds(const dbl4* pos_orig, int n, double horizon, int max_bon
         out->overflow = 2;
     }
     PD_TRY(cudaStreamSynchronize(st));
-    // live bond count
-    {
-        std::vector<int> hc(n);
-        PD_TRY(cudaMemcpy(hc.data(), out->cnt, sizeof(int) * n, cudaMemcpyDeviceToHost));
-        long long b = 0;
-        for (int i = 0; i < n; ++i) b += hc[i];
-        out->bonds = b;
-    }
-    cudaFree(cnt);
-    cudaFree(padded);
-    cudaFree(flags);
-    cudaFree(cstart);
-    cudaFree(cend);
     return cudaGetLastError();
 }
 

@@ -133,10 +133,7 @@ void Engine::free_all()
 {
     ws_free();
     hist_free();
-    void* ptrs[] = {S_.act, S_.x64, S_.v64, S_.X64, S_.x64_bk, S_.v64_bk, S_.st, S_.ost, S_.nst, S_.row_ptr,
-                    S_.cnt, S_.cnt_bk, S_.col, S_.X32, S_.u32, S_.xs4, S_.inv_d0, S_.jac, S_.jdiag, S_.force, S_.rhs, S_.sol,
-                    S_.r, S_.p, S_.y, S_.z, S_.pc, S_.sc, S_.partials, S_.counters, S_.flags, S_.lidx, S_.d0sq, S_.lim,
-                    S_.xlo4, d_perm_, d_stage_};
+    void* ptrs[] = {d_state_, S_.col, S_.inv_d0, S_.jac, S_.lidx, S_.d0sq, d_perm_, d_stage_};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     free_tiles(S_);
@@ -156,6 +153,7 @@ void Engine::free_all()
     cudaFree(contact_.list);
     contact_ = ContactBuffers{};
     S_ = DeviceState{};
+    d_state_ = nullptr;
     d_perm_ = nullptr;
     d_stage_ = nullptr;
     stage_cap_ = 0;
@@ -166,41 +164,43 @@ pd_status Engine::allocate()
     const size_t n = (size_t)n_;
     const size_t r4 = fp64_ ? sizeof(dbl4) : sizeof(float4);
     S_.n = n_;
-    CK(dalloc(&S_.act, n), "alloc act");
-    CK(dalloc(&S_.x64, n), "alloc x");
-    CK(dalloc(&S_.v64, n), "alloc v");
-    CK(dalloc(&S_.X64, n), "alloc X");
-    CK(dalloc(&S_.x64_bk, n), "alloc x backup");
-    CK(dalloc(&S_.v64_bk, n), "alloc v backup");
-    CK(dalloc(&S_.st, n), "alloc stretch");
-    CK(dalloc(&S_.ost, n), "alloc original stretch");
-    CK(dalloc(&S_.nst, n), "alloc new stretch");
-    CK(dalloc(&S_.lim, n), "alloc stretch limits");
-    CK(dalloc(&S_.row_ptr, n + 1), "alloc row_ptr");
-    CK(dalloc(&S_.cnt, n), "alloc cnt");
-    CK(dalloc(&S_.cnt_bk, n), "alloc cnt backup");
-    CK(dalloc(&S_.X32, n), "alloc X32");
-    CK(dalloc(&S_.u32, n), "alloc u32");
-    if (!fp64_) CK(dalloc(&S_.xs4, n), "alloc xs4");
-    if (!fp64_) CK(dalloc(&S_.xlo4, n), "alloc xlo4");
+    // the state in one allocation: about forty of 5 to 10 us each took most of
+    // make_ready on small bodies
+    const size_t m = n ? n : 1;
+    size_t bytes = 0;
+    struct Part {
+        void** p;
+        size_t at;
+    };
+    std::vector<Part> parts;
+    const auto add = [&](auto** p, size_t size) {
+        parts.push_back(Part{(void**)p, bytes});
+        bytes += (size + 255) / 256 * 256;
+    };
     void** vecs[] = {&S_.force, &S_.rhs, &S_.sol, &S_.r, &S_.p, &S_.y};
-    for (void** v : vecs) {
-        CK(cudaMalloc(v, r4 * (n ? n : 1)), "alloc vector");
-        CK(cudaMemsetAsync(*v, 0, r4 * (n ? n : 1), stream_), "memset vector");
-    }
-    if (fp64_) CK(dalloc(&S_.jdiag, 6 * n), "alloc jdiag");
-    if (opt_.preconditioner) {   // z and the inverse diagonal blocks (two Real4 per particle)
-        CK(cudaMalloc(&S_.z, r4 * (n ? n : 1)), "alloc z");
-        CK(cudaMemsetAsync(S_.z, 0, r4 * (n ? n : 1), stream_), "memset z");
-        CK(cudaMalloc(&S_.pc, 2 * r4 * (n ? n : 1)), "alloc preconditioner");
-    }
-    CK(dalloc(&S_.sc, 1), "alloc scalars");
-    CK(dalloc(&S_.partials, 4 * (size_t)kMaxPartials), "alloc partials");
-    CK(dalloc(&S_.counters, 8), "alloc counters");
-    CK(dalloc(&S_.flags, 4), "alloc flags");
-    CK(cudaMemsetAsync(S_.counters, 0, sizeof(unsigned) * 8, stream_), "memset counters");
-    CK(cudaMemsetAsync(S_.flags, 0, sizeof(int) * 4, stream_), "memset flags");
-    CK(cudaMemsetAsync(S_.u32, 0, sizeof(float4) * (n ? n : 1), stream_), "memset u32");
+    for (void** v : vecs) add(v, r4 * m);
+    if (opt_.preconditioner) add(&S_.z, r4 * m);
+    add(&S_.u32, sizeof(float4) * m);
+    add(&S_.counters, sizeof(unsigned) * 8);
+    add(&S_.flags, sizeof(int) * 4);
+    const size_t zeroed = bytes;
+    if (opt_.preconditioner) add(&S_.pc, 2 * r4 * m);   // the inverse diagonal blocks (two Real4 per particle)
+    add(&S_.act, sizeof(*S_.act) * m);
+    for (dbl4** v : {&S_.x64, &S_.v64, &S_.X64, &S_.x64_bk, &S_.v64_bk}) add(v, sizeof(dbl4) * m);
+    for (double** v : {&S_.st, &S_.ost, &S_.nst}) add(v, sizeof(double) * m);
+    add(&S_.lim, sizeof(*S_.lim) * m);
+    add(&S_.row_ptr, sizeof(int) * (n + 1));
+    add(&S_.cnt, sizeof(int) * m);
+    add(&S_.cnt_bk, sizeof(int) * m);
+    add(&S_.X32, sizeof(float4) * m);
+    if (!fp64_) add(&S_.xs4, sizeof(float4) * m);
+    if (!fp64_) add(&S_.xlo4, sizeof(float4) * m);
+    if (fp64_) add(&S_.jdiag, sizeof(double) * 6 * m);
+    add(&S_.sc, sizeof(CgScalars));
+    add(&S_.partials, sizeof(double) * 4 * (size_t)kMaxPartials);
+    CK(dalloc(&d_state_, bytes), "alloc state");
+    for (const Part& q : parts) *q.p = d_state_ + q.at;
+    CK(cudaMemsetAsync(d_state_, 0, zeroed, stream_), "memset state");
     return PD_OK;
 }
 
@@ -220,16 +220,12 @@ pd_status Engine::make_ready()
 
     struct Tmp {   // staging buffers in caller order, freed on every return path
         dbl4* pos = nullptr;
-        double* s0 = nullptr;
-        int* act = nullptr;
-        ~Tmp() { cudaFree(pos); cudaFree(s0); cudaFree(act); }
+        ~Tmp() { cudaFree(pos); }
     } tmp;
-    CK(dalloc(&tmp.pos, N), "alloc tmp");
-    CK(dalloc(&tmp.s0, N), "alloc tmp");
-    CK(dalloc(&tmp.act, N), "alloc tmp");
+    CK(dalloc(&tmp.pos, 2 * N + 1), "alloc tmp");
     dbl4* d_tmp4 = tmp.pos;
-    double* d_tmp1 = tmp.s0;
-    int* d_tmpi = tmp.act;
+    double* d_tmp1 = (double*)(tmp.pos + N);
+    int* d_tmpi = (int*)(d_tmp1 + N);
 
     // bonds (replaces initPeridynamicsBonds' kd-tree, simulator.cu:825-943)
     if (n > 0) CK(cudaMemcpyAsync(d_tmp4, h_pos_.data(), sizeof(dbl4) * N, cudaMemcpyHostToDevice, stream_), "upload pos");
@@ -279,12 +275,9 @@ pd_status Engine::make_ready()
         CK(cudaMemcpyAsync(d_tmpi, h_act_.data(), sizeof(int) * N, cudaMemcpyHostToDevice, stream_), "upload act");
         gather_int_to_u8(d_tmpi, d_perm_, S_.act, n, stream_);
         // s0_i = getstretch(s0) after srand(1973), in caller order (simulator.cu:852-857)
-        std::vector<double> s0 = h_s0_;
-        if (!stretch_set_) {
-            s0.assign(N, 0.0);
-            pd_sample_stretch_limits(run_.pd_stretch_limit_s0, n, s0.data());
-        }
-        CK(cudaMemcpyAsync(d_tmp1, s0.data(), sizeof(double) * N, cudaMemcpyHostToDevice, stream_), "upload s0");
+        if (stretch_set_)
+            CK(cudaMemcpyAsync(d_tmp1, h_s0_.data(), sizeof(double) * N, cudaMemcpyHostToDevice, stream_), "upload s0");
+        else CK(sample_stretch_limits(run_.pd_stretch_limit_s0, n, d_tmp1, stream_), "sample s0");
         gather_double(d_tmp1, d_perm_, S_.ost, n, stream_);
         CK(cudaMemcpyAsync(S_.st, S_.ost, sizeof(double) * N, cudaMemcpyDeviceToDevice, stream_), "copy st");
         CK(cudaMemcpyAsync(S_.nst, S_.ost, sizeof(double) * N, cudaMemcpyDeviceToDevice, stream_), "copy nst");
@@ -309,7 +302,7 @@ pd_status Engine::make_ready()
         CK(cudaMemsetAsync(S_.d0sq, 0, sizeof(float2) * slots, stream_), "memset d0sq");
         if (n > 0) {
             const int g = (int)std::min<long long>(std::max<long long>(((long long)n + kBlock - 1) / kBlock, 1), kMaxPartials);
-            launch_bond_geometry(S_, g, stream_);
+            launch_bond_geometry(S_, stream_);
             ++launches_;
             if (lat_ok_) {
                 launch_lattice_ell(S_, lat_, 1, g, stream_);
@@ -468,7 +461,7 @@ pd_status Engine::tune_spmv()
             L_.grid_bonds = grid_for_rows(c.g, row_kernel_blocks_per_sm(fp64_, c.g, c.u));
         }
     };
-    if (cand.size() == 1 || n_ < 20000 || persist_.tiled_products) {
+    if (cand.size() == 1 || n_ < 20000 || persist_.tiled_products || batch_member_) {   // (a batch times its own shape)
         // small problems: launch overhead dominates, keep the default (the
         // tiled path when it was asked for)
         // As many lanes per row as one block per SM holds: FP64 10.4 us at 500
@@ -604,7 +597,7 @@ pd_status Engine::gang_tiles(int rows, int blocks, CgPersistPlan* plan, bool* fi
     }
     if (plan->bonds == 0) {
         CK(launch_bank_order(S_, n_, plan->lanes, 4, total_slots_, stream_), "order bonds");
-        launch_bond_geometry(S_, (int)std::min<long long>(((long long)n_ + kBlock - 1) / kBlock, kMaxPartials), stream_);
+        launch_bond_geometry(S_, stream_);
         launches_ += 2;
     }
     return PD_OK;

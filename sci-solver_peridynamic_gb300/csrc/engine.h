@@ -149,6 +149,7 @@ private:
     long long total_slots_ = 0;
     long long bonds_initial_ = 0;
     DeviceState S_{};
+    unsigned char* d_state_ = nullptr;   // the per-particle state and the scalars, one allocation
     int* d_perm_ = nullptr;
     void* d_stage_ = nullptr;     // exports in caller order before the copy to the host
     size_t stage_cap_ = 0;

@@ -281,12 +281,16 @@ __global__ void __launch_bounds__(kBlock) k_refresh(StepParams P, DeviceState S)
 }
 
 // 1 / d0 and d0^2 per bond slot from the FP64 original positions (once, after the bond build)
+// eight lanes per row: 54 us for 11k particles of 70 bonds, 155 with one
+constexpr int kGeometryLanes = 8;
 __global__ void __launch_bounds__(kBlock) k_bond_geometry(int n, DeviceState S)
 {
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
+    constexpr int G = kGeometryLanes;
+    const int lane = threadIdx.x & (G - 1);
+    for (int p = (blockIdx.x * blockDim.x + threadIdx.x) / G; p < n; p += gridDim.x * blockDim.x / G) {
         const dbl4 Xp = S.X64[p];
         const int rs = S.row_ptr[p], cn = S.cnt[p];
-        for (int j = 0; j < cn; ++j) {
+        for (int j = lane; j < cn; j += G) {
             const dbl4 Xq = S.X64[S.col[rs + j]];
             const double dx = dsub(Xp.x, Xq.x), dy = dsub(Xp.y, Xq.y), dz = dsub(Xp.z, Xq.z);
             const double d0s = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
@@ -297,9 +301,10 @@ __global__ void __launch_bounds__(kBlock) k_bond_geometry(int n, DeviceState S)
     }
 }
 
-void launch_bond_geometry(const DeviceState& S, int grid, cudaStream_t st)
+void launch_bond_geometry(const DeviceState& S, cudaStream_t st)
 {
-    k_bond_geometry<<<grid, kBlock, 0, st>>>(S.n, S);
+    const long long blocks = ((long long)S.n * kGeometryLanes + kBlock - 1) / kBlock;
+    k_bond_geometry<<<(int)(blocks < 65536 ? blocks : 65536), kBlock, 0, st>>>(S.n, S);
 }
 
 __global__ void __launch_bounds__(kBlock) k_stretch_limits(int n, DeviceState S)

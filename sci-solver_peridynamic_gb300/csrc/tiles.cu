@@ -28,6 +28,7 @@ namespace {
 
 constexpr int kHashBits = 13;
 constexpr int kHashCap = 1 << kHashBits;          // per-tile hash set of neighbour slots
+constexpr int kTileBuild = 1024;                  // threads of a tile: 101 us for 30 tiles of 370 rows, 290 with 256
 constexpr int kHashLimit = (kHashCap * 3) / 4;    // larger halos use the global path
 constexpr unsigned kEmpty = 0xffffffffu;
 
@@ -87,7 +88,7 @@ __device__ void sort_table(unsigned* t)
     }
 }
 
-__global__ void __launch_bounds__(kBlock) k_tile_count(DeviceState S, int n, unsigned* counts)
+__global__ void __launch_bounds__(kTileBuild) k_tile_count(DeviceState S, int n, unsigned* counts)
 {
     __shared__ unsigned table[kHashCap];
     for (int t = blockIdx.x; t < S.n_tiles; t += gridDim.x) {
@@ -101,7 +102,7 @@ __global__ void __launch_bounds__(kBlock) k_tile_count(DeviceState S, int n, uns
     }
 }
 
-__global__ void __launch_bounds__(kBlock) k_tile_fill(DeviceState S, int n)
+__global__ void __launch_bounds__(kTileBuild) k_tile_fill(DeviceState S, int n)
 {
     __shared__ unsigned table[kHashCap];
     for (int t = blockIdx.x; t < S.n_tiles; t += gridDim.x) {
@@ -366,7 +367,7 @@ cudaError_t build_tiles(DeviceState& S, int n, int* max_halo, int* unfit, cudaSt
     if (e == cudaSuccess) e = cudaMemsetAsync(counts, 0, sizeof(unsigned) * (nt + 1), st);
     const int grid = (int)(nt < 4096 ? nt : 4096);
     if (e == cudaSuccess) {
-        k_tile_count<<<grid, kBlock, 0, st>>>(S, n, counts);
+        k_tile_count<<<grid, kTileBuild, 0, st>>>(S, n, counts);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = scan_exclusive_u32(counts, (unsigned*)S.halo_ptr, (long long)nt + 1, st);
@@ -375,7 +376,7 @@ cudaError_t build_tiles(DeviceState& S, int n, int* max_halo, int* unfit, cudaSt
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e == cudaSuccess) e = cudaMalloc((void**)&S.halo, sizeof(int) * (size_t)(total > 0 ? total : 1));
     if (e == cudaSuccess) {
-        k_tile_fill<<<grid, kBlock, 0, st>>>(S, n);
+        k_tile_fill<<<grid, kTileBuild, 0, st>>>(S, n);
         e = cudaGetLastError();
     }
     std::vector<int> info(nt);
