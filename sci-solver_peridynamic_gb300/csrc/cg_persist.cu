@@ -31,6 +31,7 @@
 // sees the error.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "batch.h"
 #include "step_rows.cuh"
@@ -235,6 +236,48 @@ __device__ __forceinline__ BondGeometry bond_geometry(const float4& Xq, const fl
     return g;
 }
 
+// A halo position as 32-bit fixed point, supercell edge = 2^25, wrapping: the
+// difference of two positions less than 64 supercells apart is exact, in three
+// integer subtractions instead of the decoding of two words of supercell
+// coordinates (59 instructions per bond of the tile product, 77 with it).  The
+// offset's own rounding (2^-25 of the edge at most) is twice what the
+// conversion adds.  Blocks whose rows and halo reach farther than kFixedReach
+// supercells from their first row keep the decoding form.
+constexpr int kFixedBits = 25;
+constexpr int kFixedReach = 31;
+__device__ __forceinline__ float4 fixed_position(const float4& X, float per_edge)
+{
+    const unsigned c = (unsigned)__float_as_int(X.w);
+    const auto fix = [per_edge](float off, unsigned cell) {
+        return __int_as_float((int)((cell << kFixedBits) + (unsigned)__float2int_rn(off * per_edge)));
+    };
+    return make_float4(fix(X.x, c & 1023u), fix(X.y, (c >> 10) & 1023u), fix(X.z, (c >> 20) & 1023u), 0.f);
+}
+// (an offset outside its cell: the body has left the supercells' window)
+__device__ __forceinline__ bool farther(const float4& X, int ref, float sup)
+{
+    const int w = __float_as_int(X.w);
+    const bool inside = fabsf(X.x) <= sup && fabsf(X.y) <= sup && fabsf(X.z) <= sup;
+    return !inside || abs((w & 1023) - (ref & 1023)) > kFixedReach || abs(((w >> 10) & 1023) - ((ref >> 10) & 1023)) > kFixedReach ||
+           abs(((w >> 20) & 1023) - ((ref >> 20) & 1023)) > kFixedReach;
+}
+// `per_edge` is 2^25 / edge (a power of two): the bond vector is in units of
+// 1 / per_edge, and so is i3, which the product takes with it twice.
+__device__ __forceinline__ BondGeometry bond_geometry_fixed(const float4& Xq, const float4& xp, float per_edge,
+                                                            float inv_d0, float& a1)
+{
+    BondGeometry g;
+    g.x = (float)(__float_as_int(Xq.x) - __float_as_int(xp.x));
+    g.y = (float)(__float_as_int(Xq.y) - __float_as_int(xp.y));
+    g.z = (float)(__float_as_int(Xq.z) - __float_as_int(xp.z));
+    float inv;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(fmaf(g.x, g.x, fmaf(g.y, g.y, g.z * g.z))));
+    const float inv_d = inv * per_edge;
+    g.i3 = inv * inv * inv_d;
+    a1 = inv_d0 - inv_d;
+    return g;
+}
+
 // Four consecutive bonds' halo indices and 1/d0.
 __device__ __forceinline__ void load_bonds(const DeviceState& S, int slot, int (&l)[4], float (&id0)[4])
 {
@@ -249,11 +292,16 @@ __device__ __forceinline__ void load_bonds(const DeviceState& S, int slot, int (
 // CACHED: the bonds' geometry stays in shared memory; else the halo's
 // positions do, and the index and 1/d0 of a bond are read from global memory
 // (6 bytes per bond, from L2).  Not cached, the product is bound by the
-// shared-memory pipe and by latency (one block per SM): four consecutive bonds
-// per lane and load, the next four in flight, and the rows' order from
-// k_bank_order take an iteration at 100k particles (76 bonds) from 38.2 us to
-// 31.2; with 8 lanes per row 34.9 (37.5 without the order), with 1024 threads
-// 30.3 (but 24.0 against 21.8 at 50k and 104 bonds).
+// shared-memory pipe (7.2 wavefronts per step of 32 bonds and array when bonds
+// stood in build order) and by latency (one block per SM).  An iteration at 100k
+// particles (76 bonds) takes 25.3 us: 38.2 with scalar loads of the bonds, 31.2
+// with four per lane and load and the next four in flight, 30.4 with a round of
+// their own for the rows left over, 30.0 with fixed-point positions, 25.3 with
+// the order of k_bank_order.  Eight lanes per row: 34.9 against 31.2; 1024
+// threads 30.3 (but 24.0 against 21.8 at 50k and 104 bonds).
+template <int N>
+using Lanes = std::integral_constant<int, N>;
+
 // `epoch` is the last epoch used in the inbox and the records.  Blocks beyond the
 // last row only exchange.  Returns false when a wait ran out of time.
 template <bool CACHED, int G, int U>
@@ -301,8 +349,18 @@ __device__ __forceinline__ bool persist_solve32(const StepParams& P, const Devic
         if (!CACHED) shx[h] = S.xs4[q];
     }
     if (threadIdx.x == 0) ex.error = 0;
+    const float sup = (float)P.sup, per_edge = (float)(1 << kFixedBits) / sup;
+    bool fixed = false;
+    if (!CACHED) {   // the entries that this thread has staged
+        const int ref = nr > 0 ? __float_as_int(S.xs4[lo].w) : 0;
+        bool far = false;
+        for (int t = threadIdx.x; t < nr; t += kPersistThreads) far |= farther(S.xs4[lo + t], ref, sup);
+        for (int h = threadIdx.x; h < nh; h += kPersistThreads) far |= farther(shx[h], ref, sup);
+        fixed = !__syncthreads_or(far);
+        if (fixed)
+            for (int h = threadIdx.x; h < nh; h += kPersistThreads) shx[h] = fixed_position(shx[h], per_edge);
+    }
     __syncthreads();
-    const float sup = (float)P.sup;
     if (CACHED) {
         for (int i = threadIdx.x / G; i < nr; i += NG) {
             const int cn = scnt[i] < 0 ? 0 : scnt[i] >> 8, base = srow[i];
@@ -334,67 +392,89 @@ __device__ __forceinline__ bool persist_solve32(const StepParams& P, const Devic
         }
         __syncthreads();
         DotAcc32 acc;
-        for (int i = threadIdx.x / G; i < nr; i += NG) {
-            const int cn = scnt[i] >> 8, base = srow[i], p = lo + i;
-            int l[U];
-            float a1[U];
-            // the bond records of one step: index, and 1/d0 - 1/d (CACHED) or
-            // 1/d0; U consecutive slots in one load each (not CACHED: rows start
-            // 32-byte aligned and hold a multiple of 8 slots)
-            const auto load = [&](int j0) {
-                if constexpr (CACHED) {
+        const auto rows = [&](auto width, auto form, int from, int to) {
+            constexpr int R = decltype(width)::value;   // lanes per row
+            constexpr bool FIXED = decltype(form)::value;
+            const int rl = threadIdx.x & (R - 1);
+            const unsigned rmask = group_mask<R>();
+            for (int i = from + threadIdx.x / R; i < to; i += kPersistThreads / R) {
+                const int cn = scnt[i] >> 8, base = srow[i], p = lo + i;
+                int l[U];
+                float a1[U];
+                // the bond records of one step: index, and 1/d0 - 1/d (CACHED) or
+                // 1/d0; U consecutive slots in one load each (not CACHED: rows start
+                // 32-byte aligned and hold a multiple of 8 slots)
+                const auto load = [&](int j0) {
+                    if constexpr (CACHED) {
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            const int j = j0 + u * R;
+                            l[u] = 0;
+                            a1[u] = 0.f;
+                            if (j < cn) {
+                                l[u] = sl[base + j];
+                                a1[u] = sa1[base + j];
+                            }
+                        }
+                    } else if (j0 < cn) {
+                        load_bonds(S, base + j0, l, a1);
+                    }
+                };
+                constexpr int LS = CACHED ? 1 : U, US = CACHED ? R : 1;   // slots between lanes, between a lane's bonds
+                load(rl * LS);
+                float4 xp = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (!CACHED && cn > 0) xp = __ldg(S.xs4 + p);
+                if (FIXED) xp = fixed_position(xp, per_edge);
+                float4 w = sp[i];
+                const float4 r = sr[i];
+                w = make_float4(r.x + beta * w.x, r.y + beta * w.y, r.z + beta * w.z, 0.f);
+                float ax = 0.f, ay = 0.f, az = 0.f;
+                for (int j0 = rl * LS; j0 < cn; j0 += R * U) {
+                    int lc[U];
+                    float ac[U];
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
-                        const int j = j0 + u * G;
-                        l[u] = 0;
-                        a1[u] = 0.f;
-                        if (j < cn) {
-                            l[u] = sl[base + j];
-                            a1[u] = sa1[base + j];
-                        }
+                        lc[u] = l[u];
+                        ac[u] = a1[u];
                     }
-                } else if (j0 < cn) {
-                    load_bonds(S, base + j0, l, a1);
-                }
-            };
-            constexpr int LS = CACHED ? 1 : U, US = CACHED ? G : 1;   // slots between lanes, between a lane's bonds
-            load(lane * LS);
-            float4 xp = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (!CACHED && cn > 0) xp = __ldg(S.xs4 + p);
-            float4 w = sp[i];
-            const float4 r = sr[i];
-            w = make_float4(r.x + beta * w.x, r.y + beta * w.y, r.z + beta * w.z, 0.f);
-            float ax = 0.f, ay = 0.f, az = 0.f;
-            for (int j0 = lane * LS; j0 < cn; j0 += G * U) {
-                int lc[U];
-                float ac[U];
+                    load(j0 + R * U);   // in flight while this step's bonds are added
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    lc[u] = l[u];
-                    ac[u] = a1[u];
+                    for (int u = 0; u < U; ++u) {
+                        const int j = j0 + u * US;
+                        if (!FIXED && j >= cn) continue;
+                        const float4 Wq = sw[lc[u]];
+                        BondGeometry g;
+                        float a = ac[u];
+                        if constexpr (CACHED) g = sg[base + j];
+                        else if constexpr (FIXED) g = bond_geometry_fixed(shx[lc[u]], xp, per_edge, ac[u], a);
+                        else g = bond_geometry(shx[lc[u]], xp, sup, ac[u], a);
+                        if (FIXED && j >= cn) a = g.i3 = 0.f;   // (every slot of a row has a halo index)
+                        const float wx = w.x - Wq.x, wy = w.y - Wq.y, wz = w.z - Wq.z;
+                        const float d = fmaf(g.x, wx, fmaf(g.y, wy, g.z * wz)) * g.i3;
+                        ax = fmaf(a, wx, fmaf(d, g.x, ax));
+                        ay = fmaf(a, wy, fmaf(d, g.y, ay));
+                        az = fmaf(a, wz, fmaf(d, g.z, az));
+                    }
                 }
-                load(j0 + G * U);   // in flight while this step's bonds are added
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int j = j0 + u * US;
-                    if (j >= cn) continue;
-                    const float4 Wq = sw[lc[u]];
-                    BondGeometry g;
-                    float a = ac[u];
-                    if constexpr (CACHED) g = sg[base + j];
-                    else g = bond_geometry(shx[lc[u]], xp, sup, ac[u], a);
-                    const float wx = w.x - Wq.x, wy = w.y - Wq.y, wz = w.z - Wq.z;
-                    const float d = fmaf(g.x, wx, fmaf(g.y, wy, g.z * wz)) * g.i3;
-                    ax = fmaf(a, wx, fmaf(d, g.x, ax));
-                    ay = fmaf(a, wy, fmaf(d, g.y, ay));
-                    az = fmaf(a, wz, fmaf(d, g.z, az));
-                }
+                if (cn >= 0) spmv_finish_mixed<R, true>(P, S, p, (uint8_t)scnt[i], w, ax, ay, az, rl, rmask, sy - lo, acc);
+                else if (rl == 0) sy[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                __syncwarp(rmask);   // every lane has read sp[i]
+                if (rl == 0) sp[i] = w;
             }
-            if (cn >= 0) spmv_finish_mixed<G, true>(P, S, p, (uint8_t)scnt[i], w, ax, ay, az, lane, gmask, sy - lo, acc);
-            else if (lane == 0) sy[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            __syncwarp(gmask);   // every lane has read sp[i]
-            if (lane == 0) sp[i] = w;
-        }
+        };
+        // The rows left over from whole rounds of the block's groups take a round of
+        // their own with more lanes each.
+        const int whole = CACHED ? nr : nr / NG * NG, left = nr - whole;
+        const auto all_rows = [&](auto form) {
+            rows(Lanes<G>(), form, 0, 2 * left > NG ? nr : whole);
+            if (!CACHED && left > 0 && 2 * left <= NG) {
+                if (4 * left <= NG) rows(Lanes<4 * kTileLanes>(), form, whole, nr);
+                else rows(Lanes<2 * kTileLanes>(), form, whole, nr);
+            }
+        };
+        if constexpr (CACHED) all_rows(std::false_type());
+        else if (fixed) all_rows(std::true_type());
+        else all_rows(std::false_type());
         pAp = acc.v;
         if (!exchange_sum(ex, pAp, G, A, ++epoch, [](int, int) {})) return false;
         alpha = df_quotient(rz, pAp);
@@ -470,8 +550,8 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist32(PersistArgs
 
 // One product y = A w outside a solve by the same rows and halos, bonds read as
 // the uncached solve reads them, and bound like it.  The gather product, whose
-// every bond reads two 16-byte records through L1, takes 45.3 us at 100k
-// particles of 104 bonds, this one 38.8 (41.1 with 512 threads).
+// every bond reads two 16-byte records through L1, takes 35.3 us at 100k
+// particles of 76 bonds, this one 26.7.
 template <bool DOT>
 __global__ void __launch_bounds__(kTileBlock, 1)
     k_tile_product32(StepParams P, DeviceState S, int rows, int halo, const float4* __restrict__ in,
@@ -483,16 +563,14 @@ __global__ void __launch_bounds__(kTileBlock, 1)
     float4* shx = sw + halo;
     const int lo = blockIdx.x * rows;
     const int nr = min(rows, P.n - lo);
-    const int lane = threadIdx.x & (G - 1);
-    const unsigned gmask = group_mask<G>();
     // a row's own data and its first bonds, in flight while the halo is staged
     // (the block's later rows: while the row before them is finished)
     int rs = 0, cn = -1, l[4];
     float id0[4];
     uint8_t ab = 0;
     float4 w, xp;
-    const auto fetch = [&](int i) {
-        if (i >= nr) return;
+    const auto fetch = [&](int i, int end, int lane) {
+        if (i >= end) return;
         const int p = lo + i;
         rs = __ldg(S.row_ptr + p);
         cn = S.cnt[p];
@@ -502,48 +580,80 @@ __global__ void __launch_bounds__(kTileBlock, 1)
         if (is_dirichlet(ab & kActMask)) cn = -1;
         if (lane * 4 < cn) load_bonds(S, rs + lane * 4, l, id0);
     };
-    fetch(threadIdx.x / G);
+    // (the rows left over from whole rounds: with more lanes each, as in the solve)
+    constexpr int NG = kTileBlock / G;
+    const int left = nr % NG, whole = 2 * left > NG ? nr : nr - left;
+    if (whole > 0) fetch(threadIdx.x / G, whole, threadIdx.x & (G - 1));
     const int h0 = S.halo_ptr[blockIdx.x], nh = S.halo_ptr[blockIdx.x + 1] - h0;
+    const float sup = (float)P.sup, per_edge = (float)(1 << kFixedBits) / sup;
+    const int ref = nr > 0 ? __float_as_int(__ldg(S.xs4 + lo).w) : 0;
+    bool far = false;
+    for (int t = threadIdx.x; t < nr; t += kTileBlock) far |= farther(__ldg(S.xs4 + lo + t), ref, sup);
     for (int h = threadIdx.x; h < nh; h += kTileBlock) {
         const int q = __ldg(S.halo + h0 + h);
+        const float4 X = __ldg(S.xs4 + q);
         sw[h] = __ldg(in + q);
-        shx[h] = __ldg(S.xs4 + q);
+        far |= farther(X, ref, sup);
+        shx[h] = fixed_position(X, per_edge);
     }
-    __syncthreads();
-    const float sup = (float)P.sup;
+    const bool fixed = !__syncthreads_or(far);
+    if (!fixed) {
+        for (int h = threadIdx.x; h < nh; h += kTileBlock) shx[h] = __ldg(S.xs4 + __ldg(S.halo + h0 + h));
+        __syncthreads();
+    }
     DotAcc32 acc;
-    for (int i = threadIdx.x / G; i < nr; i += kTileBlock / G) {
-        float ax = 0.f, ay = 0.f, az = 0.f;
-        for (int j0 = lane * 4; j0 < cn; j0 += G * 4) {
-            int lc[4];
-            float ic[4];
+    const auto tile_rows = [&](auto width, auto form, int from, int to) {
+        constexpr int R = decltype(width)::value;
+        constexpr bool FIXED = decltype(form)::value;
+        const int lane = threadIdx.x & (R - 1);
+        const unsigned gmask = group_mask<R>();
+        if (from > 0 || R != G) fetch(from + threadIdx.x / R, to, lane);
+        for (int i = from + threadIdx.x / R; i < to; i += kTileBlock / R) {
+            float ax = 0.f, ay = 0.f, az = 0.f;
+            const float4 x = FIXED ? fixed_position(xp, per_edge) : xp;
+            for (int j0 = lane * 4; j0 < cn; j0 += R * 4) {
+                int lc[4];
+                float ic[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                lc[u] = l[u];
-                ic[u] = id0[u];
-            }
-            if (j0 + G * 4 < cn) load_bonds(S, rs + j0 + G * 4, l, id0);   // in flight while this step's bonds are added
+                for (int u = 0; u < 4; ++u) {
+                    lc[u] = l[u];
+                    ic[u] = id0[u];
+                }
+                if (j0 + R * 4 < cn) load_bonds(S, rs + j0 + R * 4, l, id0);   // in flight while this step's bonds are added
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (j0 + u >= cn) continue;
-                const float4 Wq = sw[lc[u]];
-                float a1;
-                const BondGeometry g = bond_geometry(shx[lc[u]], xp, sup, ic[u], a1);
-                const float wx = w.x - Wq.x, wy = w.y - Wq.y, wz = w.z - Wq.z;
-                const float d = fmaf(g.x, wx, fmaf(g.y, wy, g.z * wz)) * g.i3;
-                ax = fmaf(a1, wx, fmaf(d, g.x, ax));
-                ay = fmaf(a1, wy, fmaf(d, g.y, ay));
-                az = fmaf(a1, wz, fmaf(d, g.z, az));
+                for (int u = 0; u < 4; ++u) {
+                    if (!FIXED && j0 + u >= cn) continue;
+                    const float4 Wq = sw[lc[u]];
+                    float a1;
+                    BondGeometry g;
+                    if constexpr (FIXED) g = bond_geometry_fixed(shx[lc[u]], x, per_edge, ic[u], a1);
+                    else g = bond_geometry(shx[lc[u]], x, sup, ic[u], a1);
+                    if (FIXED && j0 + u >= cn) a1 = g.i3 = 0.f;
+                    const float wx = w.x - Wq.x, wy = w.y - Wq.y, wz = w.z - Wq.z;
+                    const float d = fmaf(g.x, wx, fmaf(g.y, wy, g.z * wz)) * g.i3;
+                    ax = fmaf(a1, wx, fmaf(d, g.x, ax));
+                    ay = fmaf(a1, wy, fmaf(d, g.y, ay));
+                    az = fmaf(a1, wz, fmaf(d, g.z, az));
+                }
             }
+            const int p = lo + i;
+            const uint8_t row_ab = ab;
+            const float4 row_w = w;
+            const bool fixed = cn < 0;
+            fetch(i + kTileBlock / R, to, lane);
+            if (!fixed) spmv_finish_mixed<R, DOT>(P, S, p, row_ab, row_w, ax, ay, az, lane, gmask, out, acc);
+            else if (lane == 0) out[p] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        const int p = lo + i;
-        const uint8_t row_ab = ab;
-        const float4 row_w = w;
-        const bool fixed = cn < 0;
-        fetch(i + kTileBlock / G);
-        if (!fixed) spmv_finish_mixed<G, DOT>(P, S, p, row_ab, row_w, ax, ay, az, lane, gmask, out, acc);
-        else if (lane == 0) out[p] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
+    };
+    const auto all_rows = [&](auto form) {
+        tile_rows(Lanes<G>(), form, 0, whole);
+        if (whole < nr) {
+            if (4 * left <= NG) tile_rows(Lanes<4 * G>(), form, whole, nr);
+            else tile_rows(Lanes<2 * G>(), form, whole, nr);
+        }
+    };
+    if (fixed) all_rows(std::true_type());
+    else all_rows(std::false_type());
     if (DOT) block_reduce_finish(acc, slot, [dot_out](double pAp) { *dot_out = pAp; });
 }
 

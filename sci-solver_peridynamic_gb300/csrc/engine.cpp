@@ -253,8 +253,8 @@ pd_status Engine::make_ready()
     // larger lattice-filled bodies are renumbered brick by brick for the stencil
     // product (mixed mode; automatic above kLatticeMinRows particles, or asked
     // for with spmv_path 3).  Other bodies keep the builder's order and the
-    // gather product.  (Per CG iteration, one launch against the stencil: 27
-    // us against 44 at 50k particles and a horizon of 3 spacings, 38 against
+    // gather product.  (Per CG iteration, one launch against the stencil: 18
+    // us against 44 at 50k particles and a horizon of 3 spacings, 25 against
     // 50 at 100k and 2.5.)
     if (opt_.spmv_path == 0 || opt_.spmv_path == 2) {
         s = persist_prepare();
@@ -561,13 +561,13 @@ pd_status Engine::persist_prepare()
         return PD_OK;
     }
     // Below kTileMinSlots bond slots the gather product is the faster one outside
-    // the solve: 12.4 us against 15.1 at 18k particles and 76 bonds each, 15.0
-    // against 16.5 at 40k and 29; above, 20.3 against 19.8 at 30k and 104, 35.9
-    // against 31.8 at 100k and 76, 45.3 against 38.8 at 100k and 104.
+    // the solve: 12.4 us against 16.4 at 18k particles and 76 bonds each, 14.5
+    // against 16.5 at 40k and 29; above, 18.5 against 16.5 at 24k and 104, 22.8
+    // against 18.6 at 40k and 76, 35.3 against 26.7 at 100k and 76.
     // (A fixed lanes_per_particle or spmv_unroll names a shape of the gather.)
     plan.tiled_products = plan.tiled_products && total_slots_ >= kTileMinSlots && !opt_.lanes_per_particle && !opt_.spmv_unroll;
     if (plan.tiled_products)
-        CK(launch_bank_order(S_, n_, plan.lanes, 4, total_slots_, stream_), "order bonds");
+        CK(launch_bank_order(S_, n_, total_slots_, stream_), "order bonds");
     const size_t inbox = 2 * (size_t)plan.grid * plan.grid, rec = (fp64_ ? 2 : 1) * (size_t)n_;
     CK(dalloc(&d_inbox_, inbox + rec), "alloc records");
     CK(cudaMemsetAsync(d_inbox_, 0, sizeof(ulonglong2) * (inbox + rec), stream_), "memset records");
@@ -596,7 +596,7 @@ pd_status Engine::gang_tiles(int rows, int blocks, CgPersistPlan* plan, bool* fi
         return PD_OK;
     }
     if (plan->bonds == 0) {
-        CK(launch_bank_order(S_, n_, plan->lanes, 4, total_slots_, stream_), "order bonds");
+        CK(launch_bank_order(S_, n_, total_slots_, stream_), "order bonds");
         launch_bond_geometry(S_, stream_);
         launches_ += 2;
     }

@@ -157,7 +157,7 @@ struct DeviceState {
 // stencil entry) streams from a table in which 0 marks "no live bond" (no
 // particle there, beyond the horizon, or broken).
 constexpr int kLatMaxOffsets = 160;  // distinct bond offsets at most
-constexpr long long kTileMinSlots = 3000000;   // bond slots from which the one-launch bodies' other products use its tiles
+constexpr long long kTileMinSlots = 2200000;   // bond slots from which the one-launch bodies' other products use its tiles
 constexpr int kLatticeMinRows = 20000;   // automatic choice: smaller bodies keep the gather product
 constexpr int kLatticeOnlyRows = 250000; // automatic choice: larger lattice bodies time only the stencil variants
 constexpr int kLatRmax = 3;          // largest offset per axis (sites)
@@ -323,9 +323,8 @@ void launch_bond_relayout(const DeviceState& S, int grid, int g_from, int u_from
 // the builder's hash set in *unfit.
 cudaError_t build_tiles(DeviceState& S, int n, int* max_halo, int* unfit, cudaStream_t st);
 // Reorders every row's bonds (col, lidx; the geometry arrays not yet formed) for
-// few bank conflicts among those that `lanes` lanes, each reading `unroll`
-// consecutive slots, look up together.
-cudaError_t launch_bank_order(const DeviceState& S, int n, int lanes, int unroll, long long slots, cudaStream_t st);
+// few bank conflicts in the look-ups of four lanes per row with four bonds each.
+cudaError_t launch_bank_order(const DeviceState& S, int n, long long slots, cudaStream_t st);
 void free_tiles(DeviceState& S);
 // Tile SpMV: blocks per SM for a shared-memory halo of halo_cap entries, and the launch.
 int tile_spmv_blocks_per_sm(int lanes, int unroll, int halo_cap);

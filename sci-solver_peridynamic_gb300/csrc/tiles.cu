@@ -135,12 +135,14 @@ __global__ void __launch_bounds__(kTileBuild) k_tile_fill(DeviceState S, int n)
 // ---- order of a row's bonds -------------------------------------------------------------
 // A halo entry is 16 bytes, so eight lanes that read entries of eight different
 // residues mod 8 take one pass through shared memory, and eight arbitrary ones
-// 2.6 on average.  Lane k of a row's G reads U consecutive slots of every G*U,
-// one after another; the bonds that the lanes read together are given different
-// residues as far as the row's bonds allow: one of each residue that is left,
-// then of the residues with most left.  Thread per row; `scratch` holds (slot,
-// local index) of the row's bonds by residue.
-__global__ void __launch_bounds__(kBlock) k_bank_order(DeviceState S, int n, int G, int U, int2* __restrict__ scratch)
+// 2.6 on average.  Such eight lanes are the four of a row and the four of the
+// next; lane k of a row reads the four slots 4 k .. 4 k + 3 of every 16, one after
+// another.  The four bonds that a row reads together are therefore given
+// different residues out of one half (0 to 3, 4 to 7), the halves in turn and the
+// other way round in the next row, as far as the row's bonds allow; of those, the
+// residues with most bonds left.  Thread per row; `scratch` holds (slot, local
+// index) of the row's bonds by residue.
+__global__ void __launch_bounds__(kBlock) k_bank_order(DeviceState S, int n, int2* __restrict__ scratch)
 {
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
         const int rs = S.row_ptr[p], cn = S.cnt[p];
@@ -156,24 +158,28 @@ __global__ void __launch_bounds__(kBlock) k_bank_order(DeviceState S, int n, int
             const int l = S.lidx[rs + j];
             scratch[at[l & 7]++] = make_int2(S.col[rs + j], l);
         }
-        for (int b = 0; b < cn; b += G * U)
-            for (int u = 0; u < U; ++u) {
-                int c = 0;
-                for (int j = b + u; j < min(b + G * U, cn); j += U) {
-                    while (c < 8 && left[c] == 0) ++c;
-                    int take = c;
-                    if (c == 8) {
-                        take = 0;
-                        for (int k = 1; k < 8; ++k)
-                            if (left[k] > left[take]) take = k;
-                    } else {
-                        ++c;
+        int half = (p % S.tile_rows) & 1;
+        for (int b = 0; b < cn; b += 16)
+            for (int u = 0; u < 4; ++u) {
+                unsigned used = 0u;
+                for (int j = b + u; j < min(b + 16, cn); j += 4) {
+                    int take = -1, best = -1;
+                    for (int c = 0; c < 8; ++c) {
+                        if (left[c] == 0) continue;
+                        // unused residues of the half, unused others, used ones
+                        const int rank = (used >> c & 1u ? 0 : (c >> 2) == half ? 2 : 1) * 65536 + left[c];
+                        if (rank > best) {
+                            best = rank;
+                            take = c;
+                        }
                     }
+                    used |= 1u << take;
                     --left[take];
                     const int2 bond = scratch[--at[take]];
                     S.col[rs + j] = bond.x;
                     S.lidx[rs + j] = (uint16_t)bond.y;
                 }
+                half ^= 1;
             }
     }
 }
@@ -338,12 +344,12 @@ int tile_blocks(int halo_cap)
 
 }  // namespace
 
-cudaError_t launch_bank_order(const DeviceState& S, int n, int lanes, int unroll, long long slots, cudaStream_t st)
+cudaError_t launch_bank_order(const DeviceState& S, int n, long long slots, cudaStream_t st)
 {
     int2* scratch = nullptr;
     cudaError_t e = cudaMalloc((void**)&scratch, sizeof(int2) * (size_t)(slots > 0 ? slots : 1));
     if (e != cudaSuccess) return e;
-    k_bank_order<<<(n + kBlock - 1) / kBlock, kBlock, 0, st>>>(S, n, lanes, unroll, scratch);
+    k_bank_order<<<(n + kBlock - 1) / kBlock, kBlock, 0, st>>>(S, n, scratch);
     e = cudaGetLastError();
     const cudaError_t f = cudaFree(scratch);
     return e != cudaSuccess ? e : f;

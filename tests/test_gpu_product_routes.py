@@ -86,3 +86,20 @@ def test_tiles_of_the_one_launch_solve(pdgb, scenes, n, coeff, jitter, tmp_path)
     assert st.bonds_alive < st.bonds_initial
     sim.dataIO_saveState(3)
     _compare(pdgb, _handle(scenes, sc, 0, load=3), _handle(scenes, sc, 2, load=3), sc.n)
+
+
+def test_a_tile_of_two_distant_pieces(pdgb, scenes, tmp_path):
+    """Rows of two blocks 300 spacings apart in one tile: more than 64 supercells,
+    where a block keeps the decoded positions (kFixedReach, csrc/cg_persist.cu)."""
+    a, b = _body(scenes, 27, 27, 27, 6.0), _body(scenes, 26, 26, 26, 6.0, seed=5)
+    a.pos = np.concatenate([a.pos, b.pos + np.array([6.0, 0.0, 0.0, 0.0])])
+    a.vel, a.act = np.concatenate([a.vel, b.vel]), np.concatenate([a.act, b.act])
+    a.sim.num_pd_particle = len(a.pos)
+    a.vel[:] = 0.0
+    rows = -(-a.n // 152)
+    assert 0 < 27 ** 3 % rows < rows   # (a tile of both, with 152 blocks)
+    sim, gather = _handle(scenes, a, 0), _handle(scenes, a, 2)
+    _compare(pdgb, sim, gather, a.n)
+    sim.advance(2)
+    st = sim.stats()
+    assert st.cg_graph_solves == 3 and st.cg_converged == 1
