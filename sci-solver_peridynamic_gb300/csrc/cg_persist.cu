@@ -82,6 +82,8 @@ struct PersistArgs {
     int bonds;                  // bond slots kept in shared memory per block (0: none)
     int max_iters;              // iterations of this launch at most
     int profile;
+    int start;                  // form r = p = b - y and its test first (y: A x of the guess)
+    int finish;                 // advance the rows when the solve has ended
 };
 
 // A block's part in a solve.
@@ -90,12 +92,13 @@ struct PersistRun {
     ulonglong2* inbox;
     int rows, halo, bonds, max_iters;
     int block, grid;            // this block among those of the solve
+    bool start;
     int* error;                 // set when a wait ran out of time
 };
 __device__ __forceinline__ PersistRun persist_run(const PersistArgs& A)
 {
     return PersistRun{A.rec, A.inbox, A.rows, A.halo, A.bonds, A.max_iters, (int)blockIdx.x, (int)gridDim.x,
-                      &A.S.sc->wait_error};
+                      A.start != 0, &A.S.sc->wait_error};
 }
 
 // Sums travel as their accumulator's own form: double-float for FP32 data.
@@ -299,6 +302,19 @@ __device__ __forceinline__ void load_bonds(const DeviceState& S, int slot, int (
 // their own for the rows left over, 30.0 with fixed-point positions, 25.3 with
 // the order of k_bank_order.  Eight lanes per row: 34.9 against 31.2; 1024
 // threads 30.3 (but 24.0 against 21.8 at 50k and 104 bonds).
+// The residual of the guess (residual_elem): zero on Dirichlet rows.
+template <typename V4>
+__device__ __forceinline__ V4 first_residual(const DeviceState& S, int p)
+{
+    V4 r = make_v4<V4>(0.0, 0.0, 0.0);
+    if (is_dirichlet(S.act[p] & kActMask)) return r;
+    const V4 b = ((const V4*)S.rhs)[p], y = ((const V4*)S.y)[p];
+    r.x = b.x - y.x;
+    r.y = b.y - y.y;
+    r.z = b.z - y.z;
+    return r;
+}
+
 template <int N>
 using Lanes = std::integral_constant<int, N>;
 
@@ -310,7 +326,7 @@ __device__ __forceinline__ bool persist_solve32(const StepParams& P, const Devic
 {
     CgScalars* sc = S.sc;
     // (the scalars change only after every block's last exchange)
-    if (((volatile CgScalars*)sc)->done) return true;
+    if (!A.start && ((volatile CgScalars*)sc)->done) return true;
     const int lo = A.block * A.rows;
     const int nr = max(0, min(A.rows, P.n - lo));
     float4* sx = (float4*)smem;
@@ -330,22 +346,28 @@ __device__ __forceinline__ bool persist_solve32(const StepParams& P, const Devic
     const int lane = threadIdx.x & (G - 1);
     const unsigned gmask = group_mask<G>();
     constexpr int NG = kPersistThreads / G;
-    const int first = CACHED && nr > 0 ? S.row_ptr[lo] : 0;
+    const int slot0 = CACHED && nr > 0 ? S.row_ptr[lo] : 0;
+    DotAcc32 first;   // <r, r> of the guess
     for (int t = threadIdx.x; t < nr; t += kPersistThreads) {
         const int p = lo + t;
         sx[t] = ((const float4*)S.sol)[p];
-        sr[t] = ((const float4*)S.r)[p];
-        sp[t] = ((const float4*)S.p)[p];
+        sr[t] = A.start ? first_residual<float4>(S, p) : ((const float4*)S.r)[p];
+        sp[t] = A.start ? sr[t] : ((const float4*)S.p)[p];
+        if (A.start) {
+            first.fma(sr[t].x, sr[t].x);
+            first.fma(sr[t].y, sr[t].y);
+            first.fma(sr[t].z, sr[t].z);
+        }
         const uint8_t ab = S.act[p];
         scnt[t] = is_dirichlet(ab & kActMask) ? -1 : S.cnt[p] << 8 | ab;
-        srow[t] = S.row_ptr[p] - first;
+        srow[t] = S.row_ptr[p] - slot0;
     }
     const int h0 = nr > 0 ? S.halo_ptr[A.block] : 0, nh = nr > 0 ? S.halo_ptr[A.block + 1] - h0 : 0;
     for (int h = threadIdx.x; h < nh; h += kPersistThreads) {
         const int q = S.halo[h0 + h];
         sq[h] = q;
-        sw[h] = ((const float4*)S.p)[q];
-        sh[h] = ((const float4*)S.r)[q];
+        sh[h] = A.start ? first_residual<float4>(S, q) : ((const float4*)S.r)[q];
+        sw[h] = A.start ? sh[h] : ((const float4*)S.p)[q];
         if (!CACHED) shx[h] = S.xs4[q];
     }
     if (threadIdx.x == 0) ex.error = 0;
@@ -366,8 +388,8 @@ __device__ __forceinline__ bool persist_solve32(const StepParams& P, const Devic
             const int cn = scnt[i] < 0 ? 0 : scnt[i] >> 8, base = srow[i];
             const float4 xp = S.xs4[lo + i];
             for (int j = lane; j < cn; j += G) {
-                const int l = S.lidx[first + base + j];
-                sg[base + j] = bond_geometry(S.xs4[sq[l]], xp, sup, S.inv_d0[first + base + j], sa1[base + j]);
+                const int l = S.lidx[slot0 + base + j];
+                sg[base + j] = bond_geometry(S.xs4[sq[l]], xp, sup, S.inv_d0[slot0 + base + j], sa1[base + j]);
                 sl[base + j] = (uint16_t)l;
             }
         }
@@ -377,9 +399,15 @@ __device__ __forceinline__ bool persist_solve32(const StepParams& P, const Devic
     const int max_iter = sc->max_iter;
     const double rz0 = sc->rz;
     DF rz{(float)rz0, (float)(rz0 - (double)(float)rz0)};
-    float alpha = 0.f, beta = (float)sc->beta;
+    float alpha = 0.f, beta = A.start ? 0.f : (float)sc->beta;
     int iter = sc->iter;
     bool done = false, converged = false;
+    if (A.start) {
+        rz = first.v;
+        if (!exchange_sum(ex, rz, 1, A, ++epoch, [](int, int) {})) return false;
+        converged = below_tolerance(df_to_double(rz), tol);
+        done = converged || iter >= max_iter;
+    }
 
     unsigned long long t_mark = 0, ns_spmv = 0, ns_vec = 0;
     DF pAp{0.f, 0.f};
@@ -545,7 +573,13 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist32(PersistArgs
     extern __shared__ __align__(32) unsigned char smem[];
     __shared__ Exchange ex;
     unsigned long long epoch = A.epoch;
-    persist_solve32<CACHED, G, U>(A.P, A.S, persist_run(A), smem, ex, epoch, A.profile && blockIdx.x == 0 && threadIdx.x == 0);
+    const PersistRun run = persist_run(A);
+    if (!persist_solve32<CACHED, G, U>(A.P, A.S, run, smem, ex, epoch, A.profile && blockIdx.x == 0 && threadIdx.x == 0)) return;
+    if (A.finish) {
+        __syncthreads();   // the block's rows of the solution
+        const int lo = blockIdx.x * A.rows, hi = min(A.P.n, lo + A.rows);
+        for (int r = lo + (int)threadIdx.x; r < hi; r += kPersistThreads) update_elem<false>(A.P, A.S, r);
+    }
 }
 
 // One product y = A w outside a solve by the same rows and halos, bonds read as
@@ -668,7 +702,7 @@ template <bool CACHED, int G, int U>
 __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist64(PersistArgs A)
 {
     CgScalars* sc = A.S.sc;
-    if (((volatile CgScalars*)sc)->done) return;
+    if (!A.start && ((volatile CgScalars*)sc)->done) return;
     extern __shared__ __align__(32) unsigned char smem[];
     __shared__ Exchange ex;
     const PersistRun run = persist_run(A);
@@ -693,7 +727,8 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist64(PersistArgs
     const int lane = threadIdx.x & (G - 1);
     const unsigned gmask = group_mask<G>();
     constexpr int NG = kPersistThreads / G;
-    const int first = CACHED ? S.row_ptr[lo] : 0;
+    const int slot0 = CACHED ? S.row_ptr[lo] : 0;
+    double first = 0.0;   // <r, r> of the guess
     const auto load3 = [](const void* v, int p) {
         const dbl4 a = ((const dbl4*)v)[p];
         return Vec3d{a.x, a.y, a.z};
@@ -701,22 +736,35 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist64(PersistArgs
     for (int t = threadIdx.x; t < nr; t += kPersistThreads) {
         const int p = lo + t;
         sx[t] = load3(S.sol, p);
-        sr[t] = load3(S.r, p);
-        sp[t] = load3(S.p, p);
+        if (A.start) {
+            const dbl4 r = first_residual<dbl4>(S, p);
+            sr[t] = Vec3d{r.x, r.y, r.z};
+            sp[t] = sr[t];
+            first = fma(r.x, r.x, fma(r.y, r.y, fma(r.z, r.z, first)));
+        } else {
+            sr[t] = load3(S.r, p);
+            sp[t] = load3(S.p, p);
+        }
         scnt[t] = is_dirichlet(S.act[p] & kActMask) ? -1 : S.cnt[p];
-        srow[t] = S.row_ptr[p] - first;
+        srow[t] = S.row_ptr[p] - slot0;
     }
     const int h0 = S.halo_ptr[blockIdx.x], nh = S.halo_ptr[blockIdx.x + 1] - h0;
     for (int h = threadIdx.x; h < nh; h += kPersistThreads) {
         const int q = S.halo[h0 + h];
         sq[h] = q;
-        sw[h] = load3(S.p, q);
-        sh[h] = load3(S.r, q);
+        if (A.start) {
+            const dbl4 r = first_residual<dbl4>(S, q);
+            sh[h] = Vec3d{r.x, r.y, r.z};
+            sw[h] = sh[h];
+        } else {
+            sw[h] = load3(S.p, q);
+            sh[h] = load3(S.r, q);
+        }
     }
     if (threadIdx.x == 0) {
         ex.error = 0;
         s_rz = sc->rz;
-        s_beta = sc->beta;
+        s_beta = A.start ? 0.0 : sc->beta;
         s_done = 0;
         s_converged = 0;
     }
@@ -725,11 +773,11 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist64(PersistArgs
         for (int i = threadIdx.x / G; i < nr; i += NG) {
             const int cn = scnt[i], base = srow[i];
             for (int j = lane; j < cn; j += G) {
-                const double2* J = (const double2*)(S.jac + 6ll * (first + base + j));
+                const double2* J = (const double2*)(S.jac + 6ll * (slot0 + base + j));
                 sJ[3 * (base + j)] = J[0];
                 sJ[3 * (base + j) + 1] = J[1];
                 sJ[3 * (base + j) + 2] = J[2];
-                sl[base + j] = S.lidx[first + base + j];
+                sl[base + j] = S.lidx[slot0 + base + j];
             }
         }
     }
@@ -738,6 +786,16 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist64(PersistArgs
     int iter = sc->iter;
 
     unsigned long long epoch = A.epoch;
+    if (A.start) {
+        __syncthreads();   // (s_rz and s_done before thread 0 sets them again)
+        if (!exchange_sum(ex, first, 1, run, ++epoch, [](int, int) {})) return;
+        if (threadIdx.x == 0) {
+            s_rz = first;
+            s_converged = below_tolerance(first, tol);
+            s_done = s_converged || iter >= max_iter;
+        }
+        __syncthreads();
+    }
     unsigned long long t_mark = 0, ns_spmv = 0, ns_vec = 0;
     const bool timed = A.profile && blockIdx.x == 0 && threadIdx.x == 0;
     double pAp = 0.0;
@@ -854,6 +912,10 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist64(PersistArgs
         sc->ns_spmv = (double)ns_spmv;
         sc->ns_vec = (double)ns_vec;
     }
+    if (A.finish) {
+        __syncthreads();   // the block's rows of the solution
+        for (int t = threadIdx.x; t < nr; t += kPersistThreads) update_elem<true>(P, S, lo + t);
+    }
 }
 
 // The solves and updates of a batch's scenes (batch.h) in one cooperative launch.
@@ -896,7 +958,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_gang_solve32(GangArgs A)
         const GangScene g = A.plan[scene];
         const StepParams P = D.P;
         const DeviceState S = D.S;
-        const PersistRun run{A.rec + g.rec, inbox, g.rows, g.halo, g.bonds, 0x7fffffff, block, A.gang, A.error};
+        const PersistRun run{A.rec + g.rec, inbox, g.rows, g.halo, g.bonds, 0x7fffffff, block, A.gang, false, A.error};
         bool ok;
         if (g.bonds == 0) ok = persist_solve32<false, kTileLanes, 4>(P, S, run, smem, ex, epoch, false);
         else if (g.lanes == 4) ok = persist_solve32<true, 4, 4>(P, S, run, smem, ex, epoch, false);
@@ -1037,9 +1099,10 @@ cudaError_t launch_tile_product(const StepParams& P, const DeviceState& S, const
 
 cudaError_t launch_cg_persist(bool fp64, const StepParams& P, const DeviceState& S, const CgPersistPlan& plan,
                               ulonglong2* rec, ulonglong2* inbox, unsigned long long epoch, int max_iters, bool profile,
-                              cudaStream_t st)
+                              bool start, bool finish, cudaStream_t st)
 {
-    PersistArgs A{P, S, rec, inbox, epoch, plan.rows, plan.halo, plan.bonds, max_iters, profile ? 1 : 0};
+    PersistArgs A{P, S, rec, inbox, epoch, plan.rows, plan.halo, plan.bonds, max_iters, profile ? 1 : 0, start ? 1 : 0,
+                  finish ? 1 : 0};
     void* args[] = {&A};
     return cudaLaunchCooperativeKernel(persist_kernel(fp64, plan), dim3(plan.grid), dim3(kPersistThreads), args, plan.smem,
                                        st);

@@ -1017,10 +1017,12 @@ pd_status Engine::integrate(bool* advanced)
     last_params_ = P;
     pd_status s = solve(P);
     if (s != PD_OK) return s;
-    mark_begin(PD_KC_UPDATE, -1);
-    launch_update(fp64_, P, S_, L_, stream_);
-    mark_end();
-    ++launches_;
+    if (!solve_updates_) {
+        mark_begin(PD_KC_UPDATE, -1);
+        launch_update(fp64_, P, S_, L_, stream_);
+        mark_end();
+        ++launches_;
+    }
     CK(cudaGetLastError(), "step launch");
     sim_time_ += P.h;
     *advanced = true;
@@ -1029,10 +1031,18 @@ pd_status Engine::integrate(bool* advanced)
 
 pd_status Engine::solve(const StepParams& P)
 {
+    // a one-launch solve from the previous solution forms the first residual
+    // itself, and updates the rows when it runs to its end (not while profiling,
+    // which times the update)
+    const bool starts = persist_.grid > 0 && opt_.warm_start != 2 && opt_.warm_start != 3 && !ws_features_needed();
+    solve_updates_ = starts && opt_.cg_loop == 0 && !profiling_;
     launch_cg_init(fp64_, P, S_, L_, stream_);
     product_of_guess(P);
-    launch_cg_residual(fp64_, P, S_, L_, stream_);
-    launches_ += 3;
+    launches_ += 2;
+    if (!starts) {
+        launch_cg_residual(fp64_, P, S_, L_, stream_);
+        ++launches_;
+    }
     if (opt_.warm_start == 3) {   // network column first, then the projection over history + column
         pd_status s = ws_before_cg(P);
         if (s == PD_OK) s = hist_project(P);
@@ -1054,7 +1064,7 @@ pd_status Engine::solve(const StepParams& P)
         launches_ += 2;
     }
     if (persist_.grid > 0) {
-        pd_status s = cg_persist_loop(P);
+        pd_status s = cg_persist_loop(P, starts);
         if (s != PD_OK) return s;
         return solve_finish(P);
     }
@@ -1228,7 +1238,7 @@ pd_status Engine::cg_host_loop(const StepParams& P)
     return PD_OK;
 }
 
-pd_status Engine::cg_persist_loop(const StepParams& P)
+pd_status Engine::cg_persist_loop(const StepParams& P, bool start)
 {
     const int check = opt_.cg_check_interval > 0 ? opt_.cg_check_interval : 8;
     const bool whole = opt_.cg_loop == 0;
@@ -1236,9 +1246,10 @@ pd_status Engine::cg_persist_loop(const StepParams& P)
     double ns_spmv = 0.0, ns_vec = 0.0;
     for (long long run = 0;;) {
         CK(launch_cg_persist(fp64_, P, S_, persist_, d_inbox_ + 2 * (size_t)persist_.grid * persist_.grid, d_inbox_,
-                             persist_epoch_, batch, profiling_, stream_),
+                             persist_epoch_, batch, profiling_, start, solve_updates_, stream_),
            "cg launch");
-        persist_epoch_ += 2ull * (unsigned long long)batch;
+        start = false;
+        persist_epoch_ += 2ull * (unsigned long long)batch + 1ull;
         ++launches_;
         CK(cudaMemcpyAsync(h_sc_, S_.sc, sizeof(CgScalars), cudaMemcpyDeviceToHost, stream_), "read cg scalars");
         CK(cudaStreamSynchronize(stream_), "cg sync");

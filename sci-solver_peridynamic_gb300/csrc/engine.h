@@ -109,7 +109,7 @@ private:
     pd_status cg_host_loop(const StepParams& P);   // the same iterations in host-checked batches
     // a small body's iterations in one cooperative launch (cg_loop 0) or in
     // host-checked batches of it (cg_loop 1)
-    pd_status cg_persist_loop(const StepParams& P);
+    pd_status cg_persist_loop(const StepParams& P, bool start);
     void hist_collect();   // the projection's statistics, after the solve's read-back
     template <typename T>
     pd_status download_scatter(const T* dev, T* host_out, size_t count_per, size_t elem_count);
@@ -206,6 +206,7 @@ private:
     CgPersistPlan persist_{};          // one-launch solve of a small body (grid 0: not used)
     ulonglong2* d_inbox_ = nullptr;    // its records: partial sums (2 grid^2), then r
     unsigned long long persist_epoch_ = 0;
+    bool solve_updates_ = false;       // the one-launch solve of this step advances the rows itself
     // profiling
     bool profiling_ = false;
     std::vector<cudaEvent_t> event_pool_;

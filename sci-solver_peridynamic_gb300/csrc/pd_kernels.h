@@ -283,10 +283,12 @@ bool cg_persist_may_fit(int rows, double reach, int device);
 // At most max_iters iterations from the state of S (x, r, p and the scalars,
 // as the residual kernel or an earlier launch left them).  rec: n records (FP64:
 // 2 n); inbox: 2 x grid^2 records; epoch: no smaller than any epoch of earlier
-// launches on them, of which a launch uses at most 2 max_iters.
+// launches on them, of which a launch uses at most 2 max_iters + 1.  start: from
+// the solution guess and y = A x of it instead (the residual kernel's part);
+// finish: the step's update of the rows, when this launch ends the solve.
 cudaError_t launch_cg_persist(bool fp64, const StepParams& P, const DeviceState& S, const CgPersistPlan& plan,
                               ulonglong2* rec, ulonglong2* inbox, unsigned long long epoch, int max_iters, bool profile,
-                              cudaStream_t st);
+                              bool start, bool finish, cudaStream_t st);
 // y = A in by the same blocks (mixed precision, a plan with a grid); *dot_out
 // (may be null) receives <in, A in>
 cudaError_t launch_tile_product(const StepParams& P, const DeviceState& S, const CgPersistPlan& plan, const void* in,
