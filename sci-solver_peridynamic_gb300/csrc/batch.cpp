@@ -465,7 +465,7 @@ pd_status Batch::tune()
     BCK(cudaEventCreate(&e1), "event");
     float best = 1e30f;
     int bl = lanes_c[0], bu = unroll_c[0], br = rows_c[0];
-    constexpr int reps = 4;
+    constexpr int reps = 2;
     for (int rows : rows_c) {
         pd_status s = build_items(rows);
         if (s != PD_OK) return s;

@@ -409,6 +409,13 @@ struct Workspace {
 
 }  // namespace
 
+size_t scan_scratch_u32(long long n) { return scan_scratch(n); }
+
+cudaError_t scan_exclusive_u32(const unsigned* in, unsigned* out, long long n, unsigned* tmp, cudaStream_t st)
+{
+    return exclusive_scan(in, out, n, tmp, st);
+}
+
 cudaError_t scan_exclusive_u32(const unsigned* in, unsigned* out, long long n, cudaStream_t st)
 {
     if (n <= 0) return cudaSuccess;

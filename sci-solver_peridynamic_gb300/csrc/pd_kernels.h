@@ -332,6 +332,9 @@ void free_tiles(DeviceState& S);
 int tile_spmv_blocks_per_sm(int lanes, int unroll, int halo_cap);
 void launch_spmv_tiled(bool dot, const StepParams& P, const DeviceState& S, const LaunchCfg& L, cudaStream_t st);
 cudaError_t scan_exclusive_u32(const unsigned* in, unsigned* out, long long n, cudaStream_t st);
+// the same with the caller's scratch of scan_scratch_u32(n) words
+size_t scan_scratch_u32(long long n);
+cudaError_t scan_exclusive_u32(const unsigned* in, unsigned* out, long long n, unsigned* tmp, cudaStream_t st);
 // Stable LSD radix sort of (key, value) pairs on the low key_bits bits, in place.
 cudaError_t sort_pairs_u32(unsigned* keys, int* vals, int n, int key_bits, cudaStream_t st);
 

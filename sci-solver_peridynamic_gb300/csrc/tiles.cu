@@ -363,12 +363,25 @@ cudaError_t build_tiles(DeviceState& S, int n, int* max_halo, int* unfit, cudaSt
     if (n <= 0 || S.tile_rows <= 0) return cudaSuccess;
     S.n_tiles = (n + S.tile_rows - 1) / S.tile_rows;
     const size_t nt = (size_t)S.n_tiles;
-    unsigned* counts = nullptr;
-    cudaError_t e = cudaMalloc((void**)&counts, sizeof(unsigned) * (nt + 1));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&S.tile_info, sizeof(int) * nt);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&S.halo_ptr, sizeof(int) * (nt + 1));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&S.tile_partials, sizeof(double) * nt);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&S.tile_ctr, sizeof(unsigned) * 2);
+    // everything but the halos in one allocation (a batch builds tiles per scene)
+    size_t bytes = 0;
+    const auto section = [&bytes](size_t size) {
+        const size_t at = bytes;
+        bytes += (size + 255) / 256 * 256;
+        return at;
+    };
+    section(sizeof(int) * nt);
+    const size_t at_ptr = section(sizeof(int) * (nt + 1)), at_sum = section(sizeof(double) * nt);
+    const size_t at_ctr = section(sizeof(unsigned) * 2), at_count = section(sizeof(unsigned) * (nt + 1));
+    const size_t at_scan = section(sizeof(unsigned) * scan_scratch_u32((long long)nt + 1));
+    unsigned char* base = nullptr;
+    cudaError_t e = cudaMalloc((void**)&base, bytes);
+    if (e != cudaSuccess) return e;
+    S.tile_info = (int*)base;
+    S.halo_ptr = (int*)(base + at_ptr);
+    S.tile_partials = (double*)(base + at_sum);
+    S.tile_ctr = (unsigned*)(base + at_ctr);
+    unsigned* counts = (unsigned*)(base + at_count);
     if (e == cudaSuccess) e = cudaMemsetAsync(S.tile_ctr, 0, sizeof(unsigned) * 2, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(counts, 0, sizeof(unsigned) * (nt + 1), st);
     const int grid = (int)(nt < 4096 ? nt : 4096);
@@ -376,7 +389,7 @@ cudaError_t build_tiles(DeviceState& S, int n, int* max_halo, int* unfit, cudaSt
         k_tile_count<<<grid, kTileBuild, 0, st>>>(S, n, counts);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = scan_exclusive_u32(counts, (unsigned*)S.halo_ptr, (long long)nt + 1, st);
+    if (e == cudaSuccess) e = scan_exclusive_u32(counts, (unsigned*)S.halo_ptr, (long long)nt + 1, (unsigned*)(base + at_scan), st);
     int total = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&total, S.halo_ptr + nt, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -388,7 +401,6 @@ cudaError_t build_tiles(DeviceState& S, int n, int* max_halo, int* unfit, cudaSt
     std::vector<int> info(nt);
     if (e == cudaSuccess) e = cudaMemcpyAsync(info.data(), S.tile_info, sizeof(int) * nt, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(counts);
     if (e != cudaSuccess) return e;
     for (int v : info) {
         *max_halo = v > *max_halo ? v : *max_halo;
@@ -400,10 +412,7 @@ cudaError_t build_tiles(DeviceState& S, int n, int* max_halo, int* unfit, cudaSt
 void free_tiles(DeviceState& S)
 {
     cudaFree(S.halo);
-    cudaFree(S.halo_ptr);
-    cudaFree(S.tile_info);
-    cudaFree(S.tile_partials);
-    cudaFree(S.tile_ctr);
+    cudaFree(S.tile_info);   // (and the arrays that share its allocation)
     S.halo = nullptr;
     S.halo_ptr = nullptr;
     S.tile_info = nullptr;
