@@ -150,13 +150,12 @@ typedef struct pd_solver_options {
      * reference's Scene fills them -- the slots are renumbered brick by
      * brick and the product walks each row's stencil of lattice offsets over
      * the brick's halo staged in shared memory (other bodies fall back to
-     * 2); 0 = automatic: 2 for bodies whose solves fit in one launch (about
-     * 130000 particles at a horizon of 2 to 2.5 spacings, less for longer
-     * ones; mixed-precision products of the larger of them use tiles of rows
-     * and their halos as 1 does), for other lattice fills from 20000
-     * particles 3, timed against the lanes x unroll shapes of 2 at make_ready
-     * (from 250000 particles a lattice body takes 3 without timing the
-     * others).
+     * 2); 0 = automatic: 3 for lattice fills from 250000 particles, else 2,
+     * where mixed-precision products of bodies from 2.2 million bond slots use
+     * large tiles of rows and their halos (unless lanes_per_particle or
+     * spmv_unroll names a shape of the gathers, which lattice fills from 20000
+     * particles time against 3) and solves of up to about 130000 particles run
+     * in one launch.
      * pd_get_options reports the path in use (1, 2 or 3). */
     int spmv_path;
     /* PD-PD contact (collectPDParticles / collidePDParticles,

@@ -589,8 +589,9 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist32(PersistArgs
 template <bool DOT>
 __global__ void __launch_bounds__(kTileBlock, 1)
     k_tile_product32(StepParams P, DeviceState S, int rows, int halo, const float4* __restrict__ in,
-                     float4* __restrict__ out, ReduceSlot slot, double* dot_out)
+                     float4* __restrict__ out, ReduceSlot slot, CgScalars* cg, double* dot_out)
 {
+    if (DOT && cg && ((volatile CgScalars*)cg)->done) return;
     constexpr int G = kTileLanes;
     extern __shared__ __align__(32) unsigned char smem[];
     float4* sw = (float4*)smem;
@@ -688,7 +689,11 @@ __global__ void __launch_bounds__(kTileBlock, 1)
     };
     if (fixed) all_rows(std::true_type());
     else all_rows(std::false_type());
-    if (DOT) block_reduce_finish(acc, slot, [dot_out](double pAp) { *dot_out = pAp; });
+    if (DOT)
+        block_reduce_finish(acc, slot, [cg, dot_out](double pAp) {
+            if (cg) cg_fin_alpha(cg, pAp);
+            if (dot_out) *dot_out = pAp;
+        });
 }
 
 struct __align__(8) Vec3d {
@@ -1069,6 +1074,29 @@ bool cg_persist_plan(bool fp64, int max_halo, int max_bonds, int device, CgPersi
     return true;
 }
 
+bool tile_product_may_fit(int rows, double reach, int device)
+{
+    int optin = 0;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    const double side = std::cbrt((double)rows) + 2.0 * reach;
+    return 2 * sizeof(float4) * side * side * side <= (double)(optin - 2048);
+}
+
+bool tile_product_plan(int max_halo, int device, CgPersistPlan* plan)
+{
+    int optin = 0;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    const int room = optin - 2048;
+    if (2 * sizeof(float4) * (size_t)max_halo > (size_t)room) return false;
+    for (const void* t : {(const void*)k_tile_product32<true>, (const void*)k_tile_product32<false>})
+        if (cudaFuncSetAttribute(t, cudaFuncAttributeMaxDynamicSharedMemorySize, room) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+    plan->halo = max_halo;
+    return true;
+}
+
 bool cg_persist_may_fit(int rows, double reach, int device)
 {
     int optin = 0;
@@ -1087,13 +1115,13 @@ cudaError_t launch_gang_solve(const GangArgs& A, int gangs, size_t smem, cudaStr
 }
 
 cudaError_t launch_tile_product(const StepParams& P, const DeviceState& S, const CgPersistPlan& plan, const void* in,
-                                void* out, ReduceSlot slot, double* dot_out, cudaStream_t st)
+                                void* out, ReduceSlot slot, CgScalars* cg, double* dot_out, cudaStream_t st)
 {
     StepParams p = P;
     DeviceState s = S;
     int rows = plan.rows, halo = plan.halo;
-    void* args[] = {&p, &s, &rows, &halo, &in, &out, &slot, &dot_out};
-    const void* k = dot_out ? (const void*)k_tile_product32<true> : (const void*)k_tile_product32<false>;
+    void* args[] = {&p, &s, &rows, &halo, &in, &out, &slot, &cg, &dot_out};
+    const void* k = cg || dot_out ? (const void*)k_tile_product32<true> : (const void*)k_tile_product32<false>;
     return cudaLaunchKernel(k, dim3(plan.grid), dim3(kTileBlock), args, 2 * sizeof(float4) * (size_t)plan.halo, st);
 }
 

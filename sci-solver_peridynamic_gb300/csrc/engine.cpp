@@ -144,6 +144,7 @@ void Engine::free_all()
     if (d_inbox_) cudaFree(d_inbox_);
     d_inbox_ = nullptr;
     persist_ = CgPersistPlan{};
+    tiles_ = CgPersistPlan{};
     L_.lattice = 0;
     L_.lat = nullptr;
     cudaFree(contact_.counts);
@@ -249,24 +250,33 @@ pd_status Engine::make_ready()
     total_slots_ = out.total;
     bonds_initial_ = out.bonds;
     sim_.pd_max_num_bonds = out.max_bonds;
-    // bodies small enough for the one-launch solve keep the builder's order;
-    // larger lattice-filled bodies are renumbered brick by brick for the stencil
-    // product (mixed mode; automatic above kLatticeMinRows particles, or asked
-    // for with spmv_path 3).  Other bodies keep the builder's order and the
-    // gather product.  (Per CG iteration, one launch against the stencil: 18
-    // us against 44 at 50k particles and a horizon of 3 spacings, 25 against
-    // 50 at 100k and 2.5.)
+    // Bodies small enough for the one-launch solve keep the builder's order (18 us
+    // per CG iteration against 44 with the stencil product at 50k particles and a
+    // horizon of 3 spacings, 25 against 50 at 100k and 2.5).  Larger bodies multiply
+    // by tiles, lattice fills from kLatticeOnlyRows particles (mixed mode, or
+    // asked for with spmv_path 3) by the stencil, their slots renumbered brick by
+    // brick: per iteration, tiles against the stencil, 48 us against 52 at 150k
+    // and 2.5, 72 against 78 at 200k and 3, but 42 against 40 at 200k and 2, 68
+    // against 62 at 250k and 2.5, 135 against 106 at 600k.  A fixed shape of the
+    // gather product is timed against the stencil from kLatticeMinRows.
+    const bool fixed_shape = opt_.lanes_per_particle || opt_.spmv_unroll;
+    const int lattice_rows = fixed_shape ? kLatticeMinRows : kLatticeOnlyRows;
     if (opt_.spmv_path == 0 || opt_.spmv_path == 2) {
         s = persist_prepare();
         if (s != PD_OK) return s;
     }
     if (!fp64_ && n > 0 && !batch_member_ &&
-        (opt_.spmv_path == 3 || (opt_.spmv_path == 0 && n >= kLatticeMinRows && persist_.grid == 0))) {
+        (opt_.spmv_path == 3 || (opt_.spmv_path == 0 && n >= lattice_rows && persist_.grid == 0))) {
         int ok = 0;
         CK(lattice_build(n, 2.0 * sim_.pd_particle_radius, S_.x64, S_.X32, d_perm_, S_.row_ptr, S_.cnt, &S_.col,
                          total_slots_, &lat_, &latb_, &ok, stream_),
            "lattice build");
         lat_ok_ = ok != 0;
+    }
+    if (persist_.tiled_products) tiles_ = persist_;
+    if (opt_.spmv_path == 0 && persist_.grid == 0 && !lat_ok_) {
+        s = tile_prepare();
+        if (s != PD_OK) return s;
     }
     if (n > 0) {
         CK(cudaMemcpyAsync(S_.X64, S_.x64, sizeof(dbl4) * N, cudaMemcpyDeviceToDevice, stream_), "copy X");
@@ -432,8 +442,8 @@ pd_status Engine::tune_spmv()
     }
     if (lat_ok_) {
         // asked for, or a large lattice body (from 250k particles the stencil
-        // product measured well ahead of every gather shape: 186 against
-        // 253 us per product at 1M), where timing the gather shapes and their
+        // product measured well ahead of every gather shape: 134 against
+        // 229 us per product at 1M), where timing the gather shapes and their
         // bond reorderings would cost make_ready ~45 ms: the stencil only
         if (opt_.spmv_path == 3 || n_ >= kLatticeOnlyRows) cand.clear();
         cand.push_back({0, 1, 1, 1});
@@ -449,7 +459,7 @@ pd_status Engine::tune_spmv()
             L_.grid_bonds = lat_.grid;
             return;
         }
-        if (c.tiled || persist_.tiled_products) relayout_bonds(1, 1);   // (the tile product has its own order)
+        if (c.tiled || tiles_.grid > 0) relayout_bonds(1, 1);   // (the tile product has its own order)
         else relayout_bonds(c.g, c.u);
         L_.tiled = c.tiled;
         L_.lanes = c.g;
@@ -461,7 +471,7 @@ pd_status Engine::tune_spmv()
             L_.grid_bonds = grid_for_rows(c.g, row_kernel_blocks_per_sm(fp64_, c.g, c.u));
         }
     };
-    if (cand.size() == 1 || n_ < 20000 || persist_.tiled_products || batch_member_) {   // (a batch times its own shape)
+    if (cand.size() == 1 || n_ < 20000 || tiles_.grid > 0 || batch_member_) {   // (a batch times its own shape)
         // small problems: launch overhead dominates, keep the default (the
         // tiled path when it was asked for)
         // As many lanes per row as one block per SM holds: FP64 10.4 us at 500
@@ -524,8 +534,8 @@ pd_status Engine::tune_spmv()
 // y = A x for the solve's first residual
 void Engine::product_of_guess(const StepParams& P)
 {
-    if (persist_.tiled_products)
-        launch_tile_product(P, S_, persist_, S_.sol, S_.y, ReduceSlot{S_.partials, S_.counters + 1}, nullptr, stream_);
+    if (tiles_.grid > 0)
+        launch_tile_product(P, S_, tiles_, S_.sol, S_.y, ReduceSlot{S_.partials, S_.counters + 1}, nullptr, nullptr, stream_);
     else launch_spmv(fp64_, false, P, S_, L_, stream_);
 }
 
@@ -535,8 +545,8 @@ void Engine::apply_op(const StepParams& P, const void* in, void* out, ReduceSlot
         launch_lattice_scatter(S_, lat_, in, stream_);
         launch_spmv_lattice(dot_out != nullptr, P, S_, lat_, out, slot, nullptr, dot_out, stream_);
         ++launches_;
-    } else if (persist_.tiled_products) {
-        launch_tile_product(P, S_, persist_, in, out, slot, dot_out, stream_);
+    } else if (tiles_.grid > 0) {
+        launch_tile_product(P, S_, tiles_, in, out, slot, nullptr, dot_out, stream_);
     }
     else launch_operator_u(fp64_, P, S_, L_.lanes, L_.unroll, L_.grid_bonds, in, out, slot, dot_out, stream_);
 }
@@ -573,6 +583,35 @@ pd_status Engine::persist_prepare()
     CK(cudaMemsetAsync(d_inbox_, 0, sizeof(ulonglong2) * (inbox + rec), stream_), "memset records");
     persist_epoch_ = 0;
     persist_ = plan;
+    return PD_OK;
+}
+
+// Products by tiles for larger bodies that are no lattice fill (mixed
+// precision): the largest tiles, a whole number of them per SM, whose halos fit.
+// 41.2 us at 200k scattered particles of 76 bonds against 61.5 for the gather,
+// 178 against 229 at 1M.
+pd_status Engine::tile_prepare()
+{
+    if (fp64_ || n_ <= 0 || batch_member_ || total_slots_ < kTileMinSlots || opt_.lanes_per_particle || opt_.spmv_unroll)
+        return PD_OK;
+    const double spacing = 2.0 * sim_.pd_particle_radius;
+    CK(dalloc(&S_.lidx, (size_t)total_slots_), "alloc local indices");
+    for (int per_sm = 1; per_sm <= kTileMaxPerSm; ++per_sm) {
+        CgPersistPlan plan;
+        plan.rows = (int)((n_ + (long long)sm_count_ * per_sm - 1) / ((long long)sm_count_ * per_sm));
+        plan.grid = (n_ + plan.rows - 1) / plan.rows;
+        if (!tile_product_may_fit(plan.rows, spacing > 0 ? sim_.pd_horizon / spacing : 0.0, device_)) continue;
+        int max_halo = 0, unfit = 0;
+        S_.tile_rows = plan.rows;
+        CK(build_tiles(S_, n_, &max_halo, &unfit, stream_), "build tiles");
+        launches_ += 2;
+        if (unfit > 0 || !tile_product_plan(max_halo, device_, &plan)) continue;
+        CK(launch_bank_order(S_, n_, total_slots_, stream_), "order bonds");
+        ++launches_;
+        tiles_ = plan;
+        return PD_OK;
+    }
+    gang_tiles_free();
     return PD_OK;
 }
 
@@ -619,6 +658,8 @@ pd_status Engine::build_halos()
     CK(build_tiles(S_, n_, &max_halo, &unfit, stream_), "build tiles");
     S_.halo_cap = std::min(max_halo, kMaxHaloCap);
     if (persist_.grid > 0 && (unfit > 0 || max_halo > persist_.halo)) persist_ = CgPersistPlan{};
+    if (persist_.grid == 0 && tiles_.grid > 0 && (unfit > 0 || !tile_product_plan(max_halo, device_, &tiles_)))
+        tiles_ = CgPersistPlan{};
     return PD_OK;
 }
 
@@ -1149,7 +1190,9 @@ void Engine::cg_iteration(const StepParams& P, int k, cudaGraphConditionalHandle
         if (sample) mark_end();
     } else {
         if (sample) mark_begin(PD_KC_SPMV, k);
-        launch_spmv(fp64_, true, P, S_, L_, stream_);
+        if (tiles_.grid > 0)
+            launch_tile_product(P, S_, tiles_, S_.p, S_.y, ReduceSlot{S_.partials, S_.counters + 1}, S_.sc, nullptr, stream_);
+        else launch_spmv(fp64_, true, P, S_, L_, stream_);
         if (sample) mark_end();
         if (sample) mark_begin(PD_KC_CG_VECTOR, k);
         if (opt_.preconditioner) {

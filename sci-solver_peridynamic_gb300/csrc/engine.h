@@ -73,6 +73,7 @@ private:
     // y = A in with this handle's product (lattice stencil or CSR rows)
     void apply_op(const StepParams& P, const void* in, void* out, ReduceSlot slot, double* dot_out);
     pd_status persist_prepare();
+    pd_status tile_prepare();
     pd_status gang_tiles(int rows, int blocks, CgPersistPlan* plan, bool* fits);
     void gang_tiles_free();
     pd_status build_halos();
@@ -205,6 +206,7 @@ private:
     bool cg_graph_failed_ = false;     // the graph could not be built: host-checked batches
     CgPersistPlan persist_{};          // one-launch solve of a small body (grid 0: not used)
     ulonglong2* d_inbox_ = nullptr;    // its records: partial sums (2 grid^2), then r
+    CgPersistPlan tiles_{};            // products by tiles (grid 0: not used)
     unsigned long long persist_epoch_ = 0;
     bool solve_updates_ = false;       // the one-launch solve of this step advances the rows itself
     // profiling

@@ -9,15 +9,14 @@
 // distinct lattice site, each bond joins two sites whose offset lies in a
 // small stencil (80 offsets for a horizon of 2.5 spacings).  The slots are
 // renumbered brick by brick (bricks of 16 x 8 x 4 sites, x fastest), and the
-// product runs one brick per block iteration: the block stages the halo of
-// the brick's sites (each particle's deviation from its site and its entry of
-// w) in shared memory, then each thread walks the stencil of one z column of
-// the brick -- its four rows at once, so that a neighbour read from shared
-// memory serves every row of the column whose stencil it is in.  Threads take
-// x-consecutive columns, so the neighbours at one stencil entry are
-// x-consecutive shared-memory words (no bank conflicts), and the only per-bond
-// stream is 1/d0 per (row, stencil entry), 0 where there is no live bond
-// (stored scaled by 2^100, see kLatScale).
+// product runs one brick per block iteration: the halo of the brick's sites
+// (each particle's entry of w and its deviation from its site) arrives in shared
+// memory by two asynchronous copies, then each thread walks the stencil columns
+// of two z-adjacent rows, so that a neighbour read from shared memory serves
+// both rows whose stencil it is in.  Threads take x-consecutive pairs, so the
+// neighbours at one stencil entry are x-consecutive shared-memory words, and the
+// only per-bond stream is 1/d0 per (row, stencil entry), 0 where there is no
+// live bond (stored scaled by 2^100, see kLatScale).
 //
 // The per-bond arithmetic is the gather product's (step_rows.cuh,
 // mixed_bond_chunk): the Jacobian applied to w_p - w_q is

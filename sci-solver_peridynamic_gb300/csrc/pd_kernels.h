@@ -158,6 +158,7 @@ struct DeviceState {
 // particle there, beyond the horizon, or broken).
 constexpr int kLatMaxOffsets = 160;  // distinct bond offsets at most
 constexpr long long kTileMinSlots = 2200000;   // bond slots from which the one-launch bodies' other products use its tiles
+constexpr int kTileMaxPerSm = 16;               // tiles per SM of larger bodies at most
 constexpr int kLatticeMinRows = 20000;   // automatic choice: smaller bodies keep the gather product
 constexpr int kLatticeOnlyRows = 250000; // automatic choice: larger lattice bodies time only the stencil variants
 constexpr int kLatRmax = 3;          // largest offset per axis (sites)
@@ -289,10 +290,14 @@ bool cg_persist_may_fit(int rows, double reach, int device);
 cudaError_t launch_cg_persist(bool fp64, const StepParams& P, const DeviceState& S, const CgPersistPlan& plan,
                               ulonglong2* rec, ulonglong2* inbox, unsigned long long epoch, int max_iters, bool profile,
                               bool start, bool finish, cudaStream_t st);
-// y = A in by the same blocks (mixed precision, a plan with a grid); *dot_out
-// (may be null) receives <in, A in>
+// y = A in by a block per tile (mixed precision); with cg (a CG iteration) alpha
+// from <in, A in>, and *dot_out (may be null) receives it
 cudaError_t launch_tile_product(const StepParams& P, const DeviceState& S, const CgPersistPlan& plan, const void* in,
-                                void* out, ReduceSlot slot, double* dot_out, cudaStream_t st);
+                                void* out, ReduceSlot slot, CgScalars* cg, double* dot_out, cudaStream_t st);
+// its plan for tiles with halos of at most max_halo (plan->grid tiles of
+// plan->rows rows); false when they do not fit in shared memory
+bool tile_product_may_fit(int rows, double reach, int device);   // likely, before the halos are known
+bool tile_product_plan(int max_halo, int device, CgPersistPlan* plan);
 // Preconditioned CG (no reference counterpart in use: the reference's
 // cusp::precond::diagonal is commented out, simulator.cu:767-769): mode 1 =
 // inverse diagonal of A, 2 = inverse 3x3 diagonal blocks; the stopping test

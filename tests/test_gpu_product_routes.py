@@ -103,3 +103,22 @@ def test_a_tile_of_two_distant_pieces(pdgb, scenes, tmp_path):
     sim.advance(2)
     st = sim.stats()
     assert st.cg_graph_solves == 3 and st.cg_converged == 1
+
+
+@pytest.mark.parametrize("n,coeff,jitter", [(56, 5.0, 0.05), (61, 5.0, 0.4), (48, 6.0, 0.4), (80, 4.0, 0.4)])
+def test_tiles_of_larger_bodies(pdgb, scenes, n, coeff, jitter, tmp_path):
+    """110k to 512k rows that take no one-launch solve (or do, at 48 and 6.0):
+    one or more tiles per SM in the products and in the CG's graph, a ragged last
+    tile, and a state that both handles load."""
+    sc = _body(scenes, n, n, n, coeff, jitter)
+    sc.run.saving_path = str(tmp_path).encode()
+    sim, gather = _handle(scenes, sc, 0), _handle(scenes, sc, 2)
+    assert sim.params()[2].spmv_path == 2
+    _compare(pdgb, sim, gather, sc.n)
+    for s in (sim, gather):
+        s.advance(1)
+        assert s.stats().cg_converged == 1
+    x, x2 = sim.get(pdgb.VAR_POSITION), gather.get(pdgb.VAR_POSITION)
+    assert np.abs(x - x2).max() <= 1e-5 * np.abs(x2).max()   # (the bound of the mixed-precision parity tests)
+    sim.dataIO_saveState(2)
+    _compare(pdgb, _handle(scenes, sc, 0, load=2), _handle(scenes, sc, 2, load=2), sc.n)
