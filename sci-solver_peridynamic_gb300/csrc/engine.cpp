@@ -481,6 +481,9 @@ pd_status Engine::tune_spmv()
         int lanes = 32;
         while (lanes > (fp64_ ? 4 : 8) && (long long)n_ * lanes > (long long)sm_count_ * kBlock) lanes /= 2;
         if (!fp64_ && lanes == 32) lanes = 16;   // (as fast, and fewer shuffles)
+        // (the gathers of an operator view of a body that multiplies by tiles: 49.9 us
+        // at 100k particles with 4 lanes, 53.6 with 8)
+        if (tiles_.grid > 0) lanes = 4;
         Cand c = cand.size() == 1 ? cand[0] : Cand{0, lanes, fp64_ ? 1 : 2};
         if (lat_ok_ && opt_.spmv_path == 3) c = Cand{0, 1, 1, 1};
         if (opt_.spmv_path == 1 && can_tile && cand.size() > 1) c = Cand{1, fixed_lanes ? fixed_lanes : 8, fixed_unroll ? fixed_unroll : 2};
@@ -1287,17 +1290,20 @@ pd_status Engine::cg_persist_loop(const StepParams& P, bool start)
     const bool whole = opt_.cg_loop == 0;
     int batch = whole ? std::max(1, opt_.cg_max_iterations) : std::max(1, predicted_iters_ - 1);
     double ns_spmv = 0.0, ns_vec = 0.0;
+    int seen = 0;   // iterations of the solve so far
     for (long long run = 0;;) {
         CK(launch_cg_persist(fp64_, P, S_, persist_, d_inbox_ + 2 * (size_t)persist_.grid * persist_.grid, d_inbox_,
                              persist_epoch_, batch, profiling_, start, solve_updates_, stream_),
            "cg launch");
-        start = false;
-        persist_epoch_ += 2ull * (unsigned long long)batch + 1ull;
         ++launches_;
         CK(cudaMemcpyAsync(h_sc_, S_.sc, sizeof(CgScalars), cudaMemcpyDeviceToHost, stream_), "read cg scalars");
         CK(cudaStreamSynchronize(stream_), "cg sync");
         ++host_syncs_;
         if (h_sc_->wait_error) break;
+        // the epochs that this launch used
+        persist_epoch_ += 2ull * (unsigned long long)(h_sc_->iter - seen) + (start ? 1ull : 0ull);
+        seen = h_sc_->iter;
+        start = false;
         ns_spmv += h_sc_->ns_spmv;
         ns_vec += h_sc_->ns_vec;
         if (h_sc_->done) break;
