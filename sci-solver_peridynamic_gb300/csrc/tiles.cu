@@ -349,7 +349,9 @@ cudaError_t launch_bank_order(const DeviceState& S, int n, long long slots, cuda
     int2* scratch = nullptr;
     cudaError_t e = cudaMalloc((void**)&scratch, sizeof(int2) * (size_t)(slots > 0 ? slots : 1));
     if (e != cudaSuccess) return e;
-    k_bank_order<<<(n + kBlock - 1) / kBlock, kBlock, 0, st>>>(S, n, scratch);
+    // (64 threads per block: a thread walks its row alone, and 11k rows are to reach
+    // every SM: 58 us, 125 with 256)
+    k_bank_order<<<(n + 63) / 64, 64, 0, st>>>(S, n, scratch);
     e = cudaGetLastError();
     const cudaError_t f = cudaFree(scratch);
     return e != cudaSuccess ? e : f;
