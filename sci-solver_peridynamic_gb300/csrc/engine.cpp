@@ -133,7 +133,7 @@ void Engine::free_all()
 {
     ws_free();
     hist_free();
-    void* ptrs[] = {d_state_, S_.col, S_.inv_d0, S_.jac, S_.lidx, S_.d0sq, d_perm_, d_stage_};
+    void* ptrs[] = {d_state_, S_.col, S_.jac, S_.lidx, S_.d0sq, d_perm_, d_stage_};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     free_tiles(S_);
@@ -306,10 +306,9 @@ pd_status Engine::make_ready()
         // 1/d0 per bond slot, and the supercell frame of the FP32 positions:
         // edge = the smallest power of two >= horizon, +-512 cells around the box centre
         const size_t slots = (size_t)std::max<long long>(total_slots_, 1);
-        CK(dalloc(&S_.inv_d0, slots), "alloc inv_d0");
-        CK(cudaMemsetAsync(S_.inv_d0, 0, sizeof(float) * slots, stream_), "memset inv_d0");
-        CK(dalloc(&S_.d0sq, slots), "alloc d0sq");
-        CK(cudaMemsetAsync(S_.d0sq, 0, sizeof(float2) * slots, stream_), "memset d0sq");
+        CK(dalloc(&S_.d0sq, slots + slots / 2 + 1), "alloc bond geometry");   // d0sq, then inv_d0
+        CK(cudaMemsetAsync(S_.d0sq, 0, sizeof(float2) * (slots + slots / 2 + 1), stream_), "memset bond geometry");
+        S_.inv_d0 = (float*)(S_.d0sq + slots);
         if (n > 0) {
             const int g = (int)std::min<long long>(std::max<long long>(((long long)n + kBlock - 1) / kBlock, 1), kMaxPartials);
             launch_bond_geometry(S_, stream_);
@@ -580,7 +579,7 @@ pd_status Engine::persist_prepare()
     // (A fixed lanes_per_particle or spmv_unroll names a shape of the gather.)
     plan.tiled_products = plan.tiled_products && total_slots_ >= kTileMinSlots && !opt_.lanes_per_particle && !opt_.spmv_unroll;
     if (plan.tiled_products)
-        CK(launch_bank_order(S_, n_, total_slots_, stream_), "order bonds");
+        CK(launch_bank_order(S_, n_, total_slots_, nullptr, stream_), "order bonds");
     const size_t inbox = 2 * (size_t)plan.grid * plan.grid, rec = (fp64_ ? 2 : 1) * (size_t)n_;
     CK(dalloc(&d_inbox_, inbox + rec), "alloc records");
     CK(cudaMemsetAsync(d_inbox_, 0, sizeof(ulonglong2) * (inbox + rec), stream_), "memset records");
@@ -609,7 +608,7 @@ pd_status Engine::tile_prepare()
         CK(build_tiles(S_, n_, &max_halo, &unfit, stream_), "build tiles");
         launches_ += 2;
         if (unfit > 0 || !tile_product_plan(max_halo, device_, &plan)) continue;
-        CK(launch_bank_order(S_, n_, total_slots_, stream_), "order bonds");
+        CK(launch_bank_order(S_, n_, total_slots_, nullptr, stream_), "order bonds");
         ++launches_;
         tiles_ = plan;
         return PD_OK;
@@ -638,7 +637,7 @@ pd_status Engine::gang_tiles(int rows, int blocks, CgPersistPlan* plan, bool* fi
         return PD_OK;
     }
     if (plan->bonds == 0) {
-        CK(launch_bank_order(S_, n_, total_slots_, stream_), "order bonds");
+        CK(launch_bank_order(S_, n_, total_slots_, S_.d0sq, stream_), "order bonds");   // (d0sq is formed again below)
         launch_bond_geometry(S_, stream_);
         launches_ += 2;
     }

@@ -331,7 +331,8 @@ void launch_bond_relayout(const DeviceState& S, int grid, int g_from, int u_from
 cudaError_t build_tiles(DeviceState& S, int n, int* max_halo, int* unfit, cudaStream_t st);
 // Reorders every row's bonds (col, lidx; the geometry arrays not yet formed) for
 // few bank conflicts in the look-ups of four lanes per row with four bonds each.
-cudaError_t launch_bank_order(const DeviceState& S, int n, long long slots, cudaStream_t st);
+// scratch: 8 bytes per bond slot (null: allocated here).
+cudaError_t launch_bank_order(const DeviceState& S, int n, long long slots, void* scratch, cudaStream_t st);
 void free_tiles(DeviceState& S);
 // Tile SpMV: blocks per SM for a shared-memory halo of halo_cap entries, and the launch.
 int tile_spmv_blocks_per_sm(int lanes, int unroll, int halo_cap);

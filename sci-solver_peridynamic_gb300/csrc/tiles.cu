@@ -344,16 +344,18 @@ int tile_blocks(int halo_cap)
 
 }  // namespace
 
-cudaError_t launch_bank_order(const DeviceState& S, int n, long long slots, cudaStream_t st)
+cudaError_t launch_bank_order(const DeviceState& S, int n, long long slots, void* scratch, cudaStream_t st)
 {
-    int2* scratch = nullptr;
-    cudaError_t e = cudaMalloc((void**)&scratch, sizeof(int2) * (size_t)(slots > 0 ? slots : 1));
-    if (e != cudaSuccess) return e;
+    int2* own = nullptr;
+    if (!scratch) {
+        const cudaError_t e = cudaMalloc((void**)&own, sizeof(int2) * (size_t)(slots > 0 ? slots : 1));
+        if (e != cudaSuccess) return e;
+    }
     // (64 threads per block: a thread walks its row alone, and 11k rows are to reach
     // every SM: 58 us, 125 with 256)
-    k_bank_order<<<(n + 63) / 64, 64, 0, st>>>(S, n, scratch);
-    e = cudaGetLastError();
-    const cudaError_t f = cudaFree(scratch);
+    k_bank_order<<<(n + 63) / 64, 64, 0, st>>>(S, n, scratch ? (int2*)scratch : own);
+    const cudaError_t e = cudaGetLastError();
+    const cudaError_t f = own ? cudaFree(own) : cudaSuccess;
     return e != cudaSuccess ? e : f;
 }
 
