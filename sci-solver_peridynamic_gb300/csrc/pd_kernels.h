@@ -157,10 +157,10 @@ struct DeviceState {
 // stencil entry) streams from a table in which 0 marks "no live bond" (no
 // particle there, beyond the horizon, or broken).
 constexpr int kLatMaxOffsets = 160;  // distinct bond offsets at most
-constexpr long long kTileMinSlots = 2200000;   // bond slots from which the one-launch bodies' other products use its tiles
+constexpr long long kTileMinSlots = 2200000;   // bond slots from which products go by tiles
 constexpr int kTileMaxPerSm = 16;               // tiles per SM of larger bodies at most
-constexpr int kLatticeMinRows = 20000;   // automatic choice: smaller bodies keep the gather product
-constexpr int kLatticeOnlyRows = 250000; // automatic choice: larger lattice bodies time only the stencil variants
+constexpr int kLatticeMinRows = 20000;   // lattice fills whose options fix a gather shape: timed against the stencil from here
+constexpr int kLatticeOnlyRows = 250000; // lattice fills take the stencil from here without timing others
 constexpr int kLatRmax = 3;          // largest offset per axis (sites)
 constexpr int kLatTab = 2 * kLatRmax + 1;
 

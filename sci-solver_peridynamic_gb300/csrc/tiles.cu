@@ -14,8 +14,8 @@
 // Built once per make_ready (bonds are never added; a broken bond only moves
 // within its row, and its local index moves with it: every slot of a row has
 // one, so a rollback that restores broken bonds finds theirs).  The one-launch
-// solve of small bodies (cg_persist.cu) uses the same halos and indices, with a
-// tile per block.
+// solve and the products by larger tiles (cg_persist.cu) use the same halos and
+// indices, with a tile per block.
 #include <vector>
 
 #include "pd_device.cuh"
