@@ -334,6 +334,7 @@ pd_status Batch::plan_gangs()
         for (auto& e : eng_) e->gang_tiles_free();
         return PD_OK;
     }
+    BCK(gang_solve_prepare(device_), "gang kernel attribute");
     std::vector<GangScene> gs(ns);
     long long rec = 0;
     gang_smem_ = 0;

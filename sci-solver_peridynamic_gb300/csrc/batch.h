@@ -115,6 +115,7 @@ struct GangArgs {
     ulonglong2* rec;        // a record per row (zero before the launch)
     int* error;
 };
+cudaError_t gang_solve_prepare(int device);   // before the first launch on the device
 cudaError_t launch_gang_solve(const GangArgs& A, int gangs, size_t smem, cudaStream_t st);
 
 // Launchers (batch.cu).  Both kernels are cooperative launches: `grid` must

@@ -1021,6 +1021,29 @@ const void* persist_kernel(bool fp64, const CgPersistPlan& pl)
     return pl.bonds > 0 ? persist_kernel64<true>(pl.lanes) : persist_kernel64<false>(pl.lanes);
 }
 
+// Dynamic shared memory that a block can have in the solves and in the products by
+// tiles.  A kernel's limit is an attribute of the kernel, not of a handle: it is
+// always set to this same value, so that no handle, in this thread or another,
+// lowers it below what another one launches with (or holds in a captured graph).
+int room_less(size_t fixed, int device)
+{
+    int optin = 0;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    return optin - (int)fixed;
+}
+int persist_room(int device) { return room_less(sizeof(Exchange) + 1024, device); }
+int tile_room(int device) { return room_less(2048, device); }
+
+bool set_tile_room(int device)
+{
+    for (const void* t : {(const void*)k_tile_product32<true>, (const void*)k_tile_product32<false>})
+        if (cudaFuncSetAttribute(t, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_room(device)) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+    return true;
+}
+
 }  // namespace
 
 CgPersistPlan cg_persist_rows(bool fp64, int n, int sm_count, int device)
@@ -1043,9 +1066,7 @@ CgPersistPlan cg_persist_rows(bool fp64, int n, int sm_count, int device)
 bool cg_persist_plan(bool fp64, int max_halo, int max_bonds, int device, CgPersistPlan* plan)
 {
     CgPersistPlan pl = *plan;
-    int optin = 0;
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-    const int room = optin - (int)sizeof(Exchange) - 1024;
+    const int room = persist_room(device);
     pl.halo = max_halo;
     const long long bonds = (long long)pl.rows * ((max_bonds + 7) / 8 * 8);
     pl.bonds = bonds < (1 << 20) && persist_smem(fp64, pl.rows, pl.halo, (int)bonds) <= (size_t)room ? (int)bonds : 0;
@@ -1064,53 +1085,40 @@ bool cg_persist_plan(bool fp64, int max_halo, int max_bonds, int device, CgPersi
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kPersistThreads, pl.smem);
     if (per_sm < 1) return false;
-    if (pl.tiled_products)
-        for (const void* t : {(const void*)k_tile_product32<true>, (const void*)k_tile_product32<false>})
-            if (cudaFuncSetAttribute(t, cudaFuncAttributeMaxDynamicSharedMemorySize, room) != cudaSuccess) {
-                cudaGetLastError();
-                return false;
-            }
+    if (pl.tiled_products && !set_tile_room(device)) return false;
     *plan = pl;
     return true;
 }
 
 bool tile_product_may_fit(int rows, double reach, int device)
 {
-    int optin = 0;
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     const double side = std::cbrt((double)rows) + 2.0 * reach;
-    return 2 * sizeof(float4) * side * side * side <= (double)(optin - 2048);
+    return 2 * sizeof(float4) * side * side * side <= (double)tile_room(device);
 }
 
 bool tile_product_plan(int max_halo, int device, CgPersistPlan* plan)
 {
-    int optin = 0;
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-    const int room = optin - 2048;
-    if (2 * sizeof(float4) * (size_t)max_halo > (size_t)room) return false;
-    for (const void* t : {(const void*)k_tile_product32<true>, (const void*)k_tile_product32<false>})
-        if (cudaFuncSetAttribute(t, cudaFuncAttributeMaxDynamicSharedMemorySize, room) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
+    if (2 * sizeof(float4) * (size_t)max_halo > (size_t)tile_room(device) || !set_tile_room(device)) return false;
     plan->halo = max_halo;
     return true;
 }
 
 bool cg_persist_may_fit(int rows, double reach, int device)
 {
-    int optin = 0;
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     const double side = std::cbrt((double)rows) + 2.0 * reach;   // a compact block of rows and its halo
-    return persist_smem(false, rows, (int)std::min(side * side * side, 1e6), 0) <= (size_t)(optin - (int)sizeof(Exchange) - 1024);
+    return persist_smem(false, rows, (int)std::min(side * side * side, 1e6), 0) <= (size_t)persist_room(device);
+}
+
+cudaError_t gang_solve_prepare(int device)
+{
+    return cudaFuncSetAttribute((const void*)k_gang_solve32, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                persist_room(device));
 }
 
 cudaError_t launch_gang_solve(const GangArgs& A, int gangs, size_t smem, cudaStream_t st)
 {
     GangArgs a = A;
     void* args[] = {&a};
-    cudaError_t e = cudaFuncSetAttribute((const void*)k_gang_solve32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
     return cudaLaunchCooperativeKernel((const void*)k_gang_solve32, dim3(gangs * A.gang), dim3(kPersistThreads), args, smem, st);
 }
 

@@ -334,8 +334,11 @@ template <int G, int U>
 int tile_blocks(int halo_cap)
 {
     const size_t smem = sizeof(float4) * 2 * (size_t)halo_cap;
-    cudaFuncSetAttribute(k_spmv_tile<G, U, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_spmv_tile<G, U, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the largest halo of any handle: the limit belongs to the kernel, and a handle
+    // with small halos must not lower it below what another one launches with
+    const int most = (int)(sizeof(float4) * 2 * kMaxHaloCap);
+    cudaFuncSetAttribute(k_spmv_tile<G, U, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    cudaFuncSetAttribute(k_spmv_tile<G, U, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     int a = 0, b = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_spmv_tile<G, U, true>, kBlock, smem);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_spmv_tile<G, U, false>, kBlock, smem);
