@@ -420,6 +420,15 @@ pd_status pd_get_launch_count(pd_handle* h, long long* launches);
 pd_status pd_get_stream(pd_handle* h, void** stream);
 /* Waits until all work of the handle has finished on the device. */
 pd_status pd_synchronize(pd_handle* h);
+/* How long a kernel of this handle waits for another block's records in a
+ * one-launch solve (default 5 s) and for a copy in the lattice product (default
+ * 1 s) before it gives up; negative: the defaults; at most 3600.  A solve whose
+ * wait ran out ends there and pd_advance returns PD_ERR_CUDA; after
+ * pd_apply_operator, which only enqueues, the next pd_synchronize, pd_get or
+ * pd_advance does.  The handle's solves then fail until the next pd_make_ready.
+ * With 0 every wait counts as run out at once: a caller's test of its own error
+ * path. */
+pd_status pd_set_wait_limit(pd_handle* h, double seconds);
 
 /* ---- DataIO (src/core/dataIO.h:20-44) -------------------------------------
  * Output under run->saving_path, as the reference's DataIO: frames
@@ -580,6 +589,10 @@ pd_status pd_batch_get_config(pd_batch* b, pd_batch_config* config);
 pd_status pd_batch_get_launch_count(pd_batch* b, long long* launches);
 pd_status pd_batch_get_stream(pd_batch* b, void** stream);
 pd_status pd_batch_synchronize(pd_batch* b);
+/* As pd_set_wait_limit, for the waits of the batch's solves (default 5 s); with
+ * use_graph it takes effect at the next pd_batch_make_ready.  pd_batch_advance
+ * returns PD_ERR_CUDA, and the batch takes no further step until then. */
+pd_status pd_batch_set_wait_limit(pd_batch* b, double seconds);
 /* Last error text of a batch. */
 const char* pd_batch_last_error_message(pd_batch* b);
 

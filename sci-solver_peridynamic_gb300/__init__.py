@@ -238,6 +238,8 @@ def library(build_if_missing: bool = True):
         "pd_batch_get_launch_count": (st, [vp, P(C.c_longlong)]),
         "pd_batch_get_stream": (st, [vp, P(vp)]),
         "pd_batch_synchronize": (st, [vp]),
+        "pd_batch_set_wait_limit": (st, [vp, C.c_double]),
+        "pd_set_wait_limit": (st, [vp, C.c_double]),
         "pd_batch_last_error_message": (C.c_char_p, [vp]),
     }
     for name, (res, args) in sig.items():
@@ -557,6 +559,11 @@ class Simulator:
     def synchronize(self):
         _check(self.lib.pd_synchronize(self.h), self.h)
 
+    def set_wait_limit(self, seconds: float):
+        """Limit of the kernels' waits (negative: the defaults; 0: every wait
+        counts as run out, for tests of the error path)."""
+        _check(self.lib.pd_set_wait_limit(self.h, float(seconds)), self.h)
+
     def sph_collide(self, sph_pos, sph_vel, slip: float = 1.0) -> int:
         """SPH <-> PD collision (collideDifferentParticles) of the caller's SPH
         particles: (n, 4) float64 arrays of positions and velocities in
@@ -710,6 +717,10 @@ class Batch:
 
     def synchronize(self):
         _bcheck(self.lib.pd_batch_synchronize(self.h), self.h)
+
+    def set_wait_limit(self, seconds: float):
+        """As Simulator.set_wait_limit; with a graph, before makeReady."""
+        _bcheck(self.lib.pd_batch_set_wait_limit(self.h, float(seconds)), self.h)
 
 
 class Scene:

@@ -43,6 +43,7 @@ public:
     long long launches() const { return launches_; }
     cudaStream_t stream() const { return stream_; }
     pd_status synchronize();
+    void set_wait_limit(unsigned long long ns) { wait_ns_ = ns; }
     bool ready() const { return ready_; }
     const std::string& error() const { return err_; }
     void set_error(const std::string& e) { err_ = e; }
@@ -86,6 +87,7 @@ private:
     size_t gang_smem_ = 0, gang_zero_ = 0;   // zeroed before each launch: the first gang_zero_ bytes
     unsigned char* d_gang_ = nullptr;
     GangArgs gang_args_{};
+    unsigned long long wait_ns_ = kWaitSolveNs;
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t exec_ = nullptr;
     // learned warm start: one network for all scenes, run once per step over
@@ -252,7 +254,7 @@ BatchArgs Batch::args(int tune_reps) const
 pd_status Batch::enqueue_step()
 {
     const BatchArgs A = args(0);
-    BCK(cudaMemsetAsync(d_sync_, 0, sizeof(BatchSync), stream_), "reset barrier");
+    BCK(cudaMemsetAsync(d_sync_, 0, offsetof(BatchSync, error), stream_), "reset barrier");
     BCK(cudaMemsetAsync(d_counters_, 0, sizeof(unsigned) * eng_.size(), stream_), "reset counters");
     BCK(launch_batch_pre(fp64_, A, grid_pre_, stream_), "k_batch_pre launch");
     if (opt_.warm_start && total_rows_ > 0) {
@@ -266,6 +268,7 @@ pd_status Batch::enqueue_step()
         G.scenes = d_desc_;
         G.run = d_run_;
         G.error = &d_sync_->error;
+        G.wait_ns = wait_ns_;
         BCK(launch_gang_solve(G, gangs_, gang_smem_, stream_), "k_gang_solve32 launch");
     } else {
         BCK(launch_batch_cg(fp64_, lanes_, unroll_, A, grid_cg_, stream_), "k_batch_cg launch");
@@ -653,7 +656,7 @@ pd_status Batch::pull_state()
     }
     if (sync.error) {
         ready_ = false;
-        err_ = "batch step: a grid barrier wait timed out";
+        err_ = "batch step: a bounded wait of a kernel ran out of time";
         return PD_ERR_CUDA;
     }
     if (opt_.warm_start && mlp_tc_take_error()) {
@@ -920,6 +923,13 @@ pd_status pd_batch_get_stream(pd_batch* b, void** stream)
 {
     if (!b || !b->b || !stream) return PD_ERR_INVALID_ARGUMENT;
     *stream = (void*)b->b->stream();
+    return PD_OK;
+}
+
+pd_status pd_batch_set_wait_limit(pd_batch* b, double seconds)
+{
+    if (!b || !b->b || !(seconds <= 3600.0)) return PD_ERR_INVALID_ARGUMENT;
+    b->b->set_wait_limit(seconds < 0 ? pdgb::kWaitSolveNs : (unsigned long long)(seconds * 1e9));
     return PD_OK;
 }
 

@@ -76,9 +76,10 @@ struct WorkItem {
 struct BatchSync {
     unsigned int count;
     unsigned int gen;
-    int error;             // 1: a barrier wait ran out of time
     int pending[2];        // scenes still needing a force pass (alternating rounds)
     int running;           // scenes whose CG has not finished
+    int error;             // 1: a wait ran out of time; stays until make_ready (every later launch ends
+                           // at once): a step resets what stands before it
     int pad[2];
 };
 
@@ -114,6 +115,7 @@ struct GangArgs {
     ulonglong2* inbox;      // [gangs][2][gang][gang] (zero before the launch)
     ulonglong2* rec;        // a record per row (zero before the launch)
     int* error;
+    unsigned long long wait_ns;   // limit of a wait
 };
 cudaError_t gang_solve_prepare(int device);   // before the first launch on the device
 cudaError_t launch_gang_solve(const GangArgs& A, int gangs, size_t smem, cudaStream_t st);

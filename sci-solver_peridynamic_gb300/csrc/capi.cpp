@@ -273,6 +273,15 @@ pd_status pd_get_stream(pd_handle* h, void** stream)
     return PD_OK;
 }
 
+pd_status pd_set_wait_limit(pd_handle* h, double seconds)
+{
+    ENG(h);
+    if (!(seconds <= 3600.0)) return PD_ERR_INVALID_ARGUMENT;
+    const unsigned long long ns = seconds < 0 ? 0ull : (unsigned long long)(seconds * 1e9);
+    h->eng->set_wait_limit(seconds < 0 ? pdgb::kWaitSolveNs : ns, seconds < 0 ? pdgb::kWaitLatticeNs : ns);
+    return PD_OK;
+}
+
 pd_status pd_synchronize(pd_handle* h)
 {
     ENG(h);

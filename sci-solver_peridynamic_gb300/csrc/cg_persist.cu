@@ -26,9 +26,9 @@
 // needs what was written before or after it.  A record is overwritten only
 // after all its readers have it: the next r of a row follows the exchange of
 // <p, A p>, whose partials depend on every record read for them, and inbox
-// records alternate by epoch parity.  Every wait is bounded: after 5 s a
-// thread records the error and its block returns, and so does every block that
-// sees the error.
+// records alternate by epoch parity.  Every wait is bounded (kWaitSolveNs): a
+// thread whose wait runs out records the error and its block returns, and so
+// does every block that sees the error, in this launch and in later ones.
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
@@ -45,7 +45,6 @@ constexpr int kPersistWarps = kPersistThreads / 32;
 constexpr int kPersistMaxGrid = 256;
 constexpr int kTileLanes = 4;        // lanes per row where the bonds are read from global memory
 constexpr int kTileBlock = 1024;     // threads of a product outside a solve
-constexpr unsigned long long kPersistTimeoutNs = 5000000000ull;   // 5 s
 
 __device__ __forceinline__ unsigned long long now_ns()
 {
@@ -84,6 +83,7 @@ struct PersistArgs {
     int profile;
     int start;                  // form r = p = b - y and its test first (y: A x of the guess)
     int finish;                 // advance the rows when the solve has ended
+    unsigned long long wait_ns; // limit of a wait
 };
 
 // A block's part in a solve.
@@ -94,11 +94,12 @@ struct PersistRun {
     int block, grid;            // this block among those of the solve
     bool start;
     int* error;                 // set when a wait ran out of time
+    unsigned long long wait_ns; // limit of a wait (0: it runs out at once)
 };
 __device__ __forceinline__ PersistRun persist_run(const PersistArgs& A)
 {
     return PersistRun{A.rec, A.inbox, A.rows, A.halo, A.bonds, A.max_iters, (int)blockIdx.x, (int)gridDim.x,
-                      A.start != 0, &A.S.sc->wait_error};
+                      A.start != 0, &A.S.sc->wait_error, A.wait_ns};
 }
 
 // Sums travel as their accumulator's own form: double-float for FP32 data.
@@ -139,22 +140,23 @@ struct Exchange {
 // Polls a record until `arrived` accepts it; false when the wait ran out of
 // time (here or in another thread).
 template <typename Ok>
-__device__ __forceinline__ bool await(const ulonglong2* rec, int* error, Exchange& e, ulonglong2& r, Ok arrived)
+__device__ __forceinline__ bool await(const ulonglong2* rec, int* error, unsigned long long limit, Exchange& e, ulonglong2& r,
+                                      Ok arrived)
 {
     r = observe(rec);
-    if (arrived(r)) return true;
-    unsigned spins = 0;
+    if (limit != 0 && arrived(r)) return true;
+    unsigned spins = limit != 0 ? 0u : ~0u;
     const unsigned long long t0 = now_ns();
     for (;;) {
-        r = observe(rec);
-        if (arrived(r)) return true;
         if ((++spins & 255u) == 0) {
-            if (*(volatile int*)error || now_ns() - t0 > kPersistTimeoutNs) {
+            if (limit == 0 || *(volatile int*)error || now_ns() - t0 > limit) {
                 *(volatile int*)error = 1;
                 e.error = 1;
                 return false;
             }
         }
+        r = observe(rec);
+        if (arrived(r)) return true;
     }
 }
 
@@ -181,7 +183,7 @@ __device__ __forceinline__ bool exchange_sum(Exchange& e, T& v, int step, const 
             ulonglong2* box = A.inbox + (size_t)(epoch & 1) * grid * grid;
             publish(box + (size_t)b * grid + A.block, pack(t), epoch);
             ulonglong2 r;
-            await(box + (size_t)A.block * grid + b, A.error, e, r, [epoch](const ulonglong2& x) { return x.y == epoch; });
+            await(box + (size_t)A.block * grid + b, A.error, A.wait_ns, e, r, [epoch](const ulonglong2& x) { return x.y == epoch; });
             e.from[b] = r.x;
         }
     } else {
@@ -325,7 +327,9 @@ __device__ __forceinline__ bool persist_solve32(const StepParams& P, const Devic
                                                 unsigned char* smem, Exchange& ex, unsigned long long& epoch, bool timed)
 {
     CgScalars* sc = S.sc;
-    // (the scalars change only after every block's last exchange)
+    // (the scalars change only after every block's last exchange; an error may come
+    // from a block of this launch, which the others learn of in their waits)
+    if (__syncthreads_or(*(volatile int*)A.error)) return false;
     if (!A.start && ((volatile CgScalars*)sc)->done) return true;
     const int lo = A.block * A.rows;
     const int nr = max(0, min(A.rows, P.n - lo));
@@ -533,7 +537,7 @@ __device__ __forceinline__ bool persist_solve32(const StepParams& P, const Devic
         const auto gather = [&](int t, int threads) {   // the halo's new r
             for (int h = t; h < nh; h += threads) {
                 ulonglong2 v;
-                if (!await(A.rec + sq[h], A.error, ex, v, [tag](const ulonglong2& x) { return (unsigned)(x.y >> 32) == tag; }))
+                if (!await(A.rec + sq[h], A.error, A.wait_ns, ex, v, [tag](const ulonglong2& x) { return (unsigned)(x.y >> 32) == tag; }))
                     return;
                 const DF yx = unpack<DF>(v.x);
                 sh[h] = make_float4(yx.lo, yx.hi, __uint_as_float((unsigned)v.y), 0.f);
@@ -707,7 +711,7 @@ template <bool CACHED, int G, int U>
 __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist64(PersistArgs A)
 {
     CgScalars* sc = A.S.sc;
-    if (!A.start && ((volatile CgScalars*)sc)->done) return;
+    if (__syncthreads_or(((volatile CgScalars*)sc)->wait_error) || (!A.start && ((volatile CgScalars*)sc)->done)) return;
     extern __shared__ __align__(32) unsigned char smem[];
     __shared__ Exchange ex;
     const PersistRun run = persist_run(A);
@@ -885,7 +889,9 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist64(PersistArgs
             for (int h = t; h < nh; h += threads) {
                 const ulonglong2* rec = A.rec + 2 * (size_t)sq[h];
                 ulonglong2 a, b;
-                if (!await(rec, run.error, ex, a, arrived) || !await(rec + 1, run.error, ex, b, arrived)) return;
+                if (!await(rec, run.error, run.wait_ns, ex, a, arrived) ||
+                    !await(rec + 1, run.error, run.wait_ns, ex, b, arrived))
+                    return;
                 sh[h] = Vec3d{unpack<double>(a.x), unpack<double>((b.y << 32) | (a.y & 0xffffffffull)), unpack<double>(b.x)};
             }
         };
@@ -949,8 +955,9 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_gang_solve32(GangArgs A)
                 publish(turns + turn, (unsigned long long)s_turn, 1ull);
             } else {
                 ulonglong2 r;
-                s_turn = await(turns + turn, A.error, ex, r, [](const ulonglong2& x) { return x.y == 1ull; }) ? (int)r.x
-                                                                                                          : A.n_scenes;
+                s_turn = await(turns + turn, A.error, A.wait_ns, ex, r, [](const ulonglong2& x) { return x.y == 1ull; })
+                             ? (int)r.x
+                             : A.n_scenes;
             }
         }
         __syncthreads();
@@ -963,7 +970,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_gang_solve32(GangArgs A)
         const GangScene g = A.plan[scene];
         const StepParams P = D.P;
         const DeviceState S = D.S;
-        const PersistRun run{A.rec + g.rec, inbox, g.rows, g.halo, g.bonds, 0x7fffffff, block, A.gang, false, A.error};
+        const PersistRun run{A.rec + g.rec, inbox, g.rows, g.halo, g.bonds, 0x7fffffff, block, A.gang, false, A.error, A.wait_ns};
         bool ok;
         if (g.bonds == 0) ok = persist_solve32<false, kTileLanes, 4>(P, S, run, smem, ex, epoch, false);
         else if (g.lanes == 4) ok = persist_solve32<true, 4, 4>(P, S, run, smem, ex, epoch, false);
@@ -1135,10 +1142,10 @@ cudaError_t launch_tile_product(const StepParams& P, const DeviceState& S, const
 
 cudaError_t launch_cg_persist(bool fp64, const StepParams& P, const DeviceState& S, const CgPersistPlan& plan,
                               ulonglong2* rec, ulonglong2* inbox, unsigned long long epoch, int max_iters, bool profile,
-                              bool start, bool finish, cudaStream_t st)
+                              bool start, bool finish, unsigned long long wait_ns, cudaStream_t st)
 {
     PersistArgs A{P, S, rec, inbox, epoch, plan.rows, plan.halo, plan.bonds, max_iters, profile ? 1 : 0, start ? 1 : 0,
-                  finish ? 1 : 0};
+                  finish ? 1 : 0, wait_ns};
     void* args[] = {&A};
     return cudaLaunchCooperativeKernel(persist_kernel(fp64, plan), dim3(plan.grid), dim3(kPersistThreads), args, plan.smem,
                                        st);

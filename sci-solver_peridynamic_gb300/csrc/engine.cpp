@@ -141,6 +141,7 @@ void Engine::free_all()
     sph_buffers_free(&sph_);
     lat_ = LatticeParams{};
     lat_ok_ = false;
+    wait_unread_ = false;
     if (d_inbox_) cudaFree(d_inbox_);
     d_inbox_ = nullptr;
     persist_ = CgPersistPlan{};
@@ -272,6 +273,7 @@ pd_status Engine::make_ready()
                          total_slots_, &lat_, &latb_, &ok, stream_),
            "lattice build");
         lat_ok_ = ok != 0;
+        lat_.wait_ns = wait_lattice_ns_;
     }
     if (persist_.tiled_products) tiles_ = persist_;
     if (opt_.spmv_path == 0 && persist_.grid == 0 && !lat_ok_) {
@@ -933,7 +935,28 @@ pd_status Engine::synchronize()
 {
     CK(cudaSetDevice(device_), "cudaSetDevice");
     CK(cudaStreamSynchronize(stream_), "cudaStreamSynchronize");
-    return PD_OK;
+    return wait_check();
+}
+
+// Whether a wait of an apply_operator since the last answer ran out of time (its
+// result is then incomplete): asked by the calls that wait for the device.
+pd_status Engine::wait_check()
+{
+    if (!wait_unread_) return PD_OK;
+    int error = 0;
+    CK(cudaMemcpyAsync(&error, &S_.sc->wait_error, sizeof(int), cudaMemcpyDeviceToHost, stream_), "read wait error");
+    CK(cudaStreamSynchronize(stream_), "read wait error");
+    wait_unread_ = false;
+    if (!error) return PD_OK;
+    err_ = "apply_operator: a bounded wait of a kernel ran out of time";
+    return PD_ERR_CUDA;
+}
+
+void Engine::set_wait_limit(unsigned long long solve_ns, unsigned long long lattice_ns)
+{
+    wait_solve_ns_ = solve_ns;
+    wait_lattice_ns_ = lattice_ns;
+    if (lat_ok_) lat_.wait_ns = lattice_ns;
 }
 
 pd_status Engine::operator_view(pd_operator_view* v) const
@@ -978,6 +1001,7 @@ pd_status Engine::apply_operator(const void* d_x, void* d_y, double* d_dot)
     // counter 4 of the handle's reduction scratch is reserved for this call
     ReduceSlot slot{S_.partials, S_.counters + 4};
     apply_op(last_params_, d_x, d_y, slot, d_dot);
+    wait_unread_ |= L_.lattice != 0;
     ++launches_;
     CK(cudaGetLastError(), "apply_operator launch");
     return PD_OK;
@@ -993,6 +1017,8 @@ pd_status Engine::advance(int nsteps)
     }
     if (nsteps < 0) return PD_ERR_INVALID_ARGUMENT;
     CK(cudaSetDevice(device_), "cudaSetDevice");
+    pd_status ws = wait_check();
+    if (ws != PD_OK) return ws;
     for (int k = 0; k < nsteps; ++k) {
         if (!cg_converged_) break;
         ++step_;
@@ -1292,7 +1318,7 @@ pd_status Engine::cg_persist_loop(const StepParams& P, bool start)
     int seen = 0;   // iterations of the solve so far
     for (long long run = 0;;) {
         CK(launch_cg_persist(fp64_, P, S_, persist_, d_inbox_ + 2 * (size_t)persist_.grid * persist_.grid, d_inbox_,
-                             persist_epoch_, batch, profiling_, start, solve_updates_, stream_),
+                             persist_epoch_, batch, profiling_, start, solve_updates_, wait_solve_ns_, stream_),
            "cg launch");
         ++launches_;
         CK(cudaMemcpyAsync(h_sc_, S_.sc, sizeof(CgScalars), cudaMemcpyDeviceToHost, stream_), "read cg scalars");
@@ -1648,6 +1674,8 @@ pd_status Engine::get(pd_variable var, void* dst, size_t bytes)
         return PD_ERR_NOT_READY;
     }
     CK(cudaSetDevice(device_), "cudaSetDevice");
+    const pd_status ws = wait_check();
+    if (ws != PD_OK) return ws;
     const size_t N = (size_t)n_;
     switch (var) {
     case PD_VAR_POSITION:

@@ -41,6 +41,8 @@ public:
     long long launches() const { return launches_; }
     cudaStream_t stream() const { return stream_; }
     pd_status synchronize();
+    // ns; 0: every wait counts as run out
+    void set_wait_limit(unsigned long long solve_ns, unsigned long long lattice_ns);
     pd_status operator_view(pd_operator_view* v) const;
     pd_status apply_operator(const void* d_x, void* d_y, double* d_dot);
     pd_status ws_set_params(const float* params, size_t count);
@@ -77,6 +79,7 @@ private:
     pd_status gang_tiles(int rows, int blocks, CgPersistPlan* plan, bool* fits);
     void gang_tiles_free();
     pd_status build_halos();
+    pd_status wait_check();
     void lattice_resync(bool force);   // the lattice product's 1/d0 table from the live CSR bonds
     // mixed mode: reorders every row's live bonds for the (g, u) SpMV shape
     void relayout_bonds(int g, int u);
@@ -208,6 +211,8 @@ private:
     ulonglong2* d_inbox_ = nullptr;    // its records: partial sums (2 grid^2), then r
     CgPersistPlan tiles_{};            // products by tiles (grid 0: not used)
     unsigned long long persist_epoch_ = 0;
+    unsigned long long wait_solve_ns_ = kWaitSolveNs, wait_lattice_ns_ = kWaitLatticeNs;
+    bool wait_unread_ = false;         // a product by apply_operator whose waits no read-back has told of yet
     bool solve_updates_ = false;       // the one-launch solve of this step advances the rows itself
     // profiling
     bool profiling_ = false;

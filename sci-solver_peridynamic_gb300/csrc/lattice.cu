@@ -349,11 +349,11 @@ __global__ void __launch_bounds__(kBlock) k_lat_xpby(int n, const int* __restric
 // one stencil column (40 bytes a thread) loaded ahead the product took 150 us at
 // 1M particles however few instructions it had, 105 us without the table.
 // Entry k's bond vector is xi = d_q - (d_p - h v_k), formed in FP32 with the
-// differences of w.  Every wait is bounded (a second): on expiry the block
-// records the error in the handle's scalars, waits once more for its copies
-// and returns.
+// differences of w.  Every wait is bounded (lp.wait_ns, a second): on expiry the
+// block records the error in the handle's scalars and ends the solve there, waits
+// once more for every copy of its own still in flight (a second at most, whatever
+// the limit) and returns; later products of the handle take no bricks.
 
-constexpr unsigned long long kLatTimeoutNs = 1000000000ull;
 __device__ __forceinline__ unsigned long long lat_now_ns()
 {
     unsigned long long t;
@@ -379,13 +379,16 @@ __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity)
         : "memory");
     return done != 0;
 }
-__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity)
+// The whole warp's answer: false when a lane's wait ran out of time (a limit of 0:
+// at once).
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, unsigned long long limit)
 {
-    if (bar_try(bar, parity)) return true;
-    const unsigned long long t0 = lat_now_ns();
-    while (!bar_try(bar, parity))
-        if (lat_now_ns() - t0 > kLatTimeoutNs) return false;
-    return true;
+    bool ok = limit != 0;
+    if (ok && !bar_try(bar, parity)) {
+        const unsigned long long t0 = lat_now_ns();
+        while (ok && !bar_try(bar, parity)) ok = lat_now_ns() - t0 <= limit;
+    }
+    return __all_sync(0xffffffffu, ok);
 }
 
 // The rows of a thread: their sites' words and the sums of a1 (w_q - w_p) + g xi
@@ -479,7 +482,7 @@ __device__ __forceinline__ bool lat_columns(const LatticeParams& lp, const LatHa
     const int lane = threadIdx.x & 31;
     for (; count > 0; count -= M) {
         const int slot = s.used & 1;
-        if (!bar_wait(s.bars + 8 * slot, (s.used >> 1) & 1)) return false;
+        if (!bar_wait(s.bars + 8 * slot, (s.used >> 1) & 1, lp.wait_ns)) return false;
         ++s.used;
         const float2* e2 = ring + slot * (kLatSlabBytes / (int)sizeof(float2)) + lane;
 #pragma unroll 1
@@ -542,7 +545,8 @@ __global__ void __launch_bounds__(32 * lat_warps(R), 2)
     if (threadIdx.x == 0) {
         for (int k = 0; k < 1 + 2 * lat_warps(R); ++k) bar_init(bars + 8 * k, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        b = (int)atomicAdd(&lp.sched[0], 1u);
+        // (no bricks once a wait of the handle has run out)
+        b = ((volatile CgScalars*)S.sc)->wait_error ? lp.n_bricks : (int)atomicAdd(&lp.sched[0], 1u);
         s_ahead = b;
     }
     __syncthreads();
@@ -569,8 +573,9 @@ __global__ void __launch_bounds__(32 * lat_warps(R), 2)
     float cz[kLatTab];
 #pragma unroll
     for (int k = 0; k < kLatTab; ++k) cz[k] = lp.cz[k];
-    for (int it = 0; b < lp.n_bricks; ++it) {
-        ok = bar_wait(bars, it & 1);
+    int it = 0;   // halos waited for
+    for (; b < lp.n_bricks; ++it) {
+        ok = bar_wait(bars, it & 1, lp.wait_ns);
         const int ahead = *(volatile int*)&s_ahead;   // the next brick
         const int next = chunk_of(ahead);
         if (ok && chunk >= 0) {
@@ -609,7 +614,7 @@ __global__ void __launch_bounds__(32 * lat_warps(R), 2)
                     mixed_row_result<DOT>(P, S, p, ab, c0, t2, m, make_float4(row.w[i].x, row.w[i].y, row.wz[i], 0.f),
                                           -row.sxy[i].x, -row.sxy[i].y, -row.sz[i], out, acc);
             }
-        } else if (next >= 0) {
+        } else if (ok && next >= 0) {
             if (lane == 0)
                 for (int k = 0; k < min(2, lp.slabs); ++k) lat_issue(s, lp, next, k);
             base_n = __ldg(lp.pair_base + next * 32 + lane);
@@ -626,10 +631,12 @@ __global__ void __launch_bounds__(32 * lat_warps(R), 2)
             load_halo(b);
         }
     }
-    if (!ok) {   // record it, and wait once more for the copies in flight
+    if (!ok) {   // record it, end the solve, and wait once more for the copies in flight
         ((volatile CgScalars*)S.sc)->wait_error = 1;
-        if (lane == 0)
-            for (; s.used < s.issued; ++s.used) bar_wait(s.bars + 8 * (s.used & 1), (s.used >> 1) & 1);
+        ((volatile CgScalars*)S.sc)->done = 1;
+        bar_wait(bars, it & 1, kWaitLatticeNs);   // the halo's (its phase is over where another wait ran out)
+        const int issued = __shfl_sync(0xffffffffu, s.issued, 0);
+        for (; s.used < issued; ++s.used) bar_wait(s.bars + 8 * (s.used & 1), (s.used >> 1) & 1, kWaitLatticeNs);
     }
     __syncthreads();
     // every block has taken its last brick index: the last to arrive resets the counter
@@ -991,6 +998,7 @@ cudaError_t lattice_build(int n, double spacing, dbl4* x64, float4* X32, int* pe
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     L.grid = std::max(1, std::min(L.n_bricks, lattice_spmv_blocks_per_sm(L) * sms));
+    L.wait_ns = kWaitLatticeNs;
     *lp = L;
     *lb = t.lb;
     t.lb = LatticeBuffers{};

@@ -30,6 +30,11 @@ constexpr uint8_t kActMask = 7;
 constexpr uint8_t kActContact = 8;
 
 // Scalars of the device-resident CG (one instance per handle, device memory).
+// Limits of the kernels' waits (ns): for the copies of the lattice product, and for
+// another block's records in a one-launch solve.  pd_set_wait_limit sets others.
+constexpr unsigned long long kWaitLatticeNs = 1000000000ull;
+constexpr unsigned long long kWaitSolveNs = 5000000000ull;
+
 struct CgScalars {
     double bnorm2;     // ||P b||^2 over free rows
     double tol;        // rel_tol * ||P b||
@@ -51,7 +56,8 @@ struct CgScalars {
     int ws_rejects;        // batch: consecutive rejected guesses (and paused steps since)
     int ws_skip;           // batch: 1 while this step's learned pass is paused
     int ws_skipped;        // batch: steps whose learned pass was paused
-    int wait_error;        // a bounded wait of a kernel ran out of time (cg_persist.cu, lattice.cu)
+    int wait_error;        // a bounded wait of a kernel ran out of time (cg_persist.cu, lattice.cu); stays
+                           // until the next make_ready, and every solve of the handle ends at once
     double ns_spmv;        // cg_persist.cu, profiling: ns of the latest launch's products
     double ns_vec;         // ... and of its vector phases
 };
@@ -194,6 +200,7 @@ struct LatticeParams {
     int coff[kLatTab * kLatTab];                              // halo index offset
     float ccx[kLatTab * kLatTab], ccy[kLatTab * kLatTab];     // h dx, h dy
     float cz[kLatTab];        // h dz, dz = -kLatRmax .. kLatRmax
+    unsigned long long wait_ns;   // limit of the product's waits for its copies
 };
 
 struct LatticeBuffers {       // device allocations owned by the engine
@@ -289,7 +296,7 @@ bool cg_persist_may_fit(int rows, double reach, int device);
 // finish: the step's update of the rows, when this launch ends the solve.
 cudaError_t launch_cg_persist(bool fp64, const StepParams& P, const DeviceState& S, const CgPersistPlan& plan,
                               ulonglong2* rec, ulonglong2* inbox, unsigned long long epoch, int max_iters, bool profile,
-                              bool start, bool finish, cudaStream_t st);
+                              bool start, bool finish, unsigned long long wait_ns, cudaStream_t st);
 // y = A in by a block per tile (mixed precision); with cg (a CG iteration) alpha
 // from <in, A in>, and *dot_out (may be null) receives it
 cudaError_t launch_tile_product(const StepParams& P, const DeviceState& S, const CgPersistPlan& plan, const void* in,

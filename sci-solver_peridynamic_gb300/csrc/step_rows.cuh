@@ -826,7 +826,7 @@ __device__ __forceinline__ void cg_fin_init(CgScalars* sc, double bb)
     sc->bnorm2 = bb;
     sc->tol = 0.0 + sc->rel_tol * sqrt(bb);
     sc->iter = 0;
-    sc->done = 0;
+    sc->done = sc->wait_error;
     sc->converged = 0;
 }
 
