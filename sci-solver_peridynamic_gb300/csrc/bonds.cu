@@ -24,7 +24,6 @@ namespace pdgb {
 
 namespace {
 
-constexpr int kRowAlign = 8;        // row starts aligned to 8 ints (one 32-byte sector)
 constexpr int kSortThreads = 256;
 constexpr int kSortItems = 8;
 constexpr int kSortTile = kSortThreads * kSortItems;

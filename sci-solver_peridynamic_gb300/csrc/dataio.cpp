@@ -433,11 +433,19 @@ pd_status Engine::dataio_load_state(size_t timestep)
         return PD_ERR_FILE;
     }
     CK(cudaMemcpy(d_perm_, perm.data(), sizeof(int32_t) * N, cudaMemcpyHostToDevice), "upload perm");
-    // the lattice product's tables follow this handle's slot order: a state
-    // saved in another order continues on the gather product
+    // the lattice product's tables follow this handle's slot order and bonds: a
+    // state saved in another order, or of another body with other bond offsets,
+    // continues on the gather product
     const bool same_order = std::equal(perm.begin(), perm.end(), perm_.begin());
     perm_.assign(perm.begin(), perm.end());
     cnt_init_.assign(cinit.begin(), cinit.end());
+    bonds_initial_ = 0;   // (the sizes of the bond exports; another body's differ)
+    sim_.pd_max_num_bonds = 0;
+    for (int c : cnt_init_) {
+        bonds_initial_ += c;
+        sim_.pd_max_num_bonds = std::max(sim_.pd_max_num_bonds, c);
+    }
+    W_.max_bonds = std::max(sim_.pd_max_num_bonds, 1);
     for (size_t i = 0; i < N; ++i) inv_[(size_t)perm_[i]] = (int)i;
     saved_frame_ = frame;
     step_ = step;
@@ -464,7 +472,9 @@ pd_status Engine::dataio_load_state(size_t timestep)
         const pd_status hs = build_halos();
         if (hs != PD_OK) return hs;
     }
-    if (lat_ok_ && !same_order) {
+    int on_stencil = 1;
+    if (lat_ok_ && same_order) CK(lattice_holds(S_, lat_, &on_stencil, stream_), "lattice check");
+    if (lat_ok_ && !(same_order && on_stencil)) {
         lattice_free(&latb_);
         lat_ = LatticeParams{};
         lat_ok_ = false;

@@ -655,14 +655,25 @@ void Engine::gang_tiles_free()
 
 // The tiles' halos and local indices of the CSR rows as they are.  A body
 // whose blocks' halos no longer fit (a checkpoint in another slot order) leaves
-// the one-launch solve.
+// the one-launch solve, and so does one with more bond slots in a block than its
+// plan keeps in shared memory, or with rows that do not start on whole groups
+// of slots (both: a state of another body).
 pd_status Engine::build_halos()
 {
     int max_halo = 0, unfit = 0;
     CK(build_tiles(S_, n_, &max_halo, &unfit, stream_), "build tiles");
     S_.halo_cap = std::min(max_halo, kMaxHaloCap);
-    if (persist_.grid > 0 && (unfit > 0 || max_halo > persist_.halo)) persist_ = CgPersistPlan{};
-    if (persist_.grid == 0 && tiles_.grid > 0 && (unfit > 0 || !tile_product_plan(max_halo, device_, &tiles_)))
+    bool rows_fit = true;
+    if (persist_.grid > 0 || tiles_.grid > 0) {
+        std::vector<int> rp((size_t)n_ + 1);
+        CK(cudaMemcpyAsync(rp.data(), S_.row_ptr, sizeof(int) * rp.size(), cudaMemcpyDeviceToHost, stream_), "read rows");
+        CK(cudaStreamSynchronize(stream_), "read rows");
+        for (int v : rp) rows_fit &= v % kRowAlign == 0;
+        for (int lo = 0; persist_.bonds > 0 && lo < n_; lo += persist_.rows)
+            rows_fit &= rp[(size_t)std::min(n_, lo + persist_.rows)] - rp[(size_t)lo] <= persist_.bonds;
+    }
+    if (persist_.grid > 0 && (unfit > 0 || max_halo > persist_.halo || !rows_fit)) persist_ = CgPersistPlan{};
+    if (persist_.grid == 0 && tiles_.grid > 0 && (unfit > 0 || !rows_fit || !tile_product_plan(max_halo, device_, &tiles_)))
         tiles_ = CgPersistPlan{};
     return PD_OK;
 }

@@ -162,6 +162,25 @@ __global__ void __launch_bounds__(kBlock) k_lat_offsets(int n, const int4* __res
     if (bad) atomicOr(fail, 1);
 }
 
+// *fail set when a bond of a row, live or restorable (cnt_bk), is no entry of the stencil
+__global__ void __launch_bounds__(kBlock) k_lat_holds(DeviceState S, const __grid_constant__ LatticeParams lp,
+                                                      int* __restrict__ fail)
+{
+    int bad = 0;
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < S.n; p += gridDim.x * blockDim.x) {
+        const int4 sp = lp.site[p];
+        const int rs = S.row_ptr[p], cn = max(S.cnt[p], S.cnt_bk[p]);
+        for (int j = 0; j < cn; ++j) {
+            const int4 sq = lp.site[S.col[rs + j]];
+            const int dx = sq.x - sp.x, dy = sq.y - sp.y, dz = sq.z - sp.z;
+            if (abs(dx) > kLatRmax || abs(dy) > kLatRmax || abs(dz) > kLatRmax ||
+                lp.offk[((dz + kLatRmax) * kLatTab + (dy + kLatRmax)) * kLatTab + (dx + kLatRmax)] < 0)
+                bad = 1;
+        }
+    }
+    if (bad) atomicOr(fail, 1);
+}
+
 // shifted sites and the brick-major sort key of every slot
 __global__ void __launch_bounds__(kBlock) k_lat_keys(int n, int4* __restrict__ site, int3 lo, int bx, int3 nb,
                                                      unsigned* __restrict__ key, int* __restrict__ val)
@@ -656,6 +675,22 @@ __global__ void __launch_bounds__(32 * lat_warps(R), 2)
 }
 
 }  // namespace
+
+cudaError_t lattice_holds(const DeviceState& S, const LatticeParams& lp, int* ok, cudaStream_t st)
+{
+    int *d = nullptr, fail = 0;
+    LT_TRY(cudaMalloc(&d, sizeof(int)));
+    cudaError_t e = cudaMemsetAsync(d, 0, sizeof(int), st);
+    if (e == cudaSuccess) {
+        k_lat_holds<<<blocks_for(S.n), kBlock, 0, st>>>(S, lp, d);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&fail, d, sizeof(int), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    cudaFree(d);
+    *ok = fail == 0;
+    return e;
+}
 
 size_t lattice_smem_bytes(const LatticeParams& lp)
 {

@@ -24,6 +24,7 @@ __host__ __device__ inline dbl4 make_dbl4(double x, double y, double z, double w
 
 // Activity byte: low 3 bits = pd_activity, bit 3 = in contact with the sphere
 // during the current step (set by the force pass, read by the SpMV).
+constexpr int kRowAlign = 8;        // row starts aligned to 8 bond slots (one 32-byte sector of col)
 constexpr int kTileRows = 256;      // rows per tile of the shared-memory SpMV
 constexpr int kMaxHaloCap = 2048;   // halo entries a tile may stage (64 KB of shared memory)
 constexpr uint8_t kActMask = 7;
@@ -241,6 +242,8 @@ struct LaunchCfg {
 // spacing (2 r).  On success fills *lp (without `ell`) and *lb.
 cudaError_t lattice_build(int n, double spacing, dbl4* x64, float4* X32, int* perm, int* row_ptr, int* cnt, int** col,
                           long long total_slots, LatticeParams* lp, LatticeBuffers* lb, int* ok, cudaStream_t st);
+// *ok = 0 when a bond of the CSR rows as they are is no entry of the stencil
+cudaError_t lattice_holds(const DeviceState& S, const LatticeParams& lp, int* ok, cudaStream_t st);
 // 1/d0 table from the live CSR bonds (force = 0: only when the force pass
 // reported a broken bond, read from S.flags[1] on the device)
 void launch_lattice_ell(const DeviceState& S, const LatticeParams& lp, int force, int grid, cudaStream_t st);
