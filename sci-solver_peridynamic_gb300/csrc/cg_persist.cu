@@ -480,7 +480,9 @@ __device__ __forceinline__ bool persist_solve32(const StepParams& P, const Devic
                         if constexpr (CACHED) g = sg[base + j];
                         else if constexpr (FIXED) g = bond_geometry_fixed(shx[lc[u]], xp, per_edge, ac[u], a);
                         else g = bond_geometry(shx[lc[u]], xp, sup, ac[u], a);
-                        if (FIXED && j >= cn) a = g.i3 = 0.f;   // (every slot of a row has a halo index)
+                        // (every slot of a row has a halo index; a w that is not finite there
+                        // makes no row wrong that <p, A p> has not made so already)
+                        if (FIXED && j >= cn) a = g.i3 = 0.f;
                         const float wx = w.x - Wq.x, wy = w.y - Wq.y, wz = w.z - Wq.z;
                         const float d = fmaf(g.x, wx, fmaf(g.y, wy, g.z * wz)) * g.i3;
                         ax = fmaf(a, wx, fmaf(d, g.x, ax));
@@ -655,7 +657,10 @@ __global__ void __launch_bounds__(kTileBlock, 1)
                 float ic[4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    lc[u] = l[u];
+                    // (a slot without a live bond takes the partner of the lane's first
+                    // one, which has one: 0 times the w of a broken bond's partner, which
+                    // a caller may have left NaN, is NaN.  1.1 % of 36 us at 200k particles)
+                    lc[u] = FIXED && j0 + u >= cn ? l[0] : l[u];
                     ic[u] = id0[u];
                 }
                 if (j0 + R * 4 < cn) load_bonds(S, rs + j0 + R * 4, l, id0);   // in flight while this step's bonds are added
