@@ -398,16 +398,15 @@ __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity)
         : "memory");
     return done != 0;
 }
-// The whole warp's answer: false when a lane's wait ran out of time (a limit of 0:
-// at once).
+// A lane's own answer: lanes of a warp may differ, so none of them leaves its
+// path for it (a vote of the warp per wait: 123 against 115 us at 1M particles).
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, unsigned long long limit)
 {
-    bool ok = limit != 0;
-    if (ok && !bar_try(bar, parity)) {
-        const unsigned long long t0 = lat_now_ns();
-        while (ok && !bar_try(bar, parity)) ok = lat_now_ns() - t0 <= limit;
-    }
-    return __all_sync(0xffffffffu, ok);
+    if (bar_try(bar, parity)) return true;
+    const unsigned long long t0 = lat_now_ns();
+    while (!bar_try(bar, parity))
+        if (lat_now_ns() - t0 > limit) return false;
+    return true;
 }
 
 // The rows of a thread: their sites' words and the sums of a1 (w_q - w_p) + g xi
@@ -491,17 +490,18 @@ __device__ __forceinline__ void lat_issue(LatStream& s, const LatticeParams& lp,
 }
 
 // The stencil's columns of reach RC, the first one c, slab by slab; after a slab
-// the one two further on is asked for, of the next chunk at the end.
+// the one two further on is asked for, of the next chunk at the end.  Once a wait
+// has run out a lane waits no more and asks for nothing (ok).
 template <int R, int RC>
-__device__ __forceinline__ bool lat_columns(const LatticeParams& lp, const LatHalo& halo, int base, const float2* ring,
+__device__ __forceinline__ void lat_columns(const LatticeParams& lp, const LatHalo& halo, int base, const float2* ring,
                                             LatStream& s, int chunk, int next, int& slab, int& c, int count,
-                                            const float (&cz)[kLatTab], LatRows& row)
+                                            const float (&cz)[kLatTab], LatRows& row, bool& ok)
 {
     constexpr int N = 2 * RC + 1, M = lat_slab_columns(RC);
     const int lane = threadIdx.x & 31;
     for (; count > 0; count -= M) {
         const int slot = s.used & 1;
-        if (!bar_wait(s.bars + 8 * slot, (s.used >> 1) & 1, lp.wait_ns)) return false;
+        ok = ok && bar_wait(s.bars + 8 * slot, (s.used >> 1) & 1, lp.wait_ns);
         ++s.used;
         const float2* e2 = ring + slot * (kLatSlabBytes / (int)sizeof(float2)) + lane;
 #pragma unroll 1
@@ -513,12 +513,11 @@ __device__ __forceinline__ bool lat_columns(const LatticeParams& lp, const LatHa
         }
         __syncwarp();   // every lane is done with the slab
         const int ahead = ++slab + 1;
-        if (lane == 0) {
+        if (lane == 0 && ok) {
             if (ahead < lp.slabs) lat_issue(s, lp, chunk, ahead);
             else if (next >= 0) lat_issue(s, lp, next, ahead - lp.slabs);
         }
     }
-    return true;
 }
 
 template <int R, bool DOT>
@@ -564,8 +563,8 @@ __global__ void __launch_bounds__(32 * lat_warps(R), 2)
     if (threadIdx.x == 0) {
         for (int k = 0; k < 1 + 2 * lat_warps(R); ++k) bar_init(bars + 8 * k, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        // (no bricks once a wait of the handle has run out)
-        b = ((volatile CgScalars*)S.sc)->wait_error ? lp.n_bricks : (int)atomicAdd(&lp.sched[0], 1u);
+        b = (int)atomicAdd(&lp.sched[0], 1u);
+        if (((volatile CgScalars*)S.sc)->wait_error) b = lp.n_bricks;   // (no bricks once a wait of the handle has run out)
         s_ahead = b;
     }
     __syncthreads();
@@ -594,10 +593,10 @@ __global__ void __launch_bounds__(32 * lat_warps(R), 2)
     for (int k = 0; k < kLatTab; ++k) cz[k] = lp.cz[k];
     int it = 0;   // halos waited for
     for (; b < lp.n_bricks; ++it) {
-        ok = bar_wait(bars, it & 1, lp.wait_ns);
+        ok = lp.wait_ns != 0 && bar_wait(bars, it & 1, lp.wait_ns);
         const int ahead = *(volatile int*)&s_ahead;   // the next brick
         const int next = chunk_of(ahead);
-        if (ok && chunk >= 0) {
+        if (chunk >= 0) {
             const int base = base_n;
             const int2 slots = slots_n;
             const uint8_t ab2[2] = {slots.x >= 0 ? S.act[slots.x] : (uint8_t)0, slots.y >= 0 ? S.act[slots.y] : (uint8_t)0};
@@ -618,10 +617,10 @@ __global__ void __launch_bounds__(32 * lat_warps(R), 2)
             }
             const float2* ring2 = (const float2*)ring;
             int c = 0, slab = 0;
-            if constexpr (R >= 3) ok = ok && lat_columns<R, 3>(lp, halo, base, ring2, s, chunk, next, slab, c, lp.ncol[3], cz, row);
-            if constexpr (R >= 2) ok = ok && lat_columns<R, 2>(lp, halo, base, ring2, s, chunk, next, slab, c, lp.ncol[2], cz, row);
-            ok = ok && lat_columns<R, 1>(lp, halo, base, ring2, s, chunk, next, slab, c, lp.ncol[1], cz, row);
-            ok = ok && lat_columns<R, 0>(lp, halo, base, ring2, s, chunk, next, slab, c, lp.ncol[0], cz, row);
+            if constexpr (R >= 3) lat_columns<R, 3>(lp, halo, base, ring2, s, chunk, next, slab, c, lp.ncol[3], cz, row, ok);
+            if constexpr (R >= 2) lat_columns<R, 2>(lp, halo, base, ring2, s, chunk, next, slab, c, lp.ncol[2], cz, row, ok);
+            lat_columns<R, 1>(lp, halo, base, ring2, s, chunk, next, slab, c, lp.ncol[1], cz, row, ok);
+            lat_columns<R, 0>(lp, halo, base, ring2, s, chunk, next, slab, c, lp.ncol[0], cz, row, ok);
 #pragma unroll
             for (int i = 0; i < kLatRZ; ++i) {
                 const int p = i == 0 ? slots.x : slots.y;
@@ -633,8 +632,8 @@ __global__ void __launch_bounds__(32 * lat_warps(R), 2)
                     mixed_row_result<DOT>(P, S, p, ab, c0, t2, m, make_float4(row.w[i].x, row.w[i].y, row.wz[i], 0.f),
                                           -row.sxy[i].x, -row.sxy[i].y, -row.sz[i], out, acc);
             }
-        } else if (ok && next >= 0) {
-            if (lane == 0)
+        } else if (next >= 0) {
+            if (lane == 0 && ok)
                 for (int k = 0; k < min(2, lp.slabs); ++k) lat_issue(s, lp, next, k);
             base_n = __ldg(lp.pair_base + next * 32 + lane);
             slots_n = __ldg((const int2*)lp.pair_slot + next * 32 + lane);
@@ -654,8 +653,8 @@ __global__ void __launch_bounds__(32 * lat_warps(R), 2)
         ((volatile CgScalars*)S.sc)->wait_error = 1;
         ((volatile CgScalars*)S.sc)->done = 1;
         bar_wait(bars, it & 1, kWaitLatticeNs);   // the halo's (its phase is over where another wait ran out)
-        const int issued = __shfl_sync(0xffffffffu, s.issued, 0);
-        for (; s.used < issued; ++s.used) bar_wait(s.bars + 8 * (s.used & 1), (s.used >> 1) & 1, kWaitLatticeNs);
+        for (int k = max(0, s.issued - 2); k < s.issued; ++k)   // (lane 0's: the latest of each of its two slots)
+            bar_wait(s.bars + 8 * (k & 1), (k >> 1) & 1, kWaitLatticeNs);
     }
     __syncthreads();
     // every block has taken its last brick index: the last to arrive resets the counter
