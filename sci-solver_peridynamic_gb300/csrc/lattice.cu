@@ -491,7 +491,7 @@ __device__ __forceinline__ void lat_issue(LatStream& s, const LatticeParams& lp,
 
 // The stencil's columns of reach RC, the first one c, slab by slab; after a slab
 // the one two further on is asked for, of the next chunk at the end.  Once a wait
-// has run out a lane waits no more and asks for nothing (ok).
+// has run out a lane waits no more (but looks) and asks for nothing (ok).
 template <int R, int RC>
 __device__ __forceinline__ void lat_columns(const LatticeParams& lp, const LatHalo& halo, int base, const float2* ring,
                                             LatStream& s, int chunk, int next, int& slab, int& c, int count,
@@ -501,7 +501,7 @@ __device__ __forceinline__ void lat_columns(const LatticeParams& lp, const LatHa
     const int lane = threadIdx.x & 31;
     for (; count > 0; count -= M) {
         const int slot = s.used & 1;
-        ok = ok && bar_wait(s.bars + 8 * slot, (s.used >> 1) & 1, lp.wait_ns);
+        if (!bar_wait(s.bars + 8 * slot, (s.used >> 1) & 1, ok ? lp.wait_ns : 0ull)) ok = false;
         ++s.used;
         const float2* e2 = ring + slot * (kLatSlabBytes / (int)sizeof(float2)) + lane;
 #pragma unroll 1
@@ -520,8 +520,11 @@ __device__ __forceinline__ void lat_columns(const LatticeParams& lp, const LatHa
     }
 }
 
+// At most 112 registers, which leaves an SM room for a 256-thread block of a vector
+// kernel beside two of these: with 115, three bodies of 1M particles that each make
+// four products on a stream of their own took 480 us a body, 461 with 109.
 template <int R, bool DOT>
-__global__ void __launch_bounds__(32 * lat_warps(R), 2)
+__global__ void __maxnreg__(R <= 2 ? 112 : 128)
     k_spmv_lattice(StepParams P, DeviceState S, const __grid_constant__ LatticeParams lp, float4* __restrict__ out,
                    ReduceSlot slot, CgScalars* cg, double* dot_out)
 {
@@ -591,9 +594,10 @@ __global__ void __launch_bounds__(32 * lat_warps(R), 2)
     float cz[kLatTab];
 #pragma unroll
     for (int k = 0; k < kLatTab; ++k) cz[k] = lp.cz[k];
-    int it = 0;   // halos waited for
-    for (; b < lp.n_bricks; ++it) {
-        ok = lp.wait_ns != 0 && bar_wait(bars, it & 1, lp.wait_ns);
+    uint32_t phase = 0;   // of the halo's barrier
+    ok = lp.wait_ns != 0 || b >= lp.n_bricks;
+    while (ok && b < lp.n_bricks) {
+        ok = bar_wait(bars, phase, lp.wait_ns);
         const int ahead = *(volatile int*)&s_ahead;   // the next brick
         const int next = chunk_of(ahead);
         if (chunk >= 0) {
@@ -644,6 +648,7 @@ __global__ void __launch_bounds__(32 * lat_warps(R), 2)
         }
         b = ahead;
         chunk = next;
+        phase ^= 1u;
         if (threadIdx.x == 0 && b < lp.n_bricks) {
             s_ahead = (int)atomicAdd(&lp.sched[0], 1u);
             load_halo(b);
@@ -652,7 +657,7 @@ __global__ void __launch_bounds__(32 * lat_warps(R), 2)
     if (!ok) {   // record it, end the solve, and wait once more for the copies in flight
         ((volatile CgScalars*)S.sc)->wait_error = 1;
         ((volatile CgScalars*)S.sc)->done = 1;
-        bar_wait(bars, it & 1, kWaitLatticeNs);   // the halo's (its phase is over where another wait ran out)
+        bar_wait(bars, phase, kWaitLatticeNs);   // the halo's (its phase is over where another wait ran out)
         for (int k = max(0, s.issued - 2); k < s.issued; ++k)   // (lane 0's: the latest of each of its two slots)
             bar_wait(s.bars + 8 * (k & 1), (k >> 1) & 1, kWaitLatticeNs);
     }
