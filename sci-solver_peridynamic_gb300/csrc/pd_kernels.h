@@ -196,8 +196,8 @@ struct LatticeParams {
     float* image;             // per step, per brick: the deviations of its halo (x, y pairs, then z)
     CUtensorMap box_w;        // grid_w in boxes of a brick's halo
     double org[3];            // position of site (0, 0, 0)
-    double h;                 // lattice spacing
-    int ncol[kLatRmax + 1];   // the stencil's z columns (dx, dy) of each reach, the largest reach first in:
+    double h;                 // pitch of the sites (the lattice spacing in 21 bits)
+    int ncol[kLatRmax + 1];   // the stencil's z columns (dx, dy) of each reach, the smallest reach first in:
     int coff[kLatTab * kLatTab];                              // halo index offset
     float ccx[kLatTab * kLatTab], ccy[kLatTab * kLatTab];     // h dx, h dy
     float cz[kLatTab];        // h dz, dz = -kLatRmax .. kLatRmax
