@@ -102,7 +102,7 @@ __device__ __forceinline__ PersistRun persist_run(const PersistArgs& A)
                       A.start != 0, &A.S.sc->wait_error, A.wait_ns};
 }
 
-// Sums travel as their accumulator's own form: double-float for FP32 data.
+// Bits of the sums within a warp: double-float for FP32 data.
 __device__ __forceinline__ unsigned long long pack(DF v)
 {
     return ((unsigned long long)__float_as_uint(v.hi) << 32) | __float_as_uint(v.lo);
@@ -131,9 +131,79 @@ __device__ __forceinline__ void warp_sum(T& v, int step)
     for (int off = 16; off >= step; off >>= 1) add_to(v, shfl_xor(v, off));
 }
 
+// Beyond the warp, sums of FP32 data are integers times 2^(top - kTopOffset), `top`
+// the largest exponent among the terms of a sum: 53 bits of the largest term.
+// Double-float holds 48: with it throughout, <r, r> of 2,500 to 30,000 rows was
+// 1.2e-15 to 1.9e-15 off the sum of separate launches (FP64 from the warp on), root
+// mean square over bodies; with integers it is 0.8e-16 to 2.4e-16 off.  A warp adds
+// 32 such terms with 4 reductions (22 cycles for a maximum, 49 for a sum) where
+// double-float takes 5 steps of 60, and FP64 5 of 100 and 19 cycles of its pipe for
+// every warp; and the warps that poll form the sum once for the block.  With
+// double-float an iteration of 512 particles took 7.9 us instead of 7.3, of 16k 10.8
+// instead of 10.25, of 100k 23.9 instead of 23.3 (steps included).
+constexpr int kTopOffset = 256;
+constexpr int kTopSpecial = 511;   // not a finite number
+struct WideSum {                   // (hi 2^44 + mid 2^22 + lo) 2^(top - kTopOffset); mid, lo of 22 bits
+    int hi, mid, lo, top;
+};
+__device__ __forceinline__ float power_of_two(int k) { return __int_as_float((k + 127) << 23); }   // -126 .. 127
+__device__ __forceinline__ int top_of(DF v)
+{
+    const int field = (__float_as_int(v.hi) >> 23) & 255;   // hi is a 24-bit integer times 2^(field - 150)
+    return field == 255 ? kTopSpecial : max(field, 1) - 179 + kTopOffset;
+}
+// v 2^-(e) rounded to an integer (53 bits and the sign), e = top_of(v) - kTopOffset
+__device__ __forceinline__ long long mantissa_of(DF v)
+{
+    const int bits = __float_as_int(v.hi), field = (bits >> 23) & 255, e = max(field, 1) - 179, k = -e / 2;
+    const long long mant = (bits & 0x7fffff) | (field > 0 ? 0x800000 : 0);
+    const int lo = __float2int_rn(v.lo * power_of_two(k) * power_of_two(-e - k));   // (2^28 at most)
+    return ((bits < 0 ? -mant : mant) << 29) + lo;
+}
+// The sum over the warp of m 2^-(down), down >= 0, each term rounded to an integer
+// below 2^58; the carries are left in the sums of `mid` and `lo`.
+__device__ __forceinline__ WideSum warp_total(long long m, int down, int top)
+{
+    const int d = min(down, 63);
+    m = (m + (long long)((1ull << d) >> 1)) >> d;
+    return WideSum{__reduce_add_sync(0xffffffffu, (int)(m >> 44)),
+                   (int)__reduce_add_sync(0xffffffffu, (unsigned)(m >> 22) & 0x3fffffu),
+                   (int)__reduce_add_sync(0xffffffffu, (unsigned)m & 0x3fffffu), top};
+}
+__device__ __forceinline__ void carry(WideSum& s)
+{
+    s.mid += s.lo >> 22;
+    s.lo &= 0x3fffff;
+    s.hi += s.mid >> 22;
+    s.mid &= 0x3fffff;
+}
+__device__ __forceinline__ DF to_df(const WideSum& s)   // (carried)
+{
+    if (s.top == kTopSpecial) return DF{__int_as_float(0x7fffffff), 0.f};
+    const auto exact = [](int v) { return __int_as_float(0x4B000000 | v) - 8388608.f; };   // 22 bits
+    const float x = small_int_to_float(s.hi) * 17592186044416.f, y = exact(s.mid) * 4194304.f;   // 2^44, 2^22
+    const float t = __fadd_rn(x, y);
+    const float rest = __fadd_rn(__fsub_rn(y, __fsub_rn(t, x)), exact(s.lo));
+    const float hi = __fadd_rn(t, rest), lo = __fsub_rn(rest, __fsub_rn(hi, t));
+    const int e = s.top - kTopOffset, k = e / 2;
+    const float a = power_of_two(k), b = power_of_two(e - k);
+    return DF{hi * a * b, lo * a * b};
+}
+__device__ __forceinline__ double to_double(const WideSum& s)
+{
+    if (s.top == kTopSpecial) return __longlong_as_double(0x7ff8000000000000ll);
+    const double v = __fma_rn((double)(((long long)s.hi << 22) + s.mid), 4194304.0, (double)s.lo);
+    return v * __longlong_as_double((long long)(s.top - kTopOffset + 1023) << 52);
+}
+
 struct Exchange {
     unsigned long long warp[kPersistWarps];
-    unsigned long long from[kPersistMaxGrid];
+    unsigned long long from[kPersistMaxGrid];      // FP64: the blocks' sums
+    WideSum part[kPersistMaxGrid / 32];            // FP32 data: those of 32 blocks, carried
+    int top[kPersistMaxGrid / 32];
+    WideSum total;                                 // their sum, and as double-float
+    DF sum;
+    PersistRun run;
     int error;
 };
 
@@ -160,45 +230,106 @@ __device__ __forceinline__ bool await(const ulonglong2* rec, int* error, unsigne
     }
 }
 
-// The sum over all blocks of v (which only lanes at multiples of `step` hold);
-// every thread of the block calls it and gets the sum.  The warps that do not
-// poll the inbox run help(thread, threads) meanwhile.  Returns false when a
-// wait ran out of time.
-template <typename T, typename Help>
-__device__ __forceinline__ bool exchange_sum(Exchange& e, T& v, int step, const PersistRun& A, unsigned long long epoch,
-                                             Help help)
+// A block's own part goes into every block's inbox, and the part of block
+// threadIdx.x comes back (threads beyond the grid: nothing).  The low nine bits of a
+// record's second word belong to its value.
+__device__ __forceinline__ ulonglong2 round_trip(Exchange& e, const PersistRun& A, unsigned long long epoch,
+                                                 unsigned long long value, unsigned nine)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int grid = A.grid;
-    const int polling = (grid + 31) / 32 * 32;   // threads with an inbox record, in whole warps
+    ulonglong2 r = make_ulonglong2(0ull, 0ull);
+    const int b = threadIdx.x, grid = A.grid;
+    if (b < grid) {
+        ulonglong2* box = A.inbox + (size_t)(epoch & 1) * grid * grid;
+        publish(box + (size_t)b * grid + A.block, value, (epoch << 9) | nine);
+        await(box + (size_t)A.block * grid + b, A.error, A.wait_ns, e, r,
+              [epoch](const ulonglong2& x) { return x.y >> 9 == epoch; });
+    }
+    return r;
+}
+__device__ __forceinline__ int polling_threads(int grid) { return (grid + 31) / 32 * 32; }   // whole warps
+
+// The exchange of the warps that poll: from the warps' sums to e.total and e.sum.
+// (A call: inlined, it takes registers from the loops around it, 11.6 us at 16k.)
+__device__ __noinline__ void exchange_wide(Exchange& e, unsigned long long epoch)
+{
+    const PersistRun& A = e.run;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, polling = polling_threads(A.grid);
+    const DF w = lane < kPersistWarps ? unpack<DF>(e.warp[lane]) : DF{0.f, 0.f};
+    const int own = top_of(w), block_top = __reduce_max_sync(0xffffffffu, own);
+    const WideSum t = warp_total(mantissa_of(w), block_top - own, block_top);
+    const ulonglong2 r = round_trip(
+        e, A, epoch, (unsigned long long)(((long long)t.hi << 44) + ((long long)t.mid << 22) + t.lo), (unsigned)block_top);
+    const int its = (int)(r.y & 511u), warp_top = __reduce_max_sync(0xffffffffu, its);
+    if (lane == 0) e.top[warp] = warp_top;
+    asm volatile("bar.sync 1, %0;" ::"r"(polling) : "memory");   // the warps that poll
+    int top = e.top[0];
+    for (int k = 1; k < polling / 32; ++k) top = max(top, e.top[k]);
+    WideSum s = warp_total((long long)r.x, top - its, top);
+    carry(s);
+    if (lane == 0) e.part[warp] = s;
+    asm volatile("bar.sync 1, %0;" ::"r"(polling) : "memory");
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < polling / 32; ++k) {
+            const WideSum p = e.part[k];
+            s.hi += p.hi;
+            s.mid += p.mid;
+            s.lo += p.lo;
+        }
+        carry(s);
+        e.total = s;
+        e.sum = to_df(s);
+    }
+}
+
+// The sum over all blocks of v (which only lanes at multiples of `step` hold) in
+// `total` (FP32 data: in 48 bits, and e.total in 53); every thread of the block
+// calls it and gets the sum.  The warps that do not poll the inbox run help(thread,
+// threads) meanwhile.  Returns false when a wait ran out of time.
+template <typename Help>
+__device__ __forceinline__ bool exchange_sum(Exchange& e, DF v, DF& total, int step, const PersistRun& A,
+                                             unsigned long long epoch, Help help)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, polling = polling_threads(A.grid);
     warp_sum(v, step);
     if (lane == 0) e.warp[warp] = pack(v);
     __syncthreads();
     if ((int)threadIdx.x < polling) {
-        T t = unpack<T>(e.warp[lane & (kPersistWarps - 1)]);   // both halves of the warp form the same sum
-#pragma unroll
-        for (int off = kPersistWarps / 2; off > 0; off >>= 1) add_to(t, shfl_xor(t, off));
-        const int b = threadIdx.x;
-        if (b < grid) {
-            ulonglong2* box = A.inbox + (size_t)(epoch & 1) * grid * grid;
-            publish(box + (size_t)b * grid + A.block, pack(t), epoch);
-            ulonglong2 r;
-            await(box + (size_t)A.block * grid + b, A.error, A.wait_ns, e, r, [epoch](const ulonglong2& x) { return x.y == epoch; });
-            e.from[b] = r.x;
-        }
+        exchange_wide(e, epoch);
     } else {
         help((int)threadIdx.x - polling, kPersistThreads - polling);
     }
     __syncthreads();
-    v = T();
-    for (int b = lane; b < grid; b += 32) add_to(v, unpack<T>(e.from[b]));
-    warp_sum(v, 1);
+    total = e.sum;
+    return e.error == 0;
+}
+template <typename Help>
+__device__ __forceinline__ bool exchange_sum(Exchange& e, double v, double& total, int step, const PersistRun& A,
+                                             unsigned long long epoch, Help help)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, polling = polling_threads(A.grid);
+    warp_sum(v, step);
+    if (lane == 0) e.warp[warp] = pack(v);
+    __syncthreads();
+    if ((int)threadIdx.x < polling) {
+        double t = unpack<double>(e.warp[lane & (kPersistWarps - 1)]);   // both halves of the warp form the same sum
+#pragma unroll
+        for (int off = kPersistWarps / 2; off > 0; off >>= 1) add_to(t, shfl_xor(t, off));
+        const ulonglong2 r = round_trip(e, A, epoch, pack(t), 0u);
+        if ((int)threadIdx.x < A.grid) e.from[threadIdx.x] = r.x;
+    } else {
+        help((int)threadIdx.x - polling, kPersistThreads - polling);
+    }
+    __syncthreads();
+    total = 0.0;
+    for (int b = lane; b < A.grid; b += 32) add_to(total, unpack<double>(e.from[b]));
+    warp_sum(total, 1);
     return e.error == 0;
 }
 
-// The quotient a / b rounded to FP32 (a, b in double-float): the FP32 quotient
-// and one correction by its remainder, as accurate as the rounded FP64
-// quotient to 2^-40, at a fifth of an FP64 division's latency (573 cycles).
+// The quotient a / b rounded to FP32 (a, b in double-float): the FP32 quotient and
+// one correction by its remainder, at a fifth of an FP64 division's latency (573
+// cycles).  Of 10^8 pairs, on the CPU, 11 differ from the rounded FP64 quotient, all
+// within 0.0002 units of a tie: at most 0.5002 units off where that is 0.5.
 // Sums whose FP32 words leave the range of the steps take the FP64 division.
 __device__ __forceinline__ float df_quotient(DF a, DF b)
 {
@@ -374,7 +505,10 @@ __device__ __forceinline__ bool persist_solve32(const StepParams& P, const Devic
         sw[h] = A.start ? sh[h] : ((const float4*)S.p)[q];
         if (!CACHED) shx[h] = S.xs4[q];
     }
-    if (threadIdx.x == 0) ex.error = 0;
+    if (threadIdx.x == 0) {
+        ex.error = 0;
+        ex.run = A;
+    }
     const float sup = (float)P.sup, per_edge = (float)(1 << kFixedBits) / sup;
     bool fixed = false;
     if (!CACHED) {   // the entries that this thread has staged
@@ -402,19 +536,17 @@ __device__ __forceinline__ bool persist_solve32(const StepParams& P, const Devic
     const float tol2_far = (float)(tol * tol * 1.0001);   // a sum of squares above it is above tol^2
     const int max_iter = sc->max_iter;
     const double rz0 = sc->rz;
-    DF rz{(float)rz0, (float)(rz0 - (double)(float)rz0)};
+    DF rz{(float)rz0, (float)(rz0 - (double)(float)rz0)}, pAp{0.f, 0.f};   // for the quotients (48 bits)
     float alpha = 0.f, beta = A.start ? 0.f : (float)sc->beta;
     int iter = sc->iter;
     bool done = false, converged = false;
     if (A.start) {
-        rz = first.v;
-        if (!exchange_sum(ex, rz, 1, A, ++epoch, [](int, int) {})) return false;
-        converged = below_tolerance(df_to_double(rz), tol);
+        if (!exchange_sum(ex, first.v, rz, 1, A, ++epoch, [](int, int) {})) return false;
+        converged = below_tolerance(to_double(ex.total), tol);
         done = converged || iter >= max_iter;
     }
 
     unsigned long long t_mark = 0, ns_spmv = 0, ns_vec = 0;
-    DF pAp{0.f, 0.f};
     for (int it = 0; it < A.max_iters && !done; ++it) {
         if (timed) t_mark = now_ns();
         // ---- p = r + beta p of the halo and the own rows; y = A p
@@ -509,8 +641,7 @@ __device__ __forceinline__ bool persist_solve32(const StepParams& P, const Devic
         if constexpr (CACHED) all_rows(std::false_type());
         else if (fixed) all_rows(std::true_type());
         else all_rows(std::false_type());
-        pAp = acc.v;
-        if (!exchange_sum(ex, pAp, G, A, ++epoch, [](int, int) {})) return false;
+        if (!exchange_sum(ex, acc.v, pAp, G, A, ++epoch, [](int, int) {})) return false;
         alpha = df_quotient(rz, pAp);
         if (timed) {
             const unsigned long long t = now_ns();
@@ -535,7 +666,6 @@ __device__ __forceinline__ bool persist_solve32(const StepParams& P, const Devic
                 rr.fma(rv.z, rv.z);
             }
         }
-        DF total = rr.v;
         const auto gather = [&](int t, int threads) {   // the halo's new r
             for (int h = t; h < nh; h += threads) {
                 ulonglong2 v;
@@ -545,11 +675,12 @@ __device__ __forceinline__ bool persist_solve32(const StepParams& P, const Devic
                 sh[h] = make_float4(yx.lo, yx.hi, __uint_as_float((unsigned)v.y), 0.f);
             }
         };
-        if (!exchange_sum(ex, total, G, A, epoch, gather)) return false;
+        DF total;
+        if (!exchange_sum(ex, rr.v, total, G, A, epoch, gather)) return false;
         beta = df_quotient(total, rz);
         rz = total;
         ++iter;
-        if (!(total.hi > tol2_far)) converged = below_tolerance(df_to_double(total), tol);
+        if (!(total.hi > tol2_far)) converged = below_tolerance(to_double(ex.total), tol);
         done = converged || iter >= max_iter;
         if (timed) ns_vec += now_ns() - t_mark;
     }
@@ -560,7 +691,7 @@ __device__ __forceinline__ bool persist_solve32(const StepParams& P, const Devic
     }
     if (A.block == 0 && threadIdx.x == 0) {
         sc->pAp = df_to_double(pAp);
-        sc->rz = df_to_double(rz);
+        sc->rz = to_double(ex.total);
         sc->alpha = alpha;
         sc->beta = beta;
         sc->rnorm = sqrt(sc->rz);
@@ -802,7 +933,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist64(PersistArgs
     unsigned long long epoch = A.epoch;
     if (A.start) {
         __syncthreads();   // (s_rz and s_done before thread 0 sets them again)
-        if (!exchange_sum(ex, first, 1, run, ++epoch, [](int, int) {})) return;
+        if (!exchange_sum(ex, first, first, 1, run, ++epoch, [](int, int) {})) return;
         if (threadIdx.x == 0) {
             s_rz = first;
             s_converged = below_tolerance(first, tol);
@@ -862,8 +993,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist64(PersistArgs
                 acc = fma(wk, y, acc);
             }
         }
-        pAp = acc;
-        if (!exchange_sum(ex, pAp, 1, run, ++epoch, [](int, int) {})) return;
+        if (!exchange_sum(ex, acc, pAp, 1, run, ++epoch, [](int, int) {})) return;
         if (threadIdx.x == 0) s_alpha = s_rz / pAp;
         __syncthreads();
         if (timed) {
@@ -900,7 +1030,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist64(PersistArgs
                 sh[h] = Vec3d{unpack<double>(a.x), unpack<double>((b.y << 32) | (a.y & 0xffffffffull)), unpack<double>(b.x)};
             }
         };
-        if (!exchange_sum(ex, rr, 1, run, epoch, gather)) return;
+        if (!exchange_sum(ex, rr, rr, 1, run, epoch, gather)) return;
         ++iter;
         if (threadIdx.x == 0) {
             s_beta = rr / s_rz;
