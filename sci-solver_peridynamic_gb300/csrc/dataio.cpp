@@ -461,9 +461,11 @@ pd_status Engine::dataio_load_state(size_t timestep)
     predicted_iters_ = 0;
     hist_reset();   // the projection history belongs to the state that was replaced
     retries_ = 0;
-    // derived device data: FP32 positions, tile local indices
+    // derived device data: FP32 positions (rest positions too: the slot order may be
+    // another one), tile local indices
     const StepParams P = step_params();
     if (!fp64_ && n_ > 0) {
+        make_local32(S_.X64, origin_[0], origin_[1], origin_[2], S_.X32, nullptr, n_, stream_);
         launch_refresh(fp64_, P, S_, L_, stream_);
         launch_stretch_limits(S_, (int)std::min<long long>(((long long)n_ + kBlock - 1) / kBlock, 4096), stream_);
         launches_ += 2;

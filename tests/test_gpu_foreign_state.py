@@ -6,7 +6,7 @@ bond offsets.)"""
 import numpy as np
 import pytest
 
-from helpers import rel_err, same_sets
+from helpers import apply_on_device, rel_err, same_sets
 
 pytestmark = pytest.mark.gpu
 H = 0.02
@@ -91,3 +91,26 @@ def test_bond_offsets_off_the_stencil(pdgb, scenes, apart, tmp_path):
     same.dataIO_loadState(1)
     assert same.params()[2].spmv_path == 3      # (its own state keeps the stencil)
     _goes_on(pdgb, scenes, own, other, 2)
+
+
+def test_contact_rows_in_another_slot_order(pdgb, scenes, tmp_path):
+    """A state saved in the bricks' slot order, taken by a handle with the builder's:
+    the rest positions that the contact term of a row reads follow it."""
+    sc = scenes.impact_body(9000, "ball", coeff=5.0, speed=5.0, seed=2)   # (the sphere touches it)
+    sc.run.saving_path = str(tmp_path).encode()
+    x = np.zeros((sc.n, 4))
+    x[:, :3] = np.random.default_rng(2).standard_normal((sc.n, 3))
+    y = {}
+    for path in (3, 2):
+        sc.opt.spmv_path = path
+        s = scenes.make_simulator(sc)
+        s.makeReady()
+        if path == 3:
+            s.advance(2)
+            s.dataIO_saveState(2)
+        else:
+            s.dataIO_loadState(2)
+        s.advance(1)
+        y[path] = apply_on_device(pdgb, s, x)[0]
+    # (sums of at most 122 terms in 32 bits: each within 132 * 2^-24 of the largest value)
+    assert np.abs(y[2] - y[3]).max() <= 2e-5 * np.abs(y[3]).max()
