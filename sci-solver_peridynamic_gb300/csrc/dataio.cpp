@@ -471,7 +471,7 @@ pd_status Engine::dataio_load_state(size_t timestep)
         launches_ += 2;
     }
     if (S_.lidx && S_.n_tiles > 0) {
-        const pd_status hs = build_halos();
+        const pd_status hs = build_halos(!same_order);
         if (hs != PD_OK) return hs;
     }
     int on_stencil = 1;
@@ -925,7 +925,7 @@ pd_status Engine::dataio_load_state_reference(size_t timestep)
     // the rows now hold the file's order: the tuned SpMV shape's slot order is
     // laid out again from the build order
     lay_g_ = lay_u_ = 1;
-    if (!L_.lattice && !L_.tiled) relayout_bonds(L_.lanes, L_.unroll);
+    if (!L_.lattice && !L_.tiled && tiles_.grid == 0) relayout_bonds(L_.lanes, L_.unroll);
     const StepParams P = step_params();
     if (!fp64_ && n_ > 0) {
         launch_refresh(fp64_, P, S_, L_, stream_);
@@ -933,7 +933,7 @@ pd_status Engine::dataio_load_state_reference(size_t timestep)
         launches_ += 2;
     }
     if (S_.lidx && S_.n_tiles > 0) {
-        const pd_status hs = build_halos();
+        const pd_status hs = build_halos(true);
         if (hs != PD_OK) return hs;
     }
     lattice_resync(true);

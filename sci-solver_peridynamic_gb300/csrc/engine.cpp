@@ -329,7 +329,7 @@ pd_status Engine::make_ready()
         if (n > 0 && opt_.spmv_path == 1) {
             CK(dalloc(&S_.lidx, slots), "alloc local indices");
             S_.tile_rows = kTileRows;
-            s = build_halos();
+            s = build_halos(false);
             if (s != PD_OK) return s;
             launches_ += 2;
         }
@@ -657,8 +657,10 @@ void Engine::gang_tiles_free()
 // whose blocks' halos no longer fit (a checkpoint in another slot order) leaves
 // the one-launch solve, and so does one with more bond slots in a block than its
 // plan keeps in shared memory, or with rows that do not start on whole groups
-// of slots (both: a state of another body).
-pd_status Engine::build_halos()
+// of slots (both: a state of another body).  reorder: a row's live bonds come in
+// another order than that of the products by tiles (launch_bank_order), and are put
+// into it (97k particles of 76 bonds: 24.7 us per product without, 20.6 with).
+pd_status Engine::build_halos(bool reorder)
 {
     int max_halo = 0, unfit = 0;
     CK(build_tiles(S_, n_, &max_halo, &unfit, stream_), "build tiles");
@@ -675,6 +677,11 @@ pd_status Engine::build_halos()
     if (persist_.grid > 0 && (unfit > 0 || max_halo > persist_.halo || !rows_fit)) persist_ = CgPersistPlan{};
     if (persist_.grid == 0 && tiles_.grid > 0 && (unfit > 0 || !rows_fit || !tile_product_plan(max_halo, device_, &tiles_)))
         tiles_ = CgPersistPlan{};
+    if (reorder && tiles_.grid > 0) {
+        CK(launch_bank_order(S_, n_, total_slots_, nullptr, stream_), "order bonds");
+        launch_bond_geometry(S_, stream_);   // (1/d0 and d0^2 of the bonds where they stand now)
+        launches_ += 2;
+    }
     return PD_OK;
 }
 

@@ -78,7 +78,7 @@ private:
     pd_status tile_prepare();
     pd_status gang_tiles(int rows, int blocks, CgPersistPlan* plan, bool* fits);
     void gang_tiles_free();
-    pd_status build_halos();
+    pd_status build_halos(bool reorder);
     pd_status wait_check();
     void lattice_resync(bool force);   // the lattice product's 1/d0 table from the live CSR bonds
     // mixed mode: reorders every row's live bonds for the (g, u) SpMV shape
