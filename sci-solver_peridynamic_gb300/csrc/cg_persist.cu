@@ -764,8 +764,11 @@ __global__ void __launch_bounds__(kTileBlock, 1)
     for (int h = threadIdx.x; h < nh; h += kTileBlock) {
         const int q = __ldg(S.halo + h0 + h);
         const float4 X = __ldg(S.xs4 + q);
-        sw[h] = __ldg(in + q);
-        far |= farther(X, ref, sup);
+        const float4 w = __ldg(in + q);
+        sw[h] = w;
+        // (the fixed-point form takes 0 times w for a slot without a live bond, so a
+        // block that reads a w that is not finite keeps to the other, which skips it)
+        far |= farther(X, ref, sup) || !(fabsf(w.x) + fabsf(w.y) + fabsf(w.z) < INFINITY);
         shx[h] = fixed_position(X, per_edge);
     }
     const bool fixed = !__syncthreads_or(far);
@@ -788,10 +791,7 @@ __global__ void __launch_bounds__(kTileBlock, 1)
                 float ic[4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    // (a slot without a live bond takes the partner of the lane's first
-                    // one, which has one: 0 times the w of a broken bond's partner, which
-                    // a caller may have left NaN, is NaN.  1.1 % of 36 us at 200k particles)
-                    lc[u] = FIXED && j0 + u >= cn ? l[0] : l[u];
+                    lc[u] = l[u];
                     ic[u] = id0[u];
                 }
                 if (j0 + R * 4 < cn) load_bonds(S, rs + j0 + R * 4, l, id0);   // in flight while this step's bonds are added

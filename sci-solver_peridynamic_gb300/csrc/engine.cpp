@@ -659,7 +659,7 @@ void Engine::gang_tiles_free()
 // plan keeps in shared memory, or with rows that do not start on whole groups
 // of slots (both: a state of another body).  reorder: a row's live bonds come in
 // another order than that of the products by tiles (launch_bank_order), and are put
-// into it (97k particles of 76 bonds: 24.7 us per product without, 20.6 with).
+// into it (97k particles of 76 bonds: 24.7 us per product without, 20.0 with).
 pd_status Engine::build_halos(bool reorder)
 {
     int max_halo = 0, unfit = 0;

@@ -1,8 +1,8 @@
 """A state loaded in another bond order (csrc/tiles.cu, k_bank_order) is put into the
 products' own, which halves their shared-memory conflicts, and the run goes on as the
 saver's does.  Without it the body here takes 24.7 us per product after a load in the
-reference's layout and 28.8 after one in the bricks' slot order, with it 20.6 and
-22.7 (bricks make longer halos), 20.6 before.  The bounds stand between."""
+reference's layout and 28.8 after one in the bricks' slot order, with it 20.0 and
+22.7 (bricks make longer halos), 20.0 before.  The bounds stand between."""
 import numpy as np
 import pytest
 
