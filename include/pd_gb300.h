@@ -258,6 +258,16 @@ typedef struct pd_kernel_times {
     double total_ms[PD_KC_COUNT];
 } pd_kernel_times;
 
+/* How a handle's solves and products run, as make_ready chose (pd_get_routes). */
+typedef struct pd_routes {
+    int one_launch_blocks;         /* blocks of the one-launch solve, 0: not used */
+    int one_launch_bonds;          /* bond slots that one of them keeps in shared memory, 0: none */
+    int tile_blocks;               /* blocks of the product by large tiles, 0: not used */
+    int lattice;                   /* 1: products by the lattice stencil */
+    long long one_launch_solves;   /* solves in one launch so far (cg_graph_solves
+                                      counts them too, where cg_loop is 0) */
+} pd_routes;
+
 /* Device-side view of a handle's current linear system A = M + beta h^2 K
  * (beta = 1 implicit Euler, 1/4 Newmark), for applying the matrix-free
  * operator outside pd_advance: the role of the reference's
@@ -429,6 +439,12 @@ pd_status pd_synchronize(pd_handle* h);
  * With 0 every wait counts as run out at once: a caller's test of its own error
  * path. */
 pd_status pd_set_wait_limit(pd_handle* h, double seconds);
+/* The routes in use (after pd_make_ready). */
+pd_status pd_get_routes(pd_handle* h, pd_routes* routes);
+/* 0: small bodies of this handle take the CUDA graph (or, with cg_loop 1, the
+ * host-checked batches) of separate launches like larger ones; 1 (default): the
+ * one-launch solve.  Takes effect at the next pd_make_ready. */
+pd_status pd_set_one_launch(pd_handle* h, int enabled);
 
 /* ---- DataIO (src/core/dataIO.h:20-44) -------------------------------------
  * Output under run->saving_path, as the reference's DataIO: frames
@@ -593,6 +609,9 @@ pd_status pd_batch_synchronize(pd_batch* b);
  * use_graph it takes effect at the next pd_batch_make_ready.  pd_batch_advance
  * returns PD_ERR_CUDA, and the batch takes no further step until then. */
 pd_status pd_batch_set_wait_limit(pd_batch* b, double seconds);
+/* The gangs of blocks that solve the scenes one after another (after
+ * pd_batch_make_ready); *gangs = 0: the phases of all scenes between grid barriers. */
+pd_status pd_batch_get_gangs(pd_batch* b, int* gangs, int* blocks_per_gang);
 /* Last error text of a batch. */
 const char* pd_batch_last_error_message(pd_batch* b);
 

@@ -114,6 +114,12 @@ class StepStats(C.Structure):
         return {k: getattr(self, k) for k, _ in self._fields_}
 
 
+class Routes(C.Structure):
+    """pd_routes: how a handle's solves and products run."""
+    _fields_ = [("one_launch_blocks", C.c_int), ("one_launch_bonds", C.c_int), ("tile_blocks", C.c_int),
+                ("lattice", C.c_int), ("one_launch_solves", C.c_longlong)]
+
+
 class OperatorView(C.Structure):
     """pd_operator_view: device-side view of the current system operator."""
     _fields_ = [
@@ -240,6 +246,9 @@ def library(build_if_missing: bool = True):
         "pd_batch_synchronize": (st, [vp]),
         "pd_batch_set_wait_limit": (st, [vp, C.c_double]),
         "pd_set_wait_limit": (st, [vp, C.c_double]),
+        "pd_get_routes": (st, [vp, P(Routes)]),
+        "pd_set_one_launch": (st, [vp, C.c_int]),
+        "pd_batch_get_gangs": (st, [vp, P(C.c_int), P(C.c_int)]),
         "pd_batch_last_error_message": (C.c_char_p, [vp]),
     }
     for name, (res, args) in sig.items():
@@ -559,6 +568,15 @@ class Simulator:
     def synchronize(self):
         _check(self.lib.pd_synchronize(self.h), self.h)
 
+    def routes(self) -> Routes:
+        r = Routes()
+        _check(self.lib.pd_get_routes(self.h, C.byref(r)), self.h)
+        return r
+
+    def set_one_launch(self, on: bool):
+        """False, before makeReady: separate launches for small bodies too."""
+        _check(self.lib.pd_set_one_launch(self.h, 1 if on else 0), self.h)
+
     def set_wait_limit(self, seconds: float):
         """Limit of the kernels' waits (negative: the defaults; 0: every wait
         counts as run out, for tests of the error path)."""
@@ -717,6 +735,12 @@ class Batch:
 
     def synchronize(self):
         _bcheck(self.lib.pd_batch_synchronize(self.h), self.h)
+
+    def gangs(self) -> tuple[int, int]:
+        """(gangs, blocks of each); (0, 0): the phases between grid barriers."""
+        g, n = C.c_int(), C.c_int()
+        _bcheck(self.lib.pd_batch_get_gangs(self.h, C.byref(g), C.byref(n)), self.h)
+        return g.value, n.value
 
     def set_wait_limit(self, seconds: float):
         """As Simulator.set_wait_limit; with a graph, before makeReady."""

@@ -44,6 +44,7 @@ public:
     cudaStream_t stream() const { return stream_; }
     pd_status synchronize();
     void set_wait_limit(unsigned long long ns) { wait_ns_ = ns; }
+    void gangs(int* count, int* blocks) const { *count = gangs_; *blocks = gangs_ > 0 ? gang_ : 0; }
     bool ready() const { return ready_; }
     const std::string& error() const { return err_; }
     void set_error(const std::string& e) { err_ = e; }
@@ -930,6 +931,13 @@ pd_status pd_batch_set_wait_limit(pd_batch* b, double seconds)
 {
     if (!b || !b->b || !(seconds <= 3600.0)) return PD_ERR_INVALID_ARGUMENT;
     b->b->set_wait_limit(seconds < 0 ? pdgb::kWaitSolveNs : (unsigned long long)(seconds * 1e9));
+    return PD_OK;
+}
+
+pd_status pd_batch_get_gangs(pd_batch* b, int* gangs, int* blocks_per_gang)
+{
+    if (!b || !b->b || !gangs || !blocks_per_gang) return PD_ERR_INVALID_ARGUMENT;
+    b->b->gangs(gangs, blocks_per_gang);
     return PD_OK;
 }
 

@@ -282,6 +282,20 @@ pd_status pd_set_wait_limit(pd_handle* h, double seconds)
     return PD_OK;
 }
 
+pd_status pd_get_routes(pd_handle* h, pd_routes* routes)
+{
+    ENG(h);
+    if (!routes) return PD_ERR_INVALID_ARGUMENT;
+    return h->eng->routes(routes);
+}
+
+pd_status pd_set_one_launch(pd_handle* h, int enabled)
+{
+    ENG(h);
+    h->eng->set_one_launch(enabled != 0);
+    return PD_OK;
+}
+
 pd_status pd_synchronize(pd_handle* h)
 {
     ENG(h);

@@ -559,7 +559,7 @@ void Engine::apply_op(const StepParams& P, const void* in, void* out, ReduceSlot
 // cooperative launch (cg_persist.cu).
 pd_status Engine::persist_prepare()
 {
-    if (n_ <= 0 || batch_member_ || opt_.preconditioner) return PD_OK;
+    if (n_ <= 0 || batch_member_ || opt_.preconditioner || !one_launch_) return PD_OK;
     CgPersistPlan plan = cg_persist_rows(fp64_, n_, sm_count_, device_);
     if (plan.grid == 0) return PD_OK;
     int max_halo = 0, unfit = 0;
@@ -970,6 +970,13 @@ pd_status Engine::wait_check()
     return PD_ERR_CUDA;
 }
 
+pd_status Engine::routes(pd_routes* r) const
+{
+    if (!ready_) return PD_ERR_NOT_READY;
+    *r = pd_routes{persist_.grid, persist_.grid > 0 ? persist_.bonds : 0, tiles_.grid, L_.lattice ? 1 : 0, one_launch_solves_};
+    return PD_OK;
+}
+
 void Engine::set_wait_limit(unsigned long long solve_ns, unsigned long long lattice_ns)
 {
     wait_solve_ns_ = solve_ns;
@@ -1358,6 +1365,7 @@ pd_status Engine::cg_persist_loop(const StepParams& P, bool start)
         batch = (int)std::max<long long>(check, run / 8);
     }
     if (whole) ++cg_graph_solves_;
+    ++one_launch_solves_;
     if (profiling_ && h_sc_->iter > 0) {   // one sample per solve: the mean over its iterations
         const double ms = 1e-6 / h_sc_->iter;
         kc_sample_ms_[PD_KC_SPMV] += ns_spmv * ms;

@@ -41,6 +41,8 @@ public:
     long long launches() const { return launches_; }
     cudaStream_t stream() const { return stream_; }
     pd_status synchronize();
+    pd_status routes(pd_routes* r) const;
+    void set_one_launch(bool on) { one_launch_ = on; }
     // ns; 0: every wait counts as run out
     void set_wait_limit(unsigned long long solve_ns, unsigned long long lattice_ns);
     pd_status operator_view(pd_operator_view* v) const;
@@ -211,6 +213,8 @@ private:
     ulonglong2* d_inbox_ = nullptr;    // its records: partial sums (2 grid^2), then r
     CgPersistPlan tiles_{};            // products by tiles (grid 0: not used)
     unsigned long long persist_epoch_ = 0;
+    bool one_launch_ = true;           // small bodies may take it
+    long long one_launch_solves_ = 0;
     unsigned long long wait_solve_ns_ = kWaitSolveNs, wait_lattice_ns_ = kWaitLatticeNs;
     bool wait_unread_ = false;         // a product by apply_operator whose waits no read-back has told of yet
     bool solve_updates_ = false;       // the one-launch solve of this step advances the rows itself
