@@ -21,7 +21,7 @@
 // The per-bond arithmetic is the gather product's (step_rows.cuh,
 // mixed_bond_chunk): the Jacobian applied to w_p - w_q is
 //   c [ (1/d0 - 1/d) (w_p - w_q) + (xi . (w_p - w_q)) xi / d^3 ],
-// with the bond vector xi = h v_k + (d_q - d_p) from the stencil offset v_k
+// with the bond vector xi = d_q - (d_p - h v_k) from the stencil offset v_k
 // and the two deviations d from the lattice sites (per step, FP64 rounded
 // once to FP32 within half a supercell), in pairs of FP32 lanes (f32x2).
 #include <algorithm>
@@ -497,7 +497,8 @@ __device__ __forceinline__ void lat_issue(LatStream& s, const LatticeParams& lp,
 
 // The stencil's columns of reach RC, the first one c, slab by slab; after a slab
 // the one two further on is asked for, of the next chunk at the end.  Once a wait
-// has run out a lane waits no more (but looks) and asks for nothing (ok).
+// has run out (ok) a lane asks for nothing more; the waits that it still makes until
+// the block's vote, one per slab, are bounded like the first.
 template <int R, int RC>
 __device__ __forceinline__ void lat_columns(const LatticeParams& lp, const LatHalo& halo, int base, const float2* ring,
                                             LatStream& s, int chunk, int next, int& slab, int& c, int count,
@@ -507,7 +508,7 @@ __device__ __forceinline__ void lat_columns(const LatticeParams& lp, const LatHa
     const int lane = threadIdx.x & 31;
     for (; count > 0; count -= M) {
         const int slot = s.used & 1;
-        if (!bar_wait(s.bars + 8 * slot, (s.used >> 1) & 1, ok ? lp.wait_ns : 0ull)) ok = false;
+        ok &= bar_wait(s.bars + 8 * slot, (s.used >> 1) & 1, lp.wait_ns);
         ++s.used;
         const float2* e2 = ring + slot * (kLatSlabBytes / (int)sizeof(float2)) + lane;
 #pragma unroll 1
@@ -573,7 +574,8 @@ __global__ void __maxnreg__(R <= 2 ? 112 : 128)
         for (int k = 0; k < 1 + 2 * lat_warps(R); ++k) bar_init(bars + 8 * k, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         b = (int)atomicAdd(&lp.sched[0], 1u);
-        if (((volatile CgScalars*)S.sc)->wait_error) b = lp.n_bricks;   // (no bricks once a wait of the handle has run out)
+        // (no bricks once a wait of the handle has run out; in a solve `done` says so)
+        if (!(DOT && cg) && ((volatile CgScalars*)S.sc)->wait_error) b = lp.n_bricks;
         s_ahead = b;
     }
     __syncthreads();
@@ -600,10 +602,10 @@ __global__ void __maxnreg__(R <= 2 ? 112 : 128)
     float cz[kLatTab];
 #pragma unroll
     for (int k = 0; k < kLatTab; ++k) cz[k] = lp.cz[k];
-    uint32_t phase = 0;   // of the halo's barrier
+    int it = 0;   // bricks taken
     ok = lp.wait_ns != 0 || b >= lp.n_bricks;
     while (ok && b < lp.n_bricks) {
-        ok = bar_wait(bars, phase, lp.wait_ns);
+        ok = bar_wait(bars, it & 1, lp.wait_ns);
         const int ahead = *(volatile int*)&s_ahead;   // the next brick
         const int next = chunk_of(ahead);
         if (chunk >= 0) {
@@ -654,7 +656,7 @@ __global__ void __maxnreg__(R <= 2 ? 112 : 128)
         }
         b = ahead;
         chunk = next;
-        phase ^= 1u;
+        ++it;
         if (threadIdx.x == 0 && b < lp.n_bricks) {
             s_ahead = (int)atomicAdd(&lp.sched[0], 1u);
             load_halo(b);
@@ -663,7 +665,7 @@ __global__ void __maxnreg__(R <= 2 ? 112 : 128)
     if (!ok) {   // record it, end the solve, and wait once more for the copies in flight
         ((volatile CgScalars*)S.sc)->wait_error = 1;
         ((volatile CgScalars*)S.sc)->done = 1;
-        bar_wait(bars, phase, kWaitLatticeNs);   // the halo's (its phase is over where another wait ran out)
+        bar_wait(bars, it & 1, kWaitLatticeNs);   // the halo's (its phase is over where another wait ran out)
         for (int k = max(0, s.issued - 2); k < s.issued; ++k)   // (lane 0's: the latest of each of its two slots)
             bar_wait(s.bars + 8 * (k & 1), (k >> 1) & 1, kWaitLatticeNs);
     }
@@ -925,7 +927,9 @@ cudaError_t lattice_build(int n, double spacing, dbl4* x64, float4* X32, int* pe
     const long long M[3] = {NB[0] * BX + 2 * R, NB[1] * kLatBY + 2 * R, NB[2] * kLatBZ + 2 * R};
     const long long map_size = M[0] * M[1] * M[2];
     const long long bricks_total = NB[0] * NB[1] * NB[2];
-    // a dense site map of modest size (the body fills a good part of its box)
+    // dense grids of modest size: 32 bytes per site (grid_w, grid_d), so 512 per
+    // particle at most, where a particle of 80 bonds has some 2,000 elsewhere, and
+    // 134 MB for a body of few particles asked for by spmv_path 3
     if (map_size > std::max<long long>(16LL * n, 1LL << 22) || map_size >= (1LL << 31) ||
         bricks_total * BX * kLatBY * kLatBZ >= (1LL << 32))
         return cudaSuccess;
