@@ -247,6 +247,11 @@ __device__ __forceinline__ ulonglong2 round_trip(Exchange& e, const PersistRun& 
     return r;
 }
 __device__ __forceinline__ int polling_threads(int grid) { return (grid + 31) / 32 * 32; }   // whole warps
+__device__ __forceinline__ void polling_barrier(int threads)
+{
+    __syncwarp();
+    asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+}
 
 // The exchange of the warps that poll: from the warps' sums to e.total and e.sum.
 // (A call: inlined, it takes registers from the loops around it, 11.6 us at 16k.)
@@ -261,13 +266,13 @@ __device__ __noinline__ void exchange_wide(Exchange& e, unsigned long long epoch
         e, A, epoch, (unsigned long long)(((long long)t.hi << 44) + ((long long)t.mid << 22) + t.lo), (unsigned)block_top);
     const int its = (int)(r.y & 511u), warp_top = __reduce_max_sync(0xffffffffu, its);
     if (lane == 0) e.top[warp] = warp_top;
-    asm volatile("bar.sync 1, %0;" ::"r"(polling) : "memory");   // the warps that poll
+    polling_barrier(polling);
     int top = e.top[0];
     for (int k = 1; k < polling / 32; ++k) top = max(top, e.top[k]);
     WideSum s = warp_total((long long)r.x, top - its, top);
     carry(s);
     if (lane == 0) e.part[warp] = s;
-    asm volatile("bar.sync 1, %0;" ::"r"(polling) : "memory");
+    polling_barrier(polling);
     if (threadIdx.x == 0) {
         for (int k = 1; k < polling / 32; ++k) {
             const WideSum p = e.part[k];
@@ -375,10 +380,13 @@ __device__ __forceinline__ BondGeometry bond_geometry(const float4& Xq, const fl
 // A halo position as 32-bit fixed point, supercell edge = 2^25, wrapping: the
 // difference of two positions less than 64 supercells apart is exact, in three
 // integer subtractions instead of the decoding of two words of supercell
-// coordinates (59 instructions per bond of the tile product, 77 with it).  The
-// offset's own rounding (2^-25 of the edge at most) is twice what the
-// conversion adds.  Blocks whose rows and halo reach farther than kFixedReach
-// supercells from their first row keep the decoding form.
+// coordinates (59 instructions per bond of the tile product, 77 with it).  An FP32
+// offset (0 to 1 edge) is finer than 2^-25 below a quarter of the edge, but the
+// decoded difference rounds again when the cells' distance is added: over horizons
+// of 2 to 3 spacings, edges of 1 to 1.95 horizons and jitters of 0.05 and 0.4, the
+// product's error from its geometry is 0.93 to 1.00 of the decoding form's (root
+// mean square, against 64 bits, emulated).  Blocks whose rows and halo reach farther
+// than kFixedReach supercells from their first row keep the decoding form.
 constexpr int kFixedBits = 25;
 constexpr int kFixedReach = 31;
 __device__ __forceinline__ float4 fixed_position(const float4& X, float per_edge)
@@ -423,18 +431,6 @@ __device__ __forceinline__ void load_bonds(const DeviceState& S, int slot, int (
     id0[0] = d.x; id0[1] = d.y; id0[2] = d.z; id0[3] = d.w;
 }
 
-// Mixed precision, G lanes per row, U bonds in flight per lane.  The halo is
-// S.halo of a tile per block, a bond's index into it S.lidx.
-// CACHED: the bonds' geometry stays in shared memory; else the halo's
-// positions do, and the index and 1/d0 of a bond are read from global memory
-// (6 bytes per bond, from L2).  Not cached, the product is bound by the
-// shared-memory pipe (7.2 wavefronts per step of 32 bonds and array when bonds
-// stood in build order) and by latency (one block per SM).  An iteration at 100k
-// particles (76 bonds) takes 25.3 us: 38.2 with scalar loads of the bonds, 31.2
-// with four per lane and load and the next four in flight, 30.4 with a round of
-// their own for the rows left over, 30.0 with fixed-point positions, 25.3 with
-// the order of k_bank_order.  Eight lanes per row: 34.9 against 31.2; 1024
-// threads 30.3 (but 24.0 against 21.8 at 50k and 104 bonds).
 // The residual of the guess (residual_elem): zero on Dirichlet rows.
 template <typename V4>
 __device__ __forceinline__ V4 first_residual(const DeviceState& S, int p)
@@ -451,6 +447,19 @@ __device__ __forceinline__ V4 first_residual(const DeviceState& S, int p)
 template <int N>
 using Lanes = std::integral_constant<int, N>;
 
+// Mixed precision, G lanes per row, U bonds in flight per lane.  The halo is
+// S.halo of a tile per block, a bond's index into it S.lidx.
+// CACHED: the bonds' geometry stays in shared memory; else the halo's
+// positions do, and the index and 1/d0 of a bond are read from global memory
+// (6 bytes per bond, from L2).  Not cached, the product is bound by the
+// shared-memory pipe (7.2 wavefronts per step of 32 bonds and array when bonds
+// stood in build order) and by latency (one block per SM).  An iteration at 100k
+// particles (76 bonds) takes 25.3 us: 38.2 with scalar loads of the bonds, 31.2
+// with four per lane and load and the next four in flight, 30.4 with a round of
+// their own for the rows left over, 30.0 with fixed-point positions, 25.3 with
+// the order of k_bank_order.  Eight lanes per row: 34.9 against 31.2; 1024
+// threads 30.3 (but 24.0 against 21.8 at 50k and 104 bonds); 23.3 with the sums of
+// WideSum (steps included).
 // `epoch` is the last epoch used in the inbox and the records.  Blocks beyond the
 // last row only exchange.  Returns false when a wait ran out of time.
 template <bool CACHED, int G, int U>
@@ -1071,8 +1080,8 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_cg_persist64(PersistArgs
 // its own iterations.  Every block of a gang takes part in every exchange, so
 // the epochs of its inbox go on from scene to scene; which scene comes next is
 // a record of its own per turn.  Against phases of all scenes between grid
-// barriers (k_batch_cg): 12 steps of 24 bodies of 4k to 24k particles take 97 ms
-// against 226, of 8 of 1k to 4k 13.5 against 65.
+// barriers (k_batch_cg): 12 steps of 24 bodies of 4k to 24k particles take 81.5 ms
+// against 208.5, of 8 of 1k to 4k 10.7 against 65.9.
 __global__ void __launch_bounds__(kPersistThreads, 1) k_gang_solve32(GangArgs A)
 {
     extern __shared__ __align__(32) unsigned char smem[];
