@@ -1261,8 +1261,8 @@ void Engine::cg_iteration(const StepParams& P, int k, cudaGraphConditionalHandle
     }
 }
 
-// Iterations per while-node body: an even count, 4 unless cg_check_interval
-// asks otherwise.
+// Iterations per while-node body: 4, or cg_check_interval, which pd_gb300.h
+// documents as rounded up to an even count here.
 int Engine::cg_graph_body() const
 {
     const int k = opt_.cg_check_interval > 0 ? opt_.cg_check_interval : 4;

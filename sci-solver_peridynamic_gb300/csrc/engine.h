@@ -103,9 +103,8 @@ private:
     pd_status integrate(bool* advanced);
     pd_status solve(const StepParams& P);
     pd_status solve_finish(const StepParams& P);
-    // one CG iteration's launches (iteration k of the solve: on lattice bodies
-    // its parity picks the direction buffers); cond: the CG graph's while
-    // condition when captured into it, else 0
+    // one CG iteration's launches (iteration k of the solve); cond: the CG graph's
+    // while condition when captured into it, else 0
     void cg_iteration(const StepParams& P, int k, cudaGraphConditionalHandle cond, bool sample);
     int cg_kernels_per_iteration() const { return 3; }
     int cg_graph_body() const;

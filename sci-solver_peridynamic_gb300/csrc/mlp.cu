@@ -196,8 +196,10 @@ void mlp_forward(const MlpDev& m, const __nv_bfloat16* X, int B, MlpWork& ws, fl
 
 // Rows of a slice of the gradient sums: eight slices up to 20480 rows (12,000
 // rows: 45 us per layer; one slice 1.6 ms), of 2560 rows beyond.  The tensor cores
-// truncate as they accumulate: at 20,000 rows eight slices move the sums by
-// 1.7e-5 towards the exact ones, 94 slices by 1.95e-5.
+// truncate as they accumulate, so shorter slices end nearer the exact sums, and are
+// faster (94 slices of 128 rows: 23 to 31 us); eight are kept because they move the
+// sums less from those of one walk over all rows, which a caller's earlier results
+// hold (1.7e-5 at 20,000 rows, 94 slices 1.95e-5).
 static int slice_rows(int B)
 {
     const int rows = ((B + 7) / 8 + kMlpSliceRows - 1) / kMlpSliceRows * kMlpSliceRows;

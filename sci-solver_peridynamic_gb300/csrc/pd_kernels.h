@@ -326,9 +326,9 @@ void launch_cg_xpby(bool fp64, const StepParams& P, const DeviceState& S, const 
 void launch_update(bool fp64, const StepParams& P, const DeviceState& S, const LaunchCfg& L, cudaStream_t st);
 void launch_refresh(bool fp64, const StepParams& P, const DeviceState& S, const LaunchCfg& L, cudaStream_t st);
 void launch_bond_geometry(const DeviceState& S, cudaStream_t st);
-// mixed: lim[p] = limit_pair(st[p]) for every particle (after st is set)
 // pd_sample_stretch_limits on the device (stretch.cu): out in caller order
 cudaError_t sample_stretch_limits(float s0, int n, double* out, cudaStream_t st);
+// mixed: lim[p] = limit_pair(st[p]) for every particle (after st is set)
 void launch_stretch_limits(const DeviceState& S, int grid, cudaStream_t st);
 // mixed mode: live bonds of each row reordered from the (g_from, u_from)
 // SpMV shape's slot order to (g_to, u_to)'s (u = 1: build order)

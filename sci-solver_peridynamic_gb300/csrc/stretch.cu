@@ -2,7 +2,7 @@
 //
 // getstretch (simulator.cu:802-822) sums twelve values of rand() per particle
 // after srand(1973) (simulator.cu:852): 12 n steps of one serial generator, which
-// take the host 30 ms at 1M particles.  The generator (glibc_rand.h) is linear
+// take the host 12 ms at 1M particles.  The generator (glibc_rand.h) is linear
 // modulo 2^32, h[i] = h[i-31] + h[i-3], so word i + s is a fixed combination of
 // the words i .. i+30, with the coefficients of x^s modulo x^31 - x^28 - 1.  Every
 // thread jumps to its own kRun particles with the polynomial of its place in the
